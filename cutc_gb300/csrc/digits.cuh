@@ -119,10 +119,11 @@ CUTC_HD float pow2_float(int k)  // 2^k for k in [-126, 127]
 // digits are the integers q_s, returned as floats.  Scaling by 2^(8 - e) takes two
 // exact steps when 8 - e leaves the FP32 exponent range; values it makes subnormal are
 // below 2^-126, where every digit is zero.
-template <int S>
+// W: the digits' width (base 2^W), with 2^(W - 1 - e) in the place of 2^(8 - e).
+template <int S, int W = 9>
 CUTC_HD void digits_df_fp32(float hi, float lo, int e, float (&q)[S])
 {
-    const int k = 8 - e;  // -119 <= k <= 157 for FP32 hi and lo
+    const int k = W - 1 - e;  // W = 9: -119 <= k <= 157 for FP32 hi and lo
     const int k1 = k / 2, k2 = k - k1;
     const float c1 = pow2_float(k1), c2 = pow2_float(k2);
     float xh = f_mul(f_mul(hi, c1), c2), xl = f_mul(f_mul(lo, c1), c2);
@@ -138,8 +139,8 @@ CUTC_HD void digits_df_fp32(float hi, float lo, int e, float (&q)[S])
         const float sm = f_add(a, xl);
         const float bb = f_add(sm, -a);
         const float er = f_add(f_add(a, -f_add(sm, -bb)), f_add(xl, -bb));
-        xh = f_mul(sm, 512.0f);
-        xl = f_mul(er, 512.0f);
+        xh = f_mul(sm, (float)(1 << W));
+        xl = f_mul(er, (float)(1 << W));
     }
 }
 

@@ -818,7 +818,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             CUTC_TRY(launch_pair_f64(st, P));
             note_launches(2);
             if (R.precision == CUTC_SPLIT_BF16) {
-                // the split slicer reads (hi, lo) pairs: convert in place
+                // the split form's operands read (hi, lo) pairs: convert in place
                 CUTC_TRY(launch_f64_to_df(st, d_G, 4 * (int64_t)nb * n2));
                 note_launches(1);
             }
@@ -832,9 +832,6 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             P.a_ee_hi = (float)R.a_ee;
             P.a_ee_lo = (float)(R.a_ee - (double)P.a_ee_hi);
             P.G = reinterpret_cast<float2 *>(d_G); P.ldg = n2; P.plane = (int64_t)nb * n2;
-            // the kernel also leaves the row maxima the G slicer needs
-            CUTC_CUDA_TRY(cudaMemsetAsync(sp.BX.rmax, 0, 4 * (size_t)nb * 8, st));
-            P.rmax = sp.BX.rmax;
             if (sp.pair_tc) {
                 CUTC_TRY(split_pair_tile(E, R, st, sp, P, d_rn, R.a_en));
             } else {
@@ -870,8 +867,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
                 CUTC_CUDA_TRY(cudaEventRecord(tev[3], st));
         } else {
             CUTC_TRY(split_x_tile(E, R, st, sp, reinterpret_cast<const float2 *>(d_G), nb, d_Xt,
-                                  blk_rows, ib, tev ? tev[2] : nullptr, tev ? tev[3] : nullptr,
-                                  !R.pair_fp64));
+                                  blk_rows, ib, tev ? tev[2] : nullptr, tev ? tev[3] : nullptr));
         }
 
         // the tile's X rows in the reference layout X[m][i][b][a], before the int_2e share,

@@ -1,0 +1,582 @@
+// Modular contraction: residue products on tcgen05 CTA pairs, and the FP64 results from
+// their residues (moduli.cuh has the arithmetic).
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+
+#include "modular.cuh"
+#include "tc.cuh"
+
+namespace cutc {
+
+// ---------------------------------------------------------------------------
+// the residue products
+// ---------------------------------------------------------------------------
+
+// One CTA pair (a cluster of two) computes a 256 x BN tile of one modulus: the pair's
+// tcgen05.mma (cta_group::2, M = 256) takes 128 rows of A and half of B's rows from each
+// CTA's shared memory.  Against one CTA with a 128 x 256 tile this reads 8 instead of
+// 12 KB from L2 per 16-wide K step and SM, 64 B per clock at the tensor pipe's full rate.
+// Bound by the tensor pipe, the accumulators' reads beside it, and in long runs the power
+// cap: M 7260, N 16384, K 16384 with 11 moduli takes 23.6 ms, 1817 TF/s of BF16 products
+// (cuBLAS: 1898 in a burst, 1704 sustained).  The 5-slice kernel that this replaces, with
+// a 128 x 48 tile of five stacked accumulators, ran 15 products at 1551 TF/s.  The medium
+// build (n_ao 120, 25k x 80k): 1361 -> 960 ms, with 3 to 5 times smaller errors.
+constexpr int kTileM = 256, kBK = 64;     // 64 BF16 = 128-byte rows (128B swizzle)
+constexpr int kChunkBlocks = 8;           // 512 K: sums of products of residues below 2^24
+constexpr int kEpiWarps = 16;             // 4 lane quarters x 4 column groups
+constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
+constexpr int kGemmThreads = (kEpiWarps + 2) * 32;
+constexpr int kGroupN = 8;                // column tiles per raster group
+
+template <int BN>
+struct ModCfg {
+    static constexpr int kA = 128 * kBK * 2;
+    static constexpr int kB = BN / 2 * kBK * 2;
+    static constexpr int kStage = kA + kB;
+    static constexpr int kStages = 6;
+    static constexpr int kSmem = kStages * kStage + 1024 + 256;
+    static constexpr uint32_t kTmemCols = 2 * BN;  // two accumulator buffers
+    static constexpr int kCols = BN / 4;           // columns per epilogue warp
+    static_assert(kSmem <= 227 * 1024, "shared memory");
+    static_assert(kTmemCols <= 512, "tensor memory");
+};
+
+struct ModGemmParams {
+    int n_mod, M, N, tiles_m, tiles_n;
+    int nkb;                   // K blocks of the panel
+    int accumulate;            // add to the residues in out
+    short *out;                // out[i plane + n ldm + m]
+    int64_t ldm, plane;
+    float p[moduli::kMax], inv[moduli::kMax];
+    int *err;                  // set to a non-zero code if a bounded wait gave up
+};
+
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
+modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
+                    const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ModGemmParams P)
+{
+    using Cfg = ModCfg<BN>;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    // (the dynamic shared memory starts at the same offset in both CTAs)
+    const uint32_t pad = (1024u - (tc::smem_u32(smem_raw) & 1023u)) & 1023u;
+    uint8_t *smem = smem_raw + pad;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + Cfg::kStages * Cfg::kStage);
+    uint64_t *full = bars;                       // leader: both CTAs' copies of a stage landed
+    uint64_t *empty = bars + Cfg::kStages;       // each: the MMAs have read the stage
+    uint64_t *tfull = bars + 2 * Cfg::kStages;   // each: the accumulators hold a chunk
+    uint64_t *tempty = tfull + 2;                // leader: both CTAs' epilogues have read them
+    uint64_t *drain = tempty + 2;
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
+    volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = tc::cluster_rank();
+    const bool leader = rank == 0;
+
+    // tile: moduli outermost, then a grouped raster (kGroupN column tiles sweep the row
+    // tiles, so concurrent pairs share their tiles of A and B through L2)
+    const int per_mod = P.tiles_m * P.tiles_n;
+    const int task = (int)(blockIdx.x >> 1);
+    const int z = task / per_mod, t = task % per_mod;
+    const int per_group = kGroupN * P.tiles_m;
+    const int gfirst = (t / per_group) * kGroupN;
+    const int gsize = min(P.tiles_n - gfirst, kGroupN);
+    const int n0 = (gfirst + (t % per_group) % gsize) * BN;
+    const int m0 = ((t % per_group) / gsize) * kTileM + (int)rank * 128;
+    const int nkb = P.nkb;
+    const int nch = (nkb + kChunkBlocks - 1) / kChunkBlocks;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < Cfg::kStages; i++) {
+            tc::mbar_init(tc::smem_u32(&full[i]), 1);
+            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
+        }
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(tc::smem_u32(&tfull[i]), 1);
+            tc::mbar_init(tc::smem_u32(&tempty[i]), 2 * kEpiWarps);
+        }
+        tc::mbar_init(tc::smem_u32(drain), 1);
+        *s_abort = 0;
+        tc::fence_mbar_init();
+    }
+    if (warp == kMmaWarp) {
+        tc::tmem_alloc_pair(tc::smem_u32(s_tmem), Cfg::kTmemCols);
+        tc::tmem_relinquish_pair();
+    }
+    if (warp == kTmaWarp && lane == 0) {
+        tc::tma_prefetch(&tmA);
+        tc::tma_prefetch(&tmB);
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::cluster_sync();  // both CTAs' barriers are initialised
+    tc::fence_after_sync();
+    const uint32_t tbase = *s_tmem;
+
+    auto fail = [&](int code) {
+        *s_abort = 1;
+        atomicExch(P.err, code);
+    };
+
+    if (warp == kTmaWarp) {
+        if (lane == 0) {
+            int issued = 0;
+            for (int kb = 0; kb < nkb; kb++) {
+                const int stage = kb % Cfg::kStages, round = kb / Cfg::kStages;
+                if (round > 0 &&
+                    !tc::mbar_wait(tc::smem_u32(&empty[stage]), (round - 1) & 1, s_abort)) {
+                    fail(21);
+                    break;
+                }
+                const uint32_t fb = tc::smem_u32(&full[stage]);
+                if (leader)
+                    tc::mbar_arrive_expect_tx(fb, 2 * Cfg::kStage);
+                const uint32_t fl = tc::map_to_rank(fb, 0);
+                const uint32_t st = tc::smem_u32(smem + stage * Cfg::kStage);
+                tc::tma_load_3d_pair(st, &tmA, kb * kBK, m0, z, fl);
+                tc::tma_load_3d_pair(st + Cfg::kA, &tmB, kb * kBK, n0 + (int)rank * (BN / 2), z, fl);
+                issued = kb + 1;
+            }
+            if (*s_abort && leader) {
+                // let the copies already issued land before the pair goes away
+                for (int kb = max(0, issued - Cfg::kStages); kb < issued; kb++)
+                    tc::mbar_wait(tc::smem_u32(&full[kb % Cfg::kStages]),
+                                  (kb / Cfg::kStages) & 1, nullptr);
+            }
+        }
+    } else if (warp == kMmaWarp) {
+        if (leader && lane == 0) {
+            bool ok = true;
+            const uint32_t idesc = tc::idesc_bf16_f32(kTileM, BN);
+            for (int c = 0; c < nch && ok; c++) {
+                const int b = c & 1;
+                if (c >= 2 && !tc::mbar_wait(tc::smem_u32(&tempty[b]), ((c >> 1) - 1) & 1, s_abort)) {
+                    fail(22);
+                    break;
+                }
+                tc::fence_after_sync();
+                const int kb_end = min(nkb, (c + 1) * kChunkBlocks);
+                for (int kb = c * kChunkBlocks; kb < kb_end; kb++) {
+                    const int stage = kb % Cfg::kStages, round = kb / Cfg::kStages;
+                    if (!tc::mbar_wait(tc::smem_u32(&full[stage]), round & 1, s_abort)) {
+                        fail(23);
+                        ok = false;
+                        break;
+                    }
+                    tc::fence_after_sync();
+                    const uint32_t sa = tc::smem_u32(smem + stage * Cfg::kStage);
+                    const uint64_t ad = tc::smem_desc_sw128(sa);
+                    const uint64_t bd = tc::smem_desc_sw128(sa + Cfg::kA);
+#pragma unroll
+                    for (int k16 = 0; k16 < kBK / 16; k16++)  // 32 bytes further in each row
+                        tc::mma_bf16_pair(tbase + (uint32_t)(BN * b), ad + 2 * k16, bd + 2 * k16,
+                                          idesc, kb > c * kChunkBlocks || k16 > 0);
+                    tc::mma_commit_pair(tc::smem_u32(&empty[stage]));
+                }
+                if (ok)
+                    tc::mma_commit_pair(tc::smem_u32(&tfull[b]));
+            }
+            // all MMAs of the pair have completed once the drain barrier flips
+            tc::mma_commit_pair(tc::smem_u32(drain));
+            if (!tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
+                fail(25);
+        }
+    } else {
+        // ---- epilogue: running residues of the warp's 32 rows x kCols columns ----------
+        constexpr int CP = Cfg::kCols / 2;  // column pairs (one f32x2 each)
+        const int q = warp & 3, grp = warp >> 2;
+        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
+        const uint32_t coff = (uint32_t)(grp * Cfg::kCols);
+        const int m = m0 + q * 32 + lane;
+        short *dst = P.out + z * P.plane + (int64_t)(n0 + (int)coff) * P.ldm + m;
+        const int ncol = P.N - n0 - (int)coff;  // columns of this warp that exist
+        const uint64_t magic = tc::f2_dup(12582912.0f);  // 1.5 * 2^23
+        const uint64_t inv = tc::f2_dup(P.inv[z]), negp = tc::f2_dup(-P.p[z]);
+        uint64_t acc[CP];
+#pragma unroll
+        for (int j = 0; j < CP; j++)
+            acc[j] = 0ull;
+        if (P.accumulate && m < P.M) {
+#pragma unroll
+            for (int j = 0; j < CP; j++) {
+                const float a = 2 * j < ncol ? (float)dst[(int64_t)(2 * j) * P.ldm] : 0.0f;
+                const float b = 2 * j + 1 < ncol ? (float)dst[(int64_t)(2 * j + 1) * P.ldm] : 0.0f;
+                acc[j] = tc::f2_pack(__float_as_uint(a), __float_as_uint(b));
+            }
+        }
+        const uint32_t te0 = tc::map_to_rank(tc::smem_u32(&tempty[0]), 0);
+        const uint32_t te1 = tc::map_to_rank(tc::smem_u32(&tempty[1]), 0);
+        bool ok = true;
+        for (int c = 0; c < nch; c++) {
+            const int b = c & 1;
+            if (!tc::mbar_wait(tc::smem_u32(&tfull[b]), (c >> 1) & 1, s_abort)) {
+                fail(24);
+                ok = false;
+                break;
+            }
+            tc::fence_after_sync();
+            // acc <- (acc + v) mod p: |v| + |acc| < 2^24, every step exact
+#pragma unroll
+            for (int h = 0; h < Cfg::kCols / 16; h++) {
+                float v[16];
+                tc::tmem_ld16(tbase + lane_off + (uint32_t)(BN * b) + coff + 16u * h, v);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    uint64_t &a = acc[8 * h + j];
+                    const uint64_t s = tc::f2_add(a, tc::f2_pack(__float_as_uint(v[2 * j]),
+                                                                 __float_as_uint(v[2 * j + 1])));
+                    const uint64_t d = tc::f2_sub(tc::f2_fma(s, inv, magic), magic);
+                    a = tc::f2_fma(d, negp, s);
+                }
+            }
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0)
+                tc::mbar_arrive_cluster(b ? te1 : te0);
+        }
+        if (ok && m < P.M) {
+            // the low half of (residue + 1.5 2^23)'s bits is the residue as a 16-bit integer
+#pragma unroll
+            for (int j = 0; j < CP; j++) {
+                const uint64_t w = tc::f2_add(acc[j], magic);
+                if (2 * j < ncol)
+                    dst[(int64_t)(2 * j) * P.ldm] = (short)(uint32_t)w;
+                if (2 * j + 1 < ncol)
+                    dst[(int64_t)(2 * j + 1) * P.ldm] = (short)(uint32_t)(w >> 32);
+            }
+        }
+    }
+
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::cluster_sync();  // neither CTA leaves while the other may signal it or read its operands
+    tc::fence_after_sync();
+    if (warp == kMmaWarp)
+        tc::tmem_dealloc_pair(tbase, Cfg::kTmemCols);
+}
+
+// ---------------------------------------------------------------------------
+// the results
+// ---------------------------------------------------------------------------
+
+struct CombineParams {
+    int M, ncols, n0;
+    const short *res;
+    int64_t ldm, plane;
+    const int *sa, *sb;
+    ModularOut out;
+    int alpha_exp, alpha_neg, alpha_mul, beta_mode;  // beta_mode: 0, 1 or 2 (any other beta)
+    const int *err, *skip;
+};
+
+// v 2^k: the exponent field moved with integer operations when v and the result are
+// normal numbers (GB300's FP64 pipe is slow), scalbn otherwise (zeros, and results that
+// underflow to subnormals or zero or overflow to infinity)
+__device__ __forceinline__ double scale_pow2(double v, int k)
+{
+    const long long b = __double_as_longlong(v);
+    const int e = (int)((b >> 52) & 0x7ff);
+    if (e != 0 && e + k >= 1 && e + k <= 2046)
+        return __longlong_as_double(b + ((long long)k << 52));
+    return scalbn(v, k);
+}
+
+__device__ __forceinline__ int float_int(float f)  // an integer-valued float below 2^22
+{
+    return __float_as_int(f + 12582912.0f) - 0x4b400000;
+}
+
+__device__ __forceinline__ double int_double(long long v)  // |v| < 2^51, one FP64 add
+{
+    return __longlong_as_double(0x4338000000000000ll + v) - 6755399441055744.0;
+}
+
+// One mixed-radix group: sum of digits d[0..n) with radices p_{j0}, p_{j0+1}, ... (n <= 5,
+// below 2^45)
+template <int N, int J0>
+__device__ __forceinline__ long long digit_group(const float (&d)[N])
+{
+    constexpr int n = N - J0 < 5 ? N - J0 : 5;
+    auto pr = [](int i) { return moduli::prime(i); };
+    int hi = 0;
+    if constexpr (n == 5)
+        hi = float_int(d[J0 + 4]);
+    if constexpr (n >= 4) {
+        hi = hi * (moduli::prime(J0 + 2) * moduli::prime(J0 + 3 < N ? J0 + 3 : 0)) +
+             float_int(fmaf(d[J0 + (n >= 4 ? 3 : 0)], (float)pr(J0 + 2), d[J0 + 2]));
+    } else if constexpr (n == 3) {
+        hi = float_int(d[J0 + 2]);
+    }
+    const int lo = n >= 2 ? float_int(fmaf(d[J0 + (n >= 2 ? 1 : 0)], (float)pr(J0), d[J0]))
+                          : float_int(d[J0]);
+    return n >= 3 ? (long long)hi * (moduli::prime(J0) * moduli::prime(n >= 2 ? J0 + 1 : 0)) + lo
+                  : (long long)lo;
+}
+
+constexpr double radix5(int j0)  // p_{j0} ... p_{j0 + 4}, below 2^45
+{
+    double v = 1.0;
+    for (int i = 0; i < 5; i++)
+        v *= moduli::prime(j0 + i);
+    return v;
+}
+
+template <int N>
+__device__ __forceinline__ double digits_value(const float (&d)[N])
+{
+    // rounded once, at the result's own precision (to a unit that is 2^-50 of its last place)
+    double v = int_double(digit_group<N, 0>(d));
+    if constexpr (N > 10) {
+        constexpr double q0 = radix5(0), q1 = radix5(5);
+        const double g1 = int_double(digit_group<N, 5>(d)), g2 = int_double(digit_group<N, 10>(d));
+        const double u = fma(g2, q1, g1);
+        if constexpr (N > 11)  // u's rounding error, an exact integer (below 2^53 if N = 11)
+            v = fma(fma(g2, q1, -u) + g1, q0, v);
+        v = fma(u, q0, v);
+    } else if constexpr (N > 5) {
+        constexpr double q0 = radix5(0);
+        v = fma(int_double(digit_group<N, 5>(d)), q0, v);
+    }
+    return v;
+}
+
+// Residues -> mixed-radix digits (Garner; every FP32 operation exact, two rows per f32x2
+// operation) -> FP64.  Consecutive threads take consecutive m; bound by the N reads of
+// 2 bytes and the digits' N (N - 1) / 2 modular steps.
+template <int N>
+__global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
+{
+    if (P.skip && *P.skip)
+        return;
+    const int m = 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
+    if (m >= P.M)
+        return;
+    const bool failed = *P.err != 0;
+    const uint64_t magic = tc::f2_dup(12582912.0f);
+    const int s0 = P.sa[m], s1 = m + 1 < P.M ? P.sa[m + 1] : 0;
+    for (int c = blockIdx.y; c < P.ncols; c += gridDim.y) {
+        const short *src = P.res + (int64_t)c * P.ldm + m;
+        uint64_t d[N];
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const short2 v = *reinterpret_cast<const short2 *>(src + i * P.plane);
+            uint64_t t = tc::f2_pack(__float_as_uint((float)v.x), __float_as_uint((float)v.y));
+#pragma unroll
+            for (int j = 0; j < i; j++) {
+                t = tc::f2_mul(tc::f2_sub(t, d[j]), c_tab.garner[i][j]);
+                const uint64_t q = tc::f2_sub(tc::f2_fma(t, c_tab.inv[i], magic), magic);
+                t = tc::f2_fma(q, c_tab.negp[i], t);
+            }
+            d[i] = t;
+        }
+        const int sn = P.sb[c], n = P.n0 + c;
+        const int64_t col = (int64_t)(n / P.out.ncol_group) * P.out.group_stride + P.out.col0 +
+                            n % P.out.ncol_group;
+        double *dst = P.out.C + m + P.out.ldc * col;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (m + h >= P.M)
+                break;
+            float f[N];
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                f[i] = h ? tc::f2_hi(d[i]) : tc::f2_lo(d[i]);
+            const int sm = h ? s1 : s0;
+            double v;
+            if (failed || sm == kNotFinite || sn == kNotFinite) {
+                v = __longlong_as_double(0x7ff8000000000000ll);
+            } else {
+                v = scale_pow2(digits_value<N>(f), P.alpha_exp - sm - sn);
+                if (P.alpha_neg)
+                    v = __longlong_as_double(__double_as_longlong(v) ^ (1ll << 63));
+                if (P.alpha_mul)
+                    v *= P.out.alpha;
+            }
+            if (P.beta_mode == 1)
+                v += dst[h];
+            else if (P.beta_mode == 2)
+                v += P.out.beta * dst[h];
+            dst[h] = v;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
+                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static int get_encode(EncodeTiledFn *fn)
+{
+    static std::atomic<EncodeTiledFn> cached{nullptr};
+    EncodeTiledFn f = cached.load();
+    if (!f) {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
+                                                         cudaEnableDefault, &q);
+        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !p) {
+            cudaGetLastError();
+            cutc_set_error(CUTC_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
+            return CUTC_ERR_CUDA;
+        }
+        f = (EncodeTiledFn)p;
+        cached.store(f);
+    }
+    *fn = f;
+    return CUTC_OK;
+}
+
+int encode_bf16_map(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
+                    const uint64_t *strides_bytes, const uint32_t *box, int swizzle)
+{
+    EncodeTiledFn enc;
+    CUTC_TRY(get_encode(&enc));
+    cuuint64_t d[3], s[2];
+    cuuint32_t b[3] = {box[0], box[1], 1};
+    cuuint32_t estr[3] = {1, 1, 1};
+    for (int i = 0; i < rank; i++)
+        d[i] = dims[i];
+    for (int i = 0; i + 1 < rank; i++)
+        s[i] = strides_bytes[i];
+    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void *>(base), d, s, b,
+                     estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                     swizzle == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        cutc_set_error(CUTC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+        return CUTC_ERR_CUDA;
+    }
+    return CUTC_OK;
+}
+
+static int planes_map(CUtensorMap *map, int n_mod, const ResiduePlanes &o, int box_rows)
+{
+    const uint64_t dims[3] = {(uint64_t)o.kp, (uint64_t)o.rows, (uint64_t)n_mod};
+    const uint64_t strides[2] = {(uint64_t)o.pitch * 2, (uint64_t)o.pitch * 2 * (uint64_t)o.rows};
+    const uint32_t box[2] = {(uint32_t)kBK, (uint32_t)box_rows};
+    return encode_bf16_map(map, o.p, 3, dims, strides, box, 128);
+}
+
+int modular_pass_cols(int n_mod, int64_t M, int64_t N)
+{
+    const int64_t per = ((int64_t)4 << 30) / (2 * n_mod * modular_ldm(M));
+    return (int)std::min<int64_t>(N, std::max<int64_t>(256, per / 256 * 256));
+}
+
+size_t modular_out_bytes(int n_mod, int64_t M, int64_t N)
+{
+    return (size_t)2 * n_mod * modular_ldm(M) * modular_pass_cols(n_mod, M, N);
+}
+
+template <int BN>
+static int launch_gemm(cudaStream_t st, const ResiduePlanes &A, const ResiduePlanes &B,
+                       ModGemmParams P)
+{
+    using Cfg = ModCfg<BN>;
+    static std::atomic<unsigned long long> attr_done{0};
+    const unsigned long long bit = current_device_bit();
+    if (!(attr_done.load() & bit)) {
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(modular_gemm_kernel<BN>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+        attr_done.fetch_or(bit);
+    }
+    CUtensorMap ta, tb;
+    CUTC_TRY(planes_map(&ta, P.n_mod, A, 128));
+    CUTC_TRY(planes_map(&tb, P.n_mod, B, BN / 2));
+    P.tiles_m = (int)ceil_div(P.M, kTileM);
+    P.tiles_n = (int)ceil_div(P.N, BN);
+    const int64_t ctas = 2 * (int64_t)P.n_mod * P.tiles_m * P.tiles_n;
+    if (ctas > INT32_MAX) {
+        cutc_set_error(CUTC_ERR_INVALID, "modular contraction of %lld CTAs", (long long)ctas);
+        return CUTC_ERR_INVALID;
+    }
+    modular_gemm_kernel<BN><<<(unsigned)ctas, kGemmThreads, Cfg::kSmem, st>>>(ta, tb, P);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
+                 short *out, int64_t plane_cols, bool accumulate, int *err)
+{
+    if (A.rows <= 0 || B.rows <= 0 || A.kp <= 0)
+        return CUTC_OK;
+    ModGemmParams P{};
+    P.n_mod = n_mod;
+    P.M = A.rows;
+    P.N = B.rows;
+    P.nkb = (int)ceil_div(A.kp, kBK);
+    P.accumulate = accumulate ? 1 : 0;
+    P.out = out;
+    P.ldm = modular_ldm(A.rows);
+    P.plane = P.ldm * plane_cols;
+    for (int i = 0; i < n_mod; i++) {
+        P.p[i] = (float)moduli::prime(i);
+        P.inv[i] = 1.0f / (float)moduli::prime(i);
+    }
+    P.err = err;
+    // narrow tiles where wide ones would leave the 76 SM pairs short of work
+    const int64_t wide = (int64_t)n_mod * ceil_div(P.M, kTileM) * ceil_div(P.N, 256);
+    if (P.N <= 128 || wide < 76)
+        return launch_gemm<128>(st, A, B, P);
+    return launch_gemm<256>(st, A, B, P);
+}
+
+template <int N>
+static int launch_combine(cudaStream_t st, const CombineParams &P)
+{
+    dim3 grid(ceil_div(P.M, 256), (unsigned)std::min(P.ncols, 65535));
+    combine_kernel<N><<<grid, 128, 0, st>>>(P);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const short *res,
+                    const int *sa, const int *sb, const ModularOut &out, const int *err,
+                    const int *skip)
+{
+    if (M <= 0 || ncols <= 0)
+        return CUTC_OK;
+    CombineParams P;
+    P.M = M;
+    P.ncols = ncols;
+    P.n0 = n0;
+    P.res = res;
+    P.ldm = modular_ldm(M);
+    P.plane = P.ldm * ncols;
+    P.sa = sa;
+    P.sb = sb;
+    P.out = out;
+    // a power of two (1, -1/2, 1/2 in this library) scales through the exponent
+    int ae = 0;
+    const double am = std::frexp(std::fabs(out.alpha), &ae);
+    P.alpha_mul = am != 0.5;
+    P.alpha_exp = P.alpha_mul ? 0 : ae - 1;
+    P.alpha_neg = !P.alpha_mul && out.alpha < 0;
+    P.beta_mode = out.beta == 0.0 ? 0 : out.beta == 1.0 ? 1 : 2;
+    P.err = err;
+    P.skip = skip;
+    switch (n_mod) {
+    case 7: return launch_combine<7>(st, P);
+    case 9: return launch_combine<9>(st, P);
+    case 11: return launch_combine<11>(st, P);
+    case 13: return launch_combine<13>(st, P);
+    case 15: return launch_combine<15>(st, P);
+    }
+    cutc_set_error(CUTC_ERR_INVALID, "no combination of %d moduli", n_mod);
+    return CUTC_ERR_INVALID;
+}
+
+}  // namespace cutc

@@ -1,0 +1,185 @@
+// Modular contraction on the tensor cores: residue operands and entry points
+// (moduli.cuh has the arithmetic, residue.cuh the operand preparation).
+#pragma once
+
+#include <cuda.h>
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "engine.cuh"
+#include "moduli.cuh"
+
+namespace cutc {
+
+// Row scale of a row that holds an infinity or a NaN.
+constexpr int kNotFinite = INT32_MIN;
+
+// Device tables of the moduli: FP32 pairs (both lanes the same value) for f32x2.
+struct ModuliTab {
+    uint64_t chunk[moduli::kMax][moduli::kMaxChunks];  // 2^{13 j} mod p_i
+    uint64_t inv[moduli::kMax];                        // 1 / p_i
+    uint64_t negp[moduli::kMax];                       // -p_i
+    uint64_t garner[moduli::kMax][moduli::kMax];       // p_j^-1 mod p_i, j < i
+};
+
+constexpr uint32_t float_code(int v)  // the bits of a small integer as a float
+{
+    if (v == 0)
+        return 0;
+    const uint32_t sign = v < 0 ? 0x80000000u : 0u;
+    uint32_t a = (uint32_t)(v < 0 ? -v : v);
+    int e = 0;
+    for (uint32_t t = a; t > 1; t >>= 1)
+        e++;
+    return sign | ((uint32_t)(127 + e) << 23) | ((a << (23 - e)) & 0x7fffffu);
+}
+
+constexpr uint32_t inverse_code(int p)  // 1 / p rounded to nearest, 256 < p < 512
+{
+    // 1 / p = f 2^-9 with 1 < f < 2: 24-bit significand round(2^32 / p)
+    const uint64_t f = ((1ull << 32) + p / 2) / p;
+    return (uint32_t)((127 - 9) << 23) | ((uint32_t)f & 0x7fffffu);
+}
+
+constexpr uint64_t dup_code(uint32_t c) { return ((uint64_t)c << 32) | c; }
+
+constexpr ModuliTab make_moduli_tab()
+{
+    ModuliTab t{};
+    for (int i = 0; i < moduli::kMax; i++) {
+        const int p = moduli::prime(i);
+        long long w = 1;
+        for (int j = 0; j < moduli::kMaxChunks; j++) {
+            t.chunk[i][j] = dup_code(float_code(moduli::sym_mod(w, p)));
+            w = w * (1 << moduli::kChunkBits) % p;
+        }
+        t.inv[i] = dup_code(inverse_code(p));
+        t.negp[i] = dup_code(float_code(-p));
+        for (int j = 0; j < i; j++)
+            t.garner[i][j] = dup_code(float_code(moduli::inverse(moduli::prime(j), p)));
+    }
+    return t;
+}
+
+static __constant__ const ModuliTab c_tab = make_moduli_tab();
+
+// Moduli of the split form's contractions for n_slices BF16 slices (3 .. 7): operands
+// rounded at 2^-29, 2^-37, 2^-45, 2^-54, 2^-62 of their row norms, at least the precision
+// of that many 9-bit slices.
+constexpr int split_moduli(int n_slices) { return 2 * n_slices + 1; }
+// Moduli of the plain form's contractions: operands rounded at 2^-62 of their row norms,
+// below FP64's own rounding of the sums.
+constexpr int kPlainModuli = moduli::kMax;
+
+// BF16 residues of one K panel of an operand: planes[i][r][k], rows `pitch` apart.
+struct ResiduePlanes {
+    void *p = nullptr;
+    int rows = 0;
+    int64_t kp = 0, pitch = 0;
+};
+
+// Where a contraction goes: C[m + ldc col(n)] = alpha sum_k A[m, k] B[n, k] + beta C,
+// col(n) = (n / ncol_group) group_stride + col0 + n % ncol_group.
+struct ModularOut {
+    double *C;
+    int64_t ldc;
+    int ncol_group;
+    int64_t group_stride, col0;
+    double alpha, beta;
+};
+
+// Elements between the rows of a K panel of kp columns (16-byte rows for TMA, whole
+// 128-byte lines for the writers).
+inline int64_t residue_pitch(int64_t kp) { return (kp + 63) / 64 * 64; }
+
+// Bytes of the residues of a panel.
+inline size_t residue_bytes(int n_mod, int64_t rows, int64_t kp)
+{
+    return (size_t)n_mod * rows * residue_pitch(kp) * 2;
+}
+
+// Columns per pass of a contraction with M rows: the residues of the results of one pass
+// (2 bytes each and modulus) take at most 4 GiB.
+int modular_pass_cols(int n_mod, int64_t M, int64_t N);
+size_t modular_out_bytes(int n_mod, int64_t M, int64_t N);
+
+// One K panel: residues of sum_k A[m, k] B[n, k] over the panel, for m < A.rows and
+// n < B.rows, into out[i][n][m] (rows modular_ldm(A.rows) apart, planes plane_cols rows),
+// added to what is there when accumulate.  err: set when a bounded wait gave up.
+inline int64_t modular_ldm(int64_t M) { return (M + 7) / 8 * 8; }
+int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
+                 short *out, int64_t plane_cols, bool accumulate, int *err);
+
+// The FP64 results from the residues: n0 .. n0 + ncols of the output's columns; sa and sb
+// are the row scales of A and B (sb of column n0 first).  A result with a scale of
+// kNotFinite, or after a wait that gave up, is NaN.  skip (may be null): nothing is
+// written when *skip is non-zero.
+int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const short *res,
+                    const int *sa, const int *sb, const ModularOut &out, const int *err,
+                    const int *skip);
+
+// cuTensorMapEncodeTiled of BF16 arrays: box[0] x box[1] tiles of the last two
+// dimensions; swizzle in bytes (64 or 128).
+int encode_bf16_map(CUtensorMap *map, const void *base, int rank, const uint64_t *dims,
+                    const uint64_t *strides_bytes, const uint32_t *box, int swizzle);
+
+// Rows of B whose residues of a K panel fit b_bytes (at least one tile's).
+inline int modular_b_rows(int n_mod, int64_t N, int64_t kp, size_t b_bytes)
+{
+    const int64_t fit = (int64_t)(b_bytes / residue_bytes(n_mod, 1, kp)) / 256 * 256;
+    return (int)std::min<int64_t>(N, std::max<int64_t>(256, fit));
+}
+
+// True when B's residues are whole in the workspace after the contraction.
+inline bool modular_whole(int n_mod, int64_t N, int64_t K, int64_t k_panel, size_t b_bytes)
+{
+    return K <= k_panel && modular_b_rows(n_mod, N, K, b_bytes) >= N;
+}
+
+// The contraction over K panels, gen_a(k0, kp, planes) and gen_b(n0, ncols, k0, kp, planes)
+// writing the residues of a panel (B's in groups of columns whose residues fit b_bytes).
+// a_ready: A's residues of the only panel are in `a` already; b_ready: B's are in slot_b
+// (modular_whole only).
+template <class GenA, class GenB>
+int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, size_t b_bytes,
+                     int n_mod, int M, int N, int64_t K, int64_t k_panel, ResiduePlanes a,
+                     bool a_ready, bool b_ready, const int *sa, const int *sb,
+                     const ModularOut &out, int *err, const int *skip, GenA gen_a, GenB gen_b)
+{
+    if (M <= 0 || N <= 0)
+        return CUTC_OK;
+    const int pass = modular_pass_cols(n_mod, M, N);
+    const int group = std::min(pass, modular_b_rows(n_mod, N, std::min(K, k_panel), b_bytes));
+    void *p;
+    CUTC_TRY(W.get(slot_b, residue_bytes(n_mod, b_ready ? N : group, std::min(K, k_panel)), &p));
+    ResiduePlanes b;
+    b.p = p;
+    CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &p));
+    short *res = (short *)p;
+    a.rows = M;
+    for (int n0 = 0; n0 < N; n0 += pass) {
+        const int nc = std::min(pass, N - n0);
+        for (int64_t k0 = 0; k0 < K; k0 += k_panel) {
+            const int64_t kp = std::min(k_panel, K - k0);
+            a.kp = b.kp = kp;
+            a.pitch = b.pitch = residue_pitch(kp);
+            if (!a_ready)
+                CUTC_TRY(gen_a(k0, kp, a));
+            a_ready = a_ready || k_panel >= K;
+            for (int g = 0; g < nc; g += group) {
+                b.rows = std::min(group, nc - g);
+                if (!b_ready)
+                    CUTC_TRY(gen_b(n0 + g, b.rows, k0, kp, b));
+                CUTC_TRY(modular_gemm(st, n_mod, a, b, res + (int64_t)g * modular_ldm(M), nc,
+                                      k0 > 0, err));
+            }
+        }
+        CUTC_TRY(modular_combine(st, n_mod, M, n0, nc, res, sa, sb + n0, out, err, skip));
+    }
+    return CUTC_OK;
+}
+
+}  // namespace cutc

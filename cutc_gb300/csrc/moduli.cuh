@@ -1,0 +1,86 @@
+// Residue arithmetic of the modular contraction (modular.cu): the moduli, their tables
+// and the scaling of operands to integers.
+//
+// An FP64 contraction C = A B^T is computed exactly on scaled, rounded operands,
+//   t_a[m, k] = rint(A[m, k] 2^{s_m}),  t_b[n, k] = rint(B[n, k] 2^{u_n}),
+// as the integers sum_k t_a t_b modulo N pairwise coprime odd moduli p_i <= 361.  A
+// residue in [-180, 180] is an exact BF16 number and 512 products of two of them sum to
+// less than 2^24 - 181, so the tensor cores' FP32 accumulation of a 512-long chunk is
+// exact; the integer itself comes back from its N residues (Chinese remainder theorem) when
+// |sum_k t_a t_b| < M / 2, M = prod p_i.  With row scales that bound the 2-norms,
+// |t_a|_2, |t_b|_2 <= 2^beta(N), 2^{2 beta} < M / 2 (Cauchy-Schwarz), nothing else is
+// rounded: the error is that of the operands' rounding, 2^-beta of their row norms,
+// whatever K is.  One product per modulus replaces the S (S + 1) / 2 products of an
+// S-slice splitting (Ozaki, Uchino and Imamura 2025, "Ozaki scheme II"): 11 against 15
+// at the error of 5 slices, 15 at FP64's.  Larger moduli (<= 509, exact over 256 K) take
+// one product fewer at FP64's error, but the accumulators' reads from tensor memory hold
+// up the MMAs: M 7260, N 16384, K 16384 with 11 moduli took 33.5 ms in chunks of 256,
+// 23.6 in chunks of 512.
+#pragma once
+
+#include <stdint.h>
+
+#include "digits.cuh"
+
+namespace cutc {
+namespace moduli {
+
+constexpr int kMax = 15;
+constexpr int kChunkBits = 13;  // integers are cut into 13-bit chunks for the residues
+constexpr int kMaxChunks = 5;
+
+// Pairwise coprime, odd, <= 361: |residue| <= 180, running residues <= 181 (the FP32
+// quotient S / p rounds to an integer one off only within 0.003 of a tie).
+CUTC_HD constexpr int prime(int i)
+{
+    constexpr int p[kMax] = {361, 359, 355, 353, 351, 349, 347, 343,
+                              341, 337, 331, 317, 313, 311, 307};
+    return p[i];
+}
+
+// beta(n) = (log2(p_0 ... p_{n-1}) - 1) / 2, less 0.0125: the rows' log2 norm bound
+CUTC_HD constexpr float row_bits(int n)
+{
+    constexpr float b[kMax + 1] = {0.f, 3.735f, 7.979f, 12.215f, 16.446f,
+                                   20.674f, 24.898f, 29.117f, 33.328f, 37.535f,
+                                   41.733f, 45.919f, 50.073f, 54.218f, 58.358f,
+                                   62.000f};
+    return b[n];
+}
+
+// 13-bit chunks that hold |t| <= 2^beta, below 2^{13 chunks - 1}
+CUTC_HD constexpr int chunks(int n) { return n <= 9 ? 3 : n <= 11 ? 4 : 5; }
+
+CUTC_HD constexpr int sym_mod(long long a, int p)  // in [-(p - 1) / 2, (p - 1) / 2]
+{
+    long long r = a % p;
+    if (r < 0)
+        r += p;
+    return (int)(2 * r > p ? r - p : r);
+}
+
+CUTC_HD constexpr int inverse(int a, int p)  // a^-1 mod p (p small: by search)
+{
+    const int m = ((a % p) + p) % p;
+    for (int x = 1; x < p; x++)
+        if ((long long)m * x % p == 1)
+            return sym_mod(x, p);
+    return 0;
+}
+
+// rint(x 2^s) of an FP64 value with |x 2^s| < 2^63 (ties away from zero), in integer
+// arithmetic; subnormal x count as zero
+CUTC_HD long long scaled_int(double x, int s)
+{
+    const unsigned long long bits = digits::double_bits(x);
+    const int E = (int)((bits >> 52) & 0x7ff);
+    const int sh = E - 1075 + s;
+    const unsigned long long mant = (bits & ((1ull << 52) - 1)) | (1ull << 52);
+    unsigned long long T = 0;
+    if (E != 0 && sh > -54)
+        T = sh >= 0 ? mant << (sh & 63) : (mant + (1ull << (-sh - 1))) >> (-sh);
+    return (bits >> 63) ? -(long long)T : (long long)T;
+}
+
+}  // namespace moduli
+}  // namespace cutc

@@ -260,23 +260,6 @@ pair_df_kernel(PairDfArgs P)
 #pragma unroll
         for (int c = 0; c < 4; c++)
             P.G[o + c * P.plane] = w4[c];
-        if (P.rmax) {
-            // row maxima for the slicer, which needs only an exponent e with
-            // |G| < 2^e: the high word of the double |hi| (hi + lo rounds to hi,
-            // so |hi + lo| never has a larger exponent), built from the float's
-            // bits with integer operations -- no FP64 on GB300's slow FP64 pipe.
-            // Float subnormals count as 2^-126.  One atomic per converged lane
-            // group and row.
-            const unsigned mask = __activemask();
-            const bool leader = (int)(threadIdx.x & 31) == __ffs(mask) - 1;
-#pragma unroll
-            for (int c = 0; c < 4; c++) {
-                const unsigned fb = __float_as_uint(w4[c].x) & 0x7fffffffu;
-                const unsigned m = rmax_word(__reduce_max_sync(mask, fb));
-                if (leader && m)
-                    atomicMax(&P.rmax[(int64_t)c * P.n1b + row0 + r], (unsigned long long)m << 32);
-            }
-        }
     }
 }
 

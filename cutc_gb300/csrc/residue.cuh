@@ -1,0 +1,467 @@
+// Operand preparation of the modular contraction: row scales and BF16 residue planes
+// (sm_103a).  Included by the translation units that name an operand source.
+#pragma once
+
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "digits.cuh"
+#include "modular.cuh"
+#include "moduli.cuh"
+#include "tc.cuh"
+
+namespace cutc {
+
+// ---------------------------------------------------------------------------
+// operand sources: value of row r, column k of an FP64 matrix, and up(r, k) >= its
+// magnitude as a float (within 2^-21; 0 below the float range, infinity above it, NaN
+// for a NaN)
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ float abs_up(double x)
+{
+    // from the high word, with integer operations: FP64 conversions take the FP64 pipe
+    const int hi = __double2hiint(x) & 0x7fffffff;
+    if (hi >= 0x7ff00000)
+        return __int_as_float(0x7fffffff);
+    const int v = hi - 0x38000000;  // exponent bias 1023 -> 127
+    if (v < 0x00100000)
+        return 0.0f;
+    if (v >= 0x0fe00000)
+        return __int_as_float(0x7f800000);
+    return __int_as_float((v << 3) + 8);
+}
+
+struct SrcDense {  // X[r * ld + k]
+    static constexpr bool kDoubleFloat = false;
+    const double *X;
+    int64_t ld;
+    __device__ double operator()(int64_t r, int64_t k) const { return X[r * ld + k]; }
+    __device__ float up(int64_t r, int64_t k) const { return abs_up(X[r * ld + k]); }
+};
+
+struct SrcConcat {  // [X1 | X2]: X1[r * k1 + k] for k < k1, then X2[r * k2 + k - k1]
+    static constexpr bool kDoubleFloat = false;
+    const double *X1, *X2;
+    int64_t k1, k2;
+    __device__ double operator()(int64_t r, int64_t k) const
+    {
+        return k < k1 ? X1[r * k1 + k] : X2[r * k2 + (k - k1)];
+    }
+    __device__ float up(int64_t r, int64_t k) const { return abs_up((*this)(r, k)); }
+};
+
+struct SrcDenseDF {  // hi + lo of X[r * ld + k]; the residues are cut from the pair itself
+    static constexpr bool kDoubleFloat = true;
+    const float2 *X;
+    int64_t ld;
+    __device__ float2 pair(int64_t r, int64_t k) const { return X[r * ld + k]; }
+    __device__ double operator()(int64_t r, int64_t k) const
+    {
+        const float2 v = X[r * ld + k];
+        return (double)v.x + (double)v.y;
+    }
+    __device__ float up(int64_t r, int64_t k) const
+    {
+        return fabsf(X[r * ld + k].x) * 1.0000002f;
+    }
+};
+
+// The pair products take their first factor w chi_a from a table of the weighted AO
+// rows, formed once per AO (weighted_aos_kernel) instead of once per pair: FP64
+// multiplies run at 1/64 of the FP32 rate on GB300.
+struct SrcSym {  // w[k] chi_a(k) chi_b(k) = (w chi_a)(k) chi_b(k), (a, b) = pairs[r]
+    static constexpr bool kDoubleFloat = false;
+    const double *wchi, *chi;  // wchi[a * K + k] = w[k] chi_a(k); chi_b at chi[b * ldchi + k]
+    int64_t K, ldchi;
+    const int2 *pairs;
+    __device__ double operator()(int64_t r, int64_t k) const
+    {
+        const int2 ab = pairs[r];
+        return wchi[ab.x * K + k] * chi[ab.y * ldchi + k];
+    }
+    __device__ float up(int64_t r, int64_t k) const
+    {
+        const int2 ab = pairs[r];
+        return abs_up(wchi[ab.x * K + k]) * abs_up(chi[ab.y * ldchi + k]);
+    }
+};
+
+// w (chi_c d_m chi_d - chi_d d_m chi_c) as (w chi_c) d_m chi_d - (w chi_d) d_m chi_c,
+// k = m n + g, (c, d) = pairs[r]
+struct SrcAnti {
+    static constexpr bool kDoubleFloat = false;
+    const double *wchi, *aos;  // wchi[c * n + g] = w[g] chi_c(g); aos: (ld, nA, 4) with
+                               // the grid offset already applied
+    int n, nA;                 // n: grid points counted in k (g < n)
+    int64_t ld;                // grid stride of aos
+    const int2 *pairs;
+    __device__ double operator()(int64_t r, int64_t k) const
+    {
+        int m, g;
+        if (k < 0x7fffffff) {  // 32-bit division (K = 3 n)
+            const unsigned ku = (unsigned)k, mu = ku / (unsigned)n;
+            m = (int)mu;
+            g = (int)(ku - mu * (unsigned)n);
+        } else {
+            m = (int)(k / n);
+            g = (int)(k % n);
+        }
+        const int2 cd = pairs[r];
+        const int64_t comp = (int64_t)nA * ld * (m + 1);
+        return fma(wchi[(int64_t)cd.x * n + g], aos[comp + cd.y * ld + g],
+                   -(wchi[(int64_t)cd.y * n + g] * aos[comp + cd.x * ld + g]));
+    }
+    __device__ float up(int64_t r, int64_t k) const { return abs_up((*this)(r, k)); }
+};
+
+// ---------------------------------------------------------------------------
+// row scales
+// ---------------------------------------------------------------------------
+
+// |v| as its bits (non-negative doubles order like their bits)
+__device__ __forceinline__ unsigned long long abs_bits(double v)
+{
+    return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+}
+
+// The scale of a row from its maximum m and sum of squares ss in FP32 when both are well
+// inside the float range: floor(bits - log2 |row|_2).
+// Up to 2^20 columns the rounding of the sum stays far below the 0.0005.
+__device__ __forceinline__ bool scale_fast(float m, float ss, float bits, int64_t K, int *s)
+{
+    if (K > (1 << 20) || !(m >= 0x1p-50f && m <= 0x1p60f && ss <= 0x1p125f))
+        return false;
+    *s = (int)floorf(bits - 0.5f * log2f(ss) - 0.0005f);
+    return true;
+}
+
+// ... and from the largest |x| as bits otherwise (|row|_2 <= sqrt(K) max): rows of values
+// near the ends of the FP64 range, zero rows (scale 0) and rows with an infinity or a NaN
+// (kNotFinite).
+__device__ __forceinline__ int scale_slow(unsigned long long mb, float bits, int64_t K)
+{
+    const int E = (int)(mb >> 52);
+    if (E >= 0x7ff)
+        return kNotFinite;
+    if (E == 0)
+        return 0;
+    return (int)floorf(bits - 0.5f * log2f((float)K) - 0.0005f) - (E - 1022);
+}
+
+// sc[r] for every row: one block per row (a fixed summation order, so the scale never
+// depends on scheduling); reads the row once.
+template <class Src>
+__global__ void __launch_bounds__(256)
+row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc, int *bad)
+{
+    __shared__ float sm[8], sq[8];
+    __shared__ unsigned long long sb[8];
+    __shared__ int s_fast;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+        float m = 0.0f, ss = 0.0f;
+#pragma unroll 4
+        for (int64_t k = threadIdx.x; k < K; k += 256) {
+            const float v = src.up(r, k);
+            m = fmaxf(m, v);
+            ss = fmaf(v, v, ss);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        __syncthreads();  // the previous row's shared values are read
+        if (lane == 0) {
+            sm[warp] = m;
+            sq[warp] = ss;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; w++) {
+                m = fmaxf(m, sm[w]);
+                ss += sq[w];
+            }
+            int s = 0;
+            s_fast = scale_fast(m, ss, bits, K, &s);
+            if (s_fast)
+                sc[r] = s;
+        }
+        __syncthreads();
+        if (s_fast)
+            continue;
+        unsigned long long mb = 0;
+        for (int64_t k = threadIdx.x; k < K; k += 256) {
+            const unsigned long long b = abs_bits(src(r, k));
+            mb = b > mb ? b : mb;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long b = __shfl_xor_sync(0xffffffffu, mb, o);
+            mb = b > mb ? b : mb;
+        }
+        if (lane == 0)
+            sb[warp] = mb;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < 8; w++)
+                mb = sb[w] > mb ? sb[w] : mb;
+            const int s = scale_slow(mb, bits, K);
+            sc[r] = s;
+            if (s == kNotFinite && bad)
+                atomicExch(bad, 1);
+        }
+    }
+}
+
+// The residues of eight integers per thread, chunk[j][q] holding the 13-bit chunks j of
+// elements 2q and 2q + 1: every FP32 operation is exact.
+template <int N, int CH>
+__device__ __forceinline__ void store_residues(const uint64_t (&chunk)[CH][4], __nv_bfloat16 *dst,
+                                               int64_t plane)
+{
+    const uint64_t magic = tc::f2_dup(12582912.0f);  // 1.5 * 2^23: rounds to an integer
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        unsigned w[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            uint64_t S = chunk[0][q];
+#pragma unroll
+            for (int j = 1; j < CH; j++)
+                S = tc::f2_fma(chunk[j][q], c_tab.chunk[i][j], S);
+            const uint64_t d = tc::f2_sub(tc::f2_fma(S, c_tab.inv[i], magic), magic);
+            const uint64_t r = tc::f2_fma(d, c_tab.negp[i], S);
+            const __nv_bfloat162 v = __floats2bfloat162_rn(tc::f2_lo(r), tc::f2_hi(r));
+            w[q] = *reinterpret_cast<const unsigned *>(&v);
+        }
+        *reinterpret_cast<uint4 *>(dst + i * plane) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+}
+
+// chunk j of the integer rint(x 2^s) as an exact float with the integer's sign
+template <int CH>
+__device__ __forceinline__ void int_chunks(double x, int s, float (&c)[CH])
+{
+    const long long t = moduli::scaled_int(x, s);
+    const unsigned long long a = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
+    const unsigned sign = (unsigned)(__double2hiint(x)) & 0x80000000u;
+#pragma unroll
+    for (int j = 0; j < CH; j++) {
+        const unsigned u = (unsigned)(a >> (moduli::kChunkBits * j)) & 0x1fffu;
+        const float f = __uint_as_float(0x4b000000u | u) - 8388608.0f;
+        c[j] = __uint_as_float(__float_as_uint(f) ^ sign);
+    }
+}
+
+template <int N>
+__device__ __forceinline__ void pack_chunks(const float (&v)[8][moduli::chunks(N)],
+                                            uint64_t (&chunk)[moduli::chunks(N)][4])
+{
+#pragma unroll
+    for (int j = 0; j < moduli::chunks(N); j++)
+#pragma unroll
+        for (int q = 0; q < 4; q++)
+            chunk[j][q] = tc::f2_pack(__float_as_uint(v[2 * q][j]), __float_as_uint(v[2 * q + 1][j]));
+}
+
+// planes[i][r][k - k0] = residues of rint(src(r0 + r, k) 2^{sc[r0 + r]}) modulo p_i for
+// rows r < rows and k0 <= k < k0 + kp (zeros up to the row pitch).  Eight consecutive k
+// per thread: one 16-byte store per plane.  Bound by the stores: 2 N bytes are written
+// per 8-byte element read.
+template <int N, class Src>
+__global__ void __launch_bounds__(128)
+residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t pitch,
+                    const int *__restrict__ sc, __nv_bfloat16 *__restrict__ planes)
+{
+    constexpr int CH = moduli::chunks(N);
+    const int64_t kk = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
+    if (kk >= pitch)
+        return;
+    for (int r = blockIdx.y; r < rows; r += gridDim.y) {
+        const int s = max(sc[r0 + r], -4096);  // (kNotFinite: the result is NaN anyway)
+        float v[8][CH];
+#pragma unroll
+        for (int q = 0; q < 8; q++) {
+            if constexpr (Src::kDoubleFloat) {
+                const float2 x = kk + q < kp ? src.pair(r0 + r, k0 + kk + q) : make_float2(0.f, 0.f);
+                float d[CH];  // from the top: d[0] is chunk CH - 1
+                digits::digits_df_fp32<CH, moduli::kChunkBits>(
+                    x.x, x.y, moduli::kChunkBits * CH - 1 - s, d);
+#pragma unroll
+                for (int j = 0; j < CH; j++)
+                    v[q][j] = d[CH - 1 - j];
+            } else {
+                const double x = kk + q < kp ? src(r0 + r, k0 + kk + q) : 0.0;
+                int_chunks<CH>(x, s, v[q]);
+            }
+        }
+        uint64_t chunk[CH][4];
+        pack_chunks<N>(v, chunk);
+        store_residues<N, CH>(chunk, planes + (int64_t)r * pitch + kk, (int64_t)rows * pitch);
+    }
+}
+
+// Row scales of a matrix stored column by column, src[(k0 + k) ld + r]: 32 rows per block
+// (one per lane), the columns over its 32 warps.  up and abs_bits as for the sources.
+static __global__ void __launch_bounds__(1024)
+row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t K, float bits,
+                      int *__restrict__ sc, int *bad)
+{
+    __shared__ float sm[32][33], sq[32][33];
+    __shared__ unsigned long long sb[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = blockIdx.x * 32 + lane;
+    float m = 0.0f, ss = 0.0f;
+    unsigned long long mb = 0;
+    if (r < rows) {
+#pragma unroll 4
+        for (int64_t k = warp; k < K; k += 32) {
+            const double x = X[k * ld + r];
+            const float v = abs_up(x);
+            const unsigned long long b = abs_bits(x);
+            m = fmaxf(m, v);
+            ss = fmaf(v, v, ss);
+            mb = b > mb ? b : mb;
+        }
+    }
+    sm[warp][lane] = m;
+    sq[warp][lane] = ss;
+    sb[warp][lane] = mb;
+    __syncthreads();
+    if (warp != 0 || r >= rows)
+        return;
+    for (int w = 1; w < 32; w++) {
+        m = fmaxf(m, sm[w][lane]);
+        ss += sq[w][lane];
+        mb = sb[w][lane] > mb ? sb[w][lane] : mb;
+    }
+    int s = 0;
+    if (!scale_fast(m, ss, bits, K, &s))
+        s = scale_slow(mb, bits, K);
+    sc[r] = s;
+    if (s == kNotFinite && bad)
+        atomicExch(bad, 1);
+}
+
+// The residues of such a matrix, as residue_rows_kernel: 32 rows x 64 columns per block
+// through shared memory (groups of eight columns four doubles further, so that eight
+// lanes reading eight columns apart take the minimum two wavefronts), so that reads run
+// along the rows and stores along the columns.
+template <int N>
+__global__ void __launch_bounds__(256)
+residue_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t k0, int64_t kp,
+                    int64_t pitch, const int *__restrict__ sc, __nv_bfloat16 *__restrict__ planes)
+{
+    constexpr int CH = moduli::chunks(N);
+    __shared__ double tile[64 * 32 + 8 * 4];
+    const int64_t kb = (int64_t)blockIdx.x * 64;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int row = threadIdx.x >> 3, kg = threadIdx.x & 7;
+    for (int r0 = blockIdx.y * 32; r0 < rows; r0 += gridDim.y * 32) {
+        __syncthreads();
+        for (int k = warp; k < 64; k += 8)
+            tile[k * 32 + (k >> 3) * 4 + lane] =
+                (r0 + lane < rows && kb + k < kp) ? X[(k0 + kb + k) * ld + r0 + lane] : 0.0;
+        __syncthreads();
+        if (r0 + row >= rows || kb + kg * 8 >= pitch)
+            continue;
+        const int s = max(sc[r0 + row], -4096);
+        float v[8][CH];
+#pragma unroll
+        for (int q = 0; q < 8; q++)
+            int_chunks<CH>(tile[(kg * 8 + q) * 32 + kg * 4 + row], s, v[q]);
+        uint64_t chunk[CH][4];
+        pack_chunks<N>(v, chunk);
+        store_residues<N, CH>(chunk, planes + (int64_t)(r0 + row) * pitch + kb + kg * 8,
+                              (int64_t)rows * pitch);
+    }
+}
+
+// Host side: the scales of `rows` rows over all K, and the planes of one K panel.
+template <class Src>
+static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int n_mod, int *sc, int *bad)
+{
+    if (rows <= 0)
+        return CUTC_OK;
+    row_scale_kernel<Src><<<std::min(rows, 1 << 20), 256, 0, st>>>(src, rows, K,
+                                                                    moduli::row_bits(n_mod), sc, bad);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+template <int N, class Src>
+static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t k0, int64_t kp,
+                        int64_t pitch, const int *sc, void *planes)
+{
+    if (rows <= 0 || kp <= 0)
+        return CUTC_OK;
+    dim3 grid(ceil_div(pitch, 8 * 128), (unsigned)std::min(rows, 65535));
+    residue_rows_kernel<N, Src><<<grid, 128, 0, st>>>(src, r0, rows, k0, kp, pitch, sc,
+                                                      (__nv_bfloat16 *)planes);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+template <class Src>
+static int residue_rows(cudaStream_t st, int n_mod, Src src, int r0, int rows, int64_t k0,
+                        int64_t kp, int64_t pitch, const int *sc, void *planes)
+{
+    switch (n_mod) {
+    case 7: return residue_rows<7>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    case 9: return residue_rows<9>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    case 11: return residue_rows<11>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    case 13: return residue_rows<13>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    case 15: return residue_rows<15>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    }
+    cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
+    return CUTC_ERR_INVALID;
+}
+
+static inline int row_scales_cols(cudaStream_t st, const double *X, int64_t ld, int rows,
+                                  int64_t K, int n_mod, int *sc, int *bad)
+{
+    if (rows <= 0)
+        return CUTC_OK;
+    row_scale_cols_kernel<<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K,
+                                                                moduli::row_bits(n_mod), sc, bad);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+template <int N>
+static int residue_cols(cudaStream_t st, const double *X, int64_t ld, int rows, int64_t k0,
+                        int64_t kp, int64_t pitch, const int *sc, void *planes)
+{
+    if (rows <= 0 || kp <= 0)
+        return CUTC_OK;
+    dim3 grid(ceil_div(pitch, 64), std::min(ceil_div(rows, 32), 65535u));
+    residue_cols_kernel<N><<<grid, 256, 0, st>>>(X, ld, rows, k0, kp, pitch, sc,
+                                                 (__nv_bfloat16 *)planes);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+static inline int residue_cols(cudaStream_t st, int n_mod, const double *X, int64_t ld, int rows,
+                               int64_t k0, int64_t kp, int64_t pitch, const int *sc, void *planes)
+{
+    switch (n_mod) {
+    case 7: return residue_cols<7>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 9: return residue_cols<9>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 11: return residue_cols<11>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 13: return residue_cols<13>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 15: return residue_cols<15>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    }
+    cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
+    return CUTC_ERR_INVALID;
+}
+
+}  // namespace cutc

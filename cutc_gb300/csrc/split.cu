@@ -1,47 +1,21 @@
-// Split-precision contractions on the sm_103a tensor cores (tcgen05 + TMA).
+// The split form's contractions (modular.cu), its pair terms on the tensor cores
+// (tcgen05 + TMA), and the operands of both.
 //
 // Both dense contractions of the cutc_int path
 //   X_m[p, r1] = sum_r2 P[p, r2] G_m[r1, r2]                    (X build)
 //   H[p, q] = sum_r1 X_3[p, r1] S0[q, r1],
 //   N[p, l] = -1/2 sum_{m, r1} X_m[p, r1] S_m[l, r1]          (int_2e)
-// are C[M x N] = alpha * A[M x K] B[N x K]^T with FP64 operands.  Each FP64
-// operand row r is written as
+// are C[M x N] = alpha * A[M x K] B[N x K]^T with FP64 operands and run as modular
+// contractions: exact integer products of the operands rounded on their row scales,
+// one BF16 tensor-core product per modulus (moduli.cuh).  n_slices chooses the number of
+// moduli (split_moduli): the precision of at least that many 9-bit slices.
+//
+// The pair terms' short contraction (K = 4 n_nuc) keeps the splitting into S slices,
 //     A[r, k] = 2^{e_r} sum_{s < S} a_s[r, k],  a_s = q_s 2^{-8-9s},  q_s in [-256, 256]
-// (S signed 9-bit digits of the row-scaled value, rounded at the last digit:
-// relative error <= 2^{-9S}), and every digit is an exact BF16 number.  The
-// products a_s b_t with s + t <= D = S - 1 run as tcgen05.mma kind::f16 (BF16
-// in, FP32 accumulate in tensor memory), one accumulator per diagonal d = s + t:
-//   * the accumulator of diagonal d sits at tensor-memory column BN d, so the
-//     products of slice a_s with b_0 .. b_{D-s} -- the B slices stacked in
-//     shared memory -- are ONE instruction of width N = BN (D + 1 - s) that
-//     lands on diagonals s .. D: S instructions per 16-wide K step instead of
-//     S (S + 1) / 2, and A is read from shared memory once per slice, which
-//     keeps the operand traffic under the shared-memory bandwidth;
-//   * every product of diagonal d is an integer multiple of 2^{-16-9d} of
-//     magnitude <= 2^{-9d}, so the FP32 accumulator holds the exact sum while
-//     (d + 1) * Kc * 2^16 <= 2^24.  The chunk is Kc = 128: exact for d <= 1;
-//     diagonal 2 (3 * 128 * 2^16 = 1.5 * 2^24 quanta at most) can round only if
-//     a chunk sum of 384 remainder-digit products exceeds 2^24 quanta, and then
-//     by one quantum 2^-34, which over the whole K stays below 2^-41 of
-//     sum_k |a_k b_k| -- under the slicing's own representation error.  (Kc = 64
-//     keeps d = 2 provably exact but flushes twice as often: 9 % slower on the
-//     medium X contraction at the same measured error);
-//   * after each chunk the epilogue adds the d = 0, 1, 2 sums error-free into
-//     FP32 (hi, lo) register pairs (hi on a coarse grid, lo the remainder)
-//     and d >= 3 (relative size 2^-27) into a plain FP32 sum; nothing is
-//     carried across chunks in tensor memory, whose FP32 accumulation
-//     rounding would otherwise grow with K;
-//   * the accumulators are double-buffered in tensor memory, so the flush of
-//     chunk c overlaps the MMAs of chunk c + 1;
-//   * at the end the seven FP32 pieces are summed error-free (TwoSum on f32x2 pairs
-//     of columns, the small remainders in FP32), the double-float result is
-//     converted with one FP64 add, and the scale 2^{e_r + f_n} (and a power-of-two
-//     alpha) is added to the exponent bits.
-// FP64 arithmetic is used only in that conversion (and in the pair terms that feed
-// G): GB300's FP64 pipe runs at 1/64 of the FP32 rate, and a full FP64 sum of the
-// pieces cost 7 % of the contraction.
-// The scheme is the error-free splitting of Ozaki, Ogita, Oishi & Rump
-// (2012), on BF16 instead of FP64 slices, with exact FP32 chunk accumulation.
+// (S signed 9-bit digits of the row-scaled value), whose products a_s b_t, s + t < S,
+// run as BF16 tcgen05.mma with one FP32 accumulator per diagonal s + t: with K <= 80 the
+// leading diagonals are exact in FP32, and the S slices of b are read by one instruction
+// per slice of a (the error-free splitting of Ozaki, Ogita, Oishi and Rump 2012).
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -57,354 +31,25 @@
 #include "digits.cuh"
 #include "pair.cuh"
 #include "products.cuh"
+#include "residue.cuh"
 #include "split.cuh"
 #include "tc.cuh"
 
 namespace cutc {
 
-// ---------------------------------------------------------------------------
-// GEMM kernel
-// ---------------------------------------------------------------------------
-
 constexpr int kBM = 128;        // rows of A per CTA (TMEM lanes)
 constexpr int kBK = 32;         // K per TMA box: 32 BF16 = 64-byte rows (64B swizzle)
-constexpr int kChunkBlocks = 4; // exact-accumulation chunk: 128 K
-constexpr int kMaxKPerLaunch = 1 << 18;  // keeps every exact (hi, lo) sum below 2^24 units
-// Default K per launch: one launch up to kLongK; a longer contraction runs as equal
-// launches of at most kLaunchK, summed in FP64 (the C += epilogue).  On one GB300 the
-// X contraction of the 300-AO molecule (K = 200 000, 1500 r1 rows) took 1826 ms in one
-// launch and 1282 ms in five of 40 000; the medium one (K = 80 000) 1176 and 1168 ms
-// in one and two launches, and 1205 ms in three.  Over a long K loop the CTAs of a
-// wave probably drift apart and stop sharing their A and B tiles in L2.  With an A
-// operand of kBigM rows or more, launches of at most kLaunchKBigM pay: the 300-AO X
-// contraction (M = 45 150, K = 200 000) took 5141 ms per 6000 r1 rows in launches of
-// 40 000, 4995 in launches of 20 000 and 4971 in launches of 10 000, while the medium
-// one (M = 7260) was the same at 40 000 and 20 000 and 4 % slower at 10 000.
+constexpr int kMaxKPerLaunch = 1 << 18;
+// Default K per launch (one panel of residues): one launch up to kLongK; a longer
+// contraction runs as equal launches of at most kLaunchK, whose residues are added up.
+// With an A operand of kBigM rows or more, launches of at most kLaunchKBigM, which bound
+// the residues of its panel.
 constexpr int kLongK = 65536;
 constexpr int kLaunchK = 49152;
 constexpr int kBigM = 16384;
 constexpr int kLongKBigM = 32768;
 constexpr int kLaunchKBigM = 24576;
 constexpr uint32_t kTmemCols = 512;
-constexpr int kGroupN = 8;      // column tiles per raster group (B tiles shared through L2)
-
-// Output-column tile for S slices: S diagonals x 2 buffers must fit 512 columns
-// and the widest instruction (N = BN S) must not exceed 256.
-__host__ __device__ constexpr int bn_for(int S) { return S <= 5 ? 48 : 32; }
-
-struct GemmParams {
-    int M, N;
-    int Mpad, Npad;
-    int kb0, nkb;          // K blocks [kb0, kb0 + nkb) of this launch
-    const int *ea;         // row exponents of A (Mpad)
-    const int *eb;         // row exponents of B (Npad)
-    double alpha;          // result x 2^alpha_exp, negated if alpha_neg, x alpha if alpha_mul
-    int alpha_exp, alpha_neg, alpha_mul;
-    double *C;
-    int64_t ldc;           // C[m + ldc * col(n)]
-    int ncol_group;        // col(n) = (n / ncol_group) * group_stride + col0 + n % ncol_group
-    int64_t group_stride;
-    int64_t col0;
-    int accumulate;        // C += result
-    int *err;              // set to a non-zero code if a bounded wait gave up
-};
-
-template <int S>
-struct GemmCfg {
-    static constexpr int kBN = bn_for(S);
-    static constexpr int kCW = 8;                    // columns per epilogue warp
-    static constexpr int kEpiWarps = 4 * (kBN / kCW); // 4 lane quarters x column groups
-    static constexpr int kTmaWarp = kEpiWarps;
-    static constexpr int kMmaWarp = kEpiWarps + 1;
-    static constexpr int kThreads = (kEpiWarps + 2) * 32;
-    static constexpr int kBuf = kBN * S;             // tensor-memory columns per buffer
-    static constexpr int kASlice = kBM * kBK * 2;
-    static constexpr int kBSlice = kBN * kBK * 2;
-    static constexpr int kStage = S * (kASlice + kBSlice);
-    static constexpr int kStagesFit = (220 * 1024) / kStage;
-    static constexpr int kStages = kStagesFit < 4 ? kStagesFit : 4;
-    static constexpr int kBarBytes = 256;
-    static constexpr int kSmem = kStages * kStage + 1024 + kBarBytes;
-    static_assert(kStages >= 2, "not enough shared memory for two stages");
-    static_assert(2 * kBuf <= (int)kTmemCols, "accumulators exceed tensor memory");
-    static_assert(kBN * S <= 256, "instruction N exceeds 256");
-    static_assert(kBSlice % 512 == 0, "B slices must stack on 8-row swizzle atoms");
-};
-
-__device__ __forceinline__ double pow2(int e)
-{
-    e = e < -1022 ? -1022 : (e > 1023 ? 1023 : e);
-    return __longlong_as_double((long long)(1023 + e) << 52);
-}
-
-// v 2^k: the exponent field moved with integer operations when v and the result are
-// normal numbers (GB300's FP64 pipe is slow), scalbn otherwise (zeros, and results that
-// underflow to subnormals or zero or overflow to infinity)
-__device__ __forceinline__ double scale_pow2(double v, int k)
-{
-    const long long b = __double_as_longlong(v);
-    const int e = (int)((b >> 52) & 0x7ff);
-    if (e != 0 && e + k >= 1 && e + k <= 2046)
-        return __longlong_as_double(b + ((long long)k << 52));
-    return scalbn(v, k);
-}
-
-template <int S>
-__global__ void __launch_bounds__(GemmCfg<S>::kThreads, 1)
-split_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  GemmParams P)
-{
-    using Cfg = GemmCfg<S>;
-    constexpr int D = S - 1;  // highest diagonal kept
-    constexpr int BN = Cfg::kBN, CW = Cfg::kCW;
-    constexpr int kEpiWarps = Cfg::kEpiWarps, kTmaWarp = Cfg::kTmaWarp, kMmaWarp = Cfg::kMmaWarp;
-    extern __shared__ __align__(1024) uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + Cfg::kStages * Cfg::kStage);
-    uint64_t *full = bars;
-    uint64_t *empty = bars + Cfg::kStages;
-    uint64_t *tfull = bars + 2 * Cfg::kStages;
-    uint64_t *tempty = tfull + 2;
-    uint64_t *drain = tempty + 2;
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
-    volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // grouped raster: a group of kGroupN column tiles sweeps the row tiles, so the
-    // CTAs of a wave share their B tiles and a few A tiles through L2 (0.4-1% faster
-    // than groups of 8 row tiles sweeping the columns, on the large and medium X builds)
-    const int num_m = P.Mpad / kBM, num_n = P.Npad / BN;
-    const int tid = blockIdx.x;
-    const int per_group = kGroupN * num_m;
-    const int gfirst = (tid / per_group) * kGroupN;
-    const int gsize = min(num_n - gfirst, kGroupN);
-    const int n0 = (gfirst + (tid % per_group) % gsize) * BN;
-    const int m0 = ((tid % per_group) / gsize) * kBM;
-    const int nkb = P.nkb;
-    const int nch = (nkb + kChunkBlocks - 1) / kChunkBlocks;
-
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < Cfg::kStages; i++) {
-            tc::mbar_init(tc::smem_u32(&full[i]), 1);
-            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
-        }
-        for (int i = 0; i < 2; i++) {
-            tc::mbar_init(tc::smem_u32(&tfull[i]), 1);
-            tc::mbar_init(tc::smem_u32(&tempty[i]), kEpiWarps);
-        }
-        tc::mbar_init(tc::smem_u32(drain), 1);
-        *s_abort = 0;
-        tc::fence_mbar_init();
-    }
-    if (warp == kMmaWarp) {
-        tc::tmem_alloc(tc::smem_u32(s_tmem), kTmemCols);
-        tc::tmem_relinquish();
-    }
-    if (warp == kTmaWarp && lane == 0) {
-        tc::tma_prefetch(&tmA);
-        tc::tma_prefetch(&tmB);
-    }
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    const uint32_t tbase = *s_tmem;
-
-    auto fail = [&](int code) {
-        *s_abort = 1;
-        atomicExch(P.err, code);
-    };
-
-    if (warp == kTmaWarp) {
-        if (lane == 0) {
-            int issued = 0;
-            for (int kb = 0; kb < nkb; kb++) {
-                const int stage = kb % Cfg::kStages, round = kb / Cfg::kStages;
-                if (round > 0 &&
-                    !tc::mbar_wait(tc::smem_u32(&empty[stage]), (round - 1) & 1, s_abort)) {
-                    fail(1);
-                    break;
-                }
-                const uint32_t fb = tc::smem_u32(&full[stage]);
-                tc::mbar_arrive_expect_tx(fb, Cfg::kStage);
-                uint8_t *st = smem + stage * Cfg::kStage;
-                const int x = (P.kb0 + kb) * kBK;
-#pragma unroll
-                for (int s = 0; s < S; s++)
-                    tc::tma_load_2d(tc::smem_u32(st + s * Cfg::kASlice), &tmA, x, s * P.Mpad + m0, fb);
-#pragma unroll
-                for (int t = 0; t < S; t++)
-                    tc::tma_load_2d(tc::smem_u32(st + S * Cfg::kASlice + t * Cfg::kBSlice), &tmB, x,
-                                    t * P.Npad + n0, fb);
-                issued = kb + 1;
-            }
-            if (*s_abort) {
-                // let the copies already issued land before the CTA goes away
-                for (int kb = max(0, issued - Cfg::kStages); kb < issued; kb++)
-                    tc::mbar_wait(tc::smem_u32(&full[kb % Cfg::kStages]),
-                                  (kb / Cfg::kStages) & 1, nullptr);
-            }
-        }
-    } else if (warp == kMmaWarp) {
-        if (lane == 0) {
-            bool ok = true;
-            for (int c = 0; c < nch && ok; c++) {
-                const int b = c & 1;
-                if (c >= 2 && !tc::mbar_wait(tc::smem_u32(&tempty[b]), ((c >> 1) - 1) & 1, s_abort)) {
-                    fail(2);
-                    break;
-                }
-                tc::fence_after_sync();
-                bool first = true;
-                const int kb_end = min(nkb, (c + 1) * kChunkBlocks);
-                for (int kb = c * kChunkBlocks; kb < kb_end; kb++) {
-                    const int stage = kb % Cfg::kStages, round = kb / Cfg::kStages;
-                    if (!tc::mbar_wait(tc::smem_u32(&full[stage]), round & 1, s_abort)) {
-                        fail(3);
-                        ok = false;
-                        break;
-                    }
-                    tc::fence_after_sync();
-                    const uint32_t sa = tc::smem_u32(smem + stage * Cfg::kStage);
-                    const uint32_t sb = sa + S * Cfg::kASlice;
-#pragma unroll
-                    for (int k16 = 0; k16 < kBK / 16; k16++) {
-                        const uint64_t bd = tc::smem_desc_sw64(sb + k16 * 32);
-#pragma unroll
-                        for (int s = 0; s < S; s++) {
-                            // a_s x [b_0 .. b_{D-s}] -> diagonals s .. D
-                            const uint32_t idesc = tc::idesc_bf16_f32(kBM, BN * (D + 1 - s));
-                            const uint64_t ad = tc::smem_desc_sw64(sa + s * Cfg::kASlice + k16 * 32);
-                            tc::mma_bf16(tbase + (uint32_t)(Cfg::kBuf * b + BN * s), ad, bd, idesc,
-                                         first ? 0u : 1u);
-                            first = false;
-                        }
-                    }
-                    tc::mma_commit(tc::smem_u32(&empty[stage]));
-                }
-                if (ok)
-                    tc::mma_commit(tc::smem_u32(&tfull[b]));
-            }
-            // all MMAs of this CTA have completed once the drain barrier flips
-            tc::mma_commit(tc::smem_u32(drain));
-            if (!tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
-                fail(5);
-        }
-    } else {
-        // ---- epilogue: exact chunk flushes, then the error-free final sum ----
-        const int q = warp & 3, cgrp = warp >> 2;
-        const uint32_t lane_off = (uint32_t)(q * 32) << 16;
-        const uint32_t coff = (uint32_t)(CW * cgrp);
-        // column pairs packed in 64 bits: every add below is one f32x2 instruction for
-        // two columns (round to nearest in each lane, as the scalar form)
-        constexpr int CP = CW / 2;
-        uint64_t hi0[CP], lo0[CP], hi1[CP], lo1[CP], hi2[CP], lo2[CP], s3[CP];
-#pragma unroll
-        for (int j = 0; j < CP; j++)
-            hi0[j] = lo0[j] = hi1[j] = lo1[j] = hi2[j] = lo2[j] = s3[j] = 0ull;
-        // v + C - C rounds v to the grid of C's binade: C = 1.5 2^(23 + g) gives multiples of 2^g
-        const uint64_t C0 = tc::f2_pack(__float_as_uint(786432.0f), __float_as_uint(786432.0f));
-        // 1.5 * 2^19: multiples of 2^-4  (d = 0, LSB 2^-16)
-        const uint64_t C1 = tc::f2_pack(__float_as_uint(1536.0f), __float_as_uint(1536.0f));
-        // 1.5 * 2^10: multiples of 2^-13 (d = 1, LSB 2^-25)
-        const uint64_t C2 = tc::f2_pack(__float_as_uint(3.0f), __float_as_uint(3.0f));
-        // 1.5 * 2^1:  multiples of 2^-22 (d = 2, LSB 2^-34)
-        auto exact_add = [](uint64_t x, uint64_t Cg, uint64_t &hi, uint64_t &lo) {
-            const uint64_t hh = tc::f2_sub(tc::f2_add(x, Cg), Cg);
-            hi = tc::f2_add(hi, hh);
-            lo = tc::f2_add(lo, tc::f2_sub(x, hh));
-        };
-        bool ok = true;
-        for (int c = 0; c < nch; c++) {
-            const int b = c & 1;
-            if (!tc::mbar_wait(tc::smem_u32(&tfull[b]), (c >> 1) & 1, s_abort)) {
-                fail(4);
-                ok = false;
-                break;
-            }
-            tc::fence_after_sync();
-#pragma unroll
-            for (int h = 0; h < CW / 4; h++) {
-                const uint32_t cb = tbase + lane_off + (uint32_t)(Cfg::kBuf * b) + coff + 4u * h;
-                uint32_t v[4];
-                tc::tmem_ld4_nowait(cb, v);
-                tc::tmem_wait_ld();
-                exact_add(tc::f2_pack(v[0], v[1]), C0, hi0[2 * h], lo0[2 * h]);
-                exact_add(tc::f2_pack(v[2], v[3]), C0, hi0[2 * h + 1], lo0[2 * h + 1]);
-                tc::tmem_ld4_nowait(cb + BN, v);
-                tc::tmem_wait_ld();
-                exact_add(tc::f2_pack(v[0], v[1]), C1, hi1[2 * h], lo1[2 * h]);
-                exact_add(tc::f2_pack(v[2], v[3]), C1, hi1[2 * h + 1], lo1[2 * h + 1]);
-                if (D >= 2) {
-                    tc::tmem_ld4_nowait(cb + 2 * BN, v);
-                    tc::tmem_wait_ld();
-                    exact_add(tc::f2_pack(v[0], v[1]), C2, hi2[2 * h], lo2[2 * h]);
-                    exact_add(tc::f2_pack(v[2], v[3]), C2, hi2[2 * h + 1], lo2[2 * h + 1]);
-                }
-#pragma unroll
-                for (int d = 3; d <= D; d++) {
-                    tc::tmem_ld4_nowait(cb + d * BN, v);
-                    tc::tmem_wait_ld();
-                    s3[2 * h] = tc::f2_add(s3[2 * h], tc::f2_pack(v[0], v[1]));
-                    s3[2 * h + 1] = tc::f2_add(s3[2 * h + 1], tc::f2_pack(v[2], v[3]));
-                }
-            }
-            tc::fence_before_sync();
-            __syncwarp();
-            if (lane == 0)
-                tc::mbar_arrive(tc::smem_u32(&tempty[b]));
-        }
-        const int m = m0 + q * 32 + lane;
-        if (ok && m < P.M) {
-            const int em = P.ea[m];
-            // The seven exact FP32 parts of each column, two columns per f32x2 operation:
-            // hi0 + hi1 + lo0 + hi2 + lo1 by TwoSum (exact), the rounding errors and the
-            // small lo2 and s3 in FP32 (below 2^-46 of the total), then one conversion to
-            // FP64 per part and one FP64 add.  The power-of-two scale goes into the
-            // exponent bits: GB300's FP64 pipe is slow, so the epilogue keeps off it.
-            auto two_sum = [](uint64_t a, uint64_t b, uint64_t &e) -> uint64_t {
-                const uint64_t sm = tc::f2_add(a, b);
-                const uint64_t bb = tc::f2_sub(sm, a);
-                e = tc::f2_add(tc::f2_sub(a, tc::f2_sub(sm, bb)), tc::f2_sub(b, bb));
-                return sm;
-            };
-#pragma unroll
-            for (int k = 0; k < CP; k++) {
-                uint64_t e1, e2, e3, e4;
-                uint64_t sm = two_sum(hi0[k], hi1[k], e1);
-                sm = two_sum(sm, lo0[k], e2);
-                sm = two_sum(sm, hi2[k], e3);
-                sm = two_sum(sm, lo1[k], e4);
-                const uint64_t lo = tc::f2_add(tc::f2_add(tc::f2_add(e1, e2), tc::f2_add(e3, e4)),
-                                               tc::f2_add(lo2[k], s3[k]));
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int n = n0 + (int)coff + 2 * k + h;
-                    if (n >= P.N)
-                        continue;
-                    const float sh = h ? tc::f2_hi(sm) : tc::f2_lo(sm);
-                    const float sl = h ? tc::f2_hi(lo) : tc::f2_lo(lo);
-                    double val = scale_pow2((double)sh + (double)sl, em + P.eb[n] + P.alpha_exp);
-                    if (P.alpha_neg)
-                        val = __longlong_as_double(__double_as_longlong(val) ^ (1ll << 63));
-                    if (P.alpha_mul)
-                        val *= P.alpha;
-                    const int64_t col = (int64_t)(n / P.ncol_group) * P.group_stride + P.col0 +
-                                        n % P.ncol_group;
-                    double *dst = P.C + m + P.ldc * col;
-                    *dst = P.accumulate ? *dst + val : val;
-                }
-            }
-        }
-    }
-
-    tc::fence_before_sync();
-    __syncthreads();
-    tc::fence_after_sync();
-    if (warp == kMmaWarp)
-        tc::tmem_dealloc(tbase, kTmemCols);
-}
-
 
 // ---------------------------------------------------------------------------
 // Pair terms on the tensor cores (split form, Jastrow exponents in {0, 2, 3, 4})
@@ -428,8 +73,7 @@ split_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 // of the point's 16 columns, add them exactly on fixed grids into double-float
 // values, release the accumulators, then finish the pair in double-float exactly as
 // pair_df_kernel does: g12 and its gradient, the powers of
-// g, -1/2 |grad u|^2, the FP64 path near e-e coalescence, the (hi, lo) G planes and
-// the G row maxima for the slicer.  Per pair that is about 800 FP32 operations
+// g, -1/2 |grad u|^2, the FP64 path near e-e coalescence and the (hi, lo) G planes.  Per pair that is about 800 FP32 operations
 // instead of 30 df multiply-adds (~450 operations) per nucleus.
 // ---------------------------------------------------------------------------
 
@@ -704,8 +348,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 V[2 * k + 1] = df::make(tc::f2_hi(hs), tc::f2_hi(ls));
             }
             const int64_t o = (int64_t)i * P.ldg + j;
-            float2 w4[4];
             if (jok) {
+                float2 w4[4];
                 const float2 *r1p = Q.r1d + 3 * (int64_t)i;
                 const float2 r1x = r1p[0], r1y = r1p[1], r1z = r1p[2];
                 df::D dx = df::sub(df::make(r1x.x, r1x.y), df::make(x2.x, x2.y));
@@ -760,20 +404,6 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int c = 0; c < 4; c++)
                     P.G[o + c * P.plane] = w4[c];
             }
-            if (P.rmax) {
-                // row maxima for the slicer from the float bits (as pair_df_kernel)
-                const unsigned mask = __ballot_sync(0xffffffffu, jok);
-                if (jok) {
-                    const bool leader = lane == __ffs(mask) - 1;
-#pragma unroll
-                    for (int c = 0; c < 4; c++) {
-                        const unsigned fb = __float_as_uint(w4[c].x) & 0x7fffffffu;
-                        const unsigned m = rmax_word(__reduce_max_sync(mask, fb));
-                        if (leader && m)
-                            atomicMax(&P.rmax[(int64_t)c * P.n1b + i], (unsigned long long)m << 32);
-                    }
-                }
-            }
         }
     }
 
@@ -787,79 +417,6 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 // ---------------------------------------------------------------------------
 // slicing kernels
 // ---------------------------------------------------------------------------
-
-// Operand sources: value of row r, column k of an FP64 matrix.
-struct SrcDense {  // X[r * ld + k]
-    static constexpr bool kDoubleFloat = false;
-    const double *X;
-    int64_t ld;
-    __device__ double operator()(int64_t r, int64_t k) const { return X[r * ld + k]; }
-};
-
-struct SrcConcat {  // [X1 | X2]: X1[r * k1 + k] for k < k1, then X2[r * k2 + k - k1]
-    static constexpr bool kDoubleFloat = false;
-    const double *X1, *X2;
-    int64_t k1, k2;
-    __device__ double operator()(int64_t r, int64_t k) const
-    {
-        return k < k1 ? X1[r * k1 + k] : X2[r * k2 + (k - k1)];
-    }
-};
-
-struct SrcDenseDF {  // hi + lo of X[r * ld + k]; the slicer reads the pair itself
-    static constexpr bool kDoubleFloat = true;
-    const float2 *X;
-    int64_t ld;
-    __device__ float2 pair(int64_t r, int64_t k) const { return X[r * ld + k]; }
-    __device__ double operator()(int64_t r, int64_t k) const
-    {
-        const float2 v = X[r * ld + k];
-        return (double)v.x + (double)v.y;
-    }
-};
-
-// The pair products take their first factor w chi_a from a table of the weighted AO
-// rows, formed once per AO (weighted_aos_kernel) instead of once per pair: FP64
-// multiplies run at 1/64 of the FP32 rate on GB300, and these sources are evaluated
-// twice per element (row maxima, then digits).
-struct SrcSym {  // w[k] chi_a(k) chi_b(k) = (w chi_a)(k) chi_b(k), (a, b) = pairs[r]
-    static constexpr bool kDoubleFloat = false;
-    const double *wchi, *chi;  // wchi[a * K + k] = w[k] chi_a(k); chi_b at chi[b * ldchi + k]
-    int64_t K, ldchi;
-    const int2 *pairs;
-    __device__ double operator()(int64_t r, int64_t k) const
-    {
-        const int2 ab = pairs[r];
-        return wchi[ab.x * K + k] * chi[ab.y * ldchi + k];
-    }
-};
-
-// w (chi_c d_m chi_d - chi_d d_m chi_c) as (w chi_c) d_m chi_d - (w chi_d) d_m chi_c,
-// k = m n + g, (c, d) = pairs[r]
-struct SrcAnti {
-    static constexpr bool kDoubleFloat = false;
-    const double *wchi, *aos;  // wchi[c * n + g] = w[g] chi_c(g); aos: (ld, nA, 4) with
-                               // the grid offset already applied
-    int n, nA;                 // n: grid points counted in k (g < n)
-    int64_t ld;                // grid stride of aos
-    const int2 *pairs;
-    __device__ double operator()(int64_t r, int64_t k) const
-    {
-        int m, g;
-        if (k < 0x7fffffff) {  // 32-bit division (K = 3 n)
-            const unsigned ku = (unsigned)k, mu = ku / (unsigned)n;
-            m = (int)mu;
-            g = (int)(ku - mu * (unsigned)n);
-        } else {
-            m = (int)(k / n);
-            g = (int)(k % n);
-        }
-        const int2 cd = pairs[r];
-        const int64_t comp = (int64_t)nA * ld * (m + 1);
-        return fma(wchi[(int64_t)cd.x * n + g], aos[comp + cd.y * ld + g],
-                   -(wchi[(int64_t)cd.y * n + g] * aos[comp + cd.x * ld + g]));
-    }
-};
 
 // wchi[a * n + g] = w[g] chi_a(g), chi_a at chi[a * ldchi]
 __global__ void weighted_aos_kernel(int n, const double *__restrict__ w,
@@ -883,11 +440,11 @@ static int weighted_aos(cudaStream_t st, int n, int nA, const double *w, const d
     return CUTC_OK;
 }
 
-// |v| as its bits (non-negative doubles order like their bits); NaN counts as 0, as
-// fmax would skip it.  Integer work: an FP64 max would take the FP64 pipe.
-__device__ __forceinline__ unsigned long long abs_bits(double v)
+// |v| as its bits; NaN counts as 0, as fmax would skip it.  Integer work: an FP64 max
+// would take the FP64 pipe.
+__device__ __forceinline__ unsigned long long max_bits(double v)
 {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
+    const unsigned long long b = abs_bits(v);
     return b > 0x7ff0000000000000ull ? 0ull : b;
 }
 
@@ -903,7 +460,7 @@ __global__ void rowmax_kernel(Src src, int rows, int64_t K, int64_t kper,
     const int64_t k1 = min(K, k0 + kper);
     unsigned long long m = 0;
     for (int64_t k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const unsigned long long b = abs_bits(src(r, k));
+        const unsigned long long b = max_bits(src(r, k));
         m = b > m ? b : m;
     }
 #pragma unroll
@@ -925,23 +482,6 @@ __global__ void rowmax_kernel(Src src, int rows, int64_t K, int64_t kper,
         if (threadIdx.x == 0 && m > 0)
             atomicMax(&rmax[r], m);
     }
-}
-
-// Row maxima of a matrix stored column by column: src[(k0 + k) * ld + r].
-__global__ void rowmax_cols_kernel(const double *X, int64_t ld, int64_t k0, int rows, int64_t K,
-                                   int64_t kper, unsigned long long *rmax)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= rows)
-        return;
-    const int64_t ka = (int64_t)blockIdx.y * kper, kb = min(K, ka + kper);
-    unsigned long long m = 0;
-    for (int64_t k = ka; k < kb; k++) {
-        const unsigned long long b = abs_bits(X[(k0 + k) * ld + r]);
-        m = b > m ? b : m;
-    }
-    if (m > 0)
-        atomicMax(&rmax[r], m);
 }
 
 // Exponent e with |x| < 2^e for every x of the row; 0 for zero (or denormal-only) rows.
@@ -987,17 +527,8 @@ __global__ void slice_kernel(Src src, int M, int64_t K, int64_t Kpad, int Mpad,
         __nv_bfloat16 d[4][S];
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            if constexpr (Src::kDoubleFloat) {
-                const float2 v = (r < M && k + q < K) ? src.pair(r, k + q) : make_float2(0.f, 0.f);
-                float qf[S];
-                digits::digits_df_fp32<S>(v.x, v.y, e, qf);
-#pragma unroll
-                for (int s = 0; s < S; s++)
-                    d[q][s] = __float2bfloat16_rn(__fmul_rn(qf[s], exp2f((float)(-8 - 9 * s))));
-            } else {
-                const double x = (r < M && k + q < K) ? src(r, k + q) : 0.0;
-                split_digits<S>(x, e, d[q]);
-            }
+            const double x = (r < M && k + q < K) ? src(r, k + q) : 0.0;
+            split_digits<S>(x, e, d[q]);
         }
 #pragma unroll
         for (int s = 0; s < S; s++) {
@@ -1014,89 +545,21 @@ __global__ void slice_kernel(Src src, int M, int64_t K, int64_t Kpad, int Mpad,
     }
 }
 
-// Same for a matrix stored column by column, src[(k0 + k) * ld + r], through a
-// 32 x 32 shared-memory transpose so reads and writes are both coalesced.
-template <int S>
-__global__ void slice_cols_kernel(const double *X, int64_t ld, int64_t k0, int M, int64_t K,
-                                  int64_t Kpad, int Mpad, const unsigned long long *rmax,
-                                  __nv_bfloat16 *slices, int *ex)
-{
-    __shared__ double tile[32][33];
-    const int r0 = blockIdx.y * 32;
-    const int64_t kb = (int64_t)blockIdx.x * 32;
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    for (int i = ty; i < 32; i += blockDim.y) {
-        const int64_t k = kb + i;
-        const int r = r0 + tx;
-        tile[i][tx] = (r < M && k < K) ? X[(k0 + k) * ld + r] : 0.0;
-    }
-    __syncthreads();
-    for (int i = ty; i < 32; i += blockDim.y) {
-        const int r = r0 + i;
-        const int64_t k = kb + tx;
-        if (r >= Mpad || k >= Kpad)
-            continue;
-        const int e = r < M ? row_exponent(rmax[r]) : 0;
-        if (k == 0)
-            ex[r] = e;
-        __nv_bfloat16 d[S];
-        split_digits<S>(tile[tx][i], e, d);
-#pragma unroll
-        for (int s = 0; s < S; s++)
-            slices[((int64_t)s * Mpad + r) * Kpad + k] = d[s];
-    }
-}
-
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static int get_encode(EncodeTiledFn *fn)
-{
-    static EncodeTiledFn cached = nullptr;
-    if (!cached) {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        cudaError_t e = cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                                         cudaEnableDefault, &q);
-        if (e != cudaSuccess || q != cudaDriverEntryPointSuccess || !p) {
-            cudaGetLastError();
-            cutc_set_error(CUTC_ERR_CUDA, "cuTensorMapEncodeTiled unavailable");
-            return CUTC_ERR_CUDA;
-        }
-        cached = (EncodeTiledFn)p;
-    }
-    *fn = cached;
-    return CUTC_OK;
-}
-
 // 2-D map over slices [rows_total][Kpad] BF16, box = kBK x box_rows, 64B swizzle.
 static int make_tmap(CUtensorMap *map, const void *base, int64_t rows_total, int64_t Kpad,
                      int box_rows)
 {
-    EncodeTiledFn enc;
-    CUTC_TRY(get_encode(&enc));
-    cuuint64_t dims[2] = {(cuuint64_t)Kpad, (cuuint64_t)rows_total};
-    cuuint64_t strides[1] = {(cuuint64_t)Kpad * 2};
-    cuuint32_t box[2] = {(cuuint32_t)kBK, (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims,
-                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
-                     CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        cutc_set_error(CUTC_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-        return CUTC_ERR_CUDA;
-    }
-    return CUTC_OK;
+    const uint64_t dims[2] = {(uint64_t)Kpad, (uint64_t)rows_total};
+    const uint64_t strides[1] = {(uint64_t)Kpad * 2};
+    const uint32_t box[2] = {(uint32_t)kBK, (uint32_t)box_rows};
+    return encode_bf16_map(map, base, 2, dims, strides, box, 64);
 }
-
 
 static int alloc_operand(Workspace &W, int slot, int S, int M, int row_mult, int64_t K,
                          Operand &op)
@@ -1115,18 +578,15 @@ static int alloc_operand(Workspace &W, int slot, int S, int M, int row_mult, int
     return CUTC_OK;
 }
 
-// have_rmax: op.rmax already holds the row maxima (written by the producer of src)
 template <int S, class Src>
-static int slice_rows(cudaStream_t st, Src src, Operand &op, bool have_rmax = false)
+static int slice_rows(cudaStream_t st, Src src, Operand &op)
 {
-    if (!have_rmax) {
-        CUTC_CUDA_TRY(cudaMemsetAsync(op.rmax, 0, (size_t)op.Mpad * 8, st));
-        if (op.M > 0 && op.K > 0) {
-            const int64_t kper = 16384;
-            dim3 g1((unsigned)op.M, ceil_div(op.K, kper));
-            rowmax_kernel<Src><<<g1, 256, 0, st>>>(src, op.M, op.K, kper, op.rmax);
-            CUTC_CUDA_TRY(cudaGetLastError());
-        }
+    CUTC_CUDA_TRY(cudaMemsetAsync(op.rmax, 0, (size_t)op.Mpad * 8, st));
+    if (op.M > 0 && op.K > 0) {
+        const int64_t kper = 16384;
+        dim3 g1((unsigned)op.M, ceil_div(op.K, kper));
+        rowmax_kernel<Src><<<g1, 256, 0, st>>>(src, op.M, op.K, kper, op.rmax);
+        CUTC_CUDA_TRY(cudaGetLastError());
     }
     if (op.Kpad % 4) {
         cutc_set_error(CUTC_ERR_INVALID, "operand K padding %lld is not a multiple of 4",
@@ -1136,24 +596,6 @@ static int slice_rows(cudaStream_t st, Src src, Operand &op, bool have_rmax = fa
     dim3 g2(ceil_div(op.Kpad, 4 * 256), (unsigned)std::min(op.Mpad, 65535));
     slice_kernel<S, Src><<<g2, 256, 0, st>>>(src, op.M, op.K, op.Kpad, op.Mpad, op.rmax,
                                              (__nv_bfloat16 *)op.sl, op.ex);
-    CUTC_CUDA_TRY(cudaGetLastError());
-    note_launches(have_rmax ? 1 : 2);
-    return CUTC_OK;
-}
-
-template <int S>
-static int slice_cols(cudaStream_t st, const double *X, int64_t ld, int64_t k0, Operand &op)
-{
-    CUTC_CUDA_TRY(cudaMemsetAsync(op.rmax, 0, (size_t)op.Mpad * 8, st));
-    if (op.M > 0 && op.K > 0) {
-        const int64_t kper = 512;
-        dim3 g1(ceil_div(op.M, 128), ceil_div(op.K, kper));
-        rowmax_cols_kernel<<<g1, 128, 0, st>>>(X, ld, k0, op.M, op.K, kper, op.rmax);
-        CUTC_CUDA_TRY(cudaGetLastError());
-    }
-    dim3 g2(ceil_div(op.Kpad, 32), ceil_div(op.Mpad, 32));
-    slice_cols_kernel<S><<<g2, dim3(32, 8), 0, st>>>(X, ld, k0, op.M, op.K, op.Kpad, op.Mpad,
-                                                     op.rmax, (__nv_bfloat16 *)op.sl, op.ex);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(2);
     return CUTC_OK;
@@ -1171,94 +613,67 @@ int split_k_blocks_per_launch(int64_t K, int64_t M, int k_split)
     return (int)((nkb_total + launches - 1) / launches);
 }
 
-// C = alpha A B^T (+ C) over the operands' common K.
-template <int S>
-static int gemm(cudaStream_t st, const Operand &A, const Operand &B, double alpha, double *C,
-                int64_t ldc, int ncol_group, int64_t group_stride, int64_t col0, int accumulate,
-                int *err, int k_split = 0)
-{
-    using Cfg = GemmCfg<S>;
-    static std::atomic<unsigned long long> attr_done{0};
-    const unsigned long long bit = current_device_bit();
-    if (!(attr_done.load() & bit)) {
-        CUTC_CUDA_TRY(cudaFuncSetAttribute(split_gemm_kernel<S>,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
-        attr_done.fetch_or(bit);
-    }
-    CUtensorMap ta, tb;
-    CUTC_TRY(make_tmap(&ta, A.sl, (int64_t)S * A.Mpad, A.Kpad, kBM));
-    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)S * B.Mpad, B.Kpad, Cfg::kBN));
-    const int nkb_total = (int)(A.Kpad / kBK);
-    const int kb_per = split_k_blocks_per_launch(A.Kpad, A.M, k_split);
-    if (A.Mpad % kBM || B.Mpad % Cfg::kBN) {
-        cutc_set_error(CUTC_ERR_INVALID, "operand padding does not match the tile");
-        return CUTC_ERR_INVALID;
-    }
-    dim3 grid((unsigned)((int64_t)(A.Mpad / kBM) * (B.Mpad / Cfg::kBN)));
-    for (int kb0 = 0; kb0 < nkb_total; kb0 += kb_per) {
-        GemmParams P;
-        P.M = A.M;
-        P.N = B.M;
-        P.Mpad = A.Mpad;
-        P.Npad = B.Mpad;
-        P.kb0 = kb0;
-        P.nkb = std::min(kb_per, nkb_total - kb0);
-        P.ea = A.ex;
-        P.eb = B.ex;
-        // a power of two (1, -1/2, 1/2 in this library) scales through the exponent
-        int ae = 0;
-        const double am = std::frexp(std::fabs(alpha), &ae);
-        P.alpha_mul = am != 0.5;
-        P.alpha_exp = P.alpha_mul ? 0 : ae - 1;
-        P.alpha_neg = !P.alpha_mul && alpha < 0;
-        P.alpha = alpha;
-        P.C = C;
-        P.ldc = ldc;
-        P.ncol_group = ncol_group;
-        P.group_stride = group_stride;
-        P.col0 = col0;
-        P.accumulate = (accumulate || kb0 > 0) ? 1 : 0;
-        P.err = err;
-        split_gemm_kernel<S><<<grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, P);
-        CUTC_CUDA_TRY(cudaGetLastError());
-        note_launches(1);
-    }
-    return CUTC_OK;
-}
-
 // ---------------------------------------------------------------------------
 // the plan for one build
 // ---------------------------------------------------------------------------
 
 enum SplitSlot {
-    SS_PAIRS_SYM = 0, SS_PAIRS_ANTI = 1, SS_ERR = 2,
-    SS_AX = 3, SS_BX = 6, SS_AH = 9, SS_AN = 12, SS_BH = 15, SS_BN = 18,
-    SS_AF = 21, SS_BC = 24, SS_F64 = 27, SS_C64 = 28, SS_R1D = 29, SS_BSCALE = 30,
-    SS_WCHI2 = 31, SS_WCHI1 = 32,
+    SS_PAIRS_SYM = 0, SS_PAIRS_ANTI, SS_ERR,
+    SS_AX, SS_AX_SC, SS_BX, SS_BX_SC, SS_RES,              // X build
+    SS_AI, SS_AI_SC, SS_BH, SS_BH_SC, SS_BN, SS_BN_SC,     // int_2e
+    SS_AF, SS_BC = SS_AF + 3, SS_F64 = SS_BC + 3, SS_C64, SS_R1D, SS_BSCALE,  // pair terms
+    SS_WCHI2, SS_WCHI1,
 };
 
+// K panel of a contraction (one launch's K).
+static int64_t panel_k(int64_t K, int64_t M, int k_split)
+{
+    return std::min(K, (int64_t)split_k_blocks_per_launch(K, M, k_split) * kBK);
+}
+
+// Device bytes for the residues of B's columns: as many as the G tile they are formed
+// from takes (its rows are then read once per panel, in a few groups of columns), at
+// least 1 GiB, so that small contractions run in one group.
+constexpr size_t kMinResidueBytes = (size_t)1 << 30;
+static size_t x_residue_bytes(int64_t rows, int64_t n2)
+{
+    return std::max(kMinResidueBytes, (size_t)rows * 4 * (size_t)n2 * 8);
+}
+// Device bytes of each operand's residues in the int_2e contractions.
+constexpr size_t kInt2eResidueBytes = (size_t)4 << 30;
+
+// K panel of the int_2e contractions: whole tensor-core chunks (256) whose residues of the
+// np rows of A fit.
+static int64_t int2e_panel_k(int n_mod, int64_t K, int64_t np, int k_split)
+{
+    const int64_t fit = (int64_t)(kInt2eResidueBytes / (2 * (size_t)n_mod * np)) / 256 * 256;
+    const int64_t cap = k_split > 0 ? panel_k(K, np, k_split) : K;
+    return std::min(cap, std::max<int64_t>(256, fit));
+}
 
 size_t split_r1_row_bytes(const Request &R)
 {
-    // slices of the four G rows of one r1 point
-    return 2 * (size_t)R.n_slices * 4 * (size_t)round_up(R.n2, kBK) + 64;
+    return 4 * (size_t)R.n2 * 8 + 64;  // residues, as many bytes as the four G rows
 }
 
 size_t split_int2e_row_bytes(const Request &R)
 {
-    const int64_t np = n_pairs(R.nA), nl = std::max<int64_t>(1, n_strict_pairs(R.nA));
-    const int bn = bn_for(R.n_slices);
-    // the point's K columns of the int_2e operands (X_3, X_012, S0, S), and its
-    // weighted AO values w chi_a
-    return 2 * (size_t)R.n_slices * (round_up(np, kBM) * 4 + round_up(np, bn) +
-                                     3 * (size_t)round_up(nl, bn)) + 8 * (size_t)R.nA + 64;
+    return 8 * (size_t)R.nA + 64;  // the point's weighted AO values w chi_a
 }
 
 size_t split_fixed_bytes(const Request &R)
 {
-    // P slices and the weighted AO values w chi_a on r2 they are formed from
-    return 2 * (size_t)R.n_slices * round_up(n_pairs(R.nA), kBM) * round_up(R.n2, kBK) +
-           8 * (size_t)R.nA * R.n2;
+    // residues of a K panel of P, the weighted AO values w chi_a on r2 they are formed
+    // from, the int_2e operands' residues, and the residues of one pass of results
+    const int n_mod = split_moduli(R.n_slices);
+    const int64_t np = n_pairs(R.nA);
+    size_t b = residue_bytes(n_mod, np, panel_k(R.n2, np, R.k_split)) + 8 * (size_t)R.nA * R.n2 +
+               std::min(kMinResidueBytes, residue_bytes(n_mod, 4 * (int64_t)R.n1, R.n2)) +
+               modular_out_bytes(n_mod, np,
+                                 std::max<int64_t>(np, std::min<int64_t>(4 * (int64_t)R.n1, 1 << 30)));
+    if (!R.x_only)
+        b += std::min(kInt2eResidueBytes, residue_bytes(n_mod, np, 3 * (int64_t)R.n1)) * 3;
+    return b;
 }
 
 static int upload_pairs(Workspace &W, int slot, cudaStream_t st, int nA, bool strict, int2 **out)
@@ -1288,56 +703,78 @@ static int upload_pairs(Workspace &W, int slot, cudaStream_t st, int nA, bool st
         return CUTC_ERR_INVALID;                                               \
     }
 
+// Row scales of an operand.
+static int scale_slot(Workspace &W, int slot, int rows, int **sc)
+{
+    void *p;
+    CUTC_TRY(W.get(slot, std::max<size_t>(1, rows) * sizeof(int), &p));
+    *sc = (int *)p;
+    return CUTC_OK;
+}
+
 int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *wr2,
                     const double *aos2v, int64_t n1t, int slot0, SplitPlan &sp)
 {
     Workspace &W = E->ws;
-    SplitPlan &S_ = sp;
     sp.slot0 = slot0;
     sp.n_slices = R.n_slices;
     sp.n1t = n1t;
+    const int n_mod = split_moduli(R.n_slices);
     const int np = (int)n_pairs(R.nA);
     void *p;
     CUTC_TRY(W.get(slot0 + SS_ERR, 64, &p));
-    S_.err = (int *)p;
-    CUTC_CUDA_TRY(cudaMemsetAsync(S_.err, 0, 4, st));
-    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_SYM, st, R.nA, false, &S_.pairs_sym));
-    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_ANTI, st, R.nA, true, &S_.pairs_anti));
-    CUTC_TRY(alloc_operand(W, slot0 + SS_AX, R.n_slices, np, kBM, R.n2, S_.AX));
-    CUTC_TRY(alloc_operand(W, slot0 + SS_BX, R.n_slices, (int)(4 * n1t), bn_for(R.n_slices), R.n2,
-                           S_.BX));
-    if (R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == S_.AX.sl)
-        return CUTC_OK;  // the same molecule's P slices are already there
+    sp.err = (int *)p;
+    CUTC_CUDA_TRY(cudaMemsetAsync(sp.err, 0, 4, st));
+    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_SYM, st, R.nA, false, &sp.pairs_sym));
+    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_ANTI, st, R.nA, true, &sp.pairs_anti));
+    CUTC_TRY(scale_slot(W, slot0 + SS_AX_SC, np, &sp.sc_ax));
+    CUTC_TRY(scale_slot(W, slot0 + SS_BX_SC, (int)(4 * n1t), &sp.sc_bx));
+    sp.k_panel = panel_k(R.n2, np, R.k_split);
+    CUTC_TRY(W.get(slot0 + SS_AX, residue_bytes(n_mod, np, sp.k_panel), &p));
+    sp.ax.p = p;
+    sp.ax.rows = np;
     CUTC_TRY(W.get(slot0 + SS_WCHI2, std::max<size_t>(1, (size_t)R.nA * R.n2) * 8, &p));
-    double *wchi = (double *)p;
-    CUTC_TRY(weighted_aos(st, R.n2, R.nA, wr2, aos2v, (int64_t)R.n2, wchi));
-    SrcSym src{wchi, aos2v, (int64_t)R.n2, (int64_t)R.n2, S_.pairs_sym};
-    CUTC_SLICES_DISPATCH(R.n_slices, CUTC_TRY((slice_rows<S, SrcSym>(st, src, S_.AX))));
+    sp.wchi2 = (const double *)p;
+    sp.aos2v = aos2v;
+    // with K in one panel the residues of P stay for every r1 tile (and, in a scan, for
+    // every set); with several panels each tile forms them again
+    sp.ax_whole = sp.k_panel >= R.n2;
+    if (R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == sp.ax.p)
+        return CUTC_OK;  // the same molecule's scales (and residues) are already there
+    CUTC_TRY(weighted_aos(st, R.n2, R.nA, wr2, aos2v, (int64_t)R.n2, (double *)p));
+    SrcSym src{sp.wchi2, aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
+    CUTC_TRY(row_scales(st, src, np, (int64_t)R.n2, n_mod, sp.sc_ax, (int *)nullptr));
+    if (sp.ax_whole)
+        CUTC_TRY(residue_rows(st, n_mod, src, 0, np, 0, R.n2, residue_pitch(R.n2), sp.sc_ax, sp.ax.p));
     E->tag_x = R.mol_tag;
-    E->tag_x_buf = S_.AX.sl;
+    E->tag_x_buf = sp.ax.p;
     return CUTC_OK;
 }
 
 int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, const float2 *G,
                  int nb, double *Xb, int blk_rows, int ib, cudaEvent_t gemm_begin,
-                 cudaEvent_t gemm_end, bool have_rmax)
+                 cudaEvent_t gemm_end)
 {
-    (void)E;
-    SplitPlan &S_ = sp;
-    Operand B = S_.BX;
-    B.M = 4 * nb;  // rows (c, i) of this tile; Mpad keeps the allocated padding
-    B.Mpad = (int)round_up(B.M, bn_for(sp.n_slices));
+    const int n_mod = split_moduli(sp.n_slices);
     const int64_t np = n_pairs(R.nA);
-    SrcDenseDF src{G, (int64_t)R.n2};
-    CUTC_SLICES_DISPATCH(sp.n_slices, {
-        CUTC_TRY((slice_rows<S, SrcDenseDF>(st, src, B, have_rmax)));
-        if (gemm_begin)
-            CUTC_CUDA_TRY(cudaEventRecord(gemm_begin, st));
-        // column (c, i) of the tile -> column c blk_rows + ib + i of the block
-        CUTC_TRY((gemm<S>(st, S_.AX, B, 1.0, Xb, np, nb, blk_rows, ib, 0, S_.err, R.k_split)));
-        if (gemm_end)
-            CUTC_CUDA_TRY(cudaEventRecord(gemm_end, st));
-    });
+    SrcSym sa{sp.wchi2, sp.aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
+    SrcDenseDF sb{G, (int64_t)R.n2};
+    CUTC_TRY(row_scales(st, sb, 4 * nb, (int64_t)R.n2, n_mod, sp.sc_bx, (int *)nullptr));
+    if (gemm_begin)
+        CUTC_CUDA_TRY(cudaEventRecord(gemm_begin, st));
+    // column (c, i) of the tile -> column c blk_rows + ib + i of the block
+    const ModularOut out{Xb, np, nb, blk_rows, ib, 1.0, 0.0};
+    CUTC_TRY(modular_contract(
+        st, E->ws, sp.slot0 + SS_BX, sp.slot0 + SS_RES, x_residue_bytes(sp.n1t, R.n2), n_mod,
+        (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, sp.ax_whole, false, sp.sc_ax, sp.sc_bx, out, sp.err, nullptr,
+        [&](int64_t k0, int64_t kp, const ResiduePlanes &a) {
+            return residue_rows(st, n_mod, sa, 0, (int)np, k0, kp, a.pitch, sp.sc_ax, a.p);
+        },
+        [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &b) {
+            return residue_rows(st, n_mod, sb, n0, nc, k0, kp, b.pitch, sp.sc_bx, b.p);
+        }));
+    if (gemm_end)
+        CUTC_CUDA_TRY(cudaEventRecord(gemm_end, st));
     return CUTC_OK;
 }
 
@@ -1346,47 +783,65 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
                      double *H, double *N, bool first)
 {
     Workspace &W = E->ws;
-    SplitPlan &S_ = sp;
     const int slot0 = sp.slot0;
     const int nA = R.nA;
     const int np = (int)n_pairs(nA), nl = (int)n_strict_pairs(nA);
-    const int bn = bn_for(sp.n_slices);
-    Operand AH, AN, BH, BN;
-    CUTC_TRY(alloc_operand(W, slot0 + SS_AH, sp.n_slices, np, kBM, nb, AH));
-    CUTC_TRY(alloc_operand(W, slot0 + SS_AN, sp.n_slices, np, kBM, 3 * (int64_t)nb, AN));
-    CUTC_TRY(alloc_operand(W, slot0 + SS_BH, sp.n_slices, np, bn, nb, BH));
-    CUTC_TRY(alloc_operand(W, slot0 + SS_BN, sp.n_slices, std::max(nl, 1), bn, 3 * (int64_t)nb, BN));
-    BN.M = nl;
-    const int acc = first ? 0 : 1;
-    // With the whole r1 grid in one tile the B operands depend on the molecule
-    // only, and a build with the same molecule tag keeps them.
-    const bool keep_b = nb == R.n1 && R.mol_tag && E->tag_i == R.mol_tag && E->tag_i_buf == BH.sl;
+    const int n_mod = split_moduli(sp.n_slices);
+    const int64_t k3 = 3 * (int64_t)nb;
+    const int64_t pan_h = int2e_panel_k(n_mod, nb, np, R.k_split);
+    const int64_t pan_n = int2e_panel_k(n_mod, k3, np, R.k_split);
     void *p;
     CUTC_TRY(W.get(slot0 + SS_WCHI1, std::max<size_t>(1, (size_t)nA * nb) * 8, &p));
     double *wchi = (double *)p;
-    if (!keep_b)
+    int *sc_a, *sc_h, *sc_n;
+    CUTC_TRY(scale_slot(W, slot0 + SS_AI_SC, np, &sc_a));
+    CUTC_TRY(scale_slot(W, slot0 + SS_BH_SC, np, &sc_h));
+    CUTC_TRY(scale_slot(W, slot0 + SS_BN_SC, nl, &sc_n));
+    CUTC_TRY(W.get(slot0 + SS_AI, std::max(residue_bytes(n_mod, np, pan_h),
+                                           residue_bytes(n_mod, np, pan_n)), &p));
+    ResiduePlanes a;
+    a.p = p;
+    // With the whole r1 grid in one block the B operands depend on the molecule only,
+    // and a build with the same molecule tag keeps them.
+    const bool whole = modular_whole(n_mod, np, nb, pan_h, kInt2eResidueBytes) &&
+                       modular_whole(n_mod, nl, k3, pan_n, kInt2eResidueBytes) &&
+                       modular_pass_cols(n_mod, np, np) >= np;
+    const bool keep_b = whole && nb == R.n1 && R.mol_tag && E->tag_i == R.mol_tag &&
+                        E->tag_i_buf == sc_h;
+    SrcSym s0{wchi, aos1, (int64_t)nb, ld1, sp.pairs_sym};
+    SrcAnti sn{wchi, aos1, nb, nA, ld1, sp.pairs_anti};
+    if (!keep_b) {
         CUTC_TRY(weighted_aos(st, nb, nA, wr1, aos1, ld1, wchi));
-    SrcSym s0{wchi, aos1, (int64_t)nb, ld1, S_.pairs_sym};
-    SrcAnti sa{wchi, aos1, nb, nA, ld1, S_.pairs_anti};
-    CUTC_SLICES_DISPATCH(sp.n_slices, {
-        // Xt[(m nb + i) np + p]: X_3 is column block 3, X_012 the blocks 0..2
-        CUTC_TRY(slice_cols<S>(st, Xt, np, 3 * (int64_t)nb, AH));
-        CUTC_TRY(slice_cols<S>(st, Xt, np, 0, AN));
-        if (!keep_b) {
-            CUTC_TRY((slice_rows<S, SrcSym>(st, s0, BH)));
-            if (nl > 0)
-                CUTC_TRY((slice_rows<S, SrcAnti>(st, sa, BN)));
-        }
-        CUTC_TRY(gemm<S>(st, AH, BH, 1.0, H, np, np, 0, 0, acc, S_.err, R.k_split));
-        if (nl > 0)
-            CUTC_TRY(gemm<S>(st, AN, BN, -0.5, N, np, nl, 0, 0, acc, S_.err, R.k_split));
-    });
-    if (nb == R.n1) {
-        E->tag_i = R.mol_tag;
-        E->tag_i_buf = BH.sl;
-    } else {
-        E->tag_i = 0;
+        CUTC_TRY(row_scales(st, s0, np, (int64_t)nb, n_mod, sc_h, (int *)nullptr));
+        CUTC_TRY(row_scales(st, sn, nl, k3, n_mod, sc_n, (int *)nullptr));
     }
+    const double beta = first ? 0.0 : 1.0;
+    // Xt[(m nb + i) np + p]: X_3 is column block 3, X_012 the blocks 0..2
+    const double *x3 = Xt + 3 * (int64_t)nb * np;
+    CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a, nullptr));
+    CUTC_TRY(modular_contract(
+        st, W, slot0 + SS_BH, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, np, nb, pan_h, a, false, keep_b, sc_a,
+        sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err, nullptr,
+        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            return residue_cols(st, n_mod, x3, np, np, k0, kp, o.pitch, sc_a, o.p);
+        },
+        [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            return residue_rows(st, n_mod, s0, n0, nc, k0, kp, o.pitch, sc_h, o.p);
+        }));
+    if (nl > 0) {
+        CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a, nullptr));
+        CUTC_TRY(modular_contract(
+            st, W, slot0 + SS_BN, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, nl, k3, pan_n, a, false, keep_b, sc_a,
+            sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err, nullptr,
+            [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+                return residue_cols(st, n_mod, Xt, np, np, k0, kp, o.pitch, sc_a, o.p);
+            },
+            [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
+                return residue_rows(st, n_mod, sn, n0, nc, k0, kp, o.pitch, sc_n, o.p);
+            }));
+    }
+    E->tag_i = whole && nb == R.n1 ? R.mol_tag : 0;
+    E->tag_i_buf = sc_h;
     return CUTC_OK;
 }
 
@@ -1574,67 +1029,57 @@ int split_check(cudaStream_t st, SplitPlan &sp)
     return CUTC_OK;
 }
 
+// C = alpha A B^T of two sources through the split form, synchronous on st.
+template <class Src>
+static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int M, int N,
+                        int64_t K, Src sa, Src sb, double alpha, double *C, int64_t ldc)
+{
+    Workspace &W = E->ws;
+    const int n_mod = split_moduli(n_slices);
+    const int64_t pan = panel_k(K, M, 0);
+    int *sc_a, *sc_b;
+    void *p;
+    CUTC_TRY(scale_slot(W, base, M, &sc_a));
+    CUTC_TRY(scale_slot(W, base + 1, N, &sc_b));
+    CUTC_TRY(W.get(base + 2, 64, &p));
+    int *err = (int *)p;
+    CUTC_TRY(W.get(base + 3, residue_bytes(n_mod, M, pan), &p));
+    ResiduePlanes a;
+    a.p = p;
+    CUTC_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
+    CUTC_TRY(row_scales(st, sa, M, K, n_mod, sc_a, (int *)nullptr));
+    CUTC_TRY(row_scales(st, sb, N, K, n_mod, sc_b, (int *)nullptr));
+    CUTC_TRY(modular_contract(
+        st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, false, sc_a, sc_b,
+        ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err, nullptr,
+        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            return residue_rows(st, n_mod, sa, 0, M, k0, kp, o.pitch, sc_a, o.p);
+        },
+        [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            return residue_rows(st, n_mod, sb, n0, nc, k0, kp, o.pitch, sc_b, o.p);
+        }));
+    SplitPlan sp;
+    sp.err = err;
+    return split_check(st, sp);
+}
+
 // Split-precision GEMM on device arrays: C[m + ldc n] = sum_k A[m K + k] B[n K + k].
 int split_gemm_dense(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K,
                      const double *A, const double *B, double *C, int64_t ldc)
 {
-    Workspace &W = E->ws;
-    const int base = 200;
-    Operand OA, OB;
-    CUTC_TRY(alloc_operand(W, base, n_slices, M, kBM, K, OA));
-    CUTC_TRY(alloc_operand(W, base + 3, n_slices, N, bn_for(n_slices), K, OB));
-    void *p;
-    CUTC_TRY(W.get(base + 6, 64, &p));
-    int *err = (int *)p;
-    CUTC_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
-    SrcDense sa{A, K}, sb{B, K};
-    CUTC_SLICES_DISPATCH(n_slices, {
-        CUTC_TRY((slice_rows<S, SrcDense>(st, sa, OA)));
-        CUTC_TRY((slice_rows<S, SrcDense>(st, sb, OB)));
-        CUTC_TRY(gemm<S>(st, OA, OB, 1.0, C, ldc, N, 0, 0, 0, err));
-    });
-    int herr = 0;
-    CUTC_CUDA_TRY(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
-    CUTC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (herr) {
-        cutc_set_error(CUTC_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (code %d)", herr);
-        return CUTC_ERR_TIMEOUT;
-    }
-    return CUTC_OK;
+    return gemm_sources(E, st, 200, n_slices, M, N, K, SrcDense{A, K}, SrcDense{B, K}, 1.0, C, ldc);
 }
 
 // C[m + ldc n] = alpha sum_k [A1 | A2][m, k] [B1 | B2][n, k] through the split form: the
 // two products of the same output as ONE contraction over K1 + K2 (one row scale per row
-// of the concatenation, exact accumulation over all of it).  A1, B1 are K1-contiguous,
-// A2, B2 K2-contiguous (device arrays); synchronous on st.
+// of the concatenation).  A1, B1 are K1-contiguous, A2, B2 K2-contiguous (device arrays);
+// synchronous on st.
 int split_gemm_concat(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K1,
                       const double *A1, const double *B1, int64_t K2, const double *A2,
                       const double *B2, double alpha, double *C, int64_t ldc)
 {
-    Workspace &W = E->ws;
-    const int base = 210;
-    const int64_t K = K1 + K2;
-    Operand OA, OB;
-    CUTC_TRY(alloc_operand(W, base, n_slices, M, kBM, K, OA));
-    CUTC_TRY(alloc_operand(W, base + 3, n_slices, N, bn_for(n_slices), K, OB));
-    void *p;
-    CUTC_TRY(W.get(base + 6, 64, &p));
-    int *err = (int *)p;
-    CUTC_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
-    SrcConcat sa{A1, A2, K1, K2}, sb{B1, B2, K1, K2};
-    CUTC_SLICES_DISPATCH(n_slices, {
-        CUTC_TRY((slice_rows<S, SrcConcat>(st, sa, OA)));
-        CUTC_TRY((slice_rows<S, SrcConcat>(st, sb, OB)));
-        CUTC_TRY(gemm<S>(st, OA, OB, alpha, C, ldc, N, 0, 0, 0, err));
-    });
-    int herr = 0;
-    CUTC_CUDA_TRY(cudaMemcpyAsync(&herr, err, 4, cudaMemcpyDeviceToHost, st));
-    CUTC_CUDA_TRY(cudaStreamSynchronize(st));
-    if (herr) {
-        cutc_set_error(CUTC_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (code %d)", herr);
-        return CUTC_ERR_TIMEOUT;
-    }
-    return CUTC_OK;
+    return gemm_sources(E, st, 210, n_slices, M, N, K1 + K2, SrcConcat{A1, A2, K1, K2},
+                        SrcConcat{B1, B2, K1, K2}, alpha, C, ldc);
 }
 
 }  // namespace cutc

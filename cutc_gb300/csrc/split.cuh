@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "engine.cuh"
+#include "modular.cuh"
 #include "pair.cuh"
 
 namespace cutc {
@@ -12,7 +13,8 @@ namespace cutc {
 constexpr int kMaxSlices = 7;
 constexpr int kDefaultSlices = 5;
 
-// One FP64 operand as S BF16 slices [S][Mpad][Kpad] plus row exponents.
+// One FP64 operand of the pair contraction as S BF16 slices [S][Mpad][Kpad] plus row
+// exponents.
 struct Operand {
     void *sl = nullptr;               // __nv_bfloat16 slices
     int *ex = nullptr;                // row exponents (Mpad)
@@ -25,8 +27,12 @@ struct SplitPlan {
     int slot0 = 0;
     int n_slices = 0;
     int64_t n1t = 0;
-    Operand AX;                        // P slices: X-build A operand
-    Operand BX;                        // G-tile slices: X-build B operand
+    ResiduePlanes ax;                  // residues of P (a K panel, or all of K: ax_whole)
+    bool ax_whole = false;
+    int64_t k_panel = 0;               // K per launch of the X contraction
+    int *sc_ax = nullptr, *sc_bx = nullptr;  // row scales of P and of a G tile
+    const double *wchi2 = nullptr;     // w chi_a on r2, the first factor of P
+    const double *aos2v = nullptr;     // the AO values on r2, the second
     // pair terms on the tensor cores: F slices (powers of f2 on r2), the tile's
     // coefficient slices, and their FP64 sources
     bool pair_tc = false;
@@ -40,15 +46,15 @@ struct SplitPlan {
     int *err = nullptr;                // device flag set by a bounded wait that gave up
 };
 
-// Device bytes per r1 row of an X tile (slices of G).
+// Device bytes per r1 row of an X tile (residues of G).
 size_t split_r1_row_bytes(const Request &R);
 // 32-wide K blocks per tensor-core launch of a contraction over K with an A operand of
 // M rows (k_split as in cutc_options: 0 = one launch up to K = 65536, equal launches of
 // <= 49152 beyond; for M >= 16384 one launch up to 32768, launches of <= 24576 beyond).
 int split_k_blocks_per_launch(int64_t K, int64_t M, int k_split);
-// Device bytes per r1 row of an int_2e block (slices of its int_2e operands).
+// Device bytes per r1 row of an int_2e block (residues of its int_2e operands).
 size_t split_int2e_row_bytes(const Request &R);
-// Device bytes that do not depend on the tile size (the P slices).
+// Device bytes that do not depend on the tile size (a panel of P's residues, results).
 size_t split_fixed_bytes(const Request &R);
 // The bounded-wait check behind cutc_check_wait_limit: CUTC_ERR_TIMEOUT when the
 // wait gave up as designed.
@@ -57,11 +63,10 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
                     const double *aos2v, int64_t n1t, int slot0, SplitPlan &sp);
 // X of one r1 tile from the df tile G[c][i][j] ((hi, lo) pairs), written into the
 // int_2e block buffer Xb[(m blk_rows + ib + i) np + p] (the tile starts at row ib of
-// a block of blk_rows rows).  have_rmax: the row maxima of G are already in
-// sp.BX.rmax (rows c nb + i).
+// a block of blk_rows rows).
 int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, const float2 *G,
                  int nb, double *Xb, int blk_rows, int ib, cudaEvent_t gemm_begin,
-                 cudaEvent_t gemm_end, bool have_rmax = false);
+                 cudaEvent_t gemm_end);
 // Adds an r1 block's share of the int_2e contractions to H and N (overwrites when
 // first): wr1 and aos1 point at the block's first row, ld1 is the row stride of aos1,
 // Xt[(m nb + i) np + p] holds the block's X rows.
@@ -78,7 +83,7 @@ bool split_pair_tc_ok(const Request &R, const int *exps, int n_terms);
 int split_pair_prepare(Engine *E, const Request &R, cudaStream_t st, const double *f2,
                        int64_t n1t, SplitPlan &sp);
 // The pair planes G of one r1 tile (P: the tile's rows, outputs and near-coalescence
-// data, as for launch_pair_df; its rmax must be zeroed).
+// data, as for launch_pair_df).
 int split_pair_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp,
                     const PairDfArgs &P, const double *rn, double a_en);
 // Device bytes of the tensor-core pair operands: fixed (F) and per r1 row of a tile.

@@ -35,7 +35,7 @@ extern "C" {
 
 /* ---- precision forms --------------------------------------------------- */
 #define CUTC_PLAIN_FP64 0 /* FP64 contractions: the drop-in form */
-#define CUTC_SPLIT_BF16 1 /* FP64 operands split into BF16 slices on tcgen05, exact FP32 sums, FP64 result */
+#define CUTC_SPLIT_BF16 1 /* FP64 operands rounded and split into BF16 residues on tcgen05, exact sums, FP64 result */
 
 /*
  * Drop-in replacement for CuTC's cutc_int (src/cutc_int.c:15-20).
@@ -72,7 +72,8 @@ typedef struct cutc_basis {
 
 typedef struct cutc_options {
     int precision;          /* CUTC_PLAIN_FP64 or CUTC_SPLIT_BF16 */
-    int n_slices;           /* split form: BF16 slices per operand, 3..7 (default 5) */
+    int n_slices;           /* split form: precision of the operands in 9-bit slices, 3..7
+                               (default 5) */
     double a_en;            /* e-n Jastrow scale: f = a r / (1 + a r); 1.0 = reference */
     double a_ee;            /* e-e Jastrow scale; 1.0 = reference */
     int x_components;       /* X components copied out: 3 (reference) or 4 */
@@ -81,7 +82,7 @@ typedef struct cutc_options {
     void *stream;           /* cudaStream_t to run on; NULL = the engine's stream */
     int pair_fp64;          /* split form: 1 = pair terms in FP64 instead of double-float */
     int k_split;            /* split form: max K per tensor-core launch; the partial results
-                               are summed in FP64 (0 = automatic: one launch up to K = 65536,
+                               are added exactly (0 = automatic: one launch up to K = 65536,
                                equal launches of at most 49152 beyond) */
     int int2e_layout;       /* CUTC_INT2E_PQST (reference order) or CUTC_INT2E_PSQT: int_2e with
                                its 2nd and 3rd indices swapped, as trans_pqst_psqt_inplace
@@ -140,7 +141,7 @@ int cutc_int_ex(const cutc_options *opt,
  * A Jastrow-parameter scan: the build of cutc_int_ex for n_sets parameter sets
  * on one molecule.  The molecule arrays are copied to the device once and the
  * Jastrow-independent operands (the AO pair products on both grids, or their
- * BF16 slices) are built once and shared by all sets; only the pair terms and
+ * BF16 residues) are built once and shared by all sets; only the pair terms and
  * the contractions run per set.  Set s uses c/m/n/o_bh + s * size_bh * n_nuc,
  * a_en[s] and a_ee[s] (NULL: opt->a_en / opt->a_ee) and writes its outputs at
  * int2_grad1_u12_ao + s * x_components * n_grid1 * n_ao^2 and
@@ -212,8 +213,9 @@ int cutc_check_wait_limit(void);
 /*
  * The split-precision contraction alone, on device arrays of the current
  * device: C[m + ldc * n] = sum_k A[m * K + k] * B[n * K + k] for m < M, n < N,
- * with A and B FP64 row-major (K contiguous) and the product formed from
- * n_slices BF16 slices per operand on the tcgen05 tensor cores (3..7 slices).
+ * with A and B FP64 row-major (K contiguous) and the product formed
+ * exactly from operands rounded to the precision of n_slices 9-bit slices (3..7), on
+ * the tcgen05 tensor cores.  A row with an infinity or a NaN gives NaN results.
  * This is the kernel behind CUTC_SPLIT_BF16, exposed for callers that need the
  * GEMM itself.  Synchronous on the engine stream.  No reference counterpart.
  */
