@@ -31,6 +31,8 @@
 
 #include "common.cuh"
 #include "dgemm.cuh"
+#include "modular.cuh"
+#include "residue.cuh"
 
 namespace cutc {
 
@@ -86,19 +88,23 @@ struct Args {
     const double *A, *B;
     double *C;
     int64_t lda, ldb, ldc, sa, sb, sc;
-    int tiles_m, tiles_n;
+    int tiles_m, tiles_n, batch;
+    const int *only_if;
 };
 
 template <bool AK>
 __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
 {
+    if (g.only_if && *g.only_if == 0)
+        return;
     extern __shared__ __align__(16) double smem[];
     double *sA = smem;                       // kStages x kStageA
     double *sB = smem + kStages * kStageA;   // kStages x kStageB
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t per_batch = (int64_t)g.tiles_m * g.tiles_n;
-    const int64_t t = blockIdx.x;
+    // (one tile per block; a launch that waits for only_if has few blocks and walks them)
+    for (int64_t t = blockIdx.x; t < per_batch * g.batch; t += gridDim.x) {
     const int z = (int)(t / per_batch);
     const int64_t r = t - (int64_t)z * per_batch;
     const int m0 = (int)(r % g.tiles_m) * kBM;  // m fastest: a wave shares the B tiles
@@ -204,13 +210,15 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
             }
         }
     }
+    __syncthreads();  // the next tile's copies reuse the stages
+    }
 }
 
 }  // namespace
 
 int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double alpha,
               const double *A, int64_t lda, int64_t sa, const double *B, int64_t ldb, int64_t sb,
-              double beta, double *C, int64_t ldc, int64_t sc, int batch)
+              double beta, double *C, int64_t ldc, int64_t sc, int batch, const int *only_if)
 {
     if (M < 0 || N < 0 || K < 0 || batch < 0 || ldc < std::max(1, M) ||
         (K > 0 && (!A || !B || ldb < K || lda < (a_kmajor ? K : (int64_t)M))) || (M && N && !C)) {
@@ -244,6 +252,8 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
     g.sa = sa;
     g.sb = sb;
     g.sc = sc;
+    g.only_if = only_if;
+    g.batch = batch;
     g.tiles_m = (M + kBM - 1) / kBM;
     g.tiles_n = (N + kBN - 1) / kBN;
     const int64_t tiles = (int64_t)g.tiles_m * g.tiles_n * batch;
@@ -252,12 +262,138 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
                        (long long)tiles);
         return CUTC_ERR_INVALID;
     }
+    // a launch that mostly finds nothing to do has one block per SM
+    const unsigned grid = (unsigned)(only_if ? std::min<int64_t>(tiles, 152) : tiles);
     if (a_kmajor)
-        fp64_gemm_kernel<true><<<(unsigned)tiles, kThreads, kSmem, st>>>(g);
+        fp64_gemm_kernel<true><<<grid, kThreads, kSmem, st>>>(g);
     else
-        fp64_gemm_kernel<false><<<(unsigned)tiles, kThreads, kSmem, st>>>(g);
+        fp64_gemm_kernel<false><<<grid, kThreads, kSmem, st>>>(g);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
+    return CUTC_OK;
+}
+
+// ---------------------------------------------------------------------------
+// FP64 contractions on the BF16 tensor cores
+// ---------------------------------------------------------------------------
+//
+// GB300's FP64 pipe gives 1.1 TF/s; 15 residue products at about 1.8 PF/s of BF16 give
+// more than 100 TF/s, with a smaller error: the operands are rounded at 2^-62 of their
+// row norms and nothing else until the result is rounded to FP64, where a sum of K FP64
+// terms rounds K times.  Below K = 16 the DMMA kernel does no more than one of its K steps
+// (65 us a wave of tiles), which the modular contraction's launches do not beat.
+
+constexpr int kMinContractK = 16;
+constexpr size_t kAResidueBytes = (size_t)8 << 30;  // of a K panel of A
+constexpr size_t kBResidueBytes = (size_t)4 << 30;  // of a group of columns of B
+enum ContractSlot { C_FLAGS = 100, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
+
+static int64_t contract_panel(int64_t M, int64_t K)
+{
+    const int64_t fit = (int64_t)(kAResidueBytes / (2 * (size_t)kPlainModuli * std::max<int64_t>(M, 1))) /
+                        512 * 512;
+    return std::min(K, std::max<int64_t>(512, fit));
+}
+
+size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K)
+{
+    const int64_t kp = contract_panel(M, K);
+    return residue_bytes(kPlainModuli, M, kp) +
+           residue_bytes(kPlainModuli, modular_b_rows(kPlainModuli, N, kp, kBResidueBytes), kp) +
+           modular_out_bytes(kPlainModuli, M, N) + 4 * (size_t)(M + N);
+}
+
+int fp64_contract_begin(Workspace &W, cudaStream_t st, int **flags)
+{
+    void *p;
+    CUTC_TRY(W.get(C_FLAGS, 64, &p));
+    *flags = (int *)p;  // [0]: a wait gave up, [1]: an operand is not finite
+    CUTC_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
+    return CUTC_OK;
+}
+
+int fp64_contract_check(cudaStream_t st, const int *flags)
+{
+    int err = 0;
+    CUTC_CUDA_TRY(cudaMemcpyAsync(&err, flags, 4, cudaMemcpyDeviceToHost, st));
+    CUTC_CUDA_TRY(cudaStreamSynchronize(st));
+    if (err) {
+        cutc_set_error(CUTC_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (code %d)", err);
+        return CUTC_ERR_TIMEOUT;
+    }
+    return CUTC_OK;
+}
+
+// A K-contiguous (rows lda apart) or M-contiguous (columns lda apart), B K-contiguous.
+static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+                    int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
+                    const ModularOut &out)
+{
+    constexpr int n_mod = kPlainModuli;
+    int *err = flags, *bad = flags + 1;
+    const int64_t pan = contract_panel(M, K);
+    void *p;
+    CUTC_TRY(W.get(C_SCA, (size_t)M * 4, &p));
+    int *sca = (int *)p;
+    CUTC_TRY(W.get(C_SCB, (size_t)N * 4, &p));
+    int *scb = (int *)p;
+    CUTC_TRY(W.get(C_RA, residue_bytes(n_mod, M, pan), &p));
+    ResiduePlanes a;
+    a.p = p;
+    CUTC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, st));
+    const SrcDense sa{A, lda}, sb{B, ldb};
+    if (a_kmajor)
+        CUTC_TRY(row_scales(st, sa, M, K, n_mod, sca, bad));
+    else
+        CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
+    CUTC_TRY(row_scales(st, sb, N, K, n_mod, scb, bad));
+    return modular_contract(
+        st, W, C_RB, C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, false, sca, scb, out,
+        err, bad,
+        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
+            return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, k0, kp, o.pitch, sca, o.p)
+                            : residue_cols<n_mod>(st, A, lda, M, k0, kp, o.pitch, sca, o.p);
+        },
+        [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            return residue_rows<n_mod>(st, sb, n0, nc, k0, kp, o.pitch, scb, o.p);
+        });
+}
+
+int fp64_contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+                  int64_t K, double alpha, const double *A, int64_t lda, int64_t sa,
+                  const double *B, int64_t ldb, int64_t sb, double beta, double *C, int64_t ldc,
+                  int64_t sc, int batch)
+{
+    const bool joined = batch == 1 || (sa == 0 && sb == (int64_t)N * ldb && sc % ldc == 0 &&
+                                       (int64_t)N * batch <= INT32_MAX);
+    if (K < kMinContractK || M <= 0 || N <= 0 || batch <= 0 || ldc < M || ldb < K ||
+        lda < (a_kmajor ? K : (int64_t)M))  // (fp64_gemm refuses what it cannot take)
+        return fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc,
+                         batch);
+    if (!joined) {
+        for (int z = 0; z < batch; z++)
+            CUTC_TRY(fp64_contract(W, st, flags, a_kmajor, M, N, K, alpha, A + z * sa, lda, 0,
+                                   B + z * sb, ldb, 0, beta, C + z * sc, ldc, 0, 1));
+        return CUTC_OK;
+    }
+    CUTC_TRY(contract(W, st, flags, a_kmajor, M, N * batch, K, A, lda, B, ldb,
+                      ModularOut{C, ldc, N, batch > 1 ? sc / ldc : 0, 0, alpha, beta}));
+    return fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch,
+                     flags + 1);
+}
+
+int fp64_contract_rows(Workspace &W, cudaStream_t st, int *flags, int M, int N, int64_t K,
+                       const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
+                       int64_t ldc, int nrow_group, int64_t row_stride)
+{
+    if (K >= kMinContractK)
+        CUTC_TRY(contract(W, st, flags, true, M, N, K, A, lda, B, ldb,
+                          ModularOut{C, ldc, N, 0, 0, 1.0, 0.0, nrow_group, row_stride}));
+    // the groups of rows as a batch: C of group z starts z row_stride further
+    const int *only_if = K >= kMinContractK ? flags + 1 : nullptr;
+    const int groups = M / nrow_group;
+    CUTC_TRY(fp64_gemm(st, true, nrow_group, N, K, 1.0, A, lda, (int64_t)nrow_group * lda, B, ldb,
+                       0, 0.0, C, ldc, row_stride, groups, only_if));
     return CUTC_OK;
 }
 

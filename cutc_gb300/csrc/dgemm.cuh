@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "engine.cuh"
+
 namespace cutc {
 
 // C[m + ldc n] = alpha sum_k opA(m, k) B[n ldb + k] + beta C[m + ldc n]
@@ -13,8 +15,31 @@ namespace cutc {
 // B is K contiguous per column n (OP_N on a K x N column-major array).  With
 // beta == 0, C is not read.  Column-major C, as cuBLAS: the same call sites
 // keep their argument meaning.
+// only_if (may be null): the kernels return at once while *only_if is zero.
 int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double alpha,
               const double *A, int64_t lda, int64_t sa, const double *B, int64_t ldb, int64_t sb,
-              double beta, double *C, int64_t ldc, int64_t sc, int batch);
+              double beta, double *C, int64_t ldc, int64_t sc, int batch,
+              const int *only_if = nullptr);
+
+// The same contraction for callers with a workspace: a modular contraction on the BF16
+// tensor cores (modular.cuh) with operands rounded at 2^-62 of their row norms, below the
+// rounding of an FP64 sum, with fp64_gemm in its place for operands that hold an
+// infinity or a NaN (found on the device) and for K < 16.  flags: from fp64_contract_begin;
+// a bounded wait that gives up makes the results NaN and is reported by
+// fp64_contract_check.  Batches whose A is common and whose B rows follow one another
+// (sa = 0, sb = N ldb) are one contraction; others run one by one.
+int fp64_contract_begin(Workspace &W, cudaStream_t st, int **flags);
+int fp64_contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+                  int64_t K, double alpha, const double *A, int64_t lda, int64_t sa,
+                  const double *B, int64_t ldb, int64_t sb, double beta, double *C, int64_t ldc,
+                  int64_t sc, int batch);
+// C[row(m) + ldc n] = sum_k A[m lda + k] B[n ldb + k] with rows in groups of nrow_group,
+// row_stride apart (no batch).
+int fp64_contract_rows(Workspace &W, cudaStream_t st, int *flags, int M, int N, int64_t K,
+                       const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
+                       int64_t ldc, int nrow_group, int64_t row_stride);
+int fp64_contract_check(cudaStream_t st, const int *flags);
+// Device bytes fp64_contract keeps for operands of these sizes.
+size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K);
 
 }  // namespace cutc

@@ -410,8 +410,10 @@ static size_t fixed_bytes(const Request &R)
     double b = (double)nN * n2 * 8;
     if (!R.x_only)
         b += ((double)np * np + (double)np * nl) * 8;
-    if (R.precision == CUTC_PLAIN_FP64)
-        b += (double)np * n2 * 8;
+    if (R.precision == CUTC_PLAIN_FP64)  // P, and the contractions' residues
+        b += (double)np * n2 * 8 +
+             (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2),
+                              R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1));
     else
         b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2) +
              (double)split_pair_fixed_bytes(R);
@@ -708,6 +710,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     note_launches(1);
 
     SplitPlan sp;
+    int *flags = nullptr;  // of the plain form's contractions
     float2 *d_r2d = nullptr, *d_f2d = nullptr, *d_poly = nullptr;
     int pexp = 4;
     bool psparse = false;
@@ -724,6 +727,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         note_launches(1);
     }
     if (R.precision == CUTC_PLAIN_FP64) {
+        CUTC_TRY(fp64_contract_begin(W, st, &flags));
         CUTC_TRY(W.get(S_P, (size_t)np * n2 * 8, &p));
         d_P = (double *)p;
         if (!(R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == d_P)) {
@@ -860,9 +864,9 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             const double one = 1.0, zero = 0.0;
             if (tev)
                 CUTC_CUDA_TRY(cudaEventRecord(tev[2], st));
-            CUTC_TRY(fp64_gemm(st, true, (int)np, nb, n2, one, d_P, n2, 0, d_G, n2,
-                               (int64_t)nb * n2, zero, d_Xt + (int64_t)ib * np, np,
-                               (int64_t)blk_rows * np, 4));
+            CUTC_TRY(fp64_contract(W, st, flags, true, (int)np, nb, n2, one, d_P, n2, 0, d_G, n2,
+                                   (int64_t)nb * n2, zero, d_Xt + (int64_t)ib * np, np,
+                                   (int64_t)blk_rows * np, 4));
             if (tev)
                 CUTC_CUDA_TRY(cudaEventRecord(tev[3], st));
         } else {
@@ -913,12 +917,13 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
                 E->tag_i = K == n1 ? R.mol_tag : 0;
                 E->tag_i_buf = d_S0;
                 const double one = 1.0, mhalf = -0.5, beta = first_blk ? 0.0 : 1.0;
-                CUTC_TRY(fp64_gemm(st, false, (int)np, (int)np, K, one,
-                                   d_Xt + 3 * (int64_t)K * np, np, 0, d_S0, K, 0, beta, d_H, np,
-                                   0, 1));
+                CUTC_TRY(fp64_contract(W, st, flags, false, (int)np, (int)np, K, one,
+                                       d_Xt + 3 * (int64_t)K * np, np, 0, d_S0, K, 0, beta, d_H,
+                                       np, 0, 1));
                 if (nl > 0)
-                    CUTC_TRY(fp64_gemm(st, false, (int)np, (int)nl, 3 * (int64_t)K, mhalf, d_Xt,
-                                       np, 0, d_Sl, 3 * (int64_t)K, 0, beta, d_N, np, 0, 1));
+                    CUTC_TRY(fp64_contract(W, st, flags, false, (int)np, (int)nl, 3 * (int64_t)K,
+                                           mhalf, d_Xt, np, 0, d_Sl, 3 * (int64_t)K, 0, beta, d_N,
+                                           np, 0, 1));
             } else {
                 CUTC_TRY(split_int2e_tile(E, R, st, sp, w1, a1, ld_a1, K, d_Xt, d_H, d_N,
                                           first_blk));
@@ -1004,6 +1009,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     CUTC_CUDA_TRY(cudaGetLastError());
     if (R.precision == CUTC_SPLIT_BF16)
         CUTC_TRY(split_check(st, sp));
+    else
+        CUTC_TRY(fp64_contract_check(st, flags));
 
     if (stats) {
         double ms_pair = 0.0, ms_gemm = 0.0, ms_i = 0.0, ms_tiles = 0.0;

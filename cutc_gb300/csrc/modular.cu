@@ -40,8 +40,9 @@ struct ModCfg {
     static constexpr int kStage = kA + kB;
     static constexpr int kStages = 6;
     static constexpr int kSmem = kStages * kStage + 1024 + 256;
-    static constexpr uint32_t kTmemCols = 2 * BN;  // two accumulator buffers
+    static constexpr uint32_t kTmemCols = 2 * BN;  // two accumulator buffers (a power of two)
     static constexpr int kCols = BN / 4;           // columns per epilogue warp
+    static_assert(kCols % 16 == 0, "16 columns per tensor-memory load");
     static_assert(kSmem <= 227 * 1024, "shared memory");
     static_assert(kTmemCols <= 512, "tensor memory");
 };
@@ -378,11 +379,14 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
         const int sn = P.sb[c], n = P.n0 + c;
         const int64_t col = (int64_t)(n / P.out.ncol_group) * P.out.group_stride + P.out.col0 +
                             n % P.out.ncol_group;
-        double *dst = P.out.C + m + P.out.ldc * col;
 #pragma unroll
         for (int h = 0; h < 2; h++) {
             if (m + h >= P.M)
                 break;
+            const int64_t row = P.out.nrow_group ? (int64_t)((m + h) / P.out.nrow_group) * P.out.row_stride +
+                                                       (m + h) % P.out.nrow_group
+                                                 : m + h;
+            double *dst = P.out.C + row + P.out.ldc * col;
             float f[N];
 #pragma unroll
             for (int i = 0; i < N; i++)
@@ -399,10 +403,10 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
                     v *= P.out.alpha;
             }
             if (P.beta_mode == 1)
-                v += dst[h];
+                v += *dst;
             else if (P.beta_mode == 2)
-                v += P.out.beta * dst[h];
-            dst[h] = v;
+                v += P.out.beta * *dst;
+            *dst = v;
         }
     }
 }
@@ -526,8 +530,11 @@ int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const Resid
         P.inv[i] = 1.0f / (float)moduli::prime(i);
     }
     P.err = err;
-    // narrow tiles where wide ones would leave the 76 SM pairs short of work
+    // narrow tiles for few columns, and where wide ones would leave the 76 SM pairs short
+    // of work
     const int64_t wide = (int64_t)n_mod * ceil_div(P.M, kTileM) * ceil_div(P.N, 256);
+    if (P.N <= 64)
+        return launch_gemm<64>(st, A, B, P);
     if (P.N <= 128 || wide < 76)
         return launch_gemm<128>(st, A, B, P);
     return launch_gemm<256>(st, A, B, P);

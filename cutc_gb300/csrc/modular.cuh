@@ -81,19 +81,22 @@ struct ResiduePlanes {
     int64_t kp = 0, pitch = 0;
 };
 
-// Where a contraction goes: C[m + ldc col(n)] = alpha sum_k A[m, k] B[n, k] + beta C,
-// col(n) = (n / ncol_group) group_stride + col0 + n % ncol_group.
+// Where a contraction goes: C[row(m) + ldc col(n)] = alpha sum_k A[m, k] B[n, k] + beta C,
+// col(n) = (n / ncol_group) group_stride + col0 + n % ncol_group, and
+// row(m) = (m / nrow_group) row_stride + m % nrow_group (nrow_group 0: row(m) = m).
 struct ModularOut {
     double *C;
     int64_t ldc;
     int ncol_group;
     int64_t group_stride, col0;
     double alpha, beta;
+    int nrow_group = 0;
+    int64_t row_stride = 0;
 };
 
-// Elements between the rows of a K panel of kp columns (16-byte rows for TMA, whole
-// 128-byte lines for the writers).
-inline int64_t residue_pitch(int64_t kp) { return (kp + 63) / 64 * 64; }
+// Elements between the rows of a K panel of kp columns (whole 32-byte sectors; TMA takes
+// multiples of 16 bytes).
+inline int64_t residue_pitch(int64_t kp) { return (kp + 15) / 16 * 16; }
 
 // Bytes of the residues of a panel.
 inline size_t residue_bytes(int n_mod, int64_t rows, int64_t kp)

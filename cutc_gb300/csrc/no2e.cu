@@ -8,7 +8,7 @@
 // X is the MO-basis X in cutc_no's point-fastest order, X[(g + n1 m) + 3 n1 (i + n_mo j)],
 // which cutc_x_ao_to_mo writes; tmpC1 has its layout, tmpC2 and tmpD2 are
 // [g + n1 (i + n_mo j)].  The reference runs the two products as cuBLAS DGEMMs; here the
-// plain form uses the FP64 DMMA GEMM (two products, the second accumulating) and the split
+// plain form uses its FP64 contraction (two products, the second accumulating) and the split
 // form one split contraction over the concatenated K = 4 n1.  The symmetrisation and the
 // index swap run on the coalesced layout kernels.
 #include <cuda_runtime.h>
@@ -72,10 +72,13 @@ extern "C" int cutc_no_2e(const cutc_options *opt, int n_mo, int n_grid1, const 
     }
     if (opt->precision == CUTC_PLAIN_FP64) {
         // no_2e = 1/2 tmpC1^T X, then += 1/2 tmpC2^T tmpD2 (src/cutc_no.c:419-446)
-        CUTC_TRY(fp64_gemm(st, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X, k1, 0, 0.0, out,
-                           nm2, 0, 1));
-        CUTC_TRY(fp64_gemm(st, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2, n1, 0, 1.0, out,
-                           nm2, 0, 1));
+        int *flags;
+        CUTC_TRY(fp64_contract_begin(E->ws, st, &flags));
+        CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X,
+                               k1, 0, 0.0, out, nm2, 0, 1));
+        CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2,
+                               n1, 0, 1.0, out, nm2, 0, 1));
+        CUTC_TRY(fp64_contract_check(st, flags));
     } else {
         CUTC_TRY(split_gemm_concat(E, st, opt->n_slices, (int)nm2, (int)nm2, k1, C1, X, n1, C2,
                                    D2, 0.5, out, nm2));
