@@ -29,6 +29,7 @@
 #include "dgemm.cuh"
 #include "engine.cuh"
 #include "pair.cuh"
+#include "pair_tc.cuh"
 #include "products.cuh"
 #include "split.cuh"
 
@@ -376,7 +377,8 @@ enum Slot {
     S_R1, S_WR1, S_R2, S_WR2, S_RN, S_AOS1, S_AOS2, S_COEF, S_EXPS, S_OFF,
     S_T1, S_F2, S_P, S_G, S_XP, S_S0, S_SL, S_H, S_N, S_XOUT, S_XOUT1, S_IOUT, S_IOUT1,
     S_R2D, S_F2D, S_POLY, S_BASIS,
-    S_SPLIT0  // split-form slots follow
+    S_SPLIT0,      // split-form slots follow
+    S_PAIRTC = 80  // the tensor-core pair terms' slots
 };
 
 static inline double ev_ms(cudaEvent_t a, cudaEvent_t b)
@@ -401,6 +403,13 @@ static int int2e_slab_cols(int nA)
     return (int)std::min<int64_t>(n, std::max<int64_t>(nA, per));
 }
 
+// Slices of the tensor-core pair terms' operands (at most: the memory plan does not know
+// the exponents).
+static int pair_slices(const Request &R)
+{
+    return R.precision == CUTC_PLAIN_FP64 || R.pair_fp64 ? 7 : 6;
+}
+
 // Device bytes of a build that do not grow with the r1 tile (besides the
 // molecule arrays): r2 terms, the P operand, H and N, int_2e output slabs.
 static size_t fixed_bytes(const Request &R)
@@ -415,8 +424,8 @@ static size_t fixed_bytes(const Request &R)
              (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2),
                               R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1));
     else
-        b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2) +
-             (double)split_pair_fixed_bytes(R);
+        b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2);
+    b += (double)pair_tc_fixed_bytes(R.n2, R.nN, pair_slices(R));
     if (!(R.device_pointers || R.out_device) && !R.x_only)
         b += 2.0 * int2e_slab_cols(R.nA) * nA * nA * 8;
     return (size_t)b;
@@ -430,8 +439,8 @@ static size_t r1_row_bytes(const Request &R)
     if (!(R.device_pointers || R.out_device) && !R.i_only)
         b += 2 * (size_t)R.x_components * R.nA * R.nA * 8;
     if (R.precision == CUTC_SPLIT_BF16)
-        b += split_r1_row_bytes(R) + pair_df_poly_bytes(6, 1, R.nN) + split_pair_row_bytes(R);
-    return b;
+        b += split_r1_row_bytes(R) + pair_df_poly_bytes(6, 1, R.nN);
+    return b + pair_tc_row_bytes(R.nN, pair_slices(R));
 }
 
 // Device bytes per r1 row of an int_2e block: the packed X rows and the block's
@@ -638,10 +647,11 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     const uint64_t key = plan_key(R);
     // which pair-term buffers the build holds besides: the remembered plan is taken
     // only when they are the same
-    uint64_t path = 1 + (R.pair_fp64 ? 2 : 0);
-    if (R.precision == CUTC_SPLIT_BF16 && !R.pair_fp64)
-        path += 4 * (uint64_t)split_pair_tc_ok(R, exps.data(), nt) +
-                8 * (uint64_t)pair_df_max_exp(exps.data(), nt);
+    const bool pair64 = R.precision == CUTC_PLAIN_FP64 || R.pair_fp64;
+    const PairTcMode pmode = pair_tc_mode(nN, coef.data(), exps.data(), nt, pair64, R.n_slices);
+    uint64_t path = 1 + (R.pair_fp64 ? 2 : 0) + 64 * (uint64_t)pmode.rows;
+    if (!pair64)
+        path += 8 * (uint64_t)pair_df_max_exp(exps.data(), nt);
     const bool default_budget = budget == 0;
     if (default_budget && E->ws.recall(key, &memo) && memo.path == path) {
         budget = memo.budget;  // the last build of this shape: its buffers fit this plan
@@ -738,9 +748,11 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         }
     } else {
         CUTC_TRY(split_prepare_x(E, R, st, d_wr2, d_aos2v, n1t, S_SPLIT0, sp));
-        if (split_pair_tc_ok(R, exps.data(), nt))
-            CUTC_TRY(split_pair_prepare(E, R, st, d_f2, n1t, sp));
     }
+    PairTcPlan ptc;
+    if (pmode.rows)
+        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, pmode, n2, nN, d_f2, n1t,
+                                 R.precision == CUTC_PLAIN_FP64 ? flags : sp.err, ptc));
     CUTC_CUDA_TRY(cudaEventRecord(E->ev[2], st));
 
     // ---- tiles ---------------------------------------------------------------
@@ -809,18 +821,22 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         const int nb = (int)std::min<int64_t>(n1t, n1 - i0);
         const int ib = (int)(i0 - blk0);  // the tile's first row within the block
         cudaEvent_t *tev = stats ? &E->tile_ev[kTileEv * tile] : nullptr;
-        CUTC_TRY(launch_r1_terms(st, i0, nb, nN, d_r1, d_rn, R.a_en, d_t1));
         if (tev)
             CUTC_CUDA_TRY(cudaEventRecord(tev[0], st));
-        if (R.precision == CUTC_PLAIN_FP64 || R.pair_fp64) {
+        if (pair64) {
             PairArgs P;
             P.i0 = i0; P.n1b = nb; P.n2 = n2; P.nN = nN; P.n_terms = nt;
             P.r1 = d_r1; P.r2 = d_r2; P.t1 = d_t1; P.f2 = d_f2;
             P.coef = d_coef; P.exps = d_exps; P.term_off = d_off;
             P.a_ee = R.a_ee;
             P.G = d_G; P.ldg = n2; P.plane = (int64_t)nb * n2;
-            CUTC_TRY(launch_pair_f64(st, P));
-            note_launches(2);
+            if (pmode.rows) {
+                CUTC_TRY(pair_tc_tile_f64(st, ptc, P, d_rn, R.a_en, E->n_sm));
+            } else {
+                CUTC_TRY(launch_r1_terms(st, i0, nb, nN, d_r1, d_rn, R.a_en, d_t1));
+                CUTC_TRY(launch_pair_f64(st, P));
+                note_launches(2);
+            }
             if (R.precision == CUTC_SPLIT_BF16) {
                 // the split form's operands read (hi, lo) pairs: convert in place
                 CUTC_TRY(launch_f64_to_df(st, d_G, 4 * (int64_t)nb * n2));
@@ -836,11 +852,11 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             P.a_ee_hi = (float)R.a_ee;
             P.a_ee_lo = (float)(R.a_ee - (double)P.a_ee_hi);
             P.G = reinterpret_cast<float2 *>(d_G); P.ldg = n2; P.plane = (int64_t)nb * n2;
-            if (sp.pair_tc) {
-                CUTC_TRY(split_pair_tile(E, R, st, sp, P, d_rn, R.a_en));
+            if (pmode.rows) {
+                CUTC_TRY(pair_tc_tile_df(st, ptc, P, d_rn, R.a_en, E->n_sm));
             } else {
                 CUTC_TRY(launch_pair_df(st, P, pexp, psparse, d_rn, R.a_en));
-                note_launches(3);
+                note_launches(2);
             }
         }
         if (tev)
@@ -1096,15 +1112,25 @@ int run_pair_only(Engine *E, cudaStream_t st, int i0, int n1b, int n1, int j0, i
     CUTC_TRY(W.get(S_F2, (size_t)nN * n2b * 8, &p));
     double *d_f2 = (double *)p;
     const double *r2w = r2 + 3 * (int64_t)j0;  // the r2 window
-    CUTC_TRY(launch_r1_terms(st, i0, n1b, nN, r1, rn, a_en, d_t1));
     CUTC_TRY(launch_r2_terms(st, n2b, nN, r2w, rn, a_en, d_f2));
+    note_launches(1);
     PairArgs P;
     P.i0 = i0; P.n1b = n1b; P.n2 = n2b; P.nN = nN; P.n_terms = (int)exps.size();
     P.r1 = r1; P.r2 = r2w; P.t1 = d_t1; P.f2 = d_f2;
     P.coef = d_coef; P.exps = d_exps; P.term_off = d_off; P.a_ee = a_ee;
     P.G = G; P.ldg = ldg; P.plane = plane;
+    const PairTcMode mode = pair_tc_mode(nN, coef.data(), exps.data(), (int)exps.size(), true, 0);
+    if (mode.rows) {
+        int *flags;
+        CUTC_TRY(fp64_contract_begin(W, st, &flags));
+        PairTcPlan plan;
+        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, mode, n2b, nN, d_f2, n1b, flags, plan));
+        CUTC_TRY(pair_tc_tile_f64(st, plan, P, rn, a_en, E->n_sm));
+        return fp64_contract_check(st, flags);
+    }
+    CUTC_TRY(launch_r1_terms(st, i0, n1b, nN, r1, rn, a_en, d_t1));
     CUTC_TRY(launch_pair_f64(st, P));
-    note_launches(3);
+    note_launches(2);
     CUTC_CUDA_TRY(cudaStreamSynchronize(st));
     return CUTC_OK;
 }

@@ -67,14 +67,14 @@ int launch_r2_df(cudaStream_t st, int n2, int nN, const double *r2, const double
 int launch_pair_df(cudaStream_t st, const PairDfArgs &P, int E, bool sparse, const double *rn,
                    double a_en);
 
-// Operands of the tensor-core pair terms (exponents in {0, 2, 3, 4}), FP64: the powers
-// F[j * 4 nN + 4 A + q] = f2_A(r2_j)^b_q (b = 0, 2, 3, 4) and, for r1 rows [i0, i0 + n),
-// the 16 coefficient rows C[((i 16 + c) 4 nN) + 4 A + q] of each point, with the points
-// themselves in double-float, r1d[3 i + c].
-int launch_pair_tc_f(cudaStream_t st, int n2, int nN, const double *f2, double *F);
-int launch_pair_tc_coef(cudaStream_t st, int i0, int n, int nN, const double *r1, const double *rn,
-                        double a_en, const double *coef, const int *exps, const int *term_off,
-                        double *C, float2 *r1d);
+// Operands of the tensor-core pair terms, FP64: the powers of f2 on r2 (4 powers per
+// nucleus for exponents in {0, 2, 3, 4}, 7 for any) and, for r1 rows [i0, i0 + n), the 16
+// or 32 coefficient rows of each point, with the points themselves in double-float,
+// r1d[3 i + c] (pair_df.cu has the layouts).
+int launch_pair_tc_f(cudaStream_t st, int powers, int n2, int nN, const double *f2, double *F);
+int launch_pair_tc_coef(cudaStream_t st, int rows, int i0, int n, int nN, const double *r1,
+                        const double *rn, double a_en, const double *coef, const int *exps,
+                        const int *term_off, double *C, float2 *r1d);
 
 int launch_r1_terms(cudaStream_t st, int i0, int n, int nN, const double *r1, const double *rn,
                     double a, NucTerm *t1);

@@ -264,22 +264,30 @@ pair_df_kernel(PairDfArgs P)
 }
 
 // ---------------------------------------------------------------------------
-// FP64 operands of the tensor-core pair terms (exponents in {0, 2, 3, 4})
+// FP64 operands of the tensor-core pair terms
 //
-// For fixed (r1, r2) the nucleus sum of the sparse-power form is linear in the
-// powers f2_A(r2)^b, b in {0, 2, 3, 4}: with k = 4 A + q (b = kPowB[q])
+// For fixed (r1, r2) the nucleus sum is linear in the powers f2_A(r2)^b.  With exponents
+// in {0, 2, 3, 4} (NP = 4 powers per nucleus, k = NP A + q, b = power(q)):
 //   V_c(r1, r2) = sum_k C[(r1, c)][k] F[r2][k],   F[r2][k] = f2_A(r2)^b,
-//   C[(r1, c)][k] = U_A[b][o](r1) (d f1_A / dx)(r1)   c = 0..3,  o = kPowB[c]
+//   C[(r1, c)][k] = U_A[b][o](r1) (d f1_A / dx)(r1)   c = 0..3,  o = power(c)
 //                   ... d/dy for c = 4..7, d/dz for c = 8..11
 //                   W_A[b][o'](r1), o' = c - 11           c = 12..14
 //                   0                                     c = 15
 // and then, per pair (g = g12 and its gradient, as in pair_df_kernel),
 //   grad1 u = sum_o g^o V_{.,o} + g (V_12 + g (V_13 + g V_14)) grad g.
-// The contraction over k runs on the tensor cores (split.cu, pair_tc_kernel).
+// With any exponents up to 6 (NP = 7): c = 7 x + o for x = 0..2 and o = 0..6,
+// c = 21 + o' for W, zero rows up to 32, and
+//   grad1 u = sum_o g^o V_{.,o} + (sum_o' g^o' V_{21 + o'}) grad g.
+// The contraction over k runs on the tensor cores (pair_tc.cu).
 // ---------------------------------------------------------------------------
-__constant__ int kPowB[4] = {0, 2, 3, 4};
+template <int NP>
+__device__ __forceinline__ int power(int q)
+{
+    return NP == 4 && q > 0 ? q + 1 : q;
+}
 
-// F[j * 4 nN + 4 A + q] = f2[A n2 + j]^b_q, FP64
+// F[j * NP nN + NP A + q] = f2[A n2 + j]^power(q), FP64
+template <int NP>
 __global__ void pair_tc_f_kernel(int n2, int nN, const double *__restrict__ f2,
                                  double *__restrict__ F)
 {
@@ -289,23 +297,37 @@ __global__ void pair_tc_f_kernel(int n2, int nN, const double *__restrict__ f2,
     const int j = (int)(idx / nN), A = (int)(idx % nN);
     const double f = f2[(int64_t)A * n2 + j];
     const double f2v = f * f;
-    double *o = F + (int64_t)j * 4 * nN + 4 * A;
+    double *o = F + (int64_t)j * NP * nN + NP * A;
     o[0] = 1.0;
-    o[1] = f2v;
-    o[2] = f2v * f;
-    o[3] = f2v * f2v;
+    if (NP == 4) {
+        o[1] = f2v;
+        o[2] = f2v * f;
+        o[3] = f2v * f2v;
+    } else {
+        const double f3 = f2v * f;
+        o[1] = f;
+        o[2] = f2v;
+        o[3] = f3;
+        o[4] = f2v * f2v;
+        o[5] = f2v * f3;
+        o[6] = f3 * f3;
+    }
+    if (!(f - f == 0.0))  // an infinity or a NaN makes the whole row one
+        o[0] = f;
 }
 
-// C[((i 16 + c) 4 nN) + 4 A + q] for rows i of the tile, FP64; the polynomial
-// coefficients U, W are formed as in r1_poly_kernel<4>.  Also the tile's r1 points in
-// double-float, r1d[3 i + c].
+// The coefficient rows C[((i R + c) NP nN) + NP A + q] for rows i of the tile, FP64; the
+// polynomial coefficients U, W are formed as in r1_poly_kernel.  Also the tile's r1 points
+// in double-float, r1d[3 i + c].
+template <int NP>
 __global__ void pair_tc_coef_kernel(int i0, int n, int nN, const double *__restrict__ r1,
                                     const double *__restrict__ rn, double a_en,
                                     const double *__restrict__ tcoef,
                                     const int *__restrict__ texps, const int *__restrict__ toff,
                                     double *__restrict__ C, float2 *__restrict__ r1d)
 {
-    constexpr int E = 4;
+    constexpr int E = NP == 4 ? 4 : 6;
+    constexpr int R = NP == 4 ? 16 : 32;
     const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= (int64_t)n * nN)
         return;
@@ -350,44 +372,55 @@ __global__ void pair_tc_coef_kernel(int i0, int n, int nN, const double *__restr
             W[m * E + o - 1] += co * F[nn];
         }
     }
-    const int64_t K = 4 * (int64_t)nN;
-    double *row = C + (int64_t)i * 16 * K + 4 * A;
+    const int64_t K = (int64_t)NP * nN;
+    double *row = C + (int64_t)i * R * K + NP * A;
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int b = kPowB[q];
+    for (int q = 0; q < NP; q++) {
+        const int b = power<NP>(q);
 #pragma unroll
-        for (int oi = 0; oi < 4; oi++) {
-            const double u = U[b * (E + 1) + kPowB[oi]];
+        for (int oi = 0; oi < NP; oi++) {
+            const double u = U[b * (E + 1) + power<NP>(oi)];
             row[oi * K + q] = u * gx;
-            row[(4 + oi) * K + q] = u * gy;
-            row[(8 + oi) * K + q] = u * gz;
+            row[(NP + oi) * K + q] = u * gy;
+            row[(2 * NP + oi) * K + q] = u * gz;
         }
+        // W: o' = 1..3 (the factor g taken out) or o' = 0..5
+        constexpr int nw = NP == 4 ? 3 : 6, w0 = NP == 4 ? 1 : 0;
 #pragma unroll
-        for (int op = 0; op < 3; op++)
-            row[(12 + op) * K + q] = W[b * E + op + 1];
-        row[15 * K + q] = 0.0;
+        for (int op = 0; op < nw; op++)
+            row[(3 * NP + op) * K + q] = W[b * E + op + w0];
+        for (int c = 3 * NP + nw; c < R; c++)
+            row[c * K + q] = 0.0;
     }
 }
 
-int launch_pair_tc_f(cudaStream_t st, int n2, int nN, const double *f2, double *F)
+int launch_pair_tc_f(cudaStream_t st, int powers, int n2, int nN, const double *f2, double *F)
 {
     const int64_t total = (int64_t)n2 * nN;
     if (total == 0)
         return CUTC_OK;
-    pair_tc_f_kernel<<<ceil_div(total, 256), 256, 0, st>>>(n2, nN, f2, F);
+    if (powers == 4)
+        pair_tc_f_kernel<4><<<ceil_div(total, 256), 256, 0, st>>>(n2, nN, f2, F);
+    else
+        pair_tc_f_kernel<7><<<ceil_div(total, 256), 256, 0, st>>>(n2, nN, f2, F);
     CUTC_CUDA_TRY(cudaGetLastError());
     return CUTC_OK;
 }
 
-int launch_pair_tc_coef(cudaStream_t st, int i0, int n, int nN, const double *r1, const double *rn,
-                        double a_en, const double *coef, const int *exps, const int *term_off,
-                        double *C, float2 *r1d)
+int launch_pair_tc_coef(cudaStream_t st, int rows, int i0, int n, int nN, const double *r1,
+                        const double *rn, double a_en, const double *coef, const int *exps,
+                        const int *term_off, double *C, float2 *r1d)
 {
     const int64_t total = (int64_t)n * nN;
     if (total == 0)
         return CUTC_OK;
-    pair_tc_coef_kernel<<<ceil_div(total, 128), 128, 0, st>>>(i0, n, nN, r1, rn, a_en, coef,
-                                                              exps, term_off, C, r1d);
+    const unsigned grid = ceil_div(total, 128);
+    if (rows == 16)
+        pair_tc_coef_kernel<4><<<grid, 128, 0, st>>>(i0, n, nN, r1, rn, a_en, coef, exps, term_off,
+                                                     C, r1d);
+    else
+        pair_tc_coef_kernel<7><<<grid, 128, 0, st>>>(i0, n, nN, r1, rn, a_en, coef, exps, term_off,
+                                                     C, r1d);
     CUTC_CUDA_TRY(cudaGetLastError());
     return CUTC_OK;
 }

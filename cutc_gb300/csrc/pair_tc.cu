@@ -1,0 +1,917 @@
+// Pair terms grad1 u(r1, r2) on the tensor cores (tcgen05 + TMA).
+//
+// For fixed g12 the nucleus sum of grad1 u(r1, r2) is the contraction
+//   V_c(r1, r2) = sum_k C[(r1, c)][k] F[r2][k],  k over (nucleus, power of f2)
+// (pair_df.cu builds F and the coefficient rows C per r1 point in FP64), and the pair's
+// value a polynomial in g12 of the V_c: 16 rows and four powers per nucleus where every
+// Jastrow exponent is 0, 2, 3 or 4, 32 rows and seven powers for any exponents up to 6.
+// The contraction runs on operands split into S slices,
+//     A[r, k] = 2^{e_r} sum_{s < S} a_s[r, k],  a_s = q_s 2^{-8-9s},  q_s in [-256, 256]
+// (S signed 9-bit digits of the row-scaled value), whose products a_s b_t, s + t < S, run
+// as BF16 tcgen05.mma with one FP32 accumulator per diagonal d = s + t: the S slices of b
+// are stacked in shared memory, so one instruction per slice of a takes all of them (the
+// error-free splitting of Ozaki, Ogita, Oishi and Rump 2012).  A product of diagonal d is
+// a multiple of 2^{-16-9d}, at most 2^{-9d}, so the FP32 sums are exact while
+// (d + 1) K 2^16 <= 2^24: K <= 85 for d <= 2 (double-float results), K <= 64 for d <= 3
+// (FP64 results); later diagonals round at 2^-27 2^-24 and 2^-36 2^-24 of the row scales.
+//
+// A = the F slices of 128 r2 points, all of K, loaded once per CTA; B = the coefficient
+// slices in tiles of 64 rows (four r1 points, or two), streamed; one stacked accumulator
+// set in tensor memory.  The tensor-core work of a tile is a small part of its epilogue, so
+// one accumulator set and one B stage suffice: the next tile's MMAs run as soon as the
+// epilogue has read the accumulators, and one control warp issues both the TMA loads and
+// the MMAs.
+//
+// Double-float epilogue (lane = r2 point, one r1 point per warp): the S diagonals of the
+// point's columns are added exactly on fixed grids into double-float values, then g12 and
+// its gradient, the polynomial, -1/2 |grad u|^2 and the (hi, lo) G planes follow in
+// double-float, with FP64 coordinate differences near e-e coalescence.  About 800 FP32
+// operations per pair with 16 rows instead of 30 df multiply-adds (~450 operations) per
+// nucleus.
+//
+// FP64 epilogue: the diagonals down to 2^-43 of the row scales become one exact integer
+// (integer arithmetic; one FP64 add makes it a double), the rest stays in FP32 beside it,
+// and g12, its gradient and the polynomial take FP64: 66 FP64 operations per pair with 16
+// rows, whatever the number of nuclei, on a pipe of 2 per clock and SM, against about 11
+// per term in the term-by-term kernel (pair.cu).  512 x 20 011 pairs, 8 nuclei with 13
+// terms each: 19.3 -> 1.77 ms.  General exponents in double-float, 2003 x 30 011 pairs, 6
+// nuclei, against pair_df_kernel<6>: 16.6 -> 4.5 ms.
+#include <cuda.h>
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <atomic>
+#include <cmath>
+#include <cstdlib>
+
+#include "common.cuh"
+#include "dfloat.cuh"
+#include "digits.cuh"
+#include "modular.cuh"
+#include "pair_tc.cuh"
+#include "tc.cuh"
+
+namespace cutc {
+
+constexpr int kBM = 128;        // r2 points per CTA (TMEM lanes)
+constexpr int kBK = 32;         // K per TMA box: 32 BF16 = 64-byte rows (64B swizzle)
+constexpr uint32_t kTmemCols = 512;
+constexpr int kPairBN = 64;     // coefficient rows per N tile
+constexpr int kNanExponent = 1025;  // row exponent of a row with an infinity or a NaN
+
+struct PairTcParams {
+    int tiles_m, tiles_n, chunk;  // r2 tiles of 128 points, N tiles, N tiles per CTA
+    int Mpad, Npad;               // padded rows of the F and coefficient slices
+    const int *ea, *eb;           // row exponents of the F and the coefficient slices
+    const float *bscale;          // double-float: 2^(row exponent) of each coefficient row
+    const float2 *r1d;            // double-float: the tile's r1 points, [3 i + c]
+    PairDfArgs P;                 // geometry and outputs
+    double *G64;                  // FP64: in place of P.G
+    int *err;
+};
+
+// x 2^e for the scale of a value of row exponents e (clamped to the float range); NaN for
+// a row that is not finite
+__device__ __forceinline__ float pow2f(int e)
+{
+    if (e >= kNanExponent)
+        return __int_as_float(0x7fffffff);
+    e = e < -126 ? -126 : (e > 127 ? 127 : e);
+    return __int_as_float((e + 127) << 23);
+}
+
+// bscale[r] = 2^ex[r] as a float
+__global__ void exp_scale_kernel(const int *__restrict__ ex, int rows, float *__restrict__ bscale)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < rows)
+        bscale[r] = pow2f(ex[r]);
+}
+
+// R: coefficient rows per r1 point (16 or 32).
+template <int S, int KB, int R, bool F64>
+struct PairTcCfg {
+    static constexpr int kBN = kPairBN;
+    static constexpr int kPts = kBN / R;
+    // double-float with 16 rows: a warp per lane quarter and point, four warps per SM
+    // sub-partition, to hide the latency of their dependent chains; otherwise two points
+    // (or one, with 32 rows) per warp of eight, which leaves the registers
+    static constexpr int kEpiWarps = (F64 || R == 32) ? 8 : 16;
+    static constexpr int kWarpPts = 4 * kPts / kEpiWarps;
+    static constexpr int kCtlWarp = kEpiWarps;       // TMA loads and MMAs, lane 0
+    static constexpr int kThreads = (kEpiWarps + 1) * 32;
+    static constexpr int kASlice = kBM * kBK * 2;
+    static constexpr int kBSlice = kBN * kBK * 2;
+    static constexpr int kABytes = KB * S * kASlice;
+    static constexpr int kBStage = KB * S * kBSlice;
+    static constexpr int kSmem = kABytes + kBStage + 1024 + 256;
+    static constexpr int kMaxN = 256;                // widest kind::f16 instruction at M = 128
+    static_assert(kSmem <= 227 * 1024, "shared memory");
+    static_assert(kBN * S <= (int)kTmemCols, "accumulators exceed tensor memory");
+    static_assert(kMaxN % kBN == 0, "instruction splits on diagonal boundaries");
+    static_assert(kBSlice % 512 == 0, "B slices must stack on 8-row swizzle atoms");
+};
+
+// The V values of R columns of the warp's lanes, in double-float: the diagonals summed
+// exactly on grids.  In units of the row scales every diagonal sum D_d is a multiple of
+// 2^(-16-9d) and |D_0| <= K:
+//   H  = D_0 + D_1 rounded to multiples of 2^-16      (exact: below 2^7 there)
+//   L  = the rest of D_1 + D_2 rounded to 2^-25         (exact: below 2^-8 there)
+//   L2 = the rest of D_2 + D_3 + ... (FP32; below 2^-18, so off by < 2^-42)
+// Two columns share each packed f32x2 operation.
+template <int S>
+__device__ __forceinline__ void read_df16(uint32_t cb, uint64_t (&H)[8], uint64_t (&L)[8],
+                                          uint64_t (&L2)[8])
+{
+    const uint64_t C16 = tc::f2_dup(192.0f), C25 = tc::f2_dup(0.375f);
+    float v[16];
+    tc::tmem_ld16(cb, v);
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        H[k] = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
+        L[k] = L2[k] = 0ull;
+    }
+#pragma unroll
+    for (int d = 1; d < S; d++) {
+        tc::tmem_ld16(cb + (uint32_t)(kPairBN * d), v);
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const uint64_t x = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
+            if (d == 1) {
+                const uint64_t hh = tc::f2_sub(tc::f2_add(x, C16), C16);
+                H[k] = tc::f2_add(H[k], hh);
+                L[k] = tc::f2_sub(x, hh);
+            } else if (d == 2) {
+                const uint64_t hh = tc::f2_sub(tc::f2_add(x, C25), C25);
+                L[k] = tc::f2_add(L[k], hh);
+                L2[k] = tc::f2_sub(x, hh);
+            } else {
+                L2[k] = tc::f2_add(L2[k], x);
+            }
+        }
+    }
+}
+
+// V_c 2^-ea = 2^eb_c ((H + L) + L2): TwoSum of H and L, then the rest.  The F rows' scale
+// 2^ea, a power of two common to a pair's values, multiplies the results instead (the
+// polynomial is linear in V, and power-of-two scaling commutes with double-float
+// arithmetic).
+__device__ __forceinline__ void scale_df16(const uint64_t (&H)[8], const uint64_t (&L)[8],
+                                           const uint64_t (&L2)[8], const float *scr, df::D *V)
+{
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        const uint64_t sm = tc::f2_add(H[k], L[k]);
+        const uint64_t bb = tc::f2_sub(sm, H[k]);
+        uint64_t e = tc::f2_add(tc::f2_sub(H[k], tc::f2_sub(sm, bb)), tc::f2_sub(L[k], bb));
+        e = tc::f2_add(e, L2[k]);
+        const uint64_t sc = *reinterpret_cast<const uint64_t *>(scr + 2 * k);
+        const uint64_t hs = tc::f2_mul(sm, sc), ls = tc::f2_mul(e, sc);
+        V[2 * k] = df::make(tc::f2_lo(hs), tc::f2_lo(ls));
+        V[2 * k + 1] = df::make(tc::f2_hi(hs), tc::f2_hi(ls));
+    }
+}
+
+// One pair in double-float from its V values.
+template <int R>
+__device__ __forceinline__ void pair_df(const PairTcParams &Q, int i, int j, const df::D *V,
+                                        float2 x2, float2 y2, float2 z2, float sa, df::D a)
+{
+    const PairDfArgs &P = Q.P;
+    const float2 *r1p = Q.r1d + 3 * (int64_t)i;
+    const float2 r1x = r1p[0], r1y = r1p[1], r1z = r1p[2];
+    df::D dx = df::sub(df::make(r1x.x, r1x.y), df::make(x2.x, x2.y));
+    df::D dy = df::sub(df::make(r1y.x, r1y.y), df::make(y2.x, y2.y));
+    df::D dz = df::sub(df::make(r1z.x, r1z.y), df::make(z2.x, z2.y));
+    df::D d2 = df::add(df::add(df::sqr(dx), df::sqr(dy)), df::sqr(dz));
+    bool coalesced = false;
+    if (d2.hi < kNearPairR2) {
+        // near e-e coalescence the differences are taken in FP64, where they are
+        // exact (the coordinates' double-float forms keep only 48 bits); only g12
+        // and its gradient depend on them, so the rest stays as it is.  The
+        // reference's own guard, r12^2 <= 1e-15 (src/jast_bh.cu:143), gives g = 0.
+        const double *a1 = P.r1 + 3 * (int64_t)(P.i0 + i);
+        const double *a2 = P.r2 + 3 * (int64_t)j;
+        const double ex = a1[0] - a2[0], ey = a1[1] - a2[1], ez = a1[2] - a2[2];
+        dx = df::from_double(ex);
+        dy = df::from_double(ey);
+        dz = df::from_double(ez);
+        d2 = df::add(df::add(df::sqr(dx), df::sqr(dy)), df::sqr(dz));
+        coalesced = !(ex * ex + ey * ey + ez * ez > 1e-15);
+    }
+    df::D g = {0.f, 0.f}, gx = {0.f, 0.f}, gy = {0.f, 0.f}, gz = {0.f, 0.f};
+    if (!coalesced) {
+        const df::D rd = df::sqrt(d2);
+        const df::D ar = df::mul(rd, a);
+        const df::D t = df::recip(df::add_f(ar, 1.0f));
+        g = df::mul(ar, t);
+        const df::D sg = df::mul(df::mul(df::sqr(t), a), df::recip(rd));
+        gx = df::mul(sg, dx);
+        gy = df::mul(sg, dy);
+        gz = df::mul(sg, dz);
+    }
+    df::D ux, uy, uz, dudg;
+    if constexpr (R == 16) {
+        const df::D g2 = df::sqr(g);
+        // sum_o g^o V_o, o = 0, 2, 3, 4
+        ux = df::fma(df::fma(df::fma(V[3], g, V[2]), g, V[1]), g2, V[0]);
+        uy = df::fma(df::fma(df::fma(V[7], g, V[6]), g, V[5]), g2, V[4]);
+        uz = df::fma(df::fma(df::fma(V[11], g, V[10]), g, V[9]), g2, V[8]);
+        dudg = df::mul(df::fma(df::fma(V[14], g, V[13]), g, V[12]), g);
+    } else {
+        auto horner = [&](const df::D *v, int n) {
+            df::D s = v[n - 1];
+#pragma unroll
+            for (int o = n - 2; o >= 0; o--)
+                s = df::fma(s, g, v[o]);
+            return s;
+        };
+        ux = horner(V, 7);
+        uy = horner(V + 7, 7);
+        uz = horner(V + 14, 7);
+        dudg = horner(V + 21, 6);
+    }
+    ux = df::fma(dudg, gx, ux);
+    uy = df::fma(dudg, gy, uy);
+    uz = df::fma(dudg, gz, uz);
+    ux = df::make(__fmul_rn(ux.hi, sa), __fmul_rn(ux.lo, sa));
+    uy = df::make(__fmul_rn(uy.hi, sa), __fmul_rn(uy.lo, sa));
+    uz = df::make(__fmul_rn(uz.hi, sa), __fmul_rn(uz.lo, sa));
+    const df::D n2v = df::add(df::add(df::sqr(ux), df::sqr(uy)), df::sqr(uz));
+    const df::D lv = df::mul_f(n2v, -0.5f);
+    float2 *o = P.G + (int64_t)i * P.ldg + j;
+    o[0] = make_float2(ux.hi, ux.lo);
+    o[P.plane] = make_float2(uy.hi, uy.lo);
+    o[2 * P.plane] = make_float2(uz.hi, uz.lo);
+    o[3 * P.plane] = make_float2(lv.hi, lv.lo);
+}
+
+// The V values of eight columns in two parts each: hi, the diagonals down to 2^-43 of the
+// row scale as a double, and lo, the rest (below 2^-35, to 2^-60) as a float.  e: the
+// exponents of the columns' scales with the F row's added.
+//   H + L + L2 + L3 on the grids 2^-16, 2^-25, 2^-34, 2^-43 (each exact, as read_df16)
+// is an integer multiple of 2^-43 below 2^50, formed with integer operations.
+template <int S>
+__device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, double *hi, float *lo)
+{
+    static_assert(S == 7, "FP64 results take 7 slices");
+    float v[8];
+    uint64_t H[4], L[4], L2[4], L3[4], L4[4];
+    tc::tmem_ld8(cb, v);
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        H[k] = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
+    // multiples of 2^g: C = 1.5 2^(23 + g)
+    auto cut = [&](int d, float C, uint64_t (&up)[4], uint64_t (&rest)[4]) {
+        const uint64_t Cg = tc::f2_dup(C);
+        tc::tmem_ld8(cb + (uint32_t)(kPairBN * d), v);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint64_t x = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
+            const uint64_t hh = tc::f2_sub(tc::f2_add(x, Cg), Cg);
+            up[k] = tc::f2_add(up[k], hh);
+            rest[k] = tc::f2_sub(x, hh);
+        }
+    };
+    cut(1, 192.0f, H, L);
+    cut(2, 0.375f, L, L2);
+    cut(3, 0.375f * 0x1p-9f, L2, L3);
+    cut(4, 0.375f * 0x1p-18f, L3, L4);
+#pragma unroll
+    for (int d = 5; d < S; d++) {
+        tc::tmem_ld8(cb + (uint32_t)(kPairBN * d), v);
+#pragma unroll
+        for (int k = 0; k < 4; k++)
+            L4[k] = tc::f2_add(L4[k], tc::f2_pack(__float_as_uint(v[2 * k]),
+                                                  __float_as_uint(v[2 * k + 1])));
+    }
+    auto grid_int = [](float x, float s) {  // x s, an integer below 2^22
+        return __float_as_int(__fmaf_rn(x, s, 12582912.0f)) - 0x4b400000;
+    };
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        auto part = [&](const uint64_t (&p)[4]) { return k & 1 ? tc::f2_hi(p[k / 2]) : tc::f2_lo(p[k / 2]); };
+        const int ih = __float2int_rn(part(H) * 65536.0f);
+        const int il = grid_int(part(L), 0x1p25f);
+        const int il2 = grid_int(part(L2), 0x1p34f), il3 = grid_int(part(L3), 0x1p43f);
+        const long long I = ((long long)ih << 27) + ((long long)il << 18) + (long long)(il2 * 512 + il3);
+        // I as a double (one FP64 add), then 2^(e - 43) on its exponent field
+        const double x = __longlong_as_double(0x4338000000000000ll + I) - 6755399441055744.0;
+        const int e = eb[k] + ea;
+        const int ef = ((__double2hiint(x) >> 20) & 0x7ff) + e - 43;
+        double y;
+        if (eb[k] >= kNanExponent || ea >= kNanExponent)
+            y = __longlong_as_double(0x7ff8000000000000ll);
+        else if (I == 0 || ef < 1)
+            y = 0.0;
+        else if (ef > 2046)
+            y = __hiloint2double((__double2hiint(x) & 0x80000000) | 0x7ff00000, 0);
+        else
+            y = __hiloint2double(__double2hiint(x) + ((e - 43) << 20), __double2loint(x));
+        hi[k] = y;
+        lo[k] = part(L4) * pow2f(min(e, 127));
+    }
+}
+
+// a double as a float, truncated, with integer operations (0 below the float range)
+__device__ __forceinline__ float trunc_float(double x)
+{
+    const int hi = __double2hiint(x);
+    const int v = (hi & 0x7fffffff) - 0x38000000;
+    const unsigned m = ((unsigned)max(v, 0) << 3) | ((unsigned)__double2loint(x) >> 29);
+    const unsigned f = v < 0x00100000 ? 0u : v >= 0x0ff00000 ? 0x7f7fffffu : m;
+    return __uint_as_float(f | ((unsigned)hi & 0x80000000u));
+}
+
+// a positive normal float as a double, with integer operations
+__device__ __forceinline__ double exact_double(float x)
+{
+    const unsigned b = __float_as_uint(x);
+    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+}
+
+// One pair in FP64 from its V values (hi + lo).  The reciprocal square root and the
+// reciprocal are FP32 seeds with one step each of third order in FP64 (the seeds' relative
+// errors of 2^-22 and 2^-23 become 2^-63 and below).
+template <int R>
+__device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, const double *V,
+                                         const float *W, double x2, double y2, double z2)
+{
+    const PairDfArgs &P = Q.P;
+    const double *r1p = P.r1 + 3 * (int64_t)(P.i0 + i);
+    const double a = P.a_ee;
+    const double dx = r1p[0] - x2, dy = r1p[1] - y2, dz = r1p[2] - z2;
+    const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    const int hw = __double2hiint(d2);
+    double g = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
+    if (d2 > 1e-15) {
+        double y, z, d, ad;
+        if (hw < (1023 + 120) << 20) {
+            const double y0 = exact_double(rsqrtf(trunc_float(d2)));
+            const double e = fma(-(d2 * y0), y0, 1.0);
+            y = fma(e * y0, fma(e, 0.375, 0.5), y0);
+            d = d2 * y;
+            ad = a * d;
+        } else {  // distances beyond 2^60, and infinities
+            d = sqrt(d2);
+            y = 1.0 / d;
+            ad = a * d;
+        }
+        const double den = 1.0 + ad;
+        if (__double2hiint(den) < (1023 + 120) << 20) {
+            const double z0 = exact_double(__frcp_rn(trunc_float(den)));
+            const double e = fma(-den, z0, 1.0);
+            z = fma(z0, fma(e, e, e), z0);
+        } else {
+            z = 1.0 / den;
+        }
+        g = ad * z;
+        const double s = (a * z) * (z * y);
+        gx = s * dx;
+        gy = s * dy;
+        gz = s * dz;
+    }
+    const float gf = trunc_float(g);
+    double ux, uy, uz, dudg;
+    float lx, ly, lz, lg;
+    if constexpr (R == 16) {
+        const double g2 = g * g;
+        const float gf2 = gf * gf;
+        auto poly = [&](int c) { return fma(fma(fma(V[c + 3], g, V[c + 2]), g, V[c + 1]), g2, V[c]); };
+        auto low = [&](int c) { return fmaf(fmaf(fmaf(W[c + 3], gf, W[c + 2]), gf, W[c + 1]), gf2, W[c]); };
+        ux = poly(0);
+        uy = poly(4);
+        uz = poly(8);
+        dudg = fma(fma(V[14], g, V[13]), g, V[12]) * g;
+        lx = low(0);
+        ly = low(4);
+        lz = low(8);
+        lg = fmaf(fmaf(W[14], gf, W[13]), gf, W[12]) * gf;
+    } else {
+        auto poly = [&](int c, int n) {
+            double s = V[c + n - 1];
+#pragma unroll
+            for (int o = n - 2; o >= 0; o--)
+                s = fma(s, g, V[c + o]);
+            return s;
+        };
+        auto low = [&](int c, int n) {
+            float s = W[c + n - 1];
+#pragma unroll
+            for (int o = n - 2; o >= 0; o--)
+                s = fmaf(s, gf, W[c + o]);
+            return s;
+        };
+        ux = poly(0, 7);
+        uy = poly(7, 7);
+        uz = poly(14, 7);
+        dudg = poly(21, 6);
+        lx = low(0, 7);
+        ly = low(7, 7);
+        lz = low(14, 7);
+        lg = low(21, 6);
+    }
+    ux = fma(dudg, gx, ux) + (double)fmaf(lg, trunc_float(gx), lx);
+    uy = fma(dudg, gy, uy) + (double)fmaf(lg, trunc_float(gy), ly);
+    uz = fma(dudg, gz, uz) + (double)fmaf(lg, trunc_float(gz), lz);
+    double *o = Q.G64 + (int64_t)i * P.ldg + j;
+    o[0] = ux;
+    o[P.plane] = uy;
+    o[2 * P.plane] = uz;
+    o[3 * P.plane] = -0.5 * fma(ux, ux, fma(uy, uy, uz * uz));
+}
+
+template <int S, int KB, int R, bool F64>
+__global__ void __launch_bounds__(PairTcCfg<S, KB, R, F64>::kThreads, 1)
+pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+               const __grid_constant__ PairTcParams Q)
+{
+    using Cfg = PairTcCfg<S, KB, R, F64>;
+    constexpr int D = S - 1, BN = Cfg::kBN;
+    constexpr int kEpiWarps = Cfg::kEpiWarps, kCtlWarp = Cfg::kCtlWarp;
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>(
+        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *sA = smem;
+    uint8_t *sB = smem + Cfg::kABytes;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + Cfg::kBStage);
+    uint64_t *afull = bars;      // the F tile has landed
+    uint64_t *full = bars + 1;   // the B stage holds tile q
+    uint64_t *empty = bars + 2;  // the MMAs of tile q are done with the B stage
+    uint64_t *tfull = bars + 3;  // the accumulators hold tile q
+    uint64_t *tempty = bars + 4; // every epilogue warp has read tile q's accumulators
+    uint64_t *drain = bars + 5;
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
+    volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
+
+    const PairDfArgs &P = Q.P;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = (int)(blockIdx.x % Q.tiles_m) * kBM;
+    const int t_begin = (int)(blockIdx.x / Q.tiles_m) * Q.chunk;
+    const int ntiles = min(Q.tiles_n, t_begin + Q.chunk) - t_begin;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 5; i++)
+            tc::mbar_init(tc::smem_u32(&bars[i]), i == 4 ? kEpiWarps : 1);
+        tc::mbar_init(tc::smem_u32(drain), 1);
+        *s_abort = 0;
+        tc::fence_mbar_init();
+    }
+    if (warp == kCtlWarp) {
+        tc::tmem_alloc(tc::smem_u32(s_tmem), kTmemCols);
+        tc::tmem_relinquish();
+        if (lane == 0) {
+            tc::tma_prefetch(&tmA);
+            tc::tma_prefetch(&tmB);
+        }
+    }
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tbase = *s_tmem;
+
+    auto fail = [&](int code) {
+        *s_abort = 1;
+        atomicExch(Q.err, code);
+    };
+
+    if (warp == kCtlWarp) {
+        if (lane == 0) {
+            auto load_b = [&](int q) {
+                const uint32_t fb = tc::smem_u32(full);
+                tc::mbar_arrive_expect_tx(fb, Cfg::kBStage);
+                const int n0 = (t_begin + q) * BN;
+#pragma unroll
+                for (int kb = 0; kb < KB; kb++)
+#pragma unroll
+                    for (int t = 0; t < S; t++)
+                        tc::tma_load_2d(tc::smem_u32(sB + (kb * S + t) * Cfg::kBSlice), &tmB,
+                                        kb * kBK, t * Q.Npad + n0, fb);
+            };
+            const uint32_t ab = tc::smem_u32(afull);
+            tc::mbar_arrive_expect_tx(ab, Cfg::kABytes);
+#pragma unroll
+            for (int kb = 0; kb < KB; kb++)
+#pragma unroll
+                for (int s = 0; s < S; s++)
+                    tc::tma_load_2d(tc::smem_u32(sA + (kb * S + s) * Cfg::kASlice), &tmA, kb * kBK,
+                                    s * Q.Mpad + m0, ab);
+            int loaded = 0;  // B tiles issued into the stage
+            if (ntiles > 0) {
+                load_b(0);
+                loaded = 1;
+            }
+            bool ok = tc::mbar_wait(ab, 0, s_abort);
+            if (!ok)
+                fail(12);
+            for (int q = 0; q < ntiles && ok; q++) {
+                // the accumulators are free once every epilogue warp has read tile q - 1
+                if (q >= 1 && !tc::mbar_wait(tc::smem_u32(tempty), (q - 1) & 1, s_abort)) {
+                    fail(13);
+                    break;
+                }
+                if (!tc::mbar_wait(tc::smem_u32(full), q & 1, s_abort)) {
+                    fail(14);
+                    break;
+                }
+                tc::fence_after_sync();
+                const uint32_t sb0 = tc::smem_u32(sB);
+                const uint32_t sa0 = tc::smem_u32(sA);
+                bool first = true;
+#pragma unroll
+                for (int kb = 0; kb < KB; kb++) {
+#pragma unroll
+                    for (int k16 = 0; k16 < kBK / 16; k16++) {
+#pragma unroll
+                        for (int s = 0; s < S; s++) {
+                            // a_s x [b_0 .. b_{D-s}] -> diagonals s .. D, in instructions of
+                            // at most kMaxN columns
+                            const uint64_t ad = tc::smem_desc_sw64(
+                                sa0 + (kb * S + s) * Cfg::kASlice + k16 * 32);
+#pragma unroll
+                            for (int t0 = 0; t0 <= D - s; t0 += Cfg::kMaxN / BN) {
+                                const int nt = min(Cfg::kMaxN / BN, D - s + 1 - t0);
+                                const uint64_t bd = tc::smem_desc_sw64(
+                                    sb0 + (kb * S + t0) * Cfg::kBSlice + k16 * 32);
+                                tc::mma_bf16(tbase + (uint32_t)(BN * (s + t0)), ad, bd,
+                                             tc::idesc_bf16_f32(kBM, BN * nt), first ? 0u : 1u);
+                            }
+                            first = false;
+                        }
+                    }
+                }
+                tc::mma_commit(tc::smem_u32(empty));
+                tc::mma_commit(tc::smem_u32(tfull));
+                // refill the B stage for tile q + 1 once these MMAs have read it
+                if (q + 1 < ntiles) {
+                    if (!tc::mbar_wait(tc::smem_u32(empty), q & 1, s_abort)) {
+                        fail(11);
+                        break;
+                    }
+                    load_b(q + 1);
+                    loaded = q + 2;
+                }
+            }
+            tc::mma_commit(tc::smem_u32(drain));
+            if (!tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
+                fail(15);
+            // let the copies still in flight land before the CTA goes away
+            tc::mbar_wait(ab, 0, nullptr);
+            if (*s_abort && loaded > 0)
+                tc::mbar_wait(tc::smem_u32(full), (loaded - 1) & 1, nullptr);
+        }
+    } else {
+        // ---- epilogue: the warp's r1 points of each N tile, 32 r2 points ----------------
+        constexpr int WP = Cfg::kWarpPts;
+        const int quarter = warp & 3, pt0 = (warp >> 2) * WP;
+        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+        const int j = m0 + quarter * 32 + lane;
+        const bool jok = j < P.n2;
+        const int jc = jok ? j : 0;
+        const int ea = Q.ea[jc];  // F rows: 1 where the row maximum is f^0 = 1
+        float2 x2 = {0.f, 0.f}, y2 = {0.f, 0.f}, z2 = {0.f, 0.f};
+        double dx2 = 0.0, dy2 = 0.0, dz2 = 0.0;
+        if constexpr (F64) {
+            dx2 = P.r2[3 * (int64_t)jc];
+            dy2 = P.r2[3 * (int64_t)jc + 1];
+            dz2 = P.r2[3 * (int64_t)jc + 2];
+        } else {
+            x2 = P.r2d[jc];
+            y2 = P.r2d[P.n2 + jc];
+            z2 = P.r2d[2 * (int64_t)P.n2 + jc];
+        }
+        const float sa = F64 ? 0.f : pow2f(ea);
+        const df::D a = df::make(P.a_ee_hi, P.a_ee_lo);
+        for (int q = 0; q < ntiles; q++) {
+            if (!tc::mbar_wait(tc::smem_u32(tfull), q & 1, s_abort)) {
+                fail(16);
+                break;
+            }
+            tc::fence_after_sync();
+            const uint32_t cb = tbase + lane_off + (uint32_t)(R * pt0);
+            const int i0 = (t_begin + q) * Cfg::kPts + pt0;  // r1 row of the tile
+            if constexpr (F64) {
+                double V[WP * R];
+                float lo[WP * R];
+#pragma unroll
+                for (int c = 0; c < WP * R; c += 8)
+                    read_f64_8<S>(cb + (uint32_t)c, Q.eb + (int64_t)i0 * R + c, ea, V + c, lo + c);
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0)
+                    tc::mbar_arrive(tc::smem_u32(tempty));
+#pragma unroll
+                for (int p = 0; p < WP; p++)
+                    if (jok && i0 + p < P.n1b)
+                        pair_f64<R>(Q, i0 + p, j, V + p * R, lo + p * R, dx2, dy2, dz2);
+            } else {
+                uint64_t H[R / 16][8], L[R / 16][8], L2[R / 16][8];
+#pragma unroll
+                for (int h = 0; h < R / 16; h++)
+                    read_df16<S>(cb + 16u * h, H[h], L[h], L2[h]);
+                tc::fence_before_sync();
+                __syncwarp();
+                if (lane == 0)
+                    tc::mbar_arrive(tc::smem_u32(tempty));
+                if (jok && i0 < P.n1b) {
+                    df::D V[R];
+#pragma unroll
+                    for (int h = 0; h < R / 16; h++)
+                        scale_df16(H[h], L[h], L2[h], Q.bscale + (int64_t)i0 * R + 16 * h, V + 16 * h);
+                    pair_df<R>(Q, i0, j, V, x2, y2, z2, sa, a);
+                }
+            }
+        }
+    }
+
+    tc::fence_before_sync();
+    __syncthreads();
+    tc::fence_after_sync();
+    if (warp == kCtlWarp)
+        tc::tmem_dealloc(tbase, kTmemCols);
+}
+
+// ---------------------------------------------------------------------------
+// slicing of the operands
+// ---------------------------------------------------------------------------
+
+// Exponent e with |x| < 2^e for every x of the row; 0 for zero (or denormal-only) rows,
+// kNanExponent for a row with an infinity or a NaN.
+__device__ __forceinline__ int row_exponent(unsigned long long bits)
+{
+    const int E = (int)(bits >> 52);
+    return E == 0 ? 0 : min(E - 1022, kNanExponent);
+}
+
+// slices[(s * Mpad + r) * Kpad + k] for r < Mpad, k < Kpad = 32 KB (zeros outside M x K),
+// ex[r] = row exponent, of X[r * K + k]: one warp per row, so the row is read once.  The
+// digits are formed in integer arithmetic (digits.cuh).
+template <int S, int KB>
+__global__ void __launch_bounds__(256)
+slice_kernel(const double *__restrict__ X, int M, int K, int Mpad, __nv_bfloat16 *__restrict__ slices,
+             int *__restrict__ ex)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (r >= Mpad)
+        return;
+    double x[KB];
+    unsigned long long m = 0;
+#pragma unroll
+    for (int b = 0; b < KB; b++) {
+        const int k = 32 * b + lane;
+        x[b] = r < M && k < K ? X[r * K + k] : 0.0;
+        const unsigned long long v =
+            (unsigned long long)__double_as_longlong(x[b]) & 0x7fffffffffffffffull;
+        m = v > m ? v : m;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, o);
+        m = v > m ? v : m;
+    }
+    const int e = row_exponent(m);
+    if (lane == 0)
+        ex[r] = e;
+#pragma unroll
+    for (int b = 0; b < KB; b++) {
+        int q[S];
+        digits::digits_int<S>(e >= kNanExponent ? 0 : digits::scaled_round<S>(x[b], e), q);
+#pragma unroll
+        for (int s = 0; s < S; s++)
+            slices[((int64_t)s * Mpad + r) * (32 * KB) + 32 * b + lane] =
+                __float2bfloat16_rn(__int2float_rn(q[s]) * exp2f((float)(-8 - 9 * s)));
+    }
+}
+
+// ---------------------------------------------------------------------------
+// host side
+// ---------------------------------------------------------------------------
+
+static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
+
+// Nuclei with which the leading diagonals are exact: K = powers n_nuc at most 64 (FP64) or
+// 85 (double-float).
+static int max_nuclei(int rows, bool fp64)
+{
+    return (fp64 ? 64 : rows == 16 ? 80 : 85) / (rows == 16 ? 4 : 7);
+}
+
+PairTcMode pair_tc_mode(int n_nuc, const double *coef, const int *exps, int n_terms, bool fp64,
+                        int slices)
+{
+    PairTcMode m;
+    m.fp64 = fp64;
+    // 5 slices (representation error 2^-45, under the error of a 5-slice build's
+    // contractions), 6 for builds of 6 and 7 slices (2^-54, below the double-float
+    // epilogue), 7 for FP64 (2^-63)
+    m.slices = fp64 ? 7 : slices >= 6 ? 6 : 5;
+    const int rows = pair_df_sparse(exps, n_terms) ? 16 : 32;
+    if (n_nuc > max_nuclei(rows, fp64))
+        return m;
+    if (!fp64 && (getenv("CUTC_PAIR_DF") || getenv("CUTC_PAIR_DENSE")))
+        return m;
+    for (int k = 0; k < 3 * n_terms; k++)
+        if (!std::isfinite(coef[k]))
+            return m;
+    m.rows = rows;
+    return m;
+}
+
+size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices)
+{
+    const int64_t K = std::min<int64_t>(7 * (int64_t)n_nuc, 85);
+    return (size_t)n2 * K * 8 + 2 * (size_t)slices * round_up(n2, kBM) * round_up(K, kBK) +
+           4 * (size_t)round_up(n2, kBM);
+}
+
+size_t pair_tc_row_bytes(int n_nuc, int slices)
+{
+    const int64_t K = std::min<int64_t>(7 * (int64_t)n_nuc, 85);
+    return 32 * (size_t)K * 8 + 2 * (size_t)slices * 32 * round_up(K, kBK) + 3 * 8 + 32 * 8 + 64;
+}
+
+static int alloc_operand(Workspace &W, int slot, int S, int64_t M, int row_mult, int64_t K,
+                         SliceOperand &op)
+{
+    op.M = (int)M;
+    op.Mpad = (int)round_up(std::max<int64_t>(M, 1), row_mult);
+    op.K = K;
+    op.Kpad = round_up(std::max<int64_t>(K, 1), kBK);
+    void *p;
+    CUTC_TRY(W.get(slot, (size_t)S * op.Mpad * op.Kpad * 2, &p));
+    op.sl = p;
+    CUTC_TRY(W.get(slot + 1, (size_t)op.Mpad * 4, &p));
+    op.ex = (int *)p;
+    return CUTC_OK;
+}
+
+template <int S>
+static int slice_rows(cudaStream_t st, const double *X, const SliceOperand &op)
+{
+    const unsigned grid = ceil_div(op.Mpad, 8);
+    auto *sl = (__nv_bfloat16 *)op.sl;
+    switch ((int)(op.Kpad / kBK)) {
+    case 1: slice_kernel<S, 1><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
+    case 2: slice_kernel<S, 2><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
+    default: slice_kernel<S, 3><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
+    }
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+static int slice_rows(cudaStream_t st, int slices, const double *X, const SliceOperand &op)
+{
+    return slices == 5   ? slice_rows<5>(st, X, op)
+           : slices == 6 ? slice_rows<6>(st, X, op)
+                         : slice_rows<7>(st, X, op);
+}
+
+enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale };
+
+int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &mode, int n2,
+                    int n_nuc, const double *f2, int64_t n1t, int *err, PairTcPlan &plan)
+{
+    const int64_t K = (int64_t)mode.powers() * n_nuc;
+    const int64_t rows = (int64_t)mode.rows * n1t;
+    plan.mode = mode;
+    plan.err = err;
+    void *p;
+    CUTC_TRY(W.get(slot0 + kSlotF64, (size_t)n2 * K * 8, &p));
+    plan.Fd = (double *)p;
+    CUTC_TRY(W.get(slot0 + kSlotC64, (size_t)rows * K * 8, &p));
+    plan.Cd = (double *)p;
+    CUTC_TRY(W.get(slot0 + kSlotR1d, (size_t)3 * n1t * sizeof(float2), &p));
+    plan.r1d = (float2 *)p;
+    CUTC_TRY(W.get(slot0 + kSlotBscale, (size_t)round_up(rows, kPairBN) * 4, &p));
+    plan.bscale = (float *)p;
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotAF, mode.slices, n2, kBM, K, plan.AF));
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, mode.slices, rows, kPairBN, K, plan.BC));
+    CUTC_TRY(launch_pair_tc_f(st, mode.powers(), n2, n_nuc, f2, plan.Fd));
+    note_launches(1);
+    return slice_rows(st, mode.slices, plan.Fd, plan.AF);
+}
+
+// 2-D map over slices [rows_total][Kpad] BF16, box = kBK x box_rows, 64B swizzle.
+static int make_tmap(CUtensorMap *map, const void *base, int64_t rows_total, int64_t Kpad,
+                     int box_rows)
+{
+    const uint64_t dims[2] = {(uint64_t)Kpad, (uint64_t)rows_total};
+    const uint64_t strides[1] = {(uint64_t)Kpad * 2};
+    const uint32_t box[2] = {(uint32_t)kBK, (uint32_t)box_rows};
+    return encode_bf16_map(map, base, 2, dims, strides, box, 64);
+}
+
+template <int S, int KB, int R, bool F64>
+static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
+                         PairTcParams Q, int n_sm)
+{
+    using Cfg = PairTcCfg<S, KB, R, F64>;
+    static std::atomic<unsigned long long> attr_done{0};
+    const unsigned long long bit = current_device_bit();
+    if (!(attr_done.load() & bit)) {
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(pair_tc_kernel<S, KB, R, F64>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
+        attr_done.fetch_or(bit);
+    }
+    // about eight CTAs per SM, each walking a run of N tiles with its F tile resident
+    const int64_t want = 8 * (int64_t)n_sm;
+    const int64_t chunks = std::max<int64_t>(
+        1, std::min<int64_t>(Q.tiles_n, (want + Q.tiles_m - 1) / Q.tiles_m));
+    Q.chunk = (int)((Q.tiles_n + chunks - 1) / chunks);
+    const int64_t grid = (int64_t)Q.tiles_m * ((Q.tiles_n + Q.chunk - 1) / Q.chunk);
+    if (grid > INT32_MAX) {
+        cutc_set_error(CUTC_ERR_INVALID, "pair grid of %lld CTAs", (long long)grid);
+        return CUTC_ERR_INVALID;
+    }
+    pair_tc_kernel<S, KB, R, F64><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, Q);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
+template <int S, int R, bool F64>
+static int launch_kb(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
+                     const PairTcParams &Q, int n_sm, int KB)
+{
+    switch (KB) {
+    case 1: return launch_kernel<S, 1, R, F64>(st, ta, tb, Q, n_sm);
+    case 2: return launch_kernel<S, 2, R, F64>(st, ta, tb, Q, n_sm);
+    case 3:
+        if constexpr (!F64)
+            return launch_kernel<S, 3, R, F64>(st, ta, tb, Q, n_sm);
+        break;
+    }
+    cutc_set_error(CUTC_ERR_INVALID, "pair contraction of %d K blocks", KB);
+    return CUTC_ERR_INVALID;
+}
+
+// The tile's coefficient operand, then the kernel.
+static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const double *rn,
+                    double a_en, int n_sm)
+{
+    const PairTcMode &m = plan.mode;
+    const PairDfArgs &P = Q.P;
+    CUTC_TRY(launch_pair_tc_coef(st, m.rows, P.i0, P.n1b, P.nN, P.r1, rn, a_en, P.coef, P.exps,
+                                 P.term_off, plan.Cd, plan.r1d));
+    note_launches(1);
+    SliceOperand B = plan.BC;
+    B.M = m.rows * P.n1b;
+    B.Mpad = (int)round_up(B.M, kPairBN);
+    CUTC_TRY(slice_rows(st, m.slices, plan.Cd, B));
+    if (!m.fp64) {
+        exp_scale_kernel<<<ceil_div(B.Mpad, 256), 256, 0, st>>>(B.ex, B.Mpad, plan.bscale);
+        CUTC_CUDA_TRY(cudaGetLastError());
+        note_launches(1);
+    }
+    CUtensorMap ta, tb;
+    CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)m.slices * plan.AF.Mpad, plan.AF.Kpad, kBM));
+    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)m.slices * B.Mpad, B.Kpad, kPairBN));
+    Q.tiles_m = plan.AF.Mpad / kBM;
+    Q.tiles_n = B.Mpad / kPairBN;
+    Q.chunk = 1;
+    Q.Mpad = plan.AF.Mpad;
+    Q.Npad = B.Mpad;
+    Q.ea = plan.AF.ex;
+    Q.eb = B.ex;
+    Q.bscale = plan.bscale;
+    Q.r1d = plan.r1d;
+    Q.err = plan.err;
+    const int KB = (int)(plan.AF.Kpad / kBK);
+    if (m.fp64)
+        return m.rows == 16 ? launch_kb<7, 16, true>(st, ta, tb, Q, n_sm, KB)
+                            : launch_kb<7, 32, true>(st, ta, tb, Q, n_sm, KB);
+    if (m.slices == 6)
+        return m.rows == 16 ? launch_kb<6, 16, false>(st, ta, tb, Q, n_sm, KB)
+                            : launch_kb<6, 32, false>(st, ta, tb, Q, n_sm, KB);
+    return m.rows == 16 ? launch_kb<5, 16, false>(st, ta, tb, Q, n_sm, KB)
+                        : launch_kb<5, 32, false>(st, ta, tb, Q, n_sm, KB);
+}
+
+int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, const double *rn,
+                    double a_en, int n_sm)
+{
+    if (P.n1b <= 0 || P.n2 <= 0)
+        return CUTC_OK;
+    PairTcParams Q{};
+    Q.P = P;
+    return run_tile(st, plan, Q, rn, a_en, n_sm);
+}
+
+int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &A, const double *rn,
+                     double a_en, int n_sm)
+{
+    if (A.n1b <= 0 || A.n2 <= 0)
+        return CUTC_OK;
+    PairTcParams Q{};
+    PairDfArgs &P = Q.P;
+    P.i0 = A.i0; P.n1b = A.n1b; P.n2 = A.n2; P.nN = A.nN;
+    P.r1 = A.r1; P.r2 = A.r2; P.coef = A.coef; P.exps = A.exps; P.term_off = A.term_off;
+    P.a_ee = A.a_ee; P.ldg = A.ldg; P.plane = A.plane;
+    Q.G64 = A.G;
+    return run_tile(st, plan, Q, rn, a_en, n_sm);
+}
+
+}  // namespace cutc

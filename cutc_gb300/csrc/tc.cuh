@@ -249,6 +249,21 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
         v[i] = __uint_as_float(r[i]);
 }
 
+// The same for 8 columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
+{
+    uint32_t r[8];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n\t"
+                 "tcgen05.wait::ld.sync.aligned;"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
+                   "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+        v[i] = __uint_as_float(r[i]);
+}
+
 // Two FP32 lanes packed in 64 bits (x in the low word): round-to-nearest
 // add / sub of both lanes in one instruction (sm_100 and later).
 __device__ __forceinline__ uint64_t f2_pack(uint32_t lo, uint32_t hi)
