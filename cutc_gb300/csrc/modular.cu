@@ -49,11 +49,16 @@ struct ModCfg {
     static_assert(kTmemCols <= 512, "tensor memory");
 };
 
+// A residue r of a result is stored as the low half of the bits of the float r + kResidueBias,
+// whose high half is kResidueHigh.
+constexpr float kResidueBias = 12582912.0f + 512.0f;  // 1.5 * 2^23 + 2^9
+constexpr unsigned kResidueHigh = 0x4b40u;
+
 struct ModGemmParams {
     int n_mod, M, N, tiles_m, tiles_n;
     int nkb;                   // K blocks of the panel
     int accumulate;            // add to the residues in out
-    short *out;                // out[i plane + n ldm + m]
+    unsigned short *out;       // out[i plane + n ldm + m]
     int64_t ldm, plane;
     float p[moduli::kMax], inv[moduli::kMax];
     int *err;                  // set to a non-zero code if a bounded wait gave up
@@ -231,6 +236,7 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
         const uint32_t lane_off = (uint32_t)(q * 32) << 16;
         const uint32_t coff = (uint32_t)(grp * Cfg::kCols);
         const uint64_t magic = tc::f2_dup(12582912.0f);  // 1.5 * 2^23
+        const uint64_t bias = tc::f2_dup(kResidueBias);
         const uint32_t te0 = tc::map_to_rank(tc::smem_u32(&tempty[0]), 0);
         const uint32_t te1 = tc::map_to_rank(tc::smem_u32(&tempty[1]), 0);
         bool ok = true;
@@ -238,7 +244,7 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
         for (int task = first; task < n_tasks && ok; task = kResident ? task + stride : n_tasks) {
             const Tile o = tile(task);
             const int m = o.m0 + q * 32 + lane;
-            short *dst = P.out + o.z * P.plane + (int64_t)(o.n0 + (int)coff) * P.ldm + m;
+            unsigned short *dst = P.out + o.z * P.plane + (int64_t)(o.n0 + (int)coff) * P.ldm + m;
             const int ncol = P.N - o.n0 - (int)coff;  // columns of this warp that exist
             const uint64_t inv = tc::f2_dup(P.inv[o.z]), negp = tc::f2_dup(-P.p[o.z]);
             uint64_t acc[CP];
@@ -248,10 +254,10 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
             if (P.accumulate && m < P.M) {
 #pragma unroll
                 for (int j = 0; j < CP; j++) {
-                    const float a = 2 * j < ncol ? (float)dst[(int64_t)(2 * j) * P.ldm] : 0.0f;
-                    const float b =
-                        2 * j + 1 < ncol ? (float)dst[(int64_t)(2 * j + 1) * P.ldm] : 0.0f;
-                    acc[j] = tc::f2_pack(__float_as_uint(a), __float_as_uint(b));
+                    const unsigned a = 2 * j < ncol ? dst[(int64_t)(2 * j) * P.ldm] : 512u;
+                    const unsigned b = 2 * j + 1 < ncol ? dst[(int64_t)(2 * j + 1) * P.ldm] : 512u;
+                    acc[j] = tc::f2_sub(tc::f2_pack((kResidueHigh << 16) | a, (kResidueHigh << 16) | b),
+                                        bias);
                 }
             }
             for (int kb0 = 0; kb0 < nkb; kb0 += kChunkBlocks) {
@@ -284,14 +290,13 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                 buf ^= 1;
             }
             if (ok && m < P.M) {
-                // the low half of (residue + 1.5 2^23)'s bits is the residue as a 16-bit integer
 #pragma unroll
                 for (int j = 0; j < CP; j++) {
-                    const uint64_t w = tc::f2_add(acc[j], magic);
+                    const uint64_t w = tc::f2_add(acc[j], bias);
                     if (2 * j < ncol)
-                        dst[(int64_t)(2 * j) * P.ldm] = (short)(uint32_t)w;
+                        dst[(int64_t)(2 * j) * P.ldm] = (unsigned short)w;
                     if (2 * j + 1 < ncol)
-                        dst[(int64_t)(2 * j + 1) * P.ldm] = (short)(uint32_t)(w >> 32);
+                        dst[(int64_t)(2 * j + 1) * P.ldm] = (unsigned short)(w >> 32);
                 }
             }
         }
@@ -311,7 +316,7 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
 
 struct CombineParams {
     int M, ncols, n0;
-    const short *res;
+    const unsigned short *res;
     int64_t ldm, plane;
     const int *sa, *sb;
     ModularOut out;
@@ -319,80 +324,131 @@ struct CombineParams {
     const int *err, *skip;
 };
 
-// v 2^k: the exponent field moved with integer operations when v and the result are
-// normal numbers (GB300's FP64 pipe is slow), scalbn otherwise (zeros, and results that
-// underflow to subnormals or zero or overflow to infinity)
-__device__ __forceinline__ double scale_pow2(double v, int k)
+// Tables of the Chinese remainder theorem for N moduli: V = sum_i r_i W_i mod M with
+// W_i = (M / p_i) ((M / p_i)^-1 mod p_i), in 12-bit limbs (FP32 pairs, both lanes the same
+// value) and as fractions W_i / M.
+constexpr int kLimbBits = 12;
+constexpr int crt_limbs(int n) { return n <= 7 ? 5 : n <= 9 ? 7 : n <= 11 ? 8 : n <= 13 ? 10 : 11; }
+
+template <int N>
+struct CrtTab {
+    static constexpr int L = crt_limbs(N);
+    uint64_t w[N][L], frac[N];
+};
+
+template <int N>
+constexpr __int128 modulus()
 {
-    const long long b = __double_as_longlong(v);
-    const int e = (int)((b >> 52) & 0x7ff);
-    if (e != 0 && e + k >= 1 && e + k <= 2046)
-        return __longlong_as_double(b + ((long long)k << 52));
-    return scalbn(v, k);
+    __int128 M = 1;
+    for (int i = 0; i < N; i++)
+        M *= moduli::prime(i);
+    return M;
 }
 
-__device__ __forceinline__ int float_int(float f)  // an integer-valued float below 2^22
+constexpr uint32_t positive_code(double x)  // the bits of a positive double as a float
 {
-    return __float_as_int(f + 12582912.0f) - 0x4b400000;
-}
-
-__device__ __forceinline__ double int_double(long long v)  // |v| < 2^51, one FP64 add
-{
-    return __longlong_as_double(0x4338000000000000ll + v) - 6755399441055744.0;
-}
-
-// One mixed-radix group: sum of digits d[0..n) with radices p_{j0}, p_{j0+1}, ... (n <= 5,
-// below 2^45)
-template <int N, int J0>
-__device__ __forceinline__ long long digit_group(const float (&d)[N])
-{
-    constexpr int n = N - J0 < 5 ? N - J0 : 5;
-    auto pr = [](int i) { return moduli::prime(i); };
-    int hi = 0;
-    if constexpr (n == 5)
-        hi = float_int(d[J0 + 4]);
-    if constexpr (n >= 4) {
-        hi = hi * (moduli::prime(J0 + 2) * moduli::prime(J0 + 3 < N ? J0 + 3 : 0)) +
-             float_int(fmaf(d[J0 + (n >= 4 ? 3 : 0)], (float)pr(J0 + 2), d[J0 + 2]));
-    } else if constexpr (n == 3) {
-        hi = float_int(d[J0 + 2]);
+    int e = 0;
+    while (x >= 2.0) {
+        x *= 0.5;
+        e++;
     }
-    const int lo = n >= 2 ? float_int(fmaf(d[J0 + (n >= 2 ? 1 : 0)], (float)pr(J0), d[J0]))
-                          : float_int(d[J0]);
-    return n >= 3 ? (long long)hi * (moduli::prime(J0) * moduli::prime(n >= 2 ? J0 + 1 : 0)) + lo
-                  : (long long)lo;
-}
-
-constexpr double radix5(int j0)  // p_{j0} ... p_{j0 + 4}, below 2^45
-{
-    double v = 1.0;
-    for (int i = 0; i < 5; i++)
-        v *= moduli::prime(j0 + i);
-    return v;
+    while (x < 1.0) {
+        x *= 2.0;
+        e--;
+    }
+    return ((uint32_t)(127 + e) << 23) + (uint32_t)((x - 1.0) * 8388608.0 + 0.5);
 }
 
 template <int N>
-__device__ __forceinline__ double digits_value(const float (&d)[N])
+constexpr CrtTab<N> make_crt_tab()
 {
-    // rounded once, at the result's own precision (to a unit that is 2^-50 of its last place)
-    double v = int_double(digit_group<N, 0>(d));
-    if constexpr (N > 10) {
-        constexpr double q0 = radix5(0), q1 = radix5(5);
-        const double g1 = int_double(digit_group<N, 5>(d)), g2 = int_double(digit_group<N, 10>(d));
-        const double u = fma(g2, q1, g1);
-        if constexpr (N > 11)  // u's rounding error, an exact integer (below 2^53 if N = 11)
-            v = fma(fma(g2, q1, -u) + g1, q0, v);
-        v = fma(u, q0, v);
-    } else if constexpr (N > 5) {
-        constexpr double q0 = radix5(0);
-        v = fma(int_double(digit_group<N, 5>(d)), q0, v);
+    CrtTab<N> t{};
+    const unsigned __int128 M = (unsigned __int128)modulus<N>();
+    for (int i = 0; i < N; i++) {
+        const int p = moduli::prime(i);
+        const unsigned __int128 q = M / (unsigned)p;
+        int inv = moduli::inverse((int)(q % (unsigned)p), p);
+        if (inv < 0)
+            inv += p;
+        const unsigned __int128 W = q * (unsigned)inv;
+        for (int l = 0; l < CrtTab<N>::L; l++)
+            t.w[i][l] = dup_code(float_code((int)(W >> (kLimbBits * l)) & 0xfff));
+        t.frac[i] = dup_code(positive_code((double)W / (double)M));
     }
-    return v;
+    return t;
 }
 
-// Residues -> mixed-radix digits (Garner; every FP32 operation exact, two rows per f32x2
-// operation) -> FP64.  Consecutive threads take consecutive m; bound by the N reads of
-// 2 bytes and the digits' N (N - 1) / 2 modular steps.
+static __constant__ const CrtTab<7> c_crt7 = make_crt_tab<7>();
+static __constant__ const CrtTab<9> c_crt9 = make_crt_tab<9>();
+static __constant__ const CrtTab<11> c_crt11 = make_crt_tab<11>();
+static __constant__ const CrtTab<13> c_crt13 = make_crt_tab<13>();
+static __constant__ const CrtTab<15> c_crt15 = make_crt_tab<15>();
+
+template <int N>
+__device__ __forceinline__ const CrtTab<N> &crt_tab()
+{
+    if constexpr (N == 7)
+        return c_crt7;
+    else if constexpr (N == 9)
+        return c_crt9;
+    else if constexpr (N == 11)
+        return c_crt11;
+    else if constexpr (N == 13)
+        return c_crt13;
+    else
+        return c_crt15;
+}
+
+// v 2^k rounded to nearest even, in integer arithmetic (GB300's FP64 pipe is slow); results
+// outside the normal range by scalbn
+__device__ __forceinline__ double scaled_double(__int128 v, int k)
+{
+    const bool neg = v < 0;
+    unsigned __int128 a = (unsigned __int128)(neg ? -v : v);
+    const unsigned long long ah = (unsigned long long)(a >> 64);
+    if (a == 0)
+        return 0.0;
+    const int lz = ah ? __clzll((long long)ah) : 64 + __clzll((long long)(unsigned long long)a);
+    a <<= lz;  // the leading bit at bit 127
+    const unsigned long long h = (unsigned long long)(a >> 64), l = (unsigned long long)a;
+    unsigned long long m = h >> 11;  // 53 bits
+    const unsigned rest = (unsigned)h & 0x7ffu;
+    m += rest > 0x400u || (rest == 0x400u && (l != 0 || (m & 1))) ? 1 : 0;
+    const int E = 1023 + 127 - lz + k;
+    double r;
+    if (E >= 1 && E <= 2045)  // m's leading bit (or its carry) adds one to the exponent field
+        r = __longlong_as_double((long long)(((unsigned long long)(E - 1) << 52) + m));
+    else
+        r = scalbn(__longlong_as_double((long long)((1022ull << 52) + m)), E - 1023);
+    return neg ? -r : r;
+}
+
+// The integer of its limbs: v[l] an integer-valued float below 2^24 in magnitude.
+template <int L>
+__device__ __forceinline__ __int128 limbs_value(const float (&v)[L])
+{
+    auto half = [&](int l0, int n) {  // up to 5 limbs, below 2^(48 + 24)
+        long long s = 0;
+#pragma unroll
+        for (int l = n - 1; l >= 0; l--)
+            s = s * (1 << kLimbBits) + __float2int_rn(v[l0 + l]);
+        return s;
+    };
+    // three limbs (2^48) to a 64-bit integer
+    __int128 r = 0;
+#pragma unroll
+    for (int g = (L - 1) / 3; g >= 0; g--)
+        r = r * ((long long)1 << (3 * kLimbBits)) + half(3 * g, g == (L - 1) / 3 ? L - 3 * g : 3);
+    return r;
+}
+
+// Residues -> the integer V = sum_i r_i W_i - q M (Chinese remainder theorem) -> FP64,
+// rounded once.  The limbs' sums stay below 2^24 (15 residues of 181 times 12 bits), so
+// their FP32 operations are exact; sum_i r_i W_i / M is off by less than 0.002, and
+// |V| <= 0.4914 M by the row scales, so q is its nearest integer.
+// Consecutive threads take consecutive m, two per thread in f32x2 operations; bound by
+// these N (L + 1) operations and the integer work, where Garner's mixed-radix digits took
+// 5 N (N - 1) / 2.
 template <int N>
 __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
 {
@@ -401,24 +457,33 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
     const int m = 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (m >= P.M)
         return;
+    constexpr int L = CrtTab<N>::L;
+    const CrtTab<N> &tab = crt_tab<N>();
     const bool failed = *P.err != 0;
     const uint64_t magic = tc::f2_dup(12582912.0f);
+    const uint64_t bias = tc::f2_dup(kResidueBias);
     const int s0 = P.sa[m], s1 = m + 1 < P.M ? P.sa[m + 1] : 0;
     for (int c = blockIdx.y; c < P.ncols; c += gridDim.y) {
-        const short *src = P.res + (int64_t)c * P.ldm + m;
-        uint64_t d[N];
+        const unsigned short *src = P.res + (int64_t)c * P.ldm + m;
+        unsigned word[N];
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            word[i] = *reinterpret_cast<const unsigned *>(src + i * P.plane);
+        uint64_t v[L], t = 0ull;
+#pragma unroll
+        for (int l = 0; l < L; l++)
+            v[l] = 0ull;
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            const short2 v = *reinterpret_cast<const short2 *>(src + i * P.plane);
-            uint64_t t = tc::f2_pack(__float_as_uint((float)v.x), __float_as_uint((float)v.y));
+            const uint64_t r = tc::f2_sub(tc::f2_pack(__byte_perm(word[i], kResidueHigh, 0x5410),
+                                                      __byte_perm(word[i], kResidueHigh, 0x5432)),
+                                          bias);
+            t = tc::f2_fma(r, tab.frac[i], t);
 #pragma unroll
-            for (int j = 0; j < i; j++) {
-                t = tc::f2_mul(tc::f2_sub(t, d[j]), c_tab.garner[i][j]);
-                const uint64_t q = tc::f2_sub(tc::f2_fma(t, c_tab.inv[i], magic), magic);
-                t = tc::f2_fma(q, c_tab.negp[i], t);
-            }
-            d[i] = t;
+            for (int l = 0; l < L; l++)
+                v[l] = tc::f2_fma(r, tab.w[i][l], v[l]);
         }
+        const uint64_t q = tc::f2_add(t, magic);  // its bits: q + those of 1.5 * 2^23
         const int sn = P.sb[c], n = P.n0 + c;
         const int64_t col = (int64_t)(n / P.out.ncol_group) * P.out.group_stride + P.out.col0 +
                             n % P.out.ncol_group;
@@ -430,26 +495,29 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
                                                        (m + h) % P.out.nrow_group
                                                  : m + h;
             double *dst = P.out.C + row + P.out.ldc * col;
-            float f[N];
+            float f[L];
 #pragma unroll
-            for (int i = 0; i < N; i++)
-                f[i] = h ? tc::f2_hi(d[i]) : tc::f2_lo(d[i]);
+            for (int l = 0; l < L; l++)
+                f[l] = h ? tc::f2_hi(v[l]) : tc::f2_lo(v[l]);
             const int sm = h ? s1 : s0;
-            double v;
+            double x;
             if (failed || sm == kNotFinite || sn == kNotFinite) {
-                v = __longlong_as_double(0x7ff8000000000000ll);
+                x = __longlong_as_double(0x7ff8000000000000ll);
             } else {
-                v = scale_pow2(digits_value<N>(f), P.alpha_exp - sm - sn);
+                x = scaled_double(
+                    limbs_value<L>(f) -
+                        (__int128)((int)(h ? q >> 32 : q) - 0x4b400000) * modulus<N>(),
+                    P.alpha_exp - sm - sn);
                 if (P.alpha_neg)
-                    v = __longlong_as_double(__double_as_longlong(v) ^ (1ll << 63));
+                    x = __longlong_as_double(__double_as_longlong(x) ^ (1ll << 63));
                 if (P.alpha_mul)
-                    v *= P.out.alpha;
+                    x *= P.out.alpha;
             }
             if (P.beta_mode == 1)
-                v += *dst;
+                x += *dst;
             else if (P.beta_mode == 2)
-                v += P.out.beta * *dst;
-            *dst = v;
+                x += P.out.beta * *dst;
+            *dst = x;
         }
     }
 }
@@ -556,7 +624,7 @@ static int launch_gemm(cudaStream_t st, const ResiduePlanes &A, const ResiduePla
 }
 
 int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
-                 short *out, int64_t plane_cols, bool accumulate, int *err)
+                 unsigned short *out, int64_t plane_cols, bool accumulate, int *err)
 {
     if (A.rows <= 0 || B.rows <= 0 || A.kp <= 0)
         return CUTC_OK;
@@ -601,7 +669,7 @@ static int launch_combine(cudaStream_t st, const CombineParams &P)
     return CUTC_OK;
 }
 
-int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const short *res,
+int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
                     const int *sa, const int *sb, const ModularOut &out, const int *err,
                     const int *skip)
 {

@@ -22,7 +22,6 @@ struct ModuliTab {
     uint64_t chunk[moduli::kMax][moduli::kMaxChunks];  // 2^{13 j} mod p_i
     uint64_t inv[moduli::kMax];                        // 1 / p_i
     uint64_t negp[moduli::kMax];                       // -p_i
-    uint64_t garner[moduli::kMax][moduli::kMax];       // p_j^-1 mod p_i, j < i
 };
 
 constexpr uint32_t float_code(int v)  // the bits of a small integer as a float
@@ -58,8 +57,6 @@ constexpr ModuliTab make_moduli_tab()
         }
         t.inv[i] = dup_code(inverse_code(p));
         t.negp[i] = dup_code(float_code(-p));
-        for (int j = 0; j < i; j++)
-            t.garner[i][j] = dup_code(float_code(moduli::inverse(moduli::prime(j), p)));
     }
     return t;
 }
@@ -114,13 +111,13 @@ size_t modular_out_bytes(int n_mod, int64_t M, int64_t N);
 // added to what is there when accumulate.  err: set when a bounded wait gave up.
 inline int64_t modular_ldm(int64_t M) { return (M + 7) / 8 * 8; }
 int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
-                 short *out, int64_t plane_cols, bool accumulate, int *err);
+                 unsigned short *out, int64_t plane_cols, bool accumulate, int *err);
 
 // The FP64 results from the residues: n0 .. n0 + ncols of the output's columns; sa and sb
 // are the row scales of A and B (sb of column n0 first).  A result with a scale of
 // kNotFinite, or after a wait that gave up, is NaN.  skip (may be null): nothing is
 // written when *skip is non-zero.
-int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const short *res,
+int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
                     const int *sa, const int *sb, const ModularOut &out, const int *err,
                     const int *skip);
 
@@ -161,7 +158,7 @@ int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, si
     ResiduePlanes b;
     b.p = p;
     CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &p));
-    short *res = (short *)p;
+    unsigned short *res = (unsigned short *)p;
     a.rows = M;
     for (int n0 = 0; n0 < N; n0 += pass) {
         const int nc = std::min(pass, N - n0);

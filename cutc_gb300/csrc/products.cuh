@@ -18,7 +18,7 @@ int launch_expand_pairs(cudaStream_t st, int64_t rows, int nA, const double *Xp,
                         double *X);
 // Columns c0 <= col < c1 of int_2e = A + A^T (column-major, nA^2 rows) from the
 // packed symmetric (H) and antisymmetric (N) parts; out holds column c0 first.
-// psqt: element (p,q,s,t) goes where (p,s,q,t) would (c0 and c1 multiples of nA).
+// c0 and c1 are multiples of nA.  psqt: element (p,q,s,t) goes where (p,s,q,t) would.
 int launch_assemble_int2e(cudaStream_t st, int nA, const double *H, const double *N, int c0,
                           int c1, bool psqt, double *out);
 // a <- a + a^T (column-major n x n), and the (p,q,s,t) -> (p,s,q,t) swap of an n^4 array,
