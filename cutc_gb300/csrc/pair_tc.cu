@@ -16,9 +16,9 @@
 // (FP64 results); later diagonals round at 2^-27 2^-24 and 2^-36 2^-24 of the row scales.
 //
 // A = the F slices of 128 r2 points, all of K, loaded once per CTA; B = the coefficient
-// slices in tiles of 64 rows (four r1 points, or two), streamed; one stacked accumulator
-// set in tensor memory.  The tensor-core work of a tile is a small part of its epilogue, so
-// one accumulator set and one B stage suffice: the next tile's MMAs run as soon as the
+// slices in tiles of 64 rows (four r1 points, or two; 32 rows for FP64 results), streamed;
+// one stacked accumulator set in tensor memory (two for FP64 results).  The tensor-core work of a tile is a small part of its epilogue, so
+// one B stage per accumulator set suffices: the next tile's MMAs run as soon as the
 // epilogue has read the accumulators, and one control warp issues both the TMA loads and
 // the MMAs.
 //
@@ -30,11 +30,11 @@
 // nucleus.
 //
 // FP64 epilogue: the diagonals down to 2^-43 of the row scales become one exact integer
-// (integer arithmetic; one FP64 add makes it a double), the rest stays in FP32 beside it,
-// and g12, its gradient and the polynomial take FP64: 66 FP64 operations per pair with 16
-// rows, whatever the number of nuclei, on a pipe of 2 per clock and SM, against about 11
-// per term in the term-by-term kernel (pair.cu).  512 x 20 011 pairs, 8 nuclei with 13
-// terms each: 19.3 -> 1.77 ms.  General exponents in double-float, 2003 x 30 011 pairs, 6
+// and a double in integer arithmetic, the rest stays in FP32 beside it, and g12, its
+// gradient and the polynomial take FP64: 45 FP64 operations per pair with 16 rows, whatever
+// the number of nuclei, on a pipe of 2 per clock and SM, against about 11 per term in the
+// term-by-term kernel (pair.cu).  512 x 20 011 pairs, 8 nuclei with 13
+// terms each: 19.3 -> 1.45 ms.  General exponents in double-float, 2003 x 30 011 pairs, 6
 // nuclei, against pair_df_kernel<6>: 16.6 -> 4.5 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -92,23 +92,28 @@ __global__ void exp_scale_kernel(const int *__restrict__ ex, int rows, float *__
 // R: coefficient rows per r1 point (16 or 32).
 template <int S, int KB, int R, bool F64>
 struct PairTcCfg {
-    static constexpr int kBN = kPairBN;
+    // Double-float: one accumulator set, and a warp per lane quarter and point of a tile
+    // (16 warps with 16 rows, four per SM sub-partition, to hide the latency of their
+    // dependent chains; 8 with 32 rows).  FP64: tiles of 32 rows in two accumulator sets,
+    // each with four warps of its own that take all points of its tiles, so that one set's
+    // integer work runs beside the other's FP64 work (with one set, every warp waits for
+    // the same tile and the FP64 pipe idled 40% of the time).
+    static constexpr int kBN = F64 ? 32 : kPairBN;
+    static constexpr int kBufs = F64 ? 2 : 1;
     static constexpr int kPts = kBN / R;
-    // double-float with 16 rows: a warp per lane quarter and point, four warps per SM
-    // sub-partition, to hide the latency of their dependent chains; otherwise two points
-    // (or one, with 32 rows) per warp of eight, which leaves the registers
-    static constexpr int kEpiWarps = (F64 || R == 32) ? 8 : 16;
-    static constexpr int kWarpPts = 4 * kPts / kEpiWarps;
+    static constexpr int kEpiWarps = F64 ? 8 : 4 * kPts;
+    static constexpr int kWarpPts = F64 ? kPts : 1;
+    static constexpr int kBufWarps = kEpiWarps / kBufs;  // epilogue warps of a buffer
     static constexpr int kCtlWarp = kEpiWarps;       // TMA loads and MMAs, lane 0
     static constexpr int kThreads = (kEpiWarps + 1) * 32;
     static constexpr int kASlice = kBM * kBK * 2;
     static constexpr int kBSlice = kBN * kBK * 2;
     static constexpr int kABytes = KB * S * kASlice;
     static constexpr int kBStage = KB * S * kBSlice;
-    static constexpr int kSmem = kABytes + kBStage + 1024 + 256;
+    static constexpr int kSmem = kABytes + kBufs * kBStage + 1024 + 256;
     static constexpr int kMaxN = 256;                // widest kind::f16 instruction at M = 128
     static_assert(kSmem <= 227 * 1024, "shared memory");
-    static_assert(kBN * S <= (int)kTmemCols, "accumulators exceed tensor memory");
+    static_assert(kBufs * kBN * S <= (int)kTmemCols, "accumulators exceed tensor memory");
     static_assert(kMaxN % kBN == 0, "instruction splits on diagonal boundaries");
     static_assert(kBSlice % 512 == 0, "B slices must stack on 8-row swizzle atoms");
 };
@@ -247,12 +252,32 @@ __device__ __forceinline__ void pair_df(const PairTcParams &Q, int i, int j, con
     o[3 * P.plane] = make_float2(lv.hi, lv.lo);
 }
 
+// I 2^k for |I| < 2^53, exactly, in integer arithmetic (0 below the normal range, an
+// infinity above it)
+__device__ __forceinline__ double int_double(long long I, int k)
+{
+    const unsigned long long m = (unsigned long long)(I < 0 ? -I : I);
+    const int lz = __clzll((long long)m);  // 64 for 0
+    const int E = 1023 + 63 - lz + k;      // the exponent field
+    const unsigned long long f = m << ((lz - 11) & 63);  // leading bit at 52
+    unsigned hi = (unsigned)(f >> 32) + ((unsigned)(E - 1) << 20), lo = (unsigned)f;
+    if (m == 0 || E < 1)
+        hi = lo = 0u;
+    else if (E > 2046) {
+        hi = 0x7ff00000u;
+        lo = 0u;
+    }
+    return __hiloint2double((int)(hi | ((unsigned)(I >> 32) & 0x80000000u)), (int)lo);
+}
+
 // The V values of eight columns in two parts each: hi, the diagonals down to 2^-43 of the
 // row scale as a double, and lo, the rest (below 2^-35, to 2^-60) as a float.  e: the
 // exponents of the columns' scales with the F row's added.
 //   H + L + L2 + L3 on the grids 2^-16, 2^-25, 2^-34, 2^-43 (each exact, as read_df16)
-// is an integer multiple of 2^-43 below 2^50, formed with integer operations.
-template <int S>
+// is an integer multiple of 2^-43 below 2^50, formed and made a double with integer
+// operations (an FP64 add per value instead, on the pipe that bounds the kernel, cost 15 of
+// 67 FP64 operations a pair).
+template <int S, int BN>
 __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, double *hi, float *lo)
 {
     static_assert(S == 7, "FP64 results take 7 slices");
@@ -265,7 +290,7 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
     // multiples of 2^g: C = 1.5 2^(23 + g)
     auto cut = [&](int d, float C, uint64_t (&up)[4], uint64_t (&rest)[4]) {
         const uint64_t Cg = tc::f2_dup(C);
-        tc::tmem_ld8(cb + (uint32_t)(kPairBN * d), v);
+        tc::tmem_ld8(cb + (uint32_t)(BN * d), v);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             const uint64_t x = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
@@ -280,7 +305,7 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
     cut(4, 0.375f * 0x1p-18f, L3, L4);
 #pragma unroll
     for (int d = 5; d < S; d++) {
-        tc::tmem_ld8(cb + (uint32_t)(kPairBN * d), v);
+        tc::tmem_ld8(cb + (uint32_t)(BN * d), v);
 #pragma unroll
         for (int k = 0; k < 4; k++)
             L4[k] = tc::f2_add(L4[k], tc::f2_pack(__float_as_uint(v[2 * k]),
@@ -296,20 +321,10 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
         const int il = grid_int(part(L), 0x1p25f);
         const int il2 = grid_int(part(L2), 0x1p34f), il3 = grid_int(part(L3), 0x1p43f);
         const long long I = ((long long)ih << 27) + ((long long)il << 18) + (long long)(il2 * 512 + il3);
-        // I as a double (one FP64 add), then 2^(e - 43) on its exponent field
-        const double x = __longlong_as_double(0x4338000000000000ll + I) - 6755399441055744.0;
         const int e = eb[k] + ea;
-        const int ef = ((__double2hiint(x) >> 20) & 0x7ff) + e - 43;
-        double y;
-        if (eb[k] >= kNanExponent || ea >= kNanExponent)
-            y = __longlong_as_double(0x7ff8000000000000ll);
-        else if (I == 0 || ef < 1)
-            y = 0.0;
-        else if (ef > 2046)
-            y = __hiloint2double((__double2hiint(x) & 0x80000000) | 0x7ff00000, 0);
-        else
-            y = __hiloint2double(__double2hiint(x) + ((e - 43) << 20), __double2loint(x));
-        hi[k] = y;
+        hi[k] = eb[k] >= kNanExponent || ea >= kNanExponent
+                    ? __longlong_as_double(0x7ff8000000000000ll)
+                    : int_double(I, e - 43);
         lo[k] = part(L4) * pow2f(min(e, 127));
     }
 }
@@ -331,6 +346,25 @@ __device__ __forceinline__ double exact_double(float x)
     return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
 }
 
+// any float as a double (subnormals as zero, infinities and NaNs as infinities or NaNs)
+__device__ __forceinline__ double signed_double(float x)
+{
+    const unsigned b = __float_as_uint(x), m = b & 0x7fffffffu;
+    unsigned hi = (m >> 3) + 0x38000000u;
+    hi = m < 0x00800000u ? 0u : m >= 0x7f800000u ? (m >> 3) | 0x7ff00000u : hi;
+    return __hiloint2double((int)(hi | (b & 0x80000000u)), m < 0x00800000u ? 0 : (int)(m << 29));
+}
+
+// -x / 2 of a finite normal x, else by an FP64 multiply
+__device__ __forceinline__ double minus_half(double x)
+{
+    const int hi = __double2hiint(x);
+    const int E = (hi >> 20) & 0x7ff;
+    if (E >= 2 && E < 0x7ff)
+        return __hiloint2double((hi - 0x00100000) ^ (int)0x80000000, __double2loint(x));
+    return -0.5 * x;
+}
+
 // One pair in FP64 from its V values (hi + lo).  The reciprocal square root and the
 // reciprocal are FP32 seeds with one step each of third order in FP64 (the seeds' relative
 // errors of 2^-22 and 2^-23 become 2^-63 and below).
@@ -341,23 +375,26 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
     const PairDfArgs &P = Q.P;
     const double *r1p = P.r1 + 3 * (int64_t)(P.i0 + i);
     const double a = P.a_ee;
+    const bool a_one = __double_as_longlong(a) == 0x3ff0000000000000ll;  // the reference's scale
     const double dx = r1p[0] - x2, dy = r1p[1] - y2, dz = r1p[2] - z2;
     const double d2 = fma(dx, dx, fma(dy, dy, dz * dz));
     const int hw = __double2hiint(d2);
     double g = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-    if (d2 > 1e-15) {
-        double y, z, d, ad;
+    // d2 > 1e-15 (src/jast_bh.cu:143) on the bits: positive doubles order like them, and a
+    // NaN is not greater
+    const long long db = __double_as_longlong(d2);
+    if (db > __double_as_longlong(1e-15) && db <= 0x7ff0000000000000ll) {
+        double y, z, d;
         if (hw < (1023 + 120) << 20) {
             const double y0 = exact_double(rsqrtf(trunc_float(d2)));
             const double e = fma(-(d2 * y0), y0, 1.0);
             y = fma(e * y0, fma(e, 0.375, 0.5), y0);
             d = d2 * y;
-            ad = a * d;
         } else {  // distances beyond 2^60, and infinities
             d = sqrt(d2);
             y = 1.0 / d;
-            ad = a * d;
         }
+        const double ad = a_one ? d : a * d;
         const double den = 1.0 + ad;
         if (__double2hiint(den) < (1023 + 120) << 20) {
             const double z0 = exact_double(__frcp_rn(trunc_float(den)));
@@ -367,7 +404,9 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
             z = 1.0 / den;
         }
         g = ad * z;
-        const double s = (a * z) * (z * y);
+        double s = z * z * y;
+        if (!a_one)
+            s *= a;
         gx = s * dx;
         gy = s * dy;
         gz = s * dz;
@@ -412,14 +451,14 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
         lz = low(14, 7);
         lg = low(21, 6);
     }
-    ux = fma(dudg, gx, ux) + (double)fmaf(lg, trunc_float(gx), lx);
-    uy = fma(dudg, gy, uy) + (double)fmaf(lg, trunc_float(gy), ly);
-    uz = fma(dudg, gz, uz) + (double)fmaf(lg, trunc_float(gz), lz);
+    ux = fma(dudg, gx, ux) + signed_double(fmaf(lg, trunc_float(gx), lx));
+    uy = fma(dudg, gy, uy) + signed_double(fmaf(lg, trunc_float(gy), ly));
+    uz = fma(dudg, gz, uz) + signed_double(fmaf(lg, trunc_float(gz), lz));
     double *o = Q.G64 + (int64_t)i * P.ldg + j;
     o[0] = ux;
     o[P.plane] = uy;
     o[2 * P.plane] = uz;
-    o[3 * P.plane] = -0.5 * fma(ux, ux, fma(uy, uy, uz * uz));
+    o[3 * P.plane] = minus_half(fma(ux, ux, fma(uy, uy, uz * uz)));
 }
 
 template <int S, int KB, int R, bool F64>
@@ -429,19 +468,20 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 {
     using Cfg = PairTcCfg<S, KB, R, F64>;
     constexpr int D = S - 1, BN = Cfg::kBN;
-    constexpr int kEpiWarps = Cfg::kEpiWarps, kCtlWarp = Cfg::kCtlWarp;
+    constexpr int kCtlWarp = Cfg::kCtlWarp;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *sA = smem;
     uint8_t *sB = smem + Cfg::kABytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + Cfg::kBStage);
-    uint64_t *afull = bars;      // the F tile has landed
-    uint64_t *full = bars + 1;   // the B stage holds tile q
-    uint64_t *empty = bars + 2;  // the MMAs of tile q are done with the B stage
-    uint64_t *tfull = bars + 3;  // the accumulators hold tile q
-    uint64_t *tempty = bars + 4; // every epilogue warp has read tile q's accumulators
-    uint64_t *drain = bars + 5;
+    constexpr int NB = Cfg::kBufs;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + NB * Cfg::kBStage);
+    uint64_t *afull = bars;            // the F tile has landed
+    uint64_t *full = bars + 1;         // a B stage holds a tile
+    uint64_t *empty = full + NB;       // the MMAs of the tile are done with the B stage
+    uint64_t *tfull = empty + NB;      // the accumulators hold the tile
+    uint64_t *tempty = tfull + NB;     // its epilogue warps have read them
+    uint64_t *drain = tempty + NB;
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
 
@@ -452,8 +492,13 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int ntiles = min(Q.tiles_n, t_begin + Q.chunk) - t_begin;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 5; i++)
-            tc::mbar_init(tc::smem_u32(&bars[i]), i == 4 ? kEpiWarps : 1);
+        tc::mbar_init(tc::smem_u32(afull), 1);
+        for (int i = 0; i < NB; i++) {
+            tc::mbar_init(tc::smem_u32(&full[i]), 1);
+            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
+            tc::mbar_init(tc::smem_u32(&tfull[i]), 1);
+            tc::mbar_init(tc::smem_u32(&tempty[i]), Cfg::kBufWarps);
+        }
         tc::mbar_init(tc::smem_u32(drain), 1);
         *s_abort = 0;
         tc::fence_mbar_init();
@@ -479,15 +524,17 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == kCtlWarp) {
         if (lane == 0) {
             auto load_b = [&](int q) {
-                const uint32_t fb = tc::smem_u32(full);
+                const int b = q % NB;
+                const uint32_t fb = tc::smem_u32(&full[b]);
                 tc::mbar_arrive_expect_tx(fb, Cfg::kBStage);
                 const int n0 = (t_begin + q) * BN;
 #pragma unroll
                 for (int kb = 0; kb < KB; kb++)
 #pragma unroll
                     for (int t = 0; t < S; t++)
-                        tc::tma_load_2d(tc::smem_u32(sB + (kb * S + t) * Cfg::kBSlice), &tmB,
-                                        kb * kBK, t * Q.Npad + n0, fb);
+                        tc::tma_load_2d(
+                            tc::smem_u32(sB + b * Cfg::kBStage + (kb * S + t) * Cfg::kBSlice), &tmB,
+                            kb * kBK, t * Q.Npad + n0, fb);
             };
             const uint32_t ab = tc::smem_u32(afull);
             tc::mbar_arrive_expect_tx(ab, Cfg::kABytes);
@@ -497,26 +544,27 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int s = 0; s < S; s++)
                     tc::tma_load_2d(tc::smem_u32(sA + (kb * S + s) * Cfg::kASlice), &tmA, kb * kBK,
                                     s * Q.Mpad + m0, ab);
-            int loaded = 0;  // B tiles issued into the stage
-            if (ntiles > 0) {
-                load_b(0);
-                loaded = 1;
-            }
+            int loaded = 0;  // B tiles issued
+            for (; loaded < min(NB, ntiles); loaded++)
+                load_b(loaded);
             bool ok = tc::mbar_wait(ab, 0, s_abort);
             if (!ok)
                 fail(12);
             for (int q = 0; q < ntiles && ok; q++) {
-                // the accumulators are free once every epilogue warp has read tile q - 1
-                if (q >= 1 && !tc::mbar_wait(tc::smem_u32(tempty), (q - 1) & 1, s_abort)) {
+                const int b = q % NB, round = q / NB;
+                // the accumulators are free once their epilogue warps have read the last tile
+                if (round >= 1 &&
+                    !tc::mbar_wait(tc::smem_u32(&tempty[b]), (round - 1) & 1, s_abort)) {
                     fail(13);
                     break;
                 }
-                if (!tc::mbar_wait(tc::smem_u32(full), q & 1, s_abort)) {
+                if (!tc::mbar_wait(tc::smem_u32(&full[b]), round & 1, s_abort)) {
                     fail(14);
                     break;
                 }
                 tc::fence_after_sync();
-                const uint32_t sb0 = tc::smem_u32(sB);
+                const uint32_t sb0 = tc::smem_u32(sB + b * Cfg::kBStage);
+                const uint32_t acc = tbase + (uint32_t)(BN * S * b);
                 const uint32_t sa0 = tc::smem_u32(sA);
                 bool first = true;
 #pragma unroll
@@ -534,23 +582,22 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 const int nt = min(Cfg::kMaxN / BN, D - s + 1 - t0);
                                 const uint64_t bd = tc::smem_desc_sw64(
                                     sb0 + (kb * S + t0) * Cfg::kBSlice + k16 * 32);
-                                tc::mma_bf16(tbase + (uint32_t)(BN * (s + t0)), ad, bd,
+                                tc::mma_bf16(acc + (uint32_t)(BN * (s + t0)), ad, bd,
                                              tc::idesc_bf16_f32(kBM, BN * nt), first ? 0u : 1u);
                             }
                             first = false;
                         }
                     }
                 }
-                tc::mma_commit(tc::smem_u32(empty));
-                tc::mma_commit(tc::smem_u32(tfull));
-                // refill the B stage for tile q + 1 once these MMAs have read it
-                if (q + 1 < ntiles) {
-                    if (!tc::mbar_wait(tc::smem_u32(empty), q & 1, s_abort)) {
+                tc::mma_commit(tc::smem_u32(&empty[b]));
+                tc::mma_commit(tc::smem_u32(&tfull[b]));
+                // refill the B stage once these MMAs have read it
+                if (loaded < ntiles) {
+                    if (!tc::mbar_wait(tc::smem_u32(&empty[b]), round & 1, s_abort)) {
                         fail(11);
                         break;
                     }
-                    load_b(q + 1);
-                    loaded = q + 2;
+                    load_b(loaded++);
                 }
             }
             tc::mma_commit(tc::smem_u32(drain));
@@ -558,13 +605,15 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 fail(15);
             // let the copies still in flight land before the CTA goes away
             tc::mbar_wait(ab, 0, nullptr);
-            if (*s_abort && loaded > 0)
-                tc::mbar_wait(tc::smem_u32(full), (loaded - 1) & 1, nullptr);
+            if (*s_abort)
+                for (int q = max(0, loaded - NB); q < loaded; q++)
+                    tc::mbar_wait(tc::smem_u32(&full[q % NB]), (q / NB) & 1, nullptr);
         }
     } else {
         // ---- epilogue: the warp's r1 points of each N tile, 32 r2 points ----------------
         constexpr int WP = Cfg::kWarpPts;
-        const int quarter = warp & 3, pt0 = (warp >> 2) * WP;
+        const int quarter = warp & 3, buf = NB == 1 ? 0 : warp >> 2;
+        const int pt0 = NB == 1 ? (warp >> 2) * WP : 0;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         const int j = m0 + quarter * 32 + lane;
         const bool jok = j < P.n2;
@@ -583,24 +632,24 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         const float sa = F64 ? 0.f : pow2f(ea);
         const df::D a = df::make(P.a_ee_hi, P.a_ee_lo);
-        for (int q = 0; q < ntiles; q++) {
-            if (!tc::mbar_wait(tc::smem_u32(tfull), q & 1, s_abort)) {
+        for (int q = buf; q < ntiles; q += NB) {
+            if (!tc::mbar_wait(tc::smem_u32(&tfull[buf]), (q / NB) & 1, s_abort)) {
                 fail(16);
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t cb = tbase + lane_off + (uint32_t)(R * pt0);
+            const uint32_t cb = tbase + lane_off + (uint32_t)(BN * S * buf + R * pt0);
             const int i0 = (t_begin + q) * Cfg::kPts + pt0;  // r1 row of the tile
             if constexpr (F64) {
                 double V[WP * R];
                 float lo[WP * R];
 #pragma unroll
                 for (int c = 0; c < WP * R; c += 8)
-                    read_f64_8<S>(cb + (uint32_t)c, Q.eb + (int64_t)i0 * R + c, ea, V + c, lo + c);
+                    read_f64_8<S, BN>(cb + (uint32_t)c, Q.eb + (int64_t)i0 * R + c, ea, V + c, lo + c);
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
-                    tc::mbar_arrive(tc::smem_u32(tempty));
+                    tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
 #pragma unroll
                 for (int p = 0; p < WP; p++)
                     if (jok && i0 + p < P.n1b)
@@ -613,7 +662,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
-                    tc::mbar_arrive(tc::smem_u32(tempty));
+                    tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
                 if (jok && i0 < P.n1b) {
                     df::D V[R];
 #pragma unroll
@@ -868,9 +917,10 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     }
     CUtensorMap ta, tb;
     CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)m.slices * plan.AF.Mpad, plan.AF.Kpad, kBM));
-    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)m.slices * B.Mpad, B.Kpad, kPairBN));
+    const int bn = m.fp64 ? 32 : kPairBN;
+    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)m.slices * B.Mpad, B.Kpad, bn));
     Q.tiles_m = plan.AF.Mpad / kBM;
-    Q.tiles_n = B.Mpad / kPairBN;
+    Q.tiles_n = B.Mpad / bn;
     Q.chunk = 1;
     Q.Mpad = plan.AF.Mpad;
     Q.Npad = B.Mpad;

@@ -83,14 +83,15 @@ __global__ void expand_pairs_kernel(int64_t rows, int nA, const double *__restri
 // (c,d).  With u+- = H[p, q] +- N[p, l(q)] and w+- = H[q, p] +- N[q, l(p)] for pairs a >= b
 // and c >= d, the pair of pairs gives the four elements
 //   (a,b),(c,d): u+ + w+    (a,b),(d,c): u- + w+    (b,a),(c,d): u+ + w-    (b,a),(d,c): u- + w-
-// (one where the indices coincide).  One block takes 16 a x 16 b x 8 c and walks d: the two
+// (one where the indices coincide).  One block takes 16 a x 16 b x 4 c and walks d: the two
 // orientations of H and N are staged through shared memory, so that reads run along p or
-// along q (64-byte runs and longer) and both (a,b) and (b,a) rows are written in 128-byte
-// runs.  Bound by HBM: H and N are read twice, 8 B written per element.  180 AOs: 20.5 ms
-// with one 32 x 32 tile of A per block and a gather per element, 3.5 ms so.
+// along q (32-byte runs and longer) and both (a,b) and (b,a) rows are written in 128-byte
+// runs.  Bound by HBM and L2: H and N are read two to four times, 8 B written per element.
+// 180 AOs: 20.5 ms with one 32 x 32 tile of A per block and a gather per element, 6.4 ms so
+// (8 c per block: 6.9).
 // Columns col = c + nA d with t0 <= d < t1 are written (out holds t0 first).  PSQT: element
 // (p,q,s,t) goes where (p,s,q,t) would.
-constexpr int kAsmA = 16, kAsmC = 8;
+constexpr int kAsmA = 16, kAsmC = 4;
 constexpr int kAsmRow = kAsmA + 1;                    // doubles per b of a tile
 constexpr int kAsmPlane = kAsmA * kAsmRow + 2;        // ... per c (spreads c over the banks)
 constexpr int kAsmTile = kAsmC * kAsmPlane;
@@ -124,7 +125,7 @@ assemble_int2e_kernel(int nA, const double *__restrict__ H, const double *__rest
         // all of a thread's loads are issued before the first is stored: along p, thread =
         // (a, b) and one c each; along q, thread = (c, one of 32 pairs) and 8 pairs
         double vh[kAsmC], vn[kAsmC], wh[kAsmC], wn[kAsmC];
-        const int a = a0 + lo, b = b0 + hi, cq = c0 + (threadIdx.x & 7);
+        const int a = a0 + lo, b = b0 + hi, cq = c0 + (int)(threadIdx.x % kAsmC);
         const int64_t p = tri_index(a, b, nA), q = tri_index(cq, d, nA);
         const bool p_ok = a < nA && b <= a, q_ok = cq < c_end && cq >= d;
 #pragma unroll
@@ -133,7 +134,7 @@ assemble_int2e_kernel(int nA, const double *__restrict__ H, const double *__rest
             const bool ok = p_ok && c < c_end && c >= d;
             vh[k] = ok ? H[p + np * tri_index(c, d, nA)] : 0.0;
             vn[k] = ok && c > d ? N[p + np * stri_index(c, d, nA)] : 0.0;
-            const int pr = (int)(threadIdx.x >> 3) + 32 * k, pa = a0 + (pr & 15), pb = b0 + (pr >> 4);
+            const int pr = (int)(threadIdx.x / kAsmC) + kAsmA * kAsmA / kAsmC * k, pa = a0 + (pr & 15), pb = b0 + (pr >> 4);
             const bool okq = q_ok && pa < nA && pb <= pa;
             wh[k] = okq ? H[q + np * tri_index(pa, pb, nA)] : 0.0;
             wn[k] = okq && pa > pb ? N[q + np * stri_index(pa, pb, nA)] : 0.0;
@@ -144,8 +145,8 @@ assemble_int2e_kernel(int nA, const double *__restrict__ H, const double *__rest
             const int o = k * kAsmPlane + hi * kAsmRow + lo;
             hp[o] = vh[k];
             np_[o] = vn[k];
-            const int pr = (int)(threadIdx.x >> 3) + 32 * k;
-            const int oq = (int)(threadIdx.x & 7) * kAsmPlane + (pr >> 4) * kAsmRow + (pr & 15);
+            const int pr = (int)(threadIdx.x / kAsmC) + kAsmA * kAsmA / kAsmC * k;
+            const int oq = (int)(threadIdx.x % kAsmC) * kAsmPlane + (pr >> 4) * kAsmRow + (pr & 15);
             hq[oq] = wh[k];
             nq[oq] = wn[k];
         }
