@@ -13,6 +13,8 @@
 //   * X is accumulated per r1 tile with beta = 0, so r1 tiling is exact (the
 //     reference keeps beta = 1 across r1 passes, src/build_int2_grad1_u12_ao.cu:166);
 //   * errors are returned as status codes, never exit().
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <cmath>
@@ -146,6 +148,35 @@ static void host_copy(void *dst, const void *src, size_t bytes)
         t.join();
 }
 
+// Touches every page of an output that is about to be written, on a few threads: fresh
+// caller memory then has its pages when the copy comes (a device copy into 256 MB without
+// them took 11.8 ms, into present ones 1.5), while the device still computes.
+static void touch_pages(void *dst, size_t bytes)
+{
+    static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    const size_t kChunk = (size_t)8 << 20;
+    static const int kMaxThreads =
+        (int)std::max(2u, std::min(8u, std::thread::hardware_concurrency() / 2));
+    auto touch = [=](size_t a, size_t b) {
+        for (size_t o = a; o < b; o += page)
+            ((volatile char *)dst)[o] = 0;
+        if (b > a)
+            ((volatile char *)dst)[b - 1] = 0;
+    };
+    const int n = (int)std::min<size_t>(kMaxThreads, bytes / kChunk);
+    if (n <= 1) {
+        touch(0, bytes);
+        return;
+    }
+    const size_t per = (bytes + n - 1) / n;
+    std::vector<std::thread> th;
+    for (int k = 1; k < n; k++)
+        th.emplace_back([=] { touch(std::min(bytes, k * per), std::min(bytes, (k + 1) * per)); });
+    touch(0, per);
+    for (auto &t : th)
+        t.join();
+}
+
 // True when the device can copy into p asynchronously (pinned, registered or managed).
 static bool async_host_ptr(const void *p)
 {
@@ -212,6 +243,10 @@ int make_engine(int dev, Engine **out)
     E->device = dev;
     E->n_sm = prop.multiProcessorCount;
     E->max_threads_per_block = prop.maxThreadsPerBlock;
+    int host_pages = 0;
+    CUTC_CUDA_TRY(cudaDeviceGetAttribute(&host_pages,
+                                         cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev));
+    E->host_pages = host_pages != 0;
     for (int k = 0; k < 3; k++)
         E->max_grid[k] = prop.maxGridSize[k];
     cudaError_t e = cudaStreamCreateWithFlags(&E->stream, cudaStreamNonBlocking);
@@ -376,7 +411,7 @@ static int validate(const Request &R)
 enum Slot {
     S_R1, S_WR1, S_R2, S_WR2, S_RN, S_AOS1, S_AOS2, S_COEF, S_EXPS, S_OFF,
     S_T1, S_F2, S_P, S_G, S_XP, S_S0, S_SL, S_H, S_N, S_XOUT, S_XOUT1, S_IOUT, S_IOUT1,
-    S_R2D, S_F2D, S_POLY, S_BASIS,
+    S_R2D, S_F2D, S_POLY, S_BASIS, S_SMALL,
     S_SPLIT0,      // split-form slots follow
     S_PAIRTC = 80  // the tensor-core pair terms' slots
 };
@@ -571,12 +606,43 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     const double *d_rn = nullptr, *d_aos1 = nullptr, *d_aos2v = nullptr;
     bool aos1_deferred = false;
     void *p;
-    auto put = [&](int slot, const void *h, size_t bytes, const double **dst) -> int {
+    // Small host arrays go to the device together, in one copy from pinned memory (a copy
+    // from pageable memory holds the caller for 13 us, whatever its size).
+    constexpr size_t kSmallInput = (size_t)128 << 10;
+    struct Small {
+        const void *src;
+        size_t bytes;
+        const void **dst;
+    };
+    std::vector<Small> small;
+    auto put = [&](int slot, const void *h, size_t bytes, const void **dst) -> int {
+        if (bytes <= kSmallInput) {
+            small.push_back({h, bytes, dst});
+            return CUTC_OK;
+        }
         CUTC_TRY(W.get(slot, bytes, &p));
         CUTC_CUDA_TRY(cudaMemcpyAsync(p, h, bytes, cudaMemcpyHostToDevice, st));
-        *dst = (const double *)p;
+        *dst = p;
         return CUTC_OK;
     };
+    auto put_small = [&]() -> int {
+        size_t total = 0;
+        for (const Small &a : small)
+            total += (a.bytes + 255) & ~(size_t)255;
+        void *h, *d;
+        CUTC_TRY(E->pinned.get(4, total, &h));
+        CUTC_TRY(W.get(S_SMALL, total, &d));
+        size_t o = 0;
+        for (const Small &a : small) {
+            if (a.bytes)
+                memcpy((char *)h + o, a.src, a.bytes);
+            *a.dst = (char *)d + o;
+            o += (a.bytes + 255) & ~(size_t)255;
+        }
+        CUTC_CUDA_TRY(cudaMemcpyAsync(d, h, total, cudaMemcpyHostToDevice, st));
+        return CUTC_OK;
+    };
+    auto in = [](const double **d) { return (const void **)d; };
     const bool in_dev = R.device_pointers || R.in_device;
     const bool out_dev = R.device_pointers || R.out_device;
     if (in_dev) {
@@ -584,13 +650,15 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         d_aos1 = R.aos1;
         d_aos2v = R.aos2;  // component 0 is the first n2*nA block
     } else {
-        CUTC_TRY(put(S_R1, R.r1, 3 * (size_t)n1 * 8, &d_r1));
+        CUTC_TRY(put(S_R1, R.r1, 3 * (size_t)n1 * 8, in(&d_r1)));
         if (R.wr1)
-            CUTC_TRY(put(S_WR1, R.wr1, (size_t)n1 * 8, &d_wr1));
-        CUTC_TRY(put(S_R2, R.r2, 3 * (size_t)n2 * 8, &d_r2));
-        CUTC_TRY(put(S_WR2, R.wr2, (size_t)n2 * 8, &d_wr2));
-        CUTC_TRY(put(S_RN, R.rn, 3 * (size_t)nN * 8, &d_rn));
-        if (R.aos1 && !R.x_only) {
+            CUTC_TRY(put(S_WR1, R.wr1, (size_t)n1 * 8, in(&d_wr1)));
+        CUTC_TRY(put(S_R2, R.r2, 3 * (size_t)n2 * 8, in(&d_r2)));
+        CUTC_TRY(put(S_WR2, R.wr2, (size_t)n2 * 8, in(&d_wr2)));
+        CUTC_TRY(put(S_RN, R.rn, 3 * (size_t)nN * 8, in(&d_rn)));
+        if (R.aos1 && !R.x_only && R.ld1 <= n1 && 4 * (size_t)n1 * nA * 8 <= kSmallInput) {
+            CUTC_TRY(put(S_AOS1, R.aos1, 4 * (size_t)n1 * nA * 8, in(&d_aos1)));
+        } else if (R.aos1 && !R.x_only) {
             // the AO values on r1, the largest input, are read only by the int_2e blocks:
             // they are copied on the transfer stream once the first tile is queued
             CUTC_TRY(W.get(S_AOS1, 4 * (size_t)n1 * nA * 8, &p));
@@ -599,8 +667,15 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         }
         // only the value component of aos_data2 is used (src/long_range_integ.cu:30-35)
         if (R.aos2)
-            CUTC_TRY(put(S_AOS2, R.aos2, (size_t)n2 * nA * 8, &d_aos2v));
+            CUTC_TRY(put(S_AOS2, R.aos2, (size_t)n2 * nA * 8, in(&d_aos2v)));
     }
+    const int nt = (int)exps.size();
+    const double *d_coef = nullptr;
+    const int *d_exps = nullptr, *d_off = nullptr;
+    CUTC_TRY(put(S_COEF, coef.data(), coef.size() * 8, in(&d_coef)));
+    CUTC_TRY(put(S_EXPS, exps.data(), exps.size() * 4, (const void **)&d_exps));
+    CUTC_TRY(put(S_OFF, off.data(), off.size() * 4, (const void **)&d_off));
+    CUTC_TRY(put_small());
     if ((!R.aos1 && !R.x_only) || !R.aos2) {
         // AO values (and r1 gradients) from the basis, on the device
         BasisDev B;
@@ -619,20 +694,6 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     // leading dimension of the AO values on r1 on the device: a window of a caller's
     // device array keeps the caller's stride; uploaded or evaluated arrays are packed
     const int64_t ld_a1 = (in_dev && R.aos1 && R.ld1 > 0) ? R.ld1 : n1;
-    const int nt = (int)exps.size();
-    double *d_coef;
-    int *d_exps, *d_off;
-    CUTC_TRY(W.get(S_COEF, std::max<size_t>(1, coef.size()) * 8, &p));
-    d_coef = (double *)p;
-    CUTC_TRY(W.get(S_EXPS, std::max<size_t>(1, exps.size()) * 4, &p));
-    d_exps = (int *)p;
-    CUTC_TRY(W.get(S_OFF, off.size() * 4, &p));
-    d_off = (int *)p;
-    if (nt) {
-        CUTC_CUDA_TRY(cudaMemcpyAsync(d_coef, coef.data(), coef.size() * 8, cudaMemcpyHostToDevice, st));
-        CUTC_CUDA_TRY(cudaMemcpyAsync(d_exps, exps.data(), exps.size() * 4, cudaMemcpyHostToDevice, st));
-    }
-    CUTC_CUDA_TRY(cudaMemcpyAsync(d_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice, st));
     CUTC_CUDA_TRY(cudaEventRecord(E->ev[1], st));
 
     // ---- r1 tiling ---------------------------------------------------------
@@ -765,15 +826,20 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     StreamsDrain drain{st, E->xfer};
     cudaEvent_t ready[2] = {E->ev[3], E->ev[4]}, done[2] = {E->ev[9], E->ev[10]};
     bool busy[2] = {false, false};
+    // Where the device reads and writes pageable memory through the host's page tables
+    // (Grace), pageable outputs are copied into directly, at the pinned rate (180 GB/s; the
+    // staged copy's host threads reach 15 each), by a copy that holds the calling thread
+    // until it is done: it is issued when the rows are ready, with the next work queued.
     const bool x_direct = out_dev || R.i_only || async_host_ptr(R.X);
     const bool i_direct = out_dev || R.x_only || async_host_ptr(R.I);
+    const bool x_held = !x_direct && E->host_pages, i_held = !i_direct && E->host_pages;
     double *hpin_x[2] = {nullptr, nullptr}, *hpin_i[2] = {nullptr, nullptr};
     for (int k = 0; k < 2 && !out_dev; k++) {
-        if (!x_direct) {
+        if (!x_direct && !x_held) {
             CUTC_TRY(E->pinned.get(k, (size_t)R.x_components * n1t * nA2 * 8, &p));
             hpin_x[k] = (double *)p;
         }
-        if (!i_direct) {
+        if (!i_direct && !i_held) {
             CUTC_TRY(E->pinned.get(2 + k, (size_t)slab * nA2 * 8, &p));
             hpin_i[k] = (double *)p;
         }
@@ -786,6 +852,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         const int b = tile & 1;
         int64_t i0, nb;
         tile_rows(tile, &i0, &nb);
+        if (x_held)
+            return CUTC_OK;  // in finish_x
         CUTC_CUDA_TRY(cudaStreamWaitEvent(E->xfer, ready[b], 0));
         if (x_direct) {
             for (int m = 0; m < R.x_components; m++)
@@ -801,12 +869,24 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         busy[b] = true;
         return CUTC_OK;
     };
-    auto finish_x = [&](int tile) -> int {  // pinned -> pageable caller memory
+    auto finish_x = [&](int tile) -> int {  // into pageable caller memory
         if (x_direct)
             return CUTC_OK;
         const int b = tile & 1;
         int64_t i0, nb;
         tile_rows(tile, &i0, &nb);
+        if (x_held) {
+            for (int m = 0; m < R.x_components; m++)
+                touch_pages(R.X + ((int64_t)m * n1 + i0) * nA2, (size_t)nb * nA2 * 8);
+            CUTC_CUDA_TRY(cudaEventSynchronize(ready[b]));
+            for (int m = 0; m < R.x_components; m++)
+                CUTC_CUDA_TRY(cudaMemcpyAsync(R.X + ((int64_t)m * n1 + i0) * nA2,
+                                              stage_x[b] + (int64_t)m * nb * nA2,
+                                              (size_t)nb * nA2 * 8, cudaMemcpyDeviceToHost, E->xfer));
+            CUTC_CUDA_TRY(cudaEventRecord(done[b], E->xfer));
+            busy[b] = true;
+            return CUTC_OK;
+        }
         CUTC_CUDA_TRY(cudaEventSynchronize(done[b]));
         for (int m = 0; m < R.x_components; m++)
             host_copy(R.X + ((int64_t)m * n1 + i0) * nA2, hpin_x[b] + (int64_t)m * nb * nA2,
@@ -948,7 +1028,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         }
         if (tev)
             CUTC_CUDA_TRY(cudaEventRecord(tev[5], st));
-        // the previous tile's rows, pinned -> pageable, while the device works on this one
+        // the previous tile's rows into pageable memory, while the device works on this one
         if (!out_dev && !R.i_only && tile > 0)
             CUTC_TRY(finish_x(tile - 1));
         if (i0 + nb == blk0 + blk_rows) {  // next block
@@ -979,6 +1059,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             const int b = slab_no & 1;
             int64_t c0, c1;
             slab_cols(slab_no, &c0, &c1);
+            if (i_held)
+                return CUTC_OK;  // in finish_i
             CUTC_CUDA_TRY(cudaStreamWaitEvent(E->xfer, ready[b], 0));
             CUTC_CUDA_TRY(cudaMemcpyAsync(i_direct ? R.I + c0 * nA2 : hpin_i[b], stage_i[b],
                                           (size_t)(c1 - c0) * nA2 * 8, cudaMemcpyDeviceToHost,
@@ -993,6 +1075,16 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             const int b = slab_no & 1;
             int64_t c0, c1;
             slab_cols(slab_no, &c0, &c1);
+            if (i_held) {
+                touch_pages(R.I + c0 * nA2, (size_t)(c1 - c0) * nA2 * 8);
+                CUTC_CUDA_TRY(cudaEventSynchronize(ready[b]));
+                CUTC_CUDA_TRY(cudaMemcpyAsync(R.I + c0 * nA2, stage_i[b],
+                                              (size_t)(c1 - c0) * nA2 * 8, cudaMemcpyDeviceToHost,
+                                              E->xfer));
+                CUTC_CUDA_TRY(cudaEventRecord(done[b], E->xfer));
+                ibusy[b] = true;
+                return CUTC_OK;
+            }
             CUTC_CUDA_TRY(cudaEventSynchronize(done[b]));
             host_copy(R.I + c0 * nA2, hpin_i[b], (size_t)(c1 - c0) * nA2 * 8);
             return CUTC_OK;

@@ -13,14 +13,14 @@ namespace cutc {
 
 constexpr int kNumEvents = 12;
 
-// Grow-only pinned host buffers: outputs bound for pageable caller memory leave
-// the device through them.
+// Grow-only pinned host buffers: outputs bound for pageable caller memory leave the device
+// through them where it cannot write that memory itself, and small inputs enter it.
 struct PinnedPool {
     struct Buf {
         void *p = nullptr;
         size_t cap = 0;
     };
-    Buf bufs[4];
+    Buf bufs[5];  // X (2), int_2e (2), a call's small inputs
     int get(int k, size_t bytes, void **out);
     void release();
 };
@@ -62,6 +62,7 @@ struct Engine {
     int n_sm = 0;
     int max_threads_per_block = 1024;
     int max_grid[3] = {0, 0, 0};
+    bool host_pages = false;  // pageable host memory is read and written through its page tables
     cudaStream_t stream = nullptr;
     cudaStream_t xfer = nullptr;  // device-to-host copies of finished r1 tiles
     cudaEvent_t ev[kNumEvents];

@@ -11,7 +11,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <vector>
 
 #include "common.cuh"
 #include "products.cuh"
@@ -133,32 +132,27 @@ size_t split_fixed_bytes(const Request &R)
     return b;
 }
 
-static int upload_pairs(Workspace &W, int slot, cudaStream_t st, int nA, bool strict, int2 **out)
+// The AO pairs (a, b) in the packed order of tri_index (a >= b) or stri_index (a > b).
+__global__ void pairs_kernel(int nA, int strict, int2 *__restrict__ out)
 {
-    std::vector<int2> v;
-    for (int b = 0; b < nA; b++)
-        for (int a = strict ? b + 1 : b; a < nA; a++)
-            v.push_back(make_int2(a, b));  // packed order of tri_index / stri_index
-    void *p;
-    CUTC_TRY(W.get(slot, std::max<size_t>(1, v.size()) * sizeof(int2), &p));
-    if (!v.empty())
-        CUTC_CUDA_TRY(cudaMemcpyAsync(p, v.data(), v.size() * sizeof(int2), cudaMemcpyHostToDevice, st));
-    CUTC_CUDA_TRY(cudaStreamSynchronize(st));  // v goes out of scope
-    *out = (int2 *)p;
-    return CUTC_OK;
+    const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y;
+    if (a < nA && a >= b + strict)
+        out[strict ? stri_index(a, b, nA) : tri_index(a, b, nA)] = make_int2(a, b);
 }
 
-#define CUTC_SLICES_DISPATCH(S_, CALL)                                         \
-    switch (S_) {                                                              \
-    case 3: { constexpr int S = 3; CALL; } break;                              \
-    case 4: { constexpr int S = 4; CALL; } break;                              \
-    case 5: { constexpr int S = 5; CALL; } break;                              \
-    case 6: { constexpr int S = 6; CALL; } break;                              \
-    case 7: { constexpr int S = 7; CALL; } break;                              \
-    default:                                                                   \
-        cutc_set_error(CUTC_ERR_INVALID, "unsupported slice count %d", S_);    \
-        return CUTC_ERR_INVALID;                                               \
-    }
+static int make_pairs(Workspace &W, int slot, cudaStream_t st, int nA, bool strict, int2 **out)
+{
+    const int64_t n = strict ? n_strict_pairs(nA) : n_pairs(nA);
+    void *p;
+    CUTC_TRY(W.get(slot, std::max<size_t>(1, n) * sizeof(int2), &p));
+    *out = (int2 *)p;
+    if (n == 0)
+        return CUTC_OK;
+    pairs_kernel<<<dim3(ceil_div(nA, 128), nA), 128, 0, st>>>(nA, strict, *out);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
 
 // Row scales of an operand.
 static int scale_slot(Workspace &W, int slot, int rows, int **sc)
@@ -182,8 +176,8 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
     CUTC_TRY(W.get(slot0 + SS_ERR, 64, &p));
     sp.err = (int *)p;
     CUTC_CUDA_TRY(cudaMemsetAsync(sp.err, 0, 4, st));
-    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_SYM, st, R.nA, false, &sp.pairs_sym));
-    CUTC_TRY(upload_pairs(W, slot0 + SS_PAIRS_ANTI, st, R.nA, true, &sp.pairs_anti));
+    CUTC_TRY(make_pairs(W, slot0 + SS_PAIRS_SYM, st, R.nA, false, &sp.pairs_sym));
+    CUTC_TRY(make_pairs(W, slot0 + SS_PAIRS_ANTI, st, R.nA, true, &sp.pairs_anti));
     CUTC_TRY(scale_slot(W, slot0 + SS_AX_SC, np, &sp.sc_ax));
     CUTC_TRY(scale_slot(W, slot0 + SS_BX_SC, (int)(4 * n1t), &sp.sc_bx));
     sp.k_panel = panel_k(R.n2, np, R.k_split);
