@@ -16,8 +16,8 @@
 // (FP64 results); later diagonals round at 2^-27 2^-24 and 2^-36 2^-24 of the row scales.
 //
 // A = the F slices of 128 r2 points, all of K, loaded once per CTA; B = the coefficient
-// slices in tiles of 64 rows (four r1 points, or two; 32 rows for FP64 results), streamed;
-// one stacked accumulator set in tensor memory (two for FP64 results).  The tensor-core work of a tile is a small part of its epilogue, so
+// slices in tiles of 64 rows (four r1 points, or two; one point for FP64 results), streamed;
+// one stacked accumulator set in tensor memory (four or two for FP64 results).  The tensor-core work of a tile is a small part of its epilogue, so
 // one B stage per accumulator set suffices: the next tile's MMAs run as soon as the
 // epilogue has read the accumulators, and one control warp issues both the TMA loads and
 // the MMAs.
@@ -94,15 +94,14 @@ template <int S, int KB, int R, bool F64>
 struct PairTcCfg {
     // Double-float: one accumulator set, and a warp per lane quarter and point of a tile
     // (16 warps with 16 rows, four per SM sub-partition, to hide the latency of their
-    // dependent chains; 8 with 32 rows).  FP64: tiles of 32 rows in two accumulator sets,
-    // each with four warps of its own that take all points of its tiles, so that one set's
-    // integer work runs beside the other's FP64 work (with one set, every warp waits for
-    // the same tile and the FP64 pipe idled 40% of the time).
-    static constexpr int kBN = F64 ? 32 : kPairBN;
-    static constexpr int kBufs = F64 ? 2 : 1;
+    // dependent chains; 8 with 32 rows).  FP64: tiles of one point in four accumulator sets
+    // (two with 32 rows), each with four warps of its own, so that one set's integer work
+    // runs beside another's FP64 work (with one set, every warp waits for the same tile and
+    // the FP64 pipe idled 40% of the time).
+    static constexpr int kBN = F64 ? R : kPairBN;
+    static constexpr int kBufs = F64 ? 64 / R : 1;
     static constexpr int kPts = kBN / R;
-    static constexpr int kEpiWarps = F64 ? 8 : 4 * kPts;
-    static constexpr int kWarpPts = F64 ? kPts : 1;
+    static constexpr int kEpiWarps = F64 ? 4 * kBufs : 4 * kPts;
     static constexpr int kBufWarps = kEpiWarps / kBufs;  // epilogue warps of a buffer
     static constexpr int kCtlWarp = kEpiWarps;       // TMA loads and MMAs, lane 0
     static constexpr int kThreads = (kEpiWarps + 1) * 32;
@@ -591,9 +590,11 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 tc::mma_commit(tc::smem_u32(&empty[b]));
                 tc::mma_commit(tc::smem_u32(&tfull[b]));
-                // refill the B stage once these MMAs have read it
-                if (loaded < ntiles) {
-                    if (!tc::mbar_wait(tc::smem_u32(&empty[b]), round & 1, s_abort)) {
+                // refill a B stage once its MMAs have read it: with several stages, that of
+                // the tile before, so that this wait does not hold up the next MMAs
+                const int r = NB > 1 ? q - 1 : q;
+                if (r >= 0 && loaded < ntiles) {
+                    if (!tc::mbar_wait(tc::smem_u32(&empty[r % NB]), (r / NB) & 1, s_abort)) {
                         fail(11);
                         break;
                     }
@@ -611,9 +612,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else {
         // ---- epilogue: the warp's r1 points of each N tile, 32 r2 points ----------------
-        constexpr int WP = Cfg::kWarpPts;
         const int quarter = warp & 3, buf = NB == 1 ? 0 : warp >> 2;
-        const int pt0 = NB == 1 ? (warp >> 2) * WP : 0;
+        const int pt0 = NB == 1 ? warp >> 2 : 0;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         const int j = m0 + quarter * 32 + lane;
         const bool jok = j < P.n2;
@@ -641,19 +641,17 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const uint32_t cb = tbase + lane_off + (uint32_t)(BN * S * buf + R * pt0);
             const int i0 = (t_begin + q) * Cfg::kPts + pt0;  // r1 row of the tile
             if constexpr (F64) {
-                double V[WP * R];
-                float lo[WP * R];
+                double V[R];
+                float lo[R];
 #pragma unroll
-                for (int c = 0; c < WP * R; c += 8)
+                for (int c = 0; c < R; c += 8)
                     read_f64_8<S, BN>(cb + (uint32_t)c, Q.eb + (int64_t)i0 * R + c, ea, V + c, lo + c);
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
                     tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-#pragma unroll
-                for (int p = 0; p < WP; p++)
-                    if (jok && i0 + p < P.n1b)
-                        pair_f64<R>(Q, i0 + p, j, V + p * R, lo + p * R, dx2, dy2, dz2);
+                if (jok && i0 < P.n1b)
+                    pair_f64<R>(Q, i0, j, V, lo, dx2, dy2, dz2);
             } else {
                 uint64_t H[R / 16][8], L[R / 16][8], L2[R / 16][8];
 #pragma unroll
@@ -917,7 +915,7 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     }
     CUtensorMap ta, tb;
     CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)m.slices * plan.AF.Mpad, plan.AF.Kpad, kBM));
-    const int bn = m.fp64 ? 32 : kPairBN;
+    const int bn = m.fp64 ? m.rows : kPairBN;
     CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)m.slices * B.Mpad, B.Kpad, bn));
     Q.tiles_m = plan.AF.Mpad / kBM;
     Q.tiles_n = B.Mpad / bn;
