@@ -307,7 +307,8 @@ int fp64_contract_begin(Workspace &W, cudaStream_t st, int **flags)
 {
     void *p;
     CUTC_TRY(W.get(C_FLAGS, 64, &p));
-    *flags = (int *)p;  // [0]: a wait gave up, [1]: an operand is not finite
+    *flags = (int *)p;  // [0]: a wait gave up, [1]: an operand of the contraction at hand is
+                        // not finite
     CUTC_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
     return CUTC_OK;
 }
@@ -343,19 +344,19 @@ static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, in
     CUTC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, st));
     const SrcDense sa{A, lda}, sb{B, ldb};
     if (a_kmajor)
-        CUTC_TRY(row_scales(st, sa, M, K, n_mod, sca, bad));
+        CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca, bad));
     else
         CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
-    CUTC_TRY(row_scales(st, sb, N, K, n_mod, scb, bad));
+    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad));
     return modular_contract(
         st, W, C_RB, C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, false, sca, scb, out,
         err, bad,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
-            return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, k0, kp, o.pitch, sca, o.p)
+            return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, K, k0, kp, o.pitch, sca, o.p, bad)
                             : residue_cols<n_mod>(st, A, lda, M, k0, kp, o.pitch, sca, o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-            return residue_rows<n_mod>(st, sb, n0, nc, k0, kp, o.pitch, scb, o.p);
+            return residue_rows<n_mod>(st, sb, n0, nc, K, k0, kp, o.pitch, scb, o.p, bad);
         });
 }
 

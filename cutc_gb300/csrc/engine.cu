@@ -975,21 +975,20 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         if (R.i_only) {
             // X stays packed in the int_2e block and is not returned
         } else if (out_dev) {
-            for (int m = 0; m < R.x_components; m++)
-                CUTC_TRY(launch_expand_pairs(st, nb, nA, d_Xt + ((int64_t)m * blk_rows + ib) * np,
-                                             np, R.X + ((int64_t)m * n1 + i0) * nA2));
+            CUTC_TRY(launch_expand_pairs(st, nb, R.x_components, nA, d_Xt + (int64_t)ib * np, np,
+                                         (int64_t)blk_rows * np, R.X + (int64_t)i0 * nA2,
+                                         (int64_t)n1 * nA2));
         } else {
             const int b = tile & 1;
             if (busy[b])
                 CUTC_CUDA_TRY(cudaStreamWaitEvent(st, done[b], 0));
-            for (int m = 0; m < R.x_components; m++)
-                CUTC_TRY(launch_expand_pairs(st, nb, nA, d_Xt + ((int64_t)m * blk_rows + ib) * np,
-                                             np, stage_x[b] + (int64_t)m * nb * nA2));
+            CUTC_TRY(launch_expand_pairs(st, nb, R.x_components, nA, d_Xt + (int64_t)ib * np, np,
+                                         (int64_t)blk_rows * np, stage_x[b], (int64_t)nb * nA2));
             CUTC_CUDA_TRY(cudaEventRecord(ready[b], st));
             CUTC_TRY(copy_x(tile));
         }
         if (!R.i_only)
-            note_launches(R.x_components);
+            note_launches(1);
 
         // the block's share of int_2e once its last tile is in
         // (src/build_int_2e_ao.cu:60-67 and 97-104, packed):

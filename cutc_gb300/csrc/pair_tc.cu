@@ -863,8 +863,11 @@ static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorM
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
         attr_done.fetch_or(bit);
     }
-    // about eight CTAs per SM, each walking a run of N tiles with its F tile resident
-    const int64_t want = 8 * (int64_t)n_sm;
+    // CTAs that each walk a run of N tiles with their F tile resident: about eight per SM,
+    // down to one per SM where that leaves a CTA fewer than 16 tiles to hide its set-up
+    // behind (210 x 805 pairs in FP64: 47 us in 735 CTAs of 2 tiles)
+    const int64_t all = (int64_t)Q.tiles_m * Q.tiles_n;
+    const int64_t want = std::min<int64_t>(8, std::max<int64_t>(1, all / (16 * (int64_t)n_sm))) * n_sm;
     const int64_t chunks = std::max<int64_t>(
         1, std::min<int64_t>(Q.tiles_n, (want + Q.tiles_m - 1) / Q.tiles_m));
     Q.chunk = (int)((Q.tiles_n + chunks - 1) / chunks);

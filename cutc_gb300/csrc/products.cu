@@ -57,19 +57,19 @@ __global__ void antisym_products_kernel(int n, int nA, const double *__restrict_
     }
 }
 
-// X[(row) * nA^2 + a + nA b] = Xp[(row) * ldp + tri(max(a,b), min(a,b))] for
-// rows = m * n1 + i of the requested components.
-__global__ void expand_pairs_kernel(int64_t rows, int nA, const double *__restrict__ Xp, int64_t ldp,
-                                    double *__restrict__ X)
+// X[m * xs + i * nA^2 + a + nA b] = Xp[m * ps + i * ldp + tri(max(a,b), min(a,b))] for rows
+// i < n of the requested components m.
+__global__ void expand_pairs_kernel(int n, int64_t rows, int nA, const double *__restrict__ Xp,
+                                    int64_t ldp, int64_t ps, double *__restrict__ X, int64_t xs)
 {
-    const int64_t nA2 = (int64_t)nA * nA;
     const int64_t row = blockIdx.y + (int64_t)gridDim.y * blockIdx.z;
     if (row >= rows)
         return;
-    const double *src = Xp + row * ldp;
-    double *dst = X + row * nA2;
     // nA^2 < 2^30 (the build's argument checks): 32-bit index arithmetic, one division
-    const int n2 = (int)nA2;
+    const int n2 = nA * nA;
+    const int64_t m = row / n, i = row - m * n;
+    const double *src = Xp + m * ps + i * ldp;
+    double *dst = X + m * xs + i * n2;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n2; k += gridDim.x * blockDim.x) {
         const int b = k / nA, a = k - b * nA;
         dst[k] = src[a >= b ? tri_index(a, b, nA) : tri_index(b, a, nA)];
@@ -201,9 +201,10 @@ int launch_antisym_products(cudaStream_t st, int n, int nA, const double *w, con
     return CUTC_OK;
 }
 
-int launch_expand_pairs(cudaStream_t st, int64_t rows, int nA, const double *Xp, int64_t ldp,
-                        double *X)
+int launch_expand_pairs(cudaStream_t st, int n, int comps, int nA, const double *Xp, int64_t ldp,
+                        int64_t ps, double *X, int64_t xs)
 {
+    const int64_t rows = (int64_t)n * comps;
     if (rows <= 0)
         return CUTC_OK;
     const int64_t nA2 = (int64_t)nA * nA;
@@ -212,7 +213,7 @@ int launch_expand_pairs(cudaStream_t st, int64_t rows, int nA, const double *Xp,
         gx = 64;
     unsigned gy = rows < 65535 ? (unsigned)rows : 65535u;
     unsigned gz = ceil_div(rows, gy);
-    expand_pairs_kernel<<<dim3(gx, gy, gz), 256, 0, st>>>(rows, nA, Xp, ldp, X);
+    expand_pairs_kernel<<<dim3(gx, gy, gz), 256, 0, st>>>(n, rows, nA, Xp, ldp, ps, X, xs);
     CUTC_CUDA_TRY(cudaGetLastError());
     return CUTC_OK;
 }

@@ -13,9 +13,10 @@ int launch_sym_products(cudaStream_t st, int n, int nA, const double *w, const d
 // aos[(k nA + a) ld_aos + g] is component k of AO a at grid point g
 int launch_antisym_products(cudaStream_t st, int n, int nA, const double *w, const double *aos,
                             int64_t ld_aos, double *out, int64_t ld);
-// full AO-pair rows from packed rows
-int launch_expand_pairs(cudaStream_t st, int64_t rows, int nA, const double *Xp, int64_t ldp,
-                        double *X);
+// full AO-pair rows from packed rows: n rows of each of comps components, whose packed rows
+// start ps doubles apart (ldp each) and whose full rows xs doubles apart (nA^2 each)
+int launch_expand_pairs(cudaStream_t st, int n, int comps, int nA, const double *Xp, int64_t ldp,
+                        int64_t ps, double *X, int64_t xs);
 // Columns c0 <= col < c1 of int_2e = A + A^T (column-major, nA^2 rows) from the
 // packed symmetric (H) and antisymmetric (N) parts; out holds column c0 first.
 // c0 and c1 are multiples of nA.  psqt: element (p,q,s,t) goes where (p,s,q,t) would.

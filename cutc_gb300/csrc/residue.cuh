@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "common.cuh"
 #include "digits.cuh"
@@ -218,48 +219,6 @@ row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc,
     }
 }
 
-// The same for short rows: one warp per row (a block per row leaves most of its threads
-// without work: 600 900 rows of 100 took 0.36 ms).
-constexpr int64_t kShortRow = 1024;
-template <class Src>
-__global__ void __launch_bounds__(256)
-row_scale_short_kernel(Src src, int rows, int K, float bits, int *__restrict__ sc, int *bad)
-{
-    const int lane = threadIdx.x & 31;
-    for (int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += 8 * (int64_t)gridDim.x) {
-        float m = 0.0f, ss = 0.0f;
-#pragma unroll 4
-        for (int k = lane; k < K; k += 32) {
-            const float v = src.up(r, k);
-            m = fmaxf(m, v);
-            ss = fmaf(v, v, ss);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        }
-        int s = 0;
-        if (!scale_fast(m, ss, bits, K, &s)) {  // the same in every lane
-            unsigned long long mb = 0;
-            for (int k = lane; k < K; k += 32) {
-                const unsigned long long b = abs_bits(src(r, k));
-                mb = b > mb ? b : mb;
-            }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long b = __shfl_xor_sync(0xffffffffu, mb, o);
-                mb = b > mb ? b : mb;
-            }
-            s = scale_slow(mb, bits, K);
-            if (s == kNotFinite && bad && lane == 0)
-                atomicExch(bad, 1);
-        }
-        if (lane == 0)
-            sc[r] = s;
-    }
-}
-
 // The residues of eight integers per thread, chunk[j][q] holding the 13-bit chunks j of
 // elements 2q and 2q + 1: every FP32 operation is exact.
 template <int N, int CH>
@@ -311,6 +270,47 @@ __device__ __forceinline__ void pack_chunks(const float (&v)[8][moduli::chunks(N
             chunk[j][q] = tc::f2_pack(__float_as_uint(v[2 * q][j]), __float_as_uint(v[2 * q + 1][j]));
 }
 
+// An element as its source holds it, a bound of its magnitude, and its 13-bit chunks scaled
+// by 2^s.
+template <bool DF>
+struct ValueOf {
+    using T = double;
+};
+template <>
+struct ValueOf<true> {
+    using T = float2;
+};
+
+template <class Src>
+__device__ __forceinline__ typename ValueOf<Src::kDoubleFloat>::T value_of(const Src &src, int64_t r,
+                                                                           int64_t k)
+{
+    if constexpr (Src::kDoubleFloat)
+        return src.pair(r, k);
+    else
+        return src(r, k);
+}
+
+__device__ __forceinline__ float up_of(double x) { return abs_up(x); }
+__device__ __forceinline__ float up_of(float2 x) { return fabsf(x.x) * 1.0000002f; }
+
+template <int N>
+__device__ __forceinline__ void residue_chunks(double x, int s, float (&v)[moduli::chunks(N)])
+{
+    int_chunks<moduli::chunks(N)>(x, s, v);
+}
+
+template <int N>
+__device__ __forceinline__ void residue_chunks(float2 x, int s, float (&v)[moduli::chunks(N)])
+{
+    constexpr int CH = moduli::chunks(N);
+    float d[CH];  // from the top: d[0] is chunk CH - 1
+    digits::digits_df_fp32<CH, moduli::kChunkBits>(x.x, x.y, moduli::kChunkBits * CH - 1 - s, d);
+#pragma unroll
+    for (int j = 0; j < CH; j++)
+        v[j] = d[CH - 1 - j];
+}
+
 // planes[i][r][k - k0] = residues of rint(src(r0 + r, k) 2^{sc[r0 + r]}) modulo p_i for
 // rows r < rows and k0 <= k < k0 + kp (zeros up to the row pitch).  Eight consecutive k
 // per thread: one 16-byte store per plane.  Bound by the stores: 2 N bytes are written
@@ -328,20 +328,10 @@ residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t p
         const int s = max(sc[r0 + r], -4096);  // (kNotFinite: the result is NaN anyway)
         float v[8][CH];
 #pragma unroll
-        for (int q = 0; q < 8; q++) {
-            if constexpr (Src::kDoubleFloat) {
-                const float2 x = kk + q < kp ? src.pair(r0 + r, k0 + kk + q) : make_float2(0.f, 0.f);
-                float d[CH];  // from the top: d[0] is chunk CH - 1
-                digits::digits_df_fp32<CH, moduli::kChunkBits>(
-                    x.x, x.y, moduli::kChunkBits * CH - 1 - s, d);
-#pragma unroll
-                for (int j = 0; j < CH; j++)
-                    v[q][j] = d[CH - 1 - j];
-            } else {
-                const double x = kk + q < kp ? src(r0 + r, k0 + kk + q) : 0.0;
-                int_chunks<CH>(x, s, v[q]);
-            }
-        }
+        for (int q = 0; q < 8; q++)
+            residue_chunks<N>(kk + q < kp ? value_of(src, r0 + r, k0 + kk + q)
+                                          : typename ValueOf<Src::kDoubleFloat>::T{},
+                              s, v[q]);
         uint64_t chunk[CH][4];
         pack_chunks<N>(v, chunk);
         store_residues<N, CH>(chunk, planes + (int64_t)r * pitch + kk, (int64_t)rows * pitch);
@@ -424,47 +414,140 @@ residue_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t 
     }
 }
 
-// Host side: the scales of `rows` rows over all K, and the planes of one K panel.
-template <class Src>
-static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int n_mod, int *sc, int *bad)
+// Scales and residues of short rows in one launch: G lanes per row, eight consecutive k per
+// lane and step; a row of one step (K <= 8 G) is read once.  (A block per row for the scales
+// and another for the residues leave most of their threads without work: 600 900 rows of
+// 100 took 0.36 + 0.60 ms.)
+template <int N, int G, class Src>
+__global__ void __launch_bounds__(128)
+residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
+                     int *__restrict__ sc, int *bad, __nv_bfloat16 *__restrict__ planes)
 {
-    if (rows <= 0)
+    constexpr int CH = moduli::chunks(N);
+    constexpr int kRows = 128 / G;  // rows per block
+    using Value = typename ValueOf<Src::kDoubleFloat>::T;
+    const int gl = threadIdx.x % G;
+    const int64_t steps = ((int64_t)rows + kRows - 1) / kRows;
+    for (int64_t b = blockIdx.x; b < steps; b += gridDim.x) {
+        const int64_t r = b * kRows + threadIdx.x / G;
+        const bool ok = r < rows;  // (every lane takes part in the reductions)
+        Value x[8];
+        auto load = [&](int kk) {
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                x[q] = ok && kk + q < K ? value_of(src, r0 + r, kk + q) : Value{};
+        };
+        float m = 0.0f, ss = 0.0f;
+        for (int kk = gl * 8; kk < K; kk += 8 * G) {
+            load(kk);
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+                const float v = up_of(x[q]);
+                m = fmaxf(m, v);
+                ss = fmaf(v, v, ss);
+            }
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        int s = 0;
+        const bool fast = scale_fast(m, ss, bits, K, &s);
+        if (!__all_sync(0xffffffffu, fast)) {
+            unsigned long long mb = 0;
+            if (ok)
+                for (int k = gl; k < K; k += G) {
+                    const unsigned long long v = abs_bits(src(r0 + r, k));
+                    mb = v > mb ? v : mb;
+                }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1) {
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
+                mb = v > mb ? v : mb;
+            }
+            if (!fast)
+                s = scale_slow(mb, bits, K);
+            if (ok && s == kNotFinite && bad && gl == 0)
+                atomicExch(bad, 1);
+        }
+        if (!ok)
+            continue;
+        if (gl == 0)
+            sc[r0 + r] = s;
+        s = max(s, -4096);
+        const bool again = K > 8 * G;
+        for (int kk = gl * 8; kk < pitch; kk += 8 * G) {
+            if (again || kk >= K)
+                load(kk);
+            float v[8][CH];
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                residue_chunks<N>(x[q], s, v[q]);
+            uint64_t chunk[CH][4];
+            pack_chunks<N>(v, chunk);
+            store_residues<N, CH>(chunk, planes + r * pitch + kk, (int64_t)rows * pitch);
+        }
+    }
+}
+
+// Host side.  Rows up to kShortRow long and in one panel take their scales with their
+// residues (residue_rows, one launch fewer); others beforehand (row_scales).
+constexpr int64_t kShortRow = 1024;
+
+template <class Src>
+static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int64_t k_panel, int n_mod,
+                      int *sc, int *bad)
+{
+    if (rows <= 0 || (K <= kShortRow && k_panel >= K))
         return CUTC_OK;
-    const float bits = moduli::row_bits(n_mod);
-    if (K <= kShortRow)
-        row_scale_short_kernel<Src><<<std::min(ceil_div(rows, 8), 1u << 16), 256, 0, st>>>(
-            src, rows, (int)K, bits, sc, bad);
-    else
-        row_scale_kernel<Src><<<std::min(rows, 1 << 20), 256, 0, st>>>(src, rows, K, bits, sc, bad);
+    row_scale_kernel<Src><<<std::min(rows, 1 << 20), 256, 0, st>>>(src, rows, K,
+                                                                    moduli::row_bits(n_mod), sc, bad);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
+// The planes of the K panel [k0, k0 + kp) for rows r0 .. r0 + rows; sc holds the scales of
+// all rows (row_scales) or receives them.
 template <int N, class Src>
-static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t k0, int64_t kp,
-                        int64_t pitch, const int *sc, void *planes)
+static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t K, int64_t k0,
+                        int64_t kp, int64_t pitch, int *sc, void *planes, int *bad)
 {
     if (rows <= 0 || kp <= 0)
         return CUTC_OK;
-    dim3 grid(ceil_div(pitch, 8 * 128), (unsigned)std::min(rows, 65535));
-    residue_rows_kernel<N, Src><<<grid, 128, 0, st>>>(src, r0, rows, k0, kp, pitch, sc,
-                                                      (__nv_bfloat16 *)planes);
+    auto *out = (__nv_bfloat16 *)planes;
+    if (K <= kShortRow && kp == K) {
+        auto launch = [&](auto g) {
+            constexpr int G = decltype(g)::value;
+            residue_short_kernel<N, G, Src><<<std::min(ceil_div(rows, 128 / G), 1u << 16), 128, 0, st>>>(
+                src, r0, rows, (int)K, (int)pitch, moduli::row_bits(N), sc, bad, out);
+        };
+        if (K <= 64)
+            launch(std::integral_constant<int, 8>{});
+        else if (K <= 128)
+            launch(std::integral_constant<int, 16>{});
+        else
+            launch(std::integral_constant<int, 32>{});
+    } else {
+        dim3 grid(ceil_div(pitch, 8 * 128), (unsigned)std::min(rows, 65535));
+        residue_rows_kernel<N, Src><<<grid, 128, 0, st>>>(src, r0, rows, k0, kp, pitch, sc, out);
+    }
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
 template <class Src>
-static int residue_rows(cudaStream_t st, int n_mod, Src src, int r0, int rows, int64_t k0,
-                        int64_t kp, int64_t pitch, const int *sc, void *planes)
+static int residue_rows(cudaStream_t st, int n_mod, Src src, int r0, int rows, int64_t K,
+                        int64_t k0, int64_t kp, int64_t pitch, int *sc, void *planes, int *bad)
 {
     switch (n_mod) {
-    case 7: return residue_rows<7>(st, src, r0, rows, k0, kp, pitch, sc, planes);
-    case 9: return residue_rows<9>(st, src, r0, rows, k0, kp, pitch, sc, planes);
-    case 11: return residue_rows<11>(st, src, r0, rows, k0, kp, pitch, sc, planes);
-    case 13: return residue_rows<13>(st, src, r0, rows, k0, kp, pitch, sc, planes);
-    case 15: return residue_rows<15>(st, src, r0, rows, k0, kp, pitch, sc, planes);
+    case 7: return residue_rows<7>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 9: return residue_rows<9>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 11: return residue_rows<11>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 13: return residue_rows<13>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 15: return residue_rows<15>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     }
     cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
     return CUTC_ERR_INVALID;
