@@ -349,7 +349,7 @@ static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, in
         CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad));
     return modular_contract(
-        st, W, C_RB, C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, false, sca, scb, out,
+        st, W, C_RB, C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, sca, scb, out,
         err, bad,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
             return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, K, k0, kp, o.pitch, sca, o.p, bad)

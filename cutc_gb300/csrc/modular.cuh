@@ -140,13 +140,13 @@ inline bool modular_whole(int n_mod, int64_t N, int64_t K, int64_t k_panel, size
 }
 
 // The contraction over K panels, gen_a(k0, kp, planes) and gen_b(n0, ncols, k0, kp, planes)
-// writing the residues of a panel (B's in groups of columns whose residues fit b_bytes).
-// a_ready: A's residues of the only panel are in `a` already; b_ready: B's are in slot_b
-// (modular_whole only).
+// writing the residues of a panel (B's in groups of columns whose residues fit b_bytes);
+// gen_a may point planes.p at residues that are there already.  b_ready: B's are in slot_b
+// already (modular_whole only).
 template <class GenA, class GenB>
 int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, size_t b_bytes,
                      int n_mod, int M, int N, int64_t K, int64_t k_panel, ResiduePlanes a,
-                     bool a_ready, bool b_ready, const int *sa, const int *sb,
+                     bool b_ready, const int *sa, const int *sb,
                      const ModularOut &out, int *err, const int *skip, GenA gen_a, GenB gen_b)
 {
     if (M <= 0 || N <= 0)
@@ -160,6 +160,7 @@ int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, si
     CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &p));
     unsigned short *res = (unsigned short *)p;
     a.rows = M;
+    bool a_ready = false;  // A's only panel stays for every pass
     for (int n0 = 0; n0 < N; n0 += pass) {
         const int nc = std::min(pass, N - n0);
         for (int64_t k0 = 0; k0 < K; k0 += k_panel) {

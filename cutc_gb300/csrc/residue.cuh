@@ -338,21 +338,23 @@ residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t p
     }
 }
 
-// Row scales of a matrix stored column by column, src[(k0 + k) ld + r]: 32 rows per block
-// (one per lane), the columns over its 32 warps.  up and abs_bits as for the sources.
+// Row scales of a matrix stored column by column, src[(k0 + k) ld + r]: RB rows per block
+// (consecutive lanes), the columns over its 1024 / RB groups of lanes.
+template <int RB>
 static __global__ void __launch_bounds__(1024)
 row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t K, float bits,
                       int *__restrict__ sc, int *bad)
 {
-    __shared__ float sm[32][33], sq[32][33];
-    __shared__ unsigned long long sb[32][33];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r = blockIdx.x * 32 + lane;
+    constexpr int NG = 1024 / RB;
+    __shared__ float sm[NG][RB + 1], sq[NG][RB + 1];
+    __shared__ unsigned long long sb[NG][RB + 1];
+    const int t = threadIdx.x % RB, g = threadIdx.x / RB;
+    const int r = blockIdx.x * RB + t;
     float m = 0.0f, ss = 0.0f;
     unsigned long long mb = 0;
     if (r < rows) {
 #pragma unroll 4
-        for (int64_t k = warp; k < K; k += 32) {
+        for (int64_t k = g; k < K; k += NG) {
             const double x = X[k * ld + r];
             const float v = abs_up(x);
             const unsigned long long b = abs_bits(x);
@@ -361,20 +363,22 @@ row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_
             mb = b > mb ? b : mb;
         }
     }
-    sm[warp][lane] = m;
-    sq[warp][lane] = ss;
-    sb[warp][lane] = mb;
-    __syncthreads();
-    if (warp != 0 || r >= rows)
-        return;
-    for (int w = 1; w < 32; w++) {
-        m = fmaxf(m, sm[w][lane]);
-        ss += sq[w][lane];
-        mb = sb[w][lane] > mb ? sb[w][lane] : mb;
+    sm[g][t] = m;
+    sq[g][t] = ss;
+    sb[g][t] = mb;
+    for (int h = NG / 2; h > 0; h >>= 1) {  // a fixed order
+        __syncthreads();
+        if (g < h) {
+            sm[g][t] = fmaxf(sm[g][t], sm[g + h][t]);
+            sq[g][t] += sq[g + h][t];
+            sb[g][t] = sb[g + h][t] > sb[g][t] ? sb[g + h][t] : sb[g][t];
+        }
     }
+    if (g != 0 || r >= rows)
+        return;
     int s = 0;
-    if (!scale_fast(m, ss, bits, K, &s))
-        s = scale_slow(mb, bits, K);
+    if (!scale_fast(sm[0][t], sq[0][t], bits, K, &s))
+        s = scale_slow(sb[0][t], bits, K);
     sc[r] = s;
     if (s == kNotFinite && bad)
         atomicExch(bad, 1);
@@ -558,8 +562,13 @@ static inline int row_scales_cols(cudaStream_t st, const double *X, int64_t ld, 
 {
     if (rows <= 0)
         return CUTC_OK;
-    row_scale_cols_kernel<<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K,
-                                                                moduli::row_bits(n_mod), sc, bad);
+    // few rows: 64-byte runs and four times the blocks (300 rows of 9000: 100 us with 32 rows
+    // a block)
+    const float bits = moduli::row_bits(n_mod);
+    if (rows <= 32 * 152)
+        row_scale_cols_kernel<8><<<ceil_div(rows, 8), 1024, 0, st>>>(X, ld, rows, K, bits, sc, bad);
+    else
+        row_scale_cols_kernel<32><<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K, bits, sc, bad);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;

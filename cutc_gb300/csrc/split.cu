@@ -107,6 +107,21 @@ static int64_t int2e_panel_k(int n_mod, int64_t K, int64_t np, int k_split)
     return std::min(cap, std::max<int64_t>(256, fit));
 }
 
+// P's residues stay for every r1 tile (and, in a scan, for every set) when all K panels
+// take at most 16 GiB; otherwise each tile forms a panel again (medium build, 7260 x 80 000:
+// 2.5 ms a tile).
+constexpr size_t kResidentBytes = (size_t)16 << 30;
+static bool p_resident(int n_mod, int64_t np, int64_t n2, int64_t k_panel)
+{
+    return k_panel >= n2 || (size_t)((n2 + k_panel - 1) / k_panel) *
+                                    residue_bytes(n_mod, np, k_panel) <= kResidentBytes;
+}
+static size_t p_bytes(int n_mod, int64_t np, int64_t n2, int64_t k_panel)
+{
+    const int64_t panels = p_resident(n_mod, np, n2, k_panel) ? (n2 + k_panel - 1) / k_panel : 1;
+    return (size_t)panels * residue_bytes(n_mod, np, k_panel);
+}
+
 size_t split_r1_row_bytes(const Request &R)
 {
     return 4 * (size_t)R.n2 * 8 + 64;  // residues, as many bytes as the four G rows
@@ -119,11 +134,11 @@ size_t split_int2e_row_bytes(const Request &R)
 
 size_t split_fixed_bytes(const Request &R)
 {
-    // residues of a K panel of P, the weighted AO values w chi_a on r2 they are formed
+    // residues of P (or of a K panel), the weighted AO values w chi_a on r2 they are formed
     // from, the int_2e operands' residues, and the residues of one pass of results
     const int n_mod = split_moduli(R.n_slices);
     const int64_t np = n_pairs(R.nA);
-    size_t b = residue_bytes(n_mod, np, panel_k(R.n2, np, R.k_split)) + 8 * (size_t)R.nA * R.n2 +
+    size_t b = p_bytes(n_mod, np, R.n2, panel_k(R.n2, np, R.k_split)) + 8 * (size_t)R.nA * R.n2 +
                std::min(kMinResidueBytes, residue_bytes(n_mod, 4 * (int64_t)R.n1, R.n2)) +
                modular_out_bytes(n_mod, np,
                                  std::max<int64_t>(np, std::min<int64_t>(4 * (int64_t)R.n1, 1 << 30)));
@@ -163,6 +178,12 @@ static int scale_slot(Workspace &W, int slot, int rows, int **sc)
     return CUTC_OK;
 }
 
+// Where the residues of P's panel from k0 are (ax_whole).
+static void *p_panel(const SplitPlan &sp, int n_mod, int np, int64_t k0)
+{
+    return (char *)sp.ax.p + (k0 / sp.k_panel) * residue_bytes(n_mod, np, sp.k_panel);
+}
+
 int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *wr2,
                     const double *aos2v, int64_t n1t, int slot0, SplitPlan &sp)
 {
@@ -181,23 +202,24 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
     CUTC_TRY(scale_slot(W, slot0 + SS_AX_SC, np, &sp.sc_ax));
     CUTC_TRY(scale_slot(W, slot0 + SS_BX_SC, (int)(4 * n1t), &sp.sc_bx));
     sp.k_panel = panel_k(R.n2, np, R.k_split);
-    CUTC_TRY(W.get(slot0 + SS_AX, residue_bytes(n_mod, np, sp.k_panel), &p));
+    CUTC_TRY(W.get(slot0 + SS_AX, p_bytes(n_mod, np, R.n2, sp.k_panel), &p));
     sp.ax.p = p;
     sp.ax.rows = np;
     CUTC_TRY(W.get(slot0 + SS_WCHI2, std::max<size_t>(1, (size_t)R.nA * R.n2) * 8, &p));
     sp.wchi2 = (const double *)p;
     sp.aos2v = aos2v;
-    // with K in one panel the residues of P stay for every r1 tile (and, in a scan, for
-    // every set); with several panels each tile forms them again
-    sp.ax_whole = sp.k_panel >= R.n2;
+    sp.ax_whole = p_resident(n_mod, np, R.n2, sp.k_panel);
     if (R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == sp.ax.p)
         return CUTC_OK;  // the same molecule's scales (and residues) are already there
     CUTC_TRY(weighted_aos(st, R.n2, R.nA, wr2, aos2v, (int64_t)R.n2, (double *)p));
     SrcSym src{sp.wchi2, aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
     CUTC_TRY(row_scales(st, src, np, (int64_t)R.n2, sp.k_panel, n_mod, sp.sc_ax, (int *)nullptr));
     if (sp.ax_whole)
-        CUTC_TRY(residue_rows(st, n_mod, src, 0, np, R.n2, 0, R.n2, residue_pitch(R.n2), sp.sc_ax,
-                              sp.ax.p, (int *)nullptr));
+        for (int64_t k0 = 0; k0 < R.n2; k0 += sp.k_panel) {
+            const int64_t kp = std::min<int64_t>(sp.k_panel, R.n2 - k0);
+            CUTC_TRY(residue_rows(st, n_mod, src, 0, np, R.n2, k0, kp, residue_pitch(kp), sp.sc_ax,
+                                  p_panel(sp, n_mod, np, k0), (int *)nullptr));
+        }
     E->tag_x = R.mol_tag;
     E->tag_x_buf = sp.ax.p;
     return CUTC_OK;
@@ -218,8 +240,12 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
     const ModularOut out{Xb, np, nb, blk_rows, ib, 1.0, 0.0};
     CUTC_TRY(modular_contract(
         st, E->ws, sp.slot0 + SS_BX, sp.slot0 + SS_RES, x_residue_bytes(sp.n1t, R.n2), n_mod,
-        (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, sp.ax_whole, false, sp.sc_ax, sp.sc_bx, out, sp.err, nullptr,
-        [&](int64_t k0, int64_t kp, const ResiduePlanes &a) {
+        (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, false, sp.sc_ax, sp.sc_bx, out, sp.err, nullptr,
+        [&](int64_t k0, int64_t kp, ResiduePlanes &a) -> int {
+            if (sp.ax_whole) {
+                a.p = p_panel(sp, n_mod, (int)np, k0);
+                return CUTC_OK;
+            }
             return residue_rows(st, n_mod, sa, 0, (int)np, R.n2, k0, kp, a.pitch, sp.sc_ax, a.p,
                                 (int *)nullptr);
         },
@@ -274,7 +300,7 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     const double *x3 = Xt + 3 * (int64_t)nb * np;
     CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a, nullptr));
     CUTC_TRY(modular_contract(
-        st, W, slot0 + SS_BH, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, np, nb, pan_h, a, false, keep_b, sc_a,
+        st, W, slot0 + SS_BH, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, np, nb, pan_h, a, keep_b, sc_a,
         sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err, nullptr,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_cols(st, n_mod, x3, np, np, k0, kp, o.pitch, sc_a, o.p);
@@ -285,7 +311,7 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     if (nl > 0) {
         CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a, nullptr));
         CUTC_TRY(modular_contract(
-            st, W, slot0 + SS_BN, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, nl, k3, pan_n, a, false, keep_b, sc_a,
+            st, W, slot0 + SS_BN, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, nl, k3, pan_n, a, keep_b, sc_a,
             sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err, nullptr,
             [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
                 return residue_cols(st, n_mod, Xt, np, np, k0, kp, o.pitch, sc_a, o.p);
@@ -367,7 +393,7 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
     CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sc_a, (int *)nullptr));
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, sc_b, (int *)nullptr));
     CUTC_TRY(modular_contract(
-        st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, false, sc_a, sc_b,
+        st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
         ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err, nullptr,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_rows(st, n_mod, sa, 0, M, K, k0, kp, o.pitch, sc_a, o.p, (int *)nullptr);

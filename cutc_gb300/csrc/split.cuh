@@ -17,7 +17,7 @@ struct SplitPlan {
     int slot0 = 0;
     int n_slices = 0;
     int64_t n1t = 0;
-    ResiduePlanes ax;                  // residues of P (a K panel, or all of K: ax_whole)
+    ResiduePlanes ax;                  // residues of P (a K panel, or all panels: ax_whole)
     bool ax_whole = false;
     int64_t k_panel = 0;               // K per launch of the X contraction
     int *sc_ax = nullptr, *sc_bx = nullptr;  // row scales of P and of a G tile
