@@ -14,6 +14,9 @@
 // a multiple of 2^{-16-9d}, at most 2^{-9d}, so the FP32 sums are exact while
 // (d + 1) K 2^16 <= 2^24: K <= 85 for d <= 2 (double-float results), K <= 64 for d <= 3
 // (FP64 results); later diagonals round at 2^-27 2^-24 and 2^-36 2^-24 of the row scales.
+// With more nuclei K is cut into groups of 64, one launch each, whose V values are added
+// (FP64: as integers) through device memory: 16 to 384 bytes a pair and group, a few
+// percent of what the kernels that loop over the nuclei take.
 //
 // A = the F slices of 128 r2 points, all of K, loaded once per CTA; B = the coefficient
 // slices in tiles of 64 rows (four r1 points, or two; one point for FP64 results), streamed;
@@ -69,6 +72,13 @@ struct PairTcParams {
     PairDfArgs P;                 // geometry and outputs
     double *G64;                  // FP64: in place of P.G
     int *err;
+    // a group of K blocks of a longer contraction: from block kb0 on; the values so far are
+    // added (not for the first group), and kept (not for the last) at
+    // part[(i R + c) n2 + j] (double-float), partI and partL (FP64: integer and rest)
+    int kb0, first, last;
+    float2 *part;
+    long long *partI;
+    float *partL;
 };
 
 // x 2^e for the scale of a value of row exponents e (clamped to the float range); NaN for
@@ -269,15 +279,12 @@ __device__ __forceinline__ double int_double(long long I, int k)
     return __hiloint2double((int)(hi | ((unsigned)(I >> 32) & 0x80000000u)), (int)lo);
 }
 
-// The V values of eight columns in two parts each: hi, the diagonals down to 2^-43 of the
-// row scale as a double, and lo, the rest (below 2^-35, to 2^-60) as a float.  e: the
-// exponents of the columns' scales with the F row's added.
+// The V values of eight columns, in units of the row scales, in two parts each: an integer
+// multiple of 2^-43 and the rest (below 2^-35, to 2^-60) as a float:
 //   H + L + L2 + L3 on the grids 2^-16, 2^-25, 2^-34, 2^-43 (each exact, as read_df16)
-// is an integer multiple of 2^-43 below 2^50, formed and made a double with integer
-// operations (an FP64 add per value instead, on the pipe that bounds the kernel, cost 15 of
-// 67 FP64 operations a pair).
+// is the integer, below 2^50, formed with integer operations.
 template <int S, int BN>
-__device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, double *hi, float *lo)
+__device__ __forceinline__ void read_f64_8(uint32_t cb, long long *I, float *rest)
 {
     static_assert(S == 7, "FP64 results take 7 slices");
     float v[8];
@@ -287,7 +294,7 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
     for (int k = 0; k < 4; k++)
         H[k] = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
     // multiples of 2^g: C = 1.5 2^(23 + g)
-    auto cut = [&](int d, float C, uint64_t (&up)[4], uint64_t (&rest)[4]) {
+    auto cut = [&](int d, float C, uint64_t (&up)[4], uint64_t (&down)[4]) {
         const uint64_t Cg = tc::f2_dup(C);
         tc::tmem_ld8(cb + (uint32_t)(BN * d), v);
 #pragma unroll
@@ -295,7 +302,7 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
             const uint64_t x = tc::f2_pack(__float_as_uint(v[2 * k]), __float_as_uint(v[2 * k + 1]));
             const uint64_t hh = tc::f2_sub(tc::f2_add(x, Cg), Cg);
             up[k] = tc::f2_add(up[k], hh);
-            rest[k] = tc::f2_sub(x, hh);
+            down[k] = tc::f2_sub(x, hh);
         }
     };
     cut(1, 192.0f, H, L);
@@ -319,13 +326,20 @@ __device__ __forceinline__ void read_f64_8(uint32_t cb, const int *eb, int ea, d
         const int ih = __float2int_rn(part(H) * 65536.0f);
         const int il = grid_int(part(L), 0x1p25f);
         const int il2 = grid_int(part(L2), 0x1p34f), il3 = grid_int(part(L3), 0x1p43f);
-        const long long I = ((long long)ih << 27) + ((long long)il << 18) + (long long)(il2 * 512 + il3);
-        const int e = eb[k] + ea;
-        hi[k] = eb[k] >= kNanExponent || ea >= kNanExponent
-                    ? __longlong_as_double(0x7ff8000000000000ll)
-                    : int_double(I, e - 43);
-        lo[k] = part(L4) * pow2f(min(e, 127));
+        I[k] = ((long long)ih << 27) + ((long long)il << 18) + (long long)(il2 * 512 + il3);
+        rest[k] = part(L4);
     }
+}
+
+// Their values: hi as a double (made in integer arithmetic: an FP64 add per value instead,
+// on the pipe that bounds the kernel, cost 15 of 67 FP64 operations a pair) and lo as a
+// float.  eb: the exponents of the columns' scales, ea: the F row's.
+__device__ __forceinline__ void scale_f64(long long I, float rest, int eb, int ea, double *hi, float *lo)
+{
+    const int e = eb + ea;
+    *hi = eb >= kNanExponent || ea >= kNanExponent ? __longlong_as_double(0x7ff8000000000000ll)
+                                                   : int_double(I, e - 43);
+    *lo = rest * pow2f(min(e, 127));
 }
 
 // a double as a float, truncated, with integer operations (0 below the float range)
@@ -460,7 +474,8 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
     o[3 * P.plane] = minus_half(fma(ux, ux, fma(uy, uy, uz * uz)));
 }
 
-template <int S, int KB, int R, bool F64>
+// PART: one group of K blocks of a longer contraction (Q.kb0, Q.first, Q.last).
+template <int S, int KB, int R, bool F64, bool PART>
 __global__ void __launch_bounds__(PairTcCfg<S, KB, R, F64>::kThreads, 1)
 pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ PairTcParams Q)
@@ -522,6 +537,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     if (warp == kCtlWarp) {
         if (lane == 0) {
+            const int kb0 = PART ? Q.kb0 : 0;
             auto load_b = [&](int q) {
                 const int b = q % NB;
                 const uint32_t fb = tc::smem_u32(&full[b]);
@@ -533,7 +549,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     for (int t = 0; t < S; t++)
                         tc::tma_load_2d(
                             tc::smem_u32(sB + b * Cfg::kBStage + (kb * S + t) * Cfg::kBSlice), &tmB,
-                            kb * kBK, t * Q.Npad + n0, fb);
+                            (kb0 + kb) * kBK, t * Q.Npad + n0, fb);
             };
             const uint32_t ab = tc::smem_u32(afull);
             tc::mbar_arrive_expect_tx(ab, Cfg::kABytes);
@@ -541,8 +557,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int kb = 0; kb < KB; kb++)
 #pragma unroll
                 for (int s = 0; s < S; s++)
-                    tc::tma_load_2d(tc::smem_u32(sA + (kb * S + s) * Cfg::kASlice), &tmA, kb * kBK,
-                                    s * Q.Mpad + m0, ab);
+                    tc::tma_load_2d(tc::smem_u32(sA + (kb * S + s) * Cfg::kASlice), &tmA,
+                                    (kb0 + kb) * kBK, s * Q.Mpad + m0, ab);
             int loaded = 0;  // B tiles issued
             for (; loaded < min(NB, ntiles); loaded++)
                 load_b(loaded);
@@ -643,14 +659,37 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if constexpr (F64) {
                 double V[R];
                 float lo[R];
+                const int *eb = Q.eb + (int64_t)i0 * R;
+                const bool out = jok && i0 < P.n1b;
 #pragma unroll
-                for (int c = 0; c < R; c += 8)
-                    read_f64_8<S, BN>(cb + (uint32_t)c, Q.eb + (int64_t)i0 * R + c, ea, V + c, lo + c);
+                for (int c = 0; c < R; c += 8) {
+                    long long I[8];
+                    float rest[8];
+                    read_f64_8<S, BN>(cb + (uint32_t)c, I, rest);
+                    if constexpr (PART) {
+                        if (out)
+#pragma unroll
+                            for (int k = 0; k < 8; k++) {
+                                const int64_t o = ((int64_t)i0 * R + c + k) * P.n2 + j;
+                                if (!Q.first) {
+                                    I[k] += Q.partI[o];
+                                    rest[k] += Q.partL[o];
+                                }
+                                if (!Q.last) {
+                                    Q.partI[o] = I[k];
+                                    Q.partL[o] = rest[k];
+                                }
+                            }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 8; k++)
+                        scale_f64(I[k], rest[k], eb[c + k], ea, V + c + k, lo + c + k);
+                }
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
                     tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-                if (jok && i0 < P.n1b)
+                if (out && (!PART || Q.last))
                     pair_f64<R>(Q, i0, j, V, lo, dx2, dy2, dz2);
             } else {
                 uint64_t H[R / 16][8], L[R / 16][8], L2[R / 16][8];
@@ -666,7 +705,18 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                     for (int h = 0; h < R / 16; h++)
                         scale_df16(H[h], L[h], L2[h], Q.bscale + (int64_t)i0 * R + 16 * h, V + 16 * h);
-                    pair_df<R>(Q, i0, j, V, x2, y2, z2, sa, a);
+                    if constexpr (PART) {
+#pragma unroll
+                        for (int c = 0; c < R; c++) {
+                            float2 *o = Q.part + ((int64_t)i0 * R + c) * P.n2 + j;
+                            if (!Q.first)
+                                V[c] = df::add(V[c], df::make(o->x, o->y));
+                            if (!Q.last)
+                                *o = make_float2(V[c].hi, V[c].lo);
+                        }
+                    }
+                    if (!PART || Q.last)
+                        pair_df<R>(Q, i0, j, V, x2, y2, z2, sa, a);
                 }
             }
         }
@@ -691,26 +741,22 @@ __device__ __forceinline__ int row_exponent(unsigned long long bits)
     return E == 0 ? 0 : min(E - 1022, kNanExponent);
 }
 
-// slices[(s * Mpad + r) * Kpad + k] for r < Mpad, k < Kpad = 32 KB (zeros outside M x K),
-// ex[r] = row exponent, of X[r * K + k]: one warp per row, so the row is read once.  The
-// digits are formed in integer arithmetic (digits.cuh).
-template <int S, int KB>
+// slices[(s * Mpad + r) * Kpad + k] for r < Mpad, k < Kpad (a multiple of 32; zeros outside
+// M x K), ex[r] = row exponent, of X[r * K + k]: one warp per row.  The digits are formed in
+// integer arithmetic (digits.cuh).
+template <int S>
 __global__ void __launch_bounds__(256)
-slice_kernel(const double *__restrict__ X, int M, int K, int Mpad, __nv_bfloat16 *__restrict__ slices,
-             int *__restrict__ ex)
+slice_kernel(const double *__restrict__ X, int M, int K, int Kpad, int Mpad,
+             __nv_bfloat16 *__restrict__ slices, int *__restrict__ ex)
 {
     const int lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
     if (r >= Mpad)
         return;
-    double x[KB];
     unsigned long long m = 0;
-#pragma unroll
-    for (int b = 0; b < KB; b++) {
-        const int k = 32 * b + lane;
-        x[b] = r < M && k < K ? X[r * K + k] : 0.0;
+    for (int k = lane; k < K && r < M; k += 32) {
         const unsigned long long v =
-            (unsigned long long)__double_as_longlong(x[b]) & 0x7fffffffffffffffull;
+            (unsigned long long)__double_as_longlong(X[r * K + k]) & 0x7fffffffffffffffull;
         m = v > m ? v : m;
     }
 #pragma unroll
@@ -721,13 +767,13 @@ slice_kernel(const double *__restrict__ X, int M, int K, int Mpad, __nv_bfloat16
     const int e = row_exponent(m);
     if (lane == 0)
         ex[r] = e;
-#pragma unroll
-    for (int b = 0; b < KB; b++) {
+    for (int k = lane; k < Kpad; k += 32) {
+        const double x = r < M && k < K && e < kNanExponent ? X[r * K + k] : 0.0;
         int q[S];
-        digits::digits_int<S>(e >= kNanExponent ? 0 : digits::scaled_round<S>(x[b], e), q);
+        digits::digits_int<S>(digits::scaled_round<S>(x, e), q);
 #pragma unroll
         for (int s = 0; s < S; s++)
-            slices[((int64_t)s * Mpad + r) * (32 * KB) + 32 * b + lane] =
+            slices[((int64_t)s * Mpad + r) * Kpad + k] =
                 __float2bfloat16_rn(__int2float_rn(q[s]) * exp2f((float)(-8 - 9 * s)));
     }
 }
@@ -738,15 +784,24 @@ slice_kernel(const double *__restrict__ X, int M, int K, int Mpad, __nv_bfloat16
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
-// Nuclei with which the leading diagonals are exact: K = powers n_nuc at most 64 (FP64) or
-// 85 (double-float).
-static int max_nuclei(int rows, bool fp64)
+// The K up to which the contraction is one group: the leading diagonals are exact (and the
+// operands fit shared memory).  A longer one runs in groups of kGroupBlocks K blocks whose
+// values are added between launches.
+constexpr int kGroupBlocks = 2;
+static int one_group_k(const PairTcMode &m) { return m.fp64 ? 64 : m.rows == 16 ? 80 : 85; }
+static int64_t pad_k(const PairTcMode &m, int64_t K)
 {
-    return (fp64 ? 64 : rows == 16 ? 80 : 85) / (rows == 16 ? 4 : 7);
+    return round_up(std::max<int64_t>(K, 1), K <= one_group_k(m) ? kBK : kGroupBlocks * kBK);
 }
 
-PairTcMode pair_tc_mode(int n_nuc, const double *coef, const int *exps, int n_terms, bool fp64,
-                        int slices)
+// r1 rows per sub-tile of a contraction in groups: its values so far take at most 2 GiB.
+static int64_t group_rows(const PairTcMode &m, int64_t n2, int64_t n1b)
+{
+    const int64_t per = n2 * m.rows * (m.fp64 ? 12 : 8);
+    return std::min(n1b, std::max<int64_t>(8, (((int64_t)2 << 30) / per) / 8 * 8));
+}
+
+PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, bool fp64, int slices)
 {
     PairTcMode m;
     m.fp64 = fp64;
@@ -754,38 +809,42 @@ PairTcMode pair_tc_mode(int n_nuc, const double *coef, const int *exps, int n_te
     // contractions), 6 for builds of 6 and 7 slices (2^-54, below the double-float
     // epilogue), 7 for FP64 (2^-63)
     m.slices = fp64 ? 7 : slices >= 6 ? 6 : 5;
-    const int rows = pair_df_sparse(exps, n_terms) ? 16 : 32;
-    if (n_nuc > max_nuclei(rows, fp64))
-        return m;
     if (!fp64 && (getenv("CUTC_PAIR_DF") || getenv("CUTC_PAIR_DENSE")))
         return m;
     for (int k = 0; k < 3 * n_terms; k++)
         if (!std::isfinite(coef[k]))
             return m;
-    m.rows = rows;
+    m.rows = pair_df_sparse(exps, n_terms) ? 16 : 32;
     return m;
+}
+
+// Device bytes: per r2 point and r1 row, of K values in FP64 and in slices.
+static size_t operand_bytes(int64_t rows, int64_t K, int slices)
+{
+    return (size_t)rows * (8 * K + 2 * slices * round_up(K, kGroupBlocks * kBK) + 4);
 }
 
 size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices)
 {
-    const int64_t K = std::min<int64_t>(7 * (int64_t)n_nuc, 85);
-    return (size_t)n2 * K * 8 + 2 * (size_t)slices * round_up(n2, kBM) * round_up(K, kBK) +
-           4 * (size_t)round_up(n2, kBM);
+    const int64_t K = 7 * (int64_t)n_nuc;
+    size_t b = operand_bytes(round_up(n2, kBM), K, slices);
+    if (K > 64)  // the values so far of a sub-tile
+        b += (size_t)2 << 30;
+    return b;
 }
 
 size_t pair_tc_row_bytes(int n_nuc, int slices)
 {
-    const int64_t K = std::min<int64_t>(7 * (int64_t)n_nuc, 85);
-    return 32 * (size_t)K * 8 + 2 * (size_t)slices * 32 * round_up(K, kBK) + 3 * 8 + 32 * 8 + 64;
+    return operand_bytes(32, std::min<int64_t>(7 * (int64_t)n_nuc, 85), slices) + 3 * 8 + 32 * 4 + 64;
 }
 
 static int alloc_operand(Workspace &W, int slot, int S, int64_t M, int row_mult, int64_t K,
-                         SliceOperand &op)
+                         int64_t Kpad, SliceOperand &op)
 {
     op.M = (int)M;
     op.Mpad = (int)round_up(std::max<int64_t>(M, 1), row_mult);
     op.K = K;
-    op.Kpad = round_up(std::max<int64_t>(K, 1), kBK);
+    op.Kpad = Kpad;
     void *p;
     CUTC_TRY(W.get(slot, (size_t)S * op.Mpad * op.Kpad * 2, &p));
     op.sl = p;
@@ -797,13 +856,8 @@ static int alloc_operand(Workspace &W, int slot, int S, int64_t M, int row_mult,
 template <int S>
 static int slice_rows(cudaStream_t st, const double *X, const SliceOperand &op)
 {
-    const unsigned grid = ceil_div(op.Mpad, 8);
-    auto *sl = (__nv_bfloat16 *)op.sl;
-    switch ((int)(op.Kpad / kBK)) {
-    case 1: slice_kernel<S, 1><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
-    case 2: slice_kernel<S, 2><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
-    default: slice_kernel<S, 3><<<grid, 256, 0, st>>>(X, op.M, (int)op.K, op.Mpad, sl, op.ex); break;
-    }
+    slice_kernel<S><<<ceil_div(op.Mpad, 8), 256, 0, st>>>(X, op.M, (int)op.K, (int)op.Kpad, op.Mpad,
+                                                          (__nv_bfloat16 *)op.sl, op.ex);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
@@ -816,26 +870,31 @@ static int slice_rows(cudaStream_t st, int slices, const double *X, const SliceO
                          : slice_rows<7>(st, X, op);
 }
 
-enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale };
+enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale, kSlotPart };
 
 int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &mode, int n2,
                     int n_nuc, const double *f2, int64_t n1t, int *err, PairTcPlan &plan)
 {
-    const int64_t K = (int64_t)mode.powers() * n_nuc;
-    const int64_t rows = (int64_t)mode.rows * n1t;
+    const int64_t K = (int64_t)mode.powers() * n_nuc, Kpad = pad_k(mode, K);
     plan.mode = mode;
     plan.err = err;
+    plan.tile_rows = K <= one_group_k(mode) ? n1t : group_rows(mode, n2, n1t);
+    const int64_t rows = (int64_t)mode.rows * plan.tile_rows;
     void *p;
     CUTC_TRY(W.get(slot0 + kSlotF64, (size_t)n2 * K * 8, &p));
     plan.Fd = (double *)p;
     CUTC_TRY(W.get(slot0 + kSlotC64, (size_t)rows * K * 8, &p));
     plan.Cd = (double *)p;
-    CUTC_TRY(W.get(slot0 + kSlotR1d, (size_t)3 * n1t * sizeof(float2), &p));
+    CUTC_TRY(W.get(slot0 + kSlotR1d, (size_t)3 * plan.tile_rows * sizeof(float2), &p));
     plan.r1d = (float2 *)p;
     CUTC_TRY(W.get(slot0 + kSlotBscale, (size_t)round_up(rows, kPairBN) * 4, &p));
     plan.bscale = (float *)p;
-    CUTC_TRY(alloc_operand(W, slot0 + kSlotAF, mode.slices, n2, kBM, K, plan.AF));
-    CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, mode.slices, rows, kPairBN, K, plan.BC));
+    if (K > one_group_k(mode)) {
+        CUTC_TRY(W.get(slot0 + kSlotPart, (size_t)n2 * rows * (mode.fp64 ? 12 : 8), &p));
+        plan.part = p;
+    }
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotAF, mode.slices, n2, kBM, K, Kpad, plan.AF));
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, mode.slices, rows, kPairBN, K, Kpad, plan.BC));
     CUTC_TRY(launch_pair_tc_f(st, mode.powers(), n2, n_nuc, f2, plan.Fd));
     note_launches(1);
     return slice_rows(st, mode.slices, plan.Fd, plan.AF);
@@ -851,7 +910,7 @@ static int make_tmap(CUtensorMap *map, const void *base, int64_t rows_total, int
     return encode_bf16_map(map, base, 2, dims, strides, box, 64);
 }
 
-template <int S, int KB, int R, bool F64>
+template <int S, int KB, int R, bool F64, bool PART>
 static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
                          PairTcParams Q, int n_sm)
 {
@@ -859,7 +918,7 @@ static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorM
     static std::atomic<unsigned long long> attr_done{0};
     const unsigned long long bit = current_device_bit();
     if (!(attr_done.load() & bit)) {
-        CUTC_CUDA_TRY(cudaFuncSetAttribute(pair_tc_kernel<S, KB, R, F64>,
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(pair_tc_kernel<S, KB, R, F64, PART>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
         attr_done.fetch_or(bit);
     }
@@ -876,7 +935,7 @@ static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorM
         cutc_set_error(CUTC_ERR_INVALID, "pair grid of %lld CTAs", (long long)grid);
         return CUTC_ERR_INVALID;
     }
-    pair_tc_kernel<S, KB, R, F64><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, Q);
+    pair_tc_kernel<S, KB, R, F64, PART><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, Q);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
@@ -884,14 +943,16 @@ static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorM
 
 template <int S, int R, bool F64>
 static int launch_kb(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
-                     const PairTcParams &Q, int n_sm, int KB)
+                     const PairTcParams &Q, int n_sm, int KB, bool part)
 {
+    if (part)
+        return launch_kernel<S, kGroupBlocks, R, F64, true>(st, ta, tb, Q, n_sm);
     switch (KB) {
-    case 1: return launch_kernel<S, 1, R, F64>(st, ta, tb, Q, n_sm);
-    case 2: return launch_kernel<S, 2, R, F64>(st, ta, tb, Q, n_sm);
+    case 1: return launch_kernel<S, 1, R, F64, false>(st, ta, tb, Q, n_sm);
+    case 2: return launch_kernel<S, 2, R, F64, false>(st, ta, tb, Q, n_sm);
     case 3:
         if constexpr (!F64)
-            return launch_kernel<S, 3, R, F64>(st, ta, tb, Q, n_sm);
+            return launch_kernel<S, 3, R, F64, false>(st, ta, tb, Q, n_sm);
         break;
     }
     cutc_set_error(CUTC_ERR_INVALID, "pair contraction of %d K blocks", KB);
@@ -931,14 +992,28 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     Q.r1d = plan.r1d;
     Q.err = plan.err;
     const int KB = (int)(plan.AF.Kpad / kBK);
-    if (m.fp64)
-        return m.rows == 16 ? launch_kb<7, 16, true>(st, ta, tb, Q, n_sm, KB)
-                            : launch_kb<7, 32, true>(st, ta, tb, Q, n_sm, KB);
-    if (m.slices == 6)
-        return m.rows == 16 ? launch_kb<6, 16, false>(st, ta, tb, Q, n_sm, KB)
-                            : launch_kb<6, 32, false>(st, ta, tb, Q, n_sm, KB);
-    return m.rows == 16 ? launch_kb<5, 16, false>(st, ta, tb, Q, n_sm, KB)
-                        : launch_kb<5, 32, false>(st, ta, tb, Q, n_sm, KB);
+    const bool part = plan.AF.K > one_group_k(m);
+    Q.part = (float2 *)plan.part;
+    Q.partI = (long long *)plan.part;
+    Q.partL = (float *)(Q.partI + (m.fp64 && part ? (int64_t)P.n2 * m.rows * P.n1b : 0));
+    for (int kb = 0; kb < KB; kb += part ? kGroupBlocks : KB) {
+        Q.kb0 = kb;
+        Q.first = kb == 0;
+        Q.last = !part || kb + kGroupBlocks >= KB;
+        if (m.fp64 && m.rows == 16)
+            CUTC_TRY((launch_kb<7, 16, true>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.fp64)
+            CUTC_TRY((launch_kb<7, 32, true>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.slices == 6 && m.rows == 16)
+            CUTC_TRY((launch_kb<6, 16, false>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.slices == 6)
+            CUTC_TRY((launch_kb<6, 32, false>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.rows == 16)
+            CUTC_TRY((launch_kb<5, 16, false>(st, ta, tb, Q, n_sm, KB, part)));
+        else
+            CUTC_TRY((launch_kb<5, 32, false>(st, ta, tb, Q, n_sm, KB, part)));
+    }
+    return CUTC_OK;
 }
 
 int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, const double *rn,
@@ -946,9 +1021,15 @@ int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, cons
 {
     if (P.n1b <= 0 || P.n2 <= 0)
         return CUTC_OK;
-    PairTcParams Q{};
-    Q.P = P;
-    return run_tile(st, plan, Q, rn, a_en, n_sm);
+    for (int64_t i = 0; i < P.n1b; i += plan.tile_rows) {
+        PairTcParams Q{};
+        Q.P = P;
+        Q.P.i0 += (int)i;
+        Q.P.n1b = (int)std::min<int64_t>(plan.tile_rows, P.n1b - i);
+        Q.P.G += i * P.ldg;
+        CUTC_TRY(run_tile(st, plan, Q, rn, a_en, n_sm));
+    }
+    return CUTC_OK;
 }
 
 int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &A, const double *rn,
@@ -961,8 +1042,13 @@ int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &A, const
     P.i0 = A.i0; P.n1b = A.n1b; P.n2 = A.n2; P.nN = A.nN;
     P.r1 = A.r1; P.r2 = A.r2; P.coef = A.coef; P.exps = A.exps; P.term_off = A.term_off;
     P.a_ee = A.a_ee; P.ldg = A.ldg; P.plane = A.plane;
-    Q.G64 = A.G;
-    return run_tile(st, plan, Q, rn, a_en, n_sm);
+    for (int64_t i = 0; i < A.n1b; i += plan.tile_rows) {
+        P.i0 = A.i0 + (int)i;
+        P.n1b = (int)std::min<int64_t>(plan.tile_rows, A.n1b - i);
+        Q.G64 = A.G + i * A.ldg;
+        CUTC_TRY(run_tile(st, plan, Q, rn, a_en, n_sm));
+    }
+    return CUTC_OK;
 }
 
 }  // namespace cutc

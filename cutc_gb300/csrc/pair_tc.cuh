@@ -27,11 +27,11 @@ struct PairTcMode {
     int powers() const { return rows == 16 ? 4 : 7; }
 };
 
-// The mode for n_nuc nuclei and a term table: double-float results from `slices` slices, or
-// FP64 results.  rows == 0 where the tensor-core kernel does not apply (too many nuclei for
-// exact leading diagonals, a coefficient that is not finite, or a kernel chosen by
-// CUTC_PAIR_DF / CUTC_PAIR_DENSE for the double-float form).
-PairTcMode pair_tc_mode(int n_nuc, const double *coef, const int *exps, int n_terms, bool fp64,
+// The mode for a term table: double-float results from `slices` slices, or
+// FP64 results.  rows == 0 where the tensor-core kernel does not apply (a coefficient that
+// is not finite, or a kernel chosen by CUTC_PAIR_DF / CUTC_PAIR_DENSE for the double-float
+// form).
+PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, bool fp64,
                         int slices);
 
 struct PairTcPlan {
@@ -40,6 +40,8 @@ struct PairTcPlan {
     double *Fd = nullptr, *Cd = nullptr;
     float2 *r1d = nullptr;      // the tile's r1 points in double-float
     float *bscale = nullptr;    // 2^(row exponent) of the coefficient rows
+    void *part = nullptr;       // the V values between the groups of a long contraction
+    int64_t tile_rows = 0;      // r1 rows taken at once
     int *err = nullptr;         // device flag set by a bounded wait that gave up
 };
 

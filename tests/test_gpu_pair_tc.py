@@ -3,9 +3,10 @@
 FP64 planes against the oracle within 1e-13 of each plane's largest value, the tolerance of
 the other pair-kernel tests, for both coefficient layouts (exponents in {0, 2, 3, 4}; any up
 to 6), at the edges of the 128-point r2 tiles and of the r1 groups of a tile (4 or 2 points),
-at the largest nucleus counts that take the kernel (16 and 9) and one beyond, with e-e and
-e-n coalescence.  The double-float form with general exponents against the oracle at the
-split form's tolerance and against the double-float kernel at 1e-12."""
+at the largest nucleus counts of one contraction (16 and 9), one beyond, and three groups
+of nuclei, with e-e and e-n coalescence.  The double-float form with general exponents, or
+more nuclei than one contraction takes, against the oracle at the split form's tolerance and
+against the double-float kernel at 1e-12."""
 import numpy as np
 import pytest
 
@@ -27,8 +28,8 @@ def _problem(n_nuc, n1, n2, exps, seed, **kw):
 
 
 @pytest.mark.parametrize("n1,n2", [(1, 127), (3, 128), (5, 129), (70, 1000)])
-@pytest.mark.parametrize("n_nuc,exps", [(1, "even"), (16, "even"), (17, "even"), (2, "all"),
-                                        (9, "all"), (10, "all")])
+@pytest.mark.parametrize("n_nuc,exps", [(1, "even"), (16, "even"), (17, "even"), (40, "even"),
+                                        (2, "all"), (9, "all"), (10, "all"), (20, "all")])
 def test_fp64_planes_match_oracle(n1, n2, n_nuc, exps):
     import torch
     p = _problem(n_nuc, max(n1, n_nuc + 5), n2, exps, 50 + n_nuc)
@@ -47,10 +48,11 @@ def test_fp64_planes_match_oracle(n1, n2, n_nuc, exps):
     assert np.all(np.abs(got - ref) <= 1e-13 * scale), np.max(np.abs(got - ref) / scale)
 
 
-@pytest.mark.parametrize("n_nuc", [1, 12, 13])
+@pytest.mark.parametrize("n_nuc,exps", [(1, "all"), (12, "all"), (13, "all"), (25, "all"),
+                                        (21, "even"), (40, "even")])
 @pytest.mark.parametrize("slices", [5, 6])
-def test_general_exponents_in_the_split_form(monkeypatch, n_nuc, slices):
-    p = synth.add_coalescence(_problem(n_nuc, 130, 515, "all", 80 + n_nuc, a_en=1.1, a_ee=0.7))
+def test_double_float_form_matches_its_kernel(monkeypatch, n_nuc, exps, slices):
+    p = synth.add_coalescence(_problem(n_nuc, 130, 515, exps, 80 + n_nuc, a_en=1.1, a_ee=0.7))
     X1, I1 = cg.build_integrals(p, cg.SPLIT_BF16, n_slices=slices, x_components=4)
     monkeypatch.setenv("CUTC_PAIR_DF", "1")
     X2, I2 = cg.build_integrals(p, cg.SPLIT_BF16, n_slices=slices, x_components=4)
