@@ -124,6 +124,10 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
         *s_abort = 0;
         tc::fence_mbar_init();
     }
+    // A pair's allocation takes both CTAs: neither asks before the other has started, nor
+    // leaves (below) before the other has given its part back.  Without this, with kernels of
+    // other streams on the device, an allocation could wait for good.
+    tc::cluster_sync();
     if (warp == kMmaWarp) {
         tc::tmem_alloc_pair(tc::smem_u32(s_tmem), Cfg::kTmemCols);
         tc::tmem_relinquish_pair();
@@ -302,12 +306,17 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
         }
     }
 
+    __syncwarp();
     tc::fence_before_sync();
     __syncthreads();
+    // the drain commit is the last to signal this CTA's barriers too
+    if (!leader && threadIdx.x == 0 && !tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
+        fail(26);
     tc::cluster_sync();  // neither CTA leaves while the other may signal it or read its operands
     tc::fence_after_sync();
     if (warp == kMmaWarp)
         tc::tmem_dealloc_pair(tbase, Cfg::kTmemCols);
+    tc::cluster_sync();
 }
 
 // ---------------------------------------------------------------------------

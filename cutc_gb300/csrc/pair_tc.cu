@@ -722,6 +722,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     }
 
+    __syncwarp();
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();

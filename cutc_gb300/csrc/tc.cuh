@@ -108,6 +108,7 @@ __device__ __forceinline__ uint32_t cluster_rank()
 
 __device__ __forceinline__ void cluster_sync()
 {
+    __syncwarp();  // (.aligned)
     asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
                  "barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

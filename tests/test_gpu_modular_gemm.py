@@ -50,3 +50,23 @@ def test_rows_that_are_not_finite():
     bad = np.zeros_like(R, dtype=bool)
     bad[3], bad[:, 5] = True, True
     assert np.all(np.isnan(C[bad])) and np.array_equal(C[~bad], R[~bad])
+
+
+def test_products_of_several_streams():
+    """Builds of different sizes on four streams at a time: the CTA pairs of one stream start
+    and end beside the kernels of the others, and every result stays the same."""
+    from cutc_gb300 import synth
+    ps = [synth.make_problem(nn, na, 250 * nn, 1000 * nn, 9, 40 + nn)
+          for nn, na in ((2, 52), (8, 10), (3, 30))]
+    srv = cg.Server(n_slots=4, device_budget_bytes=32 << 30, cache_budget_bytes=1 << 30,
+                    tile_budget_bytes=1 << 30)
+    try:
+        first = None
+        for _ in range(200):
+            tickets = [srv.submit(p, k + 1, cg.SPLIT_BF16, 5) for k, p in enumerate(ps + ps[:1])]
+            out = [[a.copy() for a in srv.wait(t)[:2]] for t in tickets]
+            first = first or out
+            for got, ref in zip(out, first):
+                assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1])
+    finally:
+        srv.close()
