@@ -81,7 +81,8 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
     uint64_t *tfull = bars + 2 * Cfg::kStages;   // each: the accumulators hold a chunk
     uint64_t *tempty = tfull + 2;                // leader: both CTAs' epilogues have read them
     uint64_t *drain = tempty + 2;
-    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
+    uint64_t *gone = drain + 1;                  // each: the other has given its tensor memory back
+    uint32_t *s_tmem = reinterpret_cast<uint32_t *>(gone + 1);
     volatile int *s_abort = reinterpret_cast<volatile int *>(s_tmem + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -121,6 +122,7 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
             tc::mbar_init(tc::smem_u32(&tempty[i]), 2 * kEpiWarps);
         }
         tc::mbar_init(tc::smem_u32(drain), 1);
+        tc::mbar_init(tc::smem_u32(gone), 1);
         *s_abort = 0;
         tc::fence_mbar_init();
     }
@@ -176,6 +178,17 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                     }
                 }
             }
+            // the last MMAs have read their stages, and signalled so, before this CTA goes away
+            for (uint32_t i = 0, t = stage, ph = phase ^ 1; i < (uint32_t)Cfg::kStages && ok; i++) {
+                if (!tc::mbar_wait(tc::smem_u32(&empty[t]), ph, s_abort)) {
+                    fail(26);
+                    ok = false;
+                }
+                if (++t == Cfg::kStages) {
+                    t = 0;
+                    ph ^= 1;
+                }
+            }
             if (*s_abort && leader) {
                 // let the copies already issued land before the pair goes away
                 for (uint32_t i = 0; i < min(issued, (uint32_t)Cfg::kStages); i++) {
@@ -228,10 +241,12 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                     buf ^= 1;
                 }
             }
-            // all MMAs of the pair have completed once the drain barrier flips
-            tc::mma_commit_pair(tc::smem_u32(drain));
-            if (!tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
-                fail(25);
+            // (without a failure the copying warps wait for the last MMAs)
+            if (!ok) {
+                tc::mma_commit_pair(tc::smem_u32(drain));
+                if (!tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
+                    fail(25);
+            }
         }
     } else {
         // ---- epilogue: running residues of the warp's 32 rows x kCols columns ----------
@@ -309,14 +324,17 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
     __syncwarp();
     tc::fence_before_sync();
     __syncthreads();
-    // the drain commit is the last to signal this CTA's barriers too
-    if (!leader && threadIdx.x == 0 && !tc::mbar_wait(tc::smem_u32(drain), 0, nullptr))
-        fail(26);
     tc::cluster_sync();  // neither CTA leaves while the other may signal it or read its operands
     tc::fence_after_sync();
-    if (warp == kMmaWarp)
+    if (warp == kMmaWarp) {
         tc::tmem_dealloc_pair(tbase, Cfg::kTmemCols);
-    tc::cluster_sync();
+        __syncwarp();
+        if (lane == 0) {  // (the other waits for this arrival before it goes away)
+            tc::mbar_arrive_cluster(tc::map_to_rank(tc::smem_u32(gone), rank ^ 1));
+            if (!tc::mbar_wait(tc::smem_u32(gone), 0, nullptr))
+                fail(27);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
