@@ -70,23 +70,24 @@ extern "C" int cutc_no_2e(const cutc_options *opt, int n_mo, int n_grid1, const 
         CUTC_TRY(E->ws.get(N_OUT, bo, &p));
         out = (double *)p;
     }
+    int *flags = nullptr;
+    SplitPlan sp;
     if (opt->precision == CUTC_PLAIN_FP64) {
         // no_2e = 1/2 tmpC1^T X, then += 1/2 tmpC2^T tmpD2 (src/cutc_no.c:419-446)
-        int *flags;
         CUTC_TRY(fp64_contract_begin(E->ws, st, &flags));
         CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X,
                                k1, 0, 0.0, out, nm2, 0, 1));
         CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2,
                                n1, 0, 1.0, out, nm2, 0, 1));
-        CUTC_TRY(fp64_contract_check(st, flags));
     } else {
         CUTC_TRY(split_gemm_concat(E, st, opt->n_slices, (int)nm2, (int)nm2, k1, C1, X, n1, C2,
-                                   D2, 0.5, out, nm2));
+                                   D2, 0.5, out, nm2, sp));
     }
     CUTC_TRY(launch_add_transpose(st, out, (int)nm2));  // src/cutc_no.c:457
     CUTC_TRY(launch_swap_qs(st, out, n_mo));             // src/cutc_no.c:468
     if (!opt->device_pointers)
         CUTC_CUDA_TRY(cudaMemcpyAsync(no_2e, out, bo, cudaMemcpyDeviceToHost, st));
-    CUTC_CUDA_TRY(cudaStreamSynchronize(st));
-    return CUTC_OK;
+    // one wait for all of it (a second one between the contraction and the reordering left
+    // the device idle for the host's turn)
+    return flags ? fp64_contract_check(st, flags) : split_check(st, sp);
 }

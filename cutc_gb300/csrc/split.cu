@@ -372,10 +372,12 @@ int split_check(cudaStream_t st, SplitPlan &sp)
     return CUTC_OK;
 }
 
-// C = alpha A B^T of two sources through the split form, synchronous on st.
+// C = alpha A B^T of two sources through the split form, asynchronous on st; sp.err is set
+// for split_check.
 template <class Src>
 static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int M, int N,
-                        int64_t K, Src sa, Src sb, double alpha, double *C, int64_t ldc)
+                        int64_t K, Src sa, Src sb, double alpha, double *C, int64_t ldc,
+                        SplitPlan &sp)
 {
     Workspace &W = E->ws;
     const int n_mod = split_moduli(n_slices);
@@ -392,7 +394,8 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
     CUTC_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
     CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sc_a, (int *)nullptr));
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, sc_b, (int *)nullptr));
-    CUTC_TRY(modular_contract(
+    sp.err = err;
+    return modular_contract(
         st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
         ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err, nullptr,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
@@ -400,29 +403,29 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_rows(st, n_mod, sb, n0, nc, K, k0, kp, o.pitch, sc_b, o.p, (int *)nullptr);
-        }));
-    SplitPlan sp;
-    sp.err = err;
-    return split_check(st, sp);
+        });
 }
 
 // Split-precision GEMM on device arrays: C[m + ldc n] = sum_k A[m K + k] B[n K + k].
 int split_gemm_dense(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K,
                      const double *A, const double *B, double *C, int64_t ldc)
 {
-    return gemm_sources(E, st, 200, n_slices, M, N, K, SrcDense{A, K}, SrcDense{B, K}, 1.0, C, ldc);
+    SplitPlan sp;
+    CUTC_TRY(gemm_sources(E, st, 200, n_slices, M, N, K, SrcDense{A, K}, SrcDense{B, K}, 1.0, C, ldc,
+                          sp));
+    return split_check(st, sp);
 }
 
 // C[m + ldc n] = alpha sum_k [A1 | A2][m, k] [B1 | B2][n, k] through the split form: the
 // two products of the same output as ONE contraction over K1 + K2 (one row scale per row
 // of the concatenation).  A1, B1 are K1-contiguous, A2, B2 K2-contiguous (device arrays);
-// synchronous on st.
+// asynchronous on st (sp.err is set for split_check).
 int split_gemm_concat(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K1,
                       const double *A1, const double *B1, int64_t K2, const double *A2,
-                      const double *B2, double alpha, double *C, int64_t ldc)
+                      const double *B2, double alpha, double *C, int64_t ldc, SplitPlan &sp)
 {
     return gemm_sources(E, st, 210, n_slices, M, N, K1 + K2, SrcConcat{A1, A2, K1, K2},
-                        SrcConcat{B1, B2, K1, K2}, alpha, C, ldc);
+                        SrcConcat{B1, B2, K1, K2}, alpha, C, ldc, sp);
 }
 
 }  // namespace cutc

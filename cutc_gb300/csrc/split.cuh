@@ -61,9 +61,10 @@ int split_check(cudaStream_t st, SplitPlan &sp);
 int split_gemm_dense(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K,
                      const double *A, const double *B, double *C, int64_t ldc);
 // C[m + ldc n] = alpha (A1[m K1 + k] B1[n K1 + k] summed over k < K1 + A2 B2^T likewise
-// over K2), as one split contraction over the concatenated K (device arrays)
+// over K2), as one split contraction over the concatenated K (device arrays); asynchronous,
+// sp.err is set for split_check
 int split_gemm_concat(Engine *E, cudaStream_t st, int n_slices, int M, int N, int64_t K1,
                       const double *A1, const double *B1, int64_t K2, const double *A2,
-                      const double *B2, double alpha, double *C, int64_t ldc);
+                      const double *B2, double alpha, double *C, int64_t ldc, SplitPlan &sp);
 
 }  // namespace cutc
