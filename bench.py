@@ -14,8 +14,8 @@ sample of r1 rows, scaled to a full build.
 
 On one GPU the line also carries the rest of the metric, each measured in the
 same run: the error of both forms against the FP64 oracle (``accuracy``), the
-plain FP64 form's rate, the split form at 6 slices (the plain form's error
-class, ``split_6_slices``), the large workload as one full build and on r1
+plain FP64 form's rate, the split form at 6 slices (errors of some 1e-15,
+``split_6_slices``), the large workload as one full build and on r1
 samples (``large``), the Jastrow-parameter scan (``scan``), a prefix of the
 serving stream with p50/p99 latency (``serving``) and the split contraction
 beside cuBLAS's own FP64 emulation on the same operands (``rival``).
@@ -48,7 +48,7 @@ from cutc_gb300 import synth  # noqa: E402
 
 METRIC = "TC integral builds/s (split-precision vs FP64 at 1e-10 rel err)"
 UNIT = "builds/s"
-FP64_CLASS_SLICES = 6        # the split form's slice count with the plain form's error class
+FP64_CLASS_SLICES = 6        # the split form's slice count with errors of some 1e-15
 CPU_SAMPLE_ROWS = 256       # per step of --impl reference: about 6 s of oracle work on 16 cores
 CPU_BASELINE_ROWS = 384     # the cpu_baseline leg: about 10 s; smaller samples underrate the
                             # CPU (48 rows gave 0.00096 builds/s, 256 rows 0.00168)
@@ -121,7 +121,7 @@ def cuda_ms(fn, stream=None):
 
 
 def fp64_class_leg(cg, p, n_slices, steps=2):
-    """The split form at n_slices (6: the plain form's error class) on the full
+    """The split form at n_slices (6: errors of some 1e-15) on the full
     workload, device-resident, timed with CUDA events after one warm-up build."""
     import torch
     dev = torch.device("cuda", torch.cuda.current_device())
@@ -194,7 +194,7 @@ def plain_rate_estimate(cg, p, sizes):
     release_device()
     return {"value_est": 1e3 / t_full, "unit": UNIT, "ms_per_build_est": t_full,
             "x_gemm_fp64_tflops": gemm[-1],
-            "x_gemm_kernel": "fp64_gemm_kernel (DMMA m8n8k4 tiles, this library)",
+            "x_gemm_kernel": "modular_gemm_kernel, 15 moduli (this library)",
             "basis": "plain FP64 form, device-resident, timed on %d and %d r1 rows (%.0f and %.0f ms) "
                      "and extrapolated linearly to n_grid1=%d" % (n_a, n_b, t_a, t_b, p.n_grid1)}
 
@@ -495,18 +495,19 @@ def run_ours(args):
         achieved = per_launch_flops / (per_launch_ms * 1e-3) / 1e12
         peak = float(peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops")))
         S = args.slices
-        n_products = S * (S + 1) // 2 if prec == cg.SPLIT_BF16 else 0
+        n_products = 2 * S + 1 if prec == cg.SPLIT_BF16 else 0
         packed = p.n_ao * (p.n_ao + 1) / 2.0 / nA2
         executed = achieved * packed * n_products if n_products else None
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                     "frac": achieved / peak, "traffic": traffic_per_launch(args, p, gemm_launches),
-                    "kernel": "split_gemm_kernel (X build: the K launches of each r1 tile)",
+                    "kernel": "modular_gemm_kernel (X build: the K panels of each r1 tile, with G's "
+                              "residues and the results from their residues)",
                     "peak_source": "bf16_tflops_sustained of %s" % peak_kind,
                     "alg_flops_per_launch": per_launch_flops, "ms_per_launch": per_launch_ms,
                     "executed_bf16_tflops": executed,
                     "executed_frac": (executed / peak) if executed else None,
                     "note": ("achieved counts the dense FP64 formula 8 nA^2 n1 n2; the kernel "
-                             "executes %d BF16 slice products on the packed (a>=b) AO pairs"
+                             "executes %d BF16 residue products on the packed (a>=b) AO pairs"
                              % n_products)}
         out = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world,
                "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
@@ -557,7 +558,7 @@ def run_ours(args):
         release_device()
     if one_gpu and not args.skip_accuracy:
         log("plain FP64 rate")
-        out["plain_fp64"] = guarded(plain_rate_estimate, cg, p, (256, 512))
+        out["plain_fp64"] = guarded(plain_rate_estimate, cg, p, (2500, 5000))
         if prec == cg.SPLIT_BF16 and args.slices < FP64_CLASS_SLICES:
             log("split form at %d slices" % FP64_CLASS_SLICES)
             out["split_%d_slices" % FP64_CLASS_SLICES] = guarded(fp64_class_leg, cg, p,
@@ -755,7 +756,7 @@ def large_leg(cg, args, warmup, steps, with_accuracy, sizes=(3000, 6000), full_b
     per_launch_ms = gemm_ms / max(1, gemm_launches)
     achieved = flops_x / max(1, gemm_launches) / (per_launch_ms * 1e-3) / 1e12
     S = args.slices
-    n_products = S * (S + 1) // 2 if prec == cg.SPLIT_BF16 else 0
+    n_products = 2 * S + 1 if prec == cg.SPLIT_BF16 else 0
     packed = p.n_ao * (p.n_ao + 1) / 2.0 / nA2
     executed = achieved * packed * n_products if n_products else None
     out = {"value": value, "unit": UNIT, "ms_per_build": t_full,
@@ -767,7 +768,7 @@ def large_leg(cg, args, warmup, steps, with_accuracy, sizes=(3000, 6000), full_b
            "samples": samples, "gpu_launches": launches, "clocks": clocks,
            "roofline": {"bound": "tensor", "achieved": achieved, "peak": peak,
                         "unit": "TFLOP/s", "frac": achieved / peak,
-                        "kernel": "split_gemm_kernel (X build)",
+                        "kernel": "modular_gemm_kernel (X build)",
                         "peak_source": "bf16_tflops_sustained of %s" % peak_kind,
                         "ms_per_launch": per_launch_ms, "executed_bf16_tflops": executed,
                         "executed_frac": (executed / peak) if executed else None},
@@ -970,8 +971,8 @@ def serving_leg(cg, args, n, rate, max_ao, with_accuracy, plain_fp64_tflops):
         out["plain_projection"] = {
             "builds_per_s": len(reqs) / sum(secs), "mean_s_per_request": float(np.mean(secs)),
             "basis": "each request's packed FP64 contraction flops at the plain form's measured "
-                     "X-contraction rate (%.3f TF/s); the stream's arrival rate exceeds this "
-                     "service rate, so its latency grows without bound" % plain_fp64_tflops}
+                     "X-contraction rate (%.3f TF/s), one request at a time"
+                     % plain_fp64_tflops}
     if with_accuracy:
         ps = sorted({k: q for k, q in reqs if q.n_ao <= 200}.values(), key=lambda q: q.n_ao)
         if ps:
@@ -1142,7 +1143,7 @@ def rival_leg(cg, p, dr, Xd, n_slices, n_cols=2048, bits=(None, 40)):
 
 def traffic_per_launch(args, p, launches):
     """DRAM bytes per X-contraction launch from the committed ncu summary, or None."""
-    path = os.path.join(ROOT, "profiles", "split_gemm_traffic.json")
+    path = os.path.join(ROOT, "profiles", "modular_gemm_traffic.json")
     if not os.path.exists(path):
         return None
     try:
@@ -1185,8 +1186,8 @@ def run_kernel(args):
                "fp64_equiv_tflops": alg / ms / 1e9}
         if k == "split_gemm":
             S = args.slices
-            rec.update(slices=S, bf16_tflops_executed=alg * S * (S + 1) / 2 / ms / 1e9,
-                       note="call time includes slicing both operands")
+            rec.update(slices=S, bf16_tflops_executed=alg * (2 * S + 1) / ms / 1e9,
+                       note="call time includes both operands' residues and the results' sums")
         print(json.dumps(rec))
     elif k == "pair":
         # a molecule with the medium workload's nuclei and Jastrow terms; by default few AOs

@@ -1,14 +1,15 @@
-// FP64 GEMM of the plain form: DMMA (mma.sync m8n8k4 .f64) tiles fed by a
-// multi-stage cp.async pipeline.
+// FP64 contractions: fp64_contract, the modular contraction at FP64's precision (below),
+// and the FP64 GEMM of DMMA (mma.sync m8n8k4 .f64) tiles fed by a multi-stage cp.async
+// pipeline, which takes contractions shorter than 16, operands with infinities or NaNs and
+// cutc_fp64_gemm_dev.
 //
-// The plain form keeps every contraction of the cutc_int path in FP64, as the
-// reference does with cublasDgemm (src/build_int2_grad1_u12_ao.cu:152-159,
-// src/build_int_2e_ao.cu:60-67 and 97-104):
+// The contractions are the reference's cublasDgemm calls
+// (src/build_int2_grad1_u12_ao.cu:152-159, src/build_int_2e_ao.cu:60-67 and 97-104):
 //   X_m[p, r1] = sum_r2 P[p, r2] G_m[r1, r2]        (A K-contiguous, "OP_T")
 //   H[p, q]    = sum_r1 X_3[p, r1] S0[q, r1]        (A M-contiguous, "OP_N")
 //   N[p, l]    = -1/2 sum_{m, r1} X_m[p, r1] S_m[l, r1]
 // GB300 executes FP64 at about 2 FMA per clock per SM (1.25 TFLOP/s for the
-// chip), so these contractions are bound by the FP64 pipe and nothing else:
+// chip), so the DMMA kernel is bound by the FP64 pipe and nothing else:
 // a 128 x 128 x 16 tile step is 262 144 FMAs, ~130 000 clocks of one SM's
 // FP64 pipe, against 32 KB of operands -- 0.25 B per clock of operand
 // traffic, far below every memory limit.  What the kernel needs is the FP64

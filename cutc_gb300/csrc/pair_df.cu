@@ -1,4 +1,6 @@
-// Pair terms grad1 u(r1, r2) in double-float arithmetic (split form, sm_103a).
+// Pair terms grad1 u(r1, r2) in double-float arithmetic (sm_103a): the per-point operands of
+// the tensor-core pair terms (pair_tc.cu), and a kernel that loops over the nuclei, for
+// coefficients that are not finite and where CUTC_PAIR_DF or CUTC_PAIR_DENSE asks for it.
 //
 // Same quantity as pair.cu (the reference's cutc_int_bh_kernel,
 // src/jast_bh.cu:31-264), reorganised so that the O(n1 n2) part runs on the

@@ -112,9 +112,9 @@ typedef struct cutc_stats {
     double ms_d2h;          /* device -> host copies */
     int n_r1_tiles;         /* r1 tiles the X build was split into */
     int gpu_launches;       /* kernels of this library launched by the call */
-    double ms_x_gemm;       /* device time of the X-build contraction launches alone */
-    int n_x_gemm;           /* number of those launches: one per r1 tile (plain form),
-                               the K launches of each r1 tile (split form) */
+    double ms_x_gemm;       /* device time of the X-build contractions alone */
+    int n_x_gemm;           /* number of their K panels: one per r1 tile (plain form),
+                               those of each r1 tile (split form) */
 } cutc_stats;
 
 /* Fills the defaults: plain FP64, 5 slices, a_en = a_ee = 1, 3 X components. */
@@ -223,7 +223,7 @@ int cutc_split_gemm_dev(int n_slices, int M, int N, long long K,
                         const double *A, const double *B, double *C, long long ldc);
 
 /*
- * The plain form's FP64 contraction alone, on device arrays of the current
+ * An FP64 GEMM on the FP64 tensor cores alone, on device arrays of the current
  * device, with cuBLAS's column-major argument meaning (the reference's
  * cublasDgemm calls, src/build_int2_grad1_u12_ao.cu:152-159 and
  * src/build_int_2e_ao.cu:60-67,97-104, take these operand orders):
