@@ -170,8 +170,14 @@ static void touch_pages(void *dst, size_t bytes)
     }
     const size_t per = (bytes + n - 1) / n;
     std::vector<std::thread> th;
-    for (int k = 1; k < n; k++)
-        th.emplace_back([=] { touch(std::min(bytes, k * per), std::min(bytes, (k + 1) * per)); });
+    for (int k = 1; k < n; k++) {
+        auto part = [=] { touch(std::min(bytes, k * per), std::min(bytes, (k + 1) * per)); };
+        try {
+            th.emplace_back(part);
+        } catch (...) {  // no thread to be had
+            part();
+        }
+    }
     touch(0, per);
     for (auto &t : th)
         t.join();
