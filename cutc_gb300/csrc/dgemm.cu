@@ -287,7 +287,8 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 constexpr int kMinContractK = 16;
 constexpr size_t kAResidueBytes = (size_t)8 << 30;  // of a K panel of A
 constexpr size_t kBResidueBytes = (size_t)4 << 30;  // of a group of columns of B
-enum ContractSlot { C_FLAGS = 100, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
+enum ContractSlot { C_FLAGS, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
+static_assert(C_OUT + 1 == kContractSlots, "slots");
 
 static int64_t contract_panel(int64_t M, int64_t K)
 {
@@ -304,20 +305,21 @@ size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K)
            modular_out_bytes(kPlainModuli, M, N) + 4 * (size_t)(M + N);
 }
 
-int fp64_contract_begin(Workspace &W, cudaStream_t st, int **flags)
+int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, ContractScratch &S)
 {
     void *p;
-    CUTC_TRY(W.get(C_FLAGS, 64, &p));
-    *flags = (int *)p;  // [0]: a wait gave up, [1]: an operand of the contraction at hand is
-                        // not finite
+    CUTC_TRY(W.get(slot0 + C_FLAGS, 64, &p));
+    S.W = &W;
+    S.slot0 = slot0;
+    S.flags = (int *)p;
     CUTC_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
     return CUTC_OK;
 }
 
-int fp64_contract_check(cudaStream_t st, const int *flags)
+int fp64_contract_check(const ContractScratch &S, cudaStream_t st)
 {
     int err = 0;
-    CUTC_CUDA_TRY(cudaMemcpyAsync(&err, flags, 4, cudaMemcpyDeviceToHost, st));
+    CUTC_CUDA_TRY(cudaMemcpyAsync(&err, S.flags, 4, cudaMemcpyDeviceToHost, st));
     CUTC_CUDA_TRY(cudaStreamSynchronize(st));
     if (err) {
         cutc_set_error(CUTC_ERR_TIMEOUT, "a tensor-core pipeline wait gave up (code %d)", err);
@@ -327,19 +329,20 @@ int fp64_contract_check(cudaStream_t st, const int *flags)
 }
 
 // A K-contiguous (rows lda apart) or M-contiguous (columns lda apart), B K-contiguous.
-static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int M, int N,
                     int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
                     const ModularOut &out)
 {
     constexpr int n_mod = kPlainModuli;
-    int *err = flags, *bad = flags + 1;
+    Workspace &W = *S.W;
+    int *err = S.flags, *bad = S.flags + 1;
     const int64_t pan = contract_panel(M, K);
     void *p;
-    CUTC_TRY(W.get(C_SCA, (size_t)M * 4, &p));
+    CUTC_TRY(W.get(S.slot0 + C_SCA, (size_t)M * 4, &p));
     int *sca = (int *)p;
-    CUTC_TRY(W.get(C_SCB, (size_t)N * 4, &p));
+    CUTC_TRY(W.get(S.slot0 + C_SCB, (size_t)N * 4, &p));
     int *scb = (int *)p;
-    CUTC_TRY(W.get(C_RA, residue_bytes(n_mod, M, pan), &p));
+    CUTC_TRY(W.get(S.slot0 + C_RA, residue_bytes(n_mod, M, pan), &p));
     ResiduePlanes a;
     a.p = p;
     CUTC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, st));
@@ -350,8 +353,8 @@ static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, in
         CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad));
     return modular_contract(
-        st, W, C_RB, C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, sca, scb, out,
-        err, bad,
+        st, W, S.slot0 + C_RB, S.slot0 + C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, sca,
+        scb, out, err, bad,
         [&](int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
             return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, K, k0, kp, o.pitch, sca, o.p, bad)
                             : residue_cols<n_mod>(st, A, lda, M, k0, kp, o.pitch, sca, o.p);
@@ -361,7 +364,7 @@ static int contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, in
         });
 }
 
-int fp64_contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+int fp64_contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int M, int N,
                   int64_t K, double alpha, const double *A, int64_t lda, int64_t sa,
                   const double *B, int64_t ldb, int64_t sb, double beta, double *C, int64_t ldc,
                   int64_t sc, int batch)
@@ -374,25 +377,25 @@ int fp64_contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int 
                          batch);
     if (!joined) {
         for (int z = 0; z < batch; z++)
-            CUTC_TRY(fp64_contract(W, st, flags, a_kmajor, M, N, K, alpha, A + z * sa, lda, 0,
+            CUTC_TRY(fp64_contract(S, st, a_kmajor, M, N, K, alpha, A + z * sa, lda, 0,
                                    B + z * sb, ldb, 0, beta, C + z * sc, ldc, 0, 1));
         return CUTC_OK;
     }
-    CUTC_TRY(contract(W, st, flags, a_kmajor, M, N * batch, K, A, lda, B, ldb,
+    CUTC_TRY(contract(S, st, a_kmajor, M, N * batch, K, A, lda, B, ldb,
                       ModularOut{C, ldc, N, batch > 1 ? sc / ldc : 0, 0, alpha, beta}));
     return fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch,
-                     flags + 1);
+                     S.flags + 1);
 }
 
-int fp64_contract_rows(Workspace &W, cudaStream_t st, int *flags, int M, int N, int64_t K,
+int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, int64_t K,
                        const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
                        int64_t ldc, int nrow_group, int64_t row_stride)
 {
     if (K >= kMinContractK)
-        CUTC_TRY(contract(W, st, flags, true, M, N, K, A, lda, B, ldb,
+        CUTC_TRY(contract(S, st, true, M, N, K, A, lda, B, ldb,
                           ModularOut{C, ldc, N, 0, 0, 1.0, 0.0, nrow_group, row_stride}));
     // the groups of rows as a batch: C of group z starts z row_stride further
-    const int *only_if = K >= kMinContractK ? flags + 1 : nullptr;
+    const int *only_if = K >= kMinContractK ? S.flags + 1 : nullptr;
     const int groups = M / nrow_group;
     CUTC_TRY(fp64_gemm(st, true, nrow_group, N, K, 1.0, A, lda, (int64_t)nrow_group * lda, B, ldb,
                        0, 0.0, C, ldc, row_stride, groups, only_if));

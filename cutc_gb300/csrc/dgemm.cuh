@@ -24,21 +24,32 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // The same contraction for callers with a workspace: a modular contraction on the BF16
 // tensor cores (modular.cuh) with operands rounded at 2^-62 of their row norms, below the
 // rounding of an FP64 sum, with fp64_gemm in its place for operands that hold an
-// infinity or a NaN (found on the device) and for K < 16.  flags: from fp64_contract_begin;
-// a bounded wait that gives up makes the results NaN and is reported by
+// infinity or a NaN (found on the device) and for K < 16.  S: from fp64_contract_begin; a
+// bounded wait that gives up makes the results NaN and is reported by
 // fp64_contract_check.  Batches whose A is common and whose B rows follow one another
 // (sa = 0, sb = N ldb) are one contraction; others run one by one.
-int fp64_contract_begin(Workspace &W, cudaStream_t st, int **flags);
-int fp64_contract(Workspace &W, cudaStream_t st, int *flags, bool a_kmajor, int M, int N,
+//
+// The scratch (kContractSlots slots from the given one) belongs to one stream until its
+// work is done: calls that wait for their results share kContractSlot, a call that returns
+// while its contractions still run has slots of its own.
+struct ContractScratch {
+    Workspace *W = nullptr;
+    int slot0 = 0;
+    int *flags = nullptr;  // [0]: a wait gave up, [1]: an operand of the contraction at hand
+                           // is not finite
+};
+constexpr int kContractSlot = 100, kContractSlots = 6;
+int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, ContractScratch &S);
+int fp64_contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int M, int N,
                   int64_t K, double alpha, const double *A, int64_t lda, int64_t sa,
                   const double *B, int64_t ldb, int64_t sb, double beta, double *C, int64_t ldc,
                   int64_t sc, int batch);
 // C[row(m) + ldc n] = sum_k A[m lda + k] B[n ldb + k] with rows in groups of nrow_group,
 // row_stride apart (no batch).
-int fp64_contract_rows(Workspace &W, cudaStream_t st, int *flags, int M, int N, int64_t K,
+int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, int64_t K,
                        const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
                        int64_t ldc, int nrow_group, int64_t row_stride);
-int fp64_contract_check(cudaStream_t st, const int *flags);
+int fp64_contract_check(const ContractScratch &S, cudaStream_t st);
 // Device bytes fp64_contract keeps for operands of these sizes.
 size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K);
 

@@ -261,6 +261,8 @@ int make_engine(int dev, Engine **out)
     if (e == cudaSuccess)
         for (int k = 0; k < kNumEvents && e == cudaSuccess; k++)
             e = cudaEventCreate(&E->ev[k]);
+    if (e == cudaSuccess)
+        e = cudaEventCreateWithFlags(&E->mo_done, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         cudaGetLastError();
         cutc_set_error(CUTC_ERR_CUDA, "engine setup: %s", cudaGetErrorString(e));
@@ -283,6 +285,7 @@ void destroy_engine(Engine *E)
         cudaEventDestroy(e);
     for (int k = 0; k < kNumEvents; k++)
         cudaEventDestroy(E->ev[k]);
+    cudaEventDestroy(E->mo_done);
     cudaStreamSynchronize(E->xfer);
     cudaStreamDestroy(E->xfer);
     cudaStreamDestroy(E->stream);
@@ -787,7 +790,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     note_launches(1);
 
     SplitPlan sp;
-    int *flags = nullptr;  // of the plain form's contractions
+    ContractScratch contract;  // of the plain form's contractions
     float2 *d_r2d = nullptr, *d_f2d = nullptr, *d_poly = nullptr;
     int pexp = 4;
     bool psparse = false;
@@ -804,7 +807,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         note_launches(1);
     }
     if (R.precision == CUTC_PLAIN_FP64) {
-        CUTC_TRY(fp64_contract_begin(W, st, &flags));
+        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, contract));
         CUTC_TRY(W.get(S_P, (size_t)np * n2 * 8, &p));
         d_P = (double *)p;
         if (!(R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == d_P)) {
@@ -819,7 +822,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     PairTcPlan ptc;
     if (pmode.rows)
         CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, pmode, n2, nN, d_f2, n1t,
-                                 R.precision == CUTC_PLAIN_FP64 ? flags : sp.err, ptc));
+                                 R.precision == CUTC_PLAIN_FP64 ? contract.flags : sp.err, ptc));
     CUTC_CUDA_TRY(cudaEventRecord(E->ev[2], st));
 
     // ---- tiles ---------------------------------------------------------------
@@ -966,7 +969,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
             const double one = 1.0, zero = 0.0;
             if (tev)
                 CUTC_CUDA_TRY(cudaEventRecord(tev[2], st));
-            CUTC_TRY(fp64_contract(W, st, flags, true, (int)np, nb, n2, one, d_P, n2, 0, d_G, n2,
+            CUTC_TRY(fp64_contract(contract, st, true, (int)np, nb, n2, one, d_P, n2, 0, d_G, n2,
                                    (int64_t)nb * n2, zero, d_Xt + (int64_t)ib * np, np,
                                    (int64_t)blk_rows * np, 4));
             if (tev)
@@ -1018,11 +1021,11 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
                 E->tag_i = K == n1 ? R.mol_tag : 0;
                 E->tag_i_buf = d_S0;
                 const double one = 1.0, mhalf = -0.5, beta = first_blk ? 0.0 : 1.0;
-                CUTC_TRY(fp64_contract(W, st, flags, false, (int)np, (int)np, K, one,
+                CUTC_TRY(fp64_contract(contract, st, false, (int)np, (int)np, K, one,
                                        d_Xt + 3 * (int64_t)K * np, np, 0, d_S0, K, 0, beta, d_H,
                                        np, 0, 1));
                 if (nl > 0)
-                    CUTC_TRY(fp64_contract(W, st, flags, false, (int)np, (int)nl, 3 * (int64_t)K,
+                    CUTC_TRY(fp64_contract(contract, st, false, (int)np, (int)nl, 3 * (int64_t)K,
                                            mhalf, d_Xt, np, 0, d_Sl, 3 * (int64_t)K, 0, beta, d_N,
                                            np, 0, 1));
             } else {
@@ -1123,7 +1126,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     if (R.precision == CUTC_SPLIT_BF16)
         CUTC_TRY(split_check(st, sp));
     else
-        CUTC_TRY(fp64_contract_check(st, flags));
+        CUTC_TRY(fp64_contract_check(contract, st));
 
     if (stats) {
         double ms_pair = 0.0, ms_gemm = 0.0, ms_i = 0.0, ms_tiles = 0.0;
@@ -1218,12 +1221,12 @@ int run_pair_only(Engine *E, cudaStream_t st, int i0, int n1b, int n1, int j0, i
     P.G = G; P.ldg = ldg; P.plane = plane;
     const PairTcMode mode = pair_tc_mode(coef.data(), exps.data(), (int)exps.size(), true, 0);
     if (mode.rows) {
-        int *flags;
-        CUTC_TRY(fp64_contract_begin(W, st, &flags));
+        ContractScratch flags;  // (its wait flag alone)
+        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, flags));
         PairTcPlan plan;
-        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, mode, n2b, nN, d_f2, n1b, flags, plan));
+        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, mode, n2b, nN, d_f2, n1b, flags.flags, plan));
         CUTC_TRY(pair_tc_tile_f64(st, plan, P, rn, a_en, E->n_sm));
-        return fp64_contract_check(st, flags);
+        return fp64_contract_check(flags, st);
     }
     CUTC_TRY(launch_r1_terms(st, i0, n1b, nN, r1, rn, a_en, d_t1));
     CUTC_TRY(launch_pair_f64(st, P));

@@ -69,6 +69,8 @@ struct Engine {
     std::vector<cudaEvent_t> tile_ev;  // per-tile timing events (grown on demand)
     Workspace ws;
     PinnedPool pinned;
+    cudaEvent_t mo_done = nullptr;  // the last asynchronous AO-to-MO transform
+    bool mo_used = false;
     // Molecule-dependent operands left in the workspace by the previous build:
     // (molecule tag, buffer address) of the X-build A operand and of the int_2e
     // B operands.  A build with the same non-zero tag and the same buffer skips

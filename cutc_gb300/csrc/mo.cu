@@ -26,7 +26,8 @@
 
 namespace cutc {
 
-enum MoSlot { M_L = 180, M_R, M_T, M_XIN, M_XOUT };
+// (a device call returns while its work runs, so it shares no slot with other calls)
+enum MoSlot { M_L = 180, M_R, M_T, M_XIN, M_XOUT, M_CONTRACT };
 
 static int x_ao_to_mo(Engine *E, cudaStream_t st, int n1, int nA, int n_mo, int comps,
                       const double *L, const double *R, const double *x_ao, double *x_mo,
@@ -60,8 +61,8 @@ static int x_ao_to_mo(Engine *E, cudaStream_t st, int n1, int nA, int n_mo, int 
         CUTC_TRY(W.get(M_XOUT, (size_t)n_mo * n_mo * nb * 8, &p));
         Xout = (double *)p;
     }
-    int *flags;
-    CUTC_TRY(fp64_contract_begin(W, st, &flags));
+    ContractScratch contract;
+    CUTC_TRY(fp64_contract_begin(W, M_CONTRACT, st, contract));
     const int64_t nA2 = (int64_t)nA * nA, nm2 = (int64_t)n_mo * n_mo;
     for (int64_t q0 = 0; q0 < nq; q0 += nb) {
         const int qb = (int)std::min<int64_t>(nb, nq - q0);
@@ -71,12 +72,12 @@ static int x_ao_to_mo(Engine *E, cudaStream_t st, int n1, int nA, int n_mo, int 
             X = Xin;
         }
         // T[(b + nA q) + nA qb i]
-        CUTC_TRY(fp64_contract(W, st, flags, true, nA * qb, n_mo, nA, 1.0, X, nA, 0, dL, nA, 0, 0.0,
+        CUTC_TRY(fp64_contract(contract, st, true, nA * qb, n_mo, nA, 1.0, X, nA, 0, dL, nA, 0, 0.0,
                                T, (int64_t)nA * qb, 0, 1));
         // X_mo[q + ld (i + n_mo j)], rows m = q + qb i
         double *out = dev ? x_mo + q0 : Xout;
         const int64_t ld = dev ? nq : qb;
-        CUTC_TRY(fp64_contract_rows(W, st, flags, n_mo * qb, n_mo, nA, T, nA, dR, nA, out,
+        CUTC_TRY(fp64_contract_rows(contract, st, n_mo * qb, n_mo, nA, T, nA, dR, nA, out,
                                     ld * n_mo, qb, ld));
         if (!dev)
             CUTC_CUDA_TRY(cudaMemcpy2DAsync(x_mo + q0, (size_t)nq * 8, Xout, (size_t)qb * 8,
@@ -84,7 +85,7 @@ static int x_ao_to_mo(Engine *E, cudaStream_t st, int n1, int nA, int n_mo, int 
     }
     // (device calls stay asynchronous: a wait that gave up shows as NaN results)
     if (!dev)
-        CUTC_TRY(fp64_contract_check(st, flags));
+        CUTC_TRY(fp64_contract_check(contract, st));
     return CUTC_OK;
 }
 
@@ -108,8 +109,19 @@ extern "C" int cutc_x_ao_to_mo(int n_grid1, int n_ao, int n_mo, int components,
     CUTC_TRY(get_engine(&E));
     std::lock_guard<std::mutex> lk(E->mu);
     cudaStream_t st = stream ? (cudaStream_t)stream : E->stream;
+    // the scratch may still be in use by a transform on another stream (a captured call's
+    // order is that of its graph)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CUTC_CUDA_TRY(cudaStreamIsCapturing(st, &cap));
+    const bool eager = cap == cudaStreamCaptureStatusNone;
+    if (eager && E->mo_used)
+        CUTC_CUDA_TRY(cudaStreamWaitEvent(st, E->mo_done, 0));
     int s = x_ao_to_mo(E, st, n_grid1, n_ao, n_mo, components, mo_l_coef, mo_r_coef, x_ao, x_mo,
                        device_pointers != 0, (size_t)2 << 30);
+    if (s == CUTC_OK && eager) {
+        CUTC_CUDA_TRY(cudaEventRecord(E->mo_done, st));
+        E->mo_used = true;
+    }
     if (s != CUTC_OK)
         cudaStreamSynchronize(st);
     return s;

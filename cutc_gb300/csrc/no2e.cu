@@ -70,14 +70,14 @@ extern "C" int cutc_no_2e(const cutc_options *opt, int n_mo, int n_grid1, const 
         CUTC_TRY(E->ws.get(N_OUT, bo, &p));
         out = (double *)p;
     }
-    int *flags = nullptr;
+    ContractScratch contract;
     SplitPlan sp;
     if (opt->precision == CUTC_PLAIN_FP64) {
         // no_2e = 1/2 tmpC1^T X, then += 1/2 tmpC2^T tmpD2 (src/cutc_no.c:419-446)
-        CUTC_TRY(fp64_contract_begin(E->ws, st, &flags));
-        CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X,
+        CUTC_TRY(fp64_contract_begin(E->ws, kContractSlot, st, contract));
+        CUTC_TRY(fp64_contract(contract, st, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X,
                                k1, 0, 0.0, out, nm2, 0, 1));
-        CUTC_TRY(fp64_contract(E->ws, st, flags, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2,
+        CUTC_TRY(fp64_contract(contract, st, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2,
                                n1, 0, 1.0, out, nm2, 0, 1));
     } else {
         CUTC_TRY(split_gemm_concat(E, st, opt->n_slices, (int)nm2, (int)nm2, k1, C1, X, n1, C2,
@@ -89,5 +89,5 @@ extern "C" int cutc_no_2e(const cutc_options *opt, int n_mo, int n_grid1, const 
         CUTC_CUDA_TRY(cudaMemcpyAsync(no_2e, out, bo, cudaMemcpyDeviceToHost, st));
     // one wait for all of it (a second one between the contraction and the reordering left
     // the device idle for the host's turn)
-    return flags ? fp64_contract_check(st, flags) : split_check(st, sp);
+    return contract.flags ? fp64_contract_check(contract, st) : split_check(st, sp);
 }

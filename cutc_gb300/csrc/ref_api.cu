@@ -140,8 +140,8 @@ static int int2e_from_full_x(Engine *E, cudaStream_t st, int n1, int nA, const d
     CUTC_TRY(W.get(R_S, 3 * (size_t)K * nA2 * 8, &p));
     double *S = (double *)p;
     const double one = 1.0, mhalf = -0.5;
-    int *flags;
-    CUTC_TRY(fp64_contract_begin(W, st, &flags));
+    ContractScratch contract;
+    CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, contract));
     for (int g0 = 0; g0 < n1; g0 += K) {
         const int Kb = std::min(K, n1 - g0);
         // S0[g + Kb q], S[g + Kb m + 3 Kb q] for the block's points
@@ -149,16 +149,16 @@ static int int2e_from_full_x(Engine *E, cudaStream_t st, int n1, int nA, const d
         CUTC_TRY(launch_full_antisym(st, Kb, nA, w1 + g0, aos1 + g0, n1, S, Kb, 3 * (int64_t)Kb));
         const double beta0 = g0 == 0 ? 0.0 : 1.0;
         // I = X_3 S0 (+ I)   (src/build_int_2e_ao.cu:60-67)
-        CUTC_TRY(fp64_contract(W, st, flags, false, (int)nA2, (int)nA2, Kb, one,
+        CUTC_TRY(fp64_contract(contract, st, false, (int)nA2, (int)nA2, Kb, one,
                                X + nA2 * (3 * (int64_t)n1 + g0), nA2, 0, S0, Kb, 0, beta0, I, nA2,
                                0, 1));
         // I += -1/2 X_m S_m   (src/build_int_2e_ao.cu:97-104, one product per component)
         for (int m = 0; m < 3; m++)
-            CUTC_TRY(fp64_contract(W, st, flags, false, (int)nA2, (int)nA2, Kb, mhalf,
+            CUTC_TRY(fp64_contract(contract, st, false, (int)nA2, (int)nA2, Kb, mhalf,
                                    X + nA2 * ((int64_t)m * n1 + g0), nA2, 0, S + (int64_t)m * Kb,
                                    3 * (int64_t)Kb, 0, one, I, nA2, 0, 1));
     }
-    return fp64_contract_check(st, flags);
+    return fp64_contract_check(contract, st);
 }
 
 static void report(int status, const char *what)
