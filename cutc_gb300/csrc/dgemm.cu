@@ -351,7 +351,10 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
         CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca, bad));
     else
         CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
-    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad));
+    // Whether an operand is not finite has to be known before the first results are written:
+    // with several passes over B's columns its short rows are looked at here, not pass by pass.
+    const bool passes = modular_pass_cols(n_mod, M, N) < N;
+    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad, passes));
     return modular_contract(
         st, W, S.slot0 + C_RB, S.slot0 + C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, sca,
         scb, out, err, bad,

@@ -499,11 +499,12 @@ residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
 // residues (residue_rows, one launch fewer); others beforehand (row_scales).
 constexpr int64_t kShortRow = 1024;
 
+// always: short rows too (their residues then find the same scales again).
 template <class Src>
 static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int64_t k_panel, int n_mod,
-                      int *sc, int *bad)
+                      int *sc, int *bad, bool always = false)
 {
-    if (rows <= 0 || (K <= kShortRow && k_panel >= K))
+    if (rows <= 0 || (K <= kShortRow && k_panel >= K && !always))
         return CUTC_OK;
     row_scale_kernel<Src><<<std::min(rows, 1 << 20), 256, 0, st>>>(src, rows, K,
                                                                     moduli::row_bits(n_mod), sc, bad);
