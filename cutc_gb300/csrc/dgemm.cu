@@ -285,31 +285,56 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // (65 us a wave of tiles), which the modular contraction's launches do not beat.
 
 constexpr int kMinContractK = 16;
-constexpr size_t kAResidueBytes = (size_t)8 << 30;  // of a K panel of A
-constexpr size_t kBResidueBytes = (size_t)4 << 30;  // of a group of columns of B
+constexpr size_t kMinContractBytes = (size_t)16 << 20;  // no smaller blocks are tried
 enum ContractSlot { C_FLAGS, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
 static_assert(C_OUT + 1 == kContractSlots, "slots");
 
-static int64_t contract_panel(int64_t M, int64_t K)
+// How a contraction is cut to fit `limit` bytes: half for the residues of A's rows in a K
+// panel, a quarter each for B's columns and for the results of a pass.  All of K if that
+// fits, then K panels of whole 512-long chunks, then blocks of rows; never below 256 rows,
+// 256 columns and one chunk.
+struct ContractPlan {
+    int64_t kp;
+    ModularBlocks blk;
+    size_t a_bytes, b_bytes, out_bytes;
+};
+
+static ContractPlan contract_plan(int64_t M, int64_t N, int64_t K, size_t limit)
 {
-    const int64_t fit = (int64_t)(kAResidueBytes / (2 * (size_t)kPlainModuli * std::max<int64_t>(M, 1))) /
-                        512 * 512;
-    return std::min(K, std::max<int64_t>(512, fit));
+    constexpr int n = kPlainModuli;
+    const size_t half = limit / 2, quarter = limit / 4;
+    auto whole = [](size_t fit, int64_t all) {  // a multiple of 256, at least one, at most all
+        return (int)std::min<int64_t>(all, std::max<int64_t>(256, (int64_t)(fit / 256 * 256)));
+    };
+    ContractPlan c;
+    c.kp = K;
+    if (residue_bytes(n, M, K) > half)
+        c.kp = std::min<int64_t>(K, std::max<int64_t>(512, (int64_t)(half / residue_bytes(n, M, 16) * 16) /
+                                                               512 * 512));
+    c.blk.rows = residue_bytes(n, M, c.kp) > half ? whole(half / residue_bytes(n, 1, c.kp), M) : (int)M;
+    const int64_t least = std::min<int64_t>(N, 256);  // columns of a pass
+    if ((size_t)2 * n * modular_ldm(c.blk.rows) * least > quarter)
+        c.blk.rows = whole(quarter / (2 * n * least), c.blk.rows);
+    c.blk.pass = whole(quarter / (2 * n * modular_ldm(c.blk.rows)), N);
+    c.blk.group = std::min(c.blk.pass, whole(quarter / residue_bytes(n, 1, c.kp), N));
+    c.a_bytes = residue_bytes(n, c.blk.rows, c.kp);
+    c.b_bytes = residue_bytes(n, c.blk.group, c.kp);
+    c.out_bytes = (size_t)2 * n * modular_ldm(c.blk.rows) * c.blk.pass;
+    return c;
 }
 
-size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K)
+size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K, size_t limit)
 {
-    const int64_t kp = contract_panel(M, K);
-    return residue_bytes(kPlainModuli, M, kp) +
-           residue_bytes(kPlainModuli, modular_b_rows(kPlainModuli, N, kp, kBResidueBytes), kp) +
-           modular_out_bytes(kPlainModuli, M, N) + 4 * (size_t)(M + N);
+    const ContractPlan c = contract_plan(M, N, K, limit);
+    return c.a_bytes + c.b_bytes + c.out_bytes + 4 * (size_t)(M + N);
 }
 
-int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, ContractScratch &S)
+int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, size_t limit, ContractScratch &S)
 {
     void *p;
     CUTC_TRY(W.get(slot0 + C_FLAGS, 64, &p));
     S.W = &W;
+    S.limit = limit;
     S.slot0 = slot0;
     S.flags = (int *)p;
     CUTC_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
@@ -329,38 +354,56 @@ int fp64_contract_check(const ContractScratch &S, cudaStream_t st)
 }
 
 // A K-contiguous (rows lda apart) or M-contiguous (columns lda apart), B K-contiguous.
+// *done is false, and nothing has run, when the device memory for the residues cannot be had
+// even in the smallest blocks.
 static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int M, int N,
                     int64_t K, const double *A, int64_t lda, const double *B, int64_t ldb,
-                    const ModularOut &out)
+                    const ModularOut &out, bool *done)
 {
     constexpr int n_mod = kPlainModuli;
     Workspace &W = *S.W;
     int *err = S.flags, *bad = S.flags + 1;
-    const int64_t pan = contract_panel(M, K);
-    void *p;
-    CUTC_TRY(W.get(S.slot0 + C_SCA, (size_t)M * 4, &p));
-    int *sca = (int *)p;
-    CUTC_TRY(W.get(S.slot0 + C_SCB, (size_t)N * 4, &p));
-    int *scb = (int *)p;
-    CUTC_TRY(W.get(S.slot0 + C_RA, residue_bytes(n_mod, M, pan), &p));
+    ContractPlan c;
     ResiduePlanes a;
-    a.p = p;
+    void *b = nullptr, *res = nullptr, *psa = nullptr, *psb = nullptr;
+    *done = false;
+    for (size_t limit = S.limit;; limit /= 4) {
+        c = contract_plan(M, N, K, limit);
+        int s = W.get(S.slot0 + C_SCA, (size_t)M * 4, &psa);
+        if (s == CUTC_OK)
+            s = W.get(S.slot0 + C_SCB, (size_t)N * 4, &psb);
+        if (s == CUTC_OK)
+            s = W.get(S.slot0 + C_RA, c.a_bytes, &a.p);
+        if (s == CUTC_OK)
+            s = W.get(S.slot0 + C_RB, c.b_bytes, &b);
+        if (s == CUTC_OK)
+            s = W.get(S.slot0 + C_OUT, c.out_bytes, &res);
+        if (s == CUTC_OK)
+            break;
+        if (s != CUTC_ERR_NO_MEMORY)
+            return s;
+        if (limit < kMinContractBytes)
+            return CUTC_OK;
+    }
+    *done = true;
+    int *sca = (int *)psa, *scb = (int *)psb;
+    const int64_t pan = c.kp;
     CUTC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, st));
     const SrcDense sa{A, lda}, sb{B, ldb};
     if (a_kmajor)
-        CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca, bad));
+        CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca, bad, c.blk.rows < M));
     else
         CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
     // Whether an operand is not finite has to be known before the first results are written:
-    // with several passes over B's columns its short rows are looked at here, not pass by pass.
-    const bool passes = modular_pass_cols(n_mod, M, N) < N;
+    // with several passes over the results short rows are looked at here, not block by block.
+    const bool passes = c.blk.pass < N || c.blk.rows < M;
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad, passes));
-    return modular_contract(
-        st, W, S.slot0 + C_RB, S.slot0 + C_OUT, kBResidueBytes, n_mod, M, N, K, pan, a, false, sca,
-        scb, out, err, bad,
-        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
-            return a_kmajor ? residue_rows<n_mod>(st, sa, 0, M, K, k0, kp, o.pitch, sca, o.p, bad)
-                            : residue_cols<n_mod>(st, A, lda, M, k0, kp, o.pitch, sca, o.p);
+    return modular_contract_blocks(
+        st, n_mod, M, N, K, pan, c.blk, a, b, false, (unsigned short *)res, sca, scb, out, err, bad,
+        [&](int m0, int rows, int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
+            return a_kmajor ? residue_rows<n_mod>(st, sa, m0, rows, K, k0, kp, o.pitch, sca, o.p, bad)
+                            : residue_cols<n_mod>(st, A + m0, lda, rows, k0, kp, o.pitch, sca + m0,
+                                                  o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_rows<n_mod>(st, sb, n0, nc, K, k0, kp, o.pitch, scb, o.p, bad);
@@ -384,21 +427,23 @@ int fp64_contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int 
                                    B + z * sb, ldb, 0, beta, C + z * sc, ldc, 0, 1));
         return CUTC_OK;
     }
+    bool done;
     CUTC_TRY(contract(S, st, a_kmajor, M, N * batch, K, A, lda, B, ldb,
-                      ModularOut{C, ldc, N, batch > 1 ? sc / ldc : 0, 0, alpha, beta}));
+                      ModularOut{C, ldc, N, batch > 1 ? sc / ldc : 0, 0, alpha, beta}, &done));
     return fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch,
-                     S.flags + 1);
+                     done ? S.flags + 1 : nullptr);
 }
 
 int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, int64_t K,
                        const double *A, int64_t lda, const double *B, int64_t ldb, double *C,
                        int64_t ldc, int nrow_group, int64_t row_stride)
 {
+    bool done = false;
     if (K >= kMinContractK)
         CUTC_TRY(contract(S, st, true, M, N, K, A, lda, B, ldb,
-                          ModularOut{C, ldc, N, 0, 0, 1.0, 0.0, nrow_group, row_stride}));
+                          ModularOut{C, ldc, N, 0, 0, 1.0, 0.0, nrow_group, row_stride}, &done));
     // the groups of rows as a batch: C of group z starts z row_stride further
-    const int *only_if = K >= kMinContractK ? S.flags + 1 : nullptr;
+    const int *only_if = done ? S.flags + 1 : nullptr;
     const int groups = M / nrow_group;
     CUTC_TRY(fp64_gemm(st, true, nrow_group, N, K, 1.0, A, lda, (int64_t)nrow_group * lda, B, ldb,
                        0, 0.0, C, ldc, row_stride, groups, only_if));

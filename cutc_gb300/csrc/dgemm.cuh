@@ -29,17 +29,23 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // fp64_contract_check.  Batches whose A is common and whose B rows follow one another
 // (sa = 0, sb = N ldb) are one contraction; others run one by one.
 //
+// Its residues take about `limit` bytes at most, whatever the sizes (contract_plan);
+// where that memory cannot be had it takes less, and fp64_gemm's path without any in the end.
+// The blocks do not change the results.
+//
 // The scratch (kContractSlots slots from the given one) belongs to one stream until its
 // work is done: calls that wait for their results share kContractSlot, a call that returns
 // while its contractions still run has slots of its own.
 struct ContractScratch {
     Workspace *W = nullptr;
     int slot0 = 0;
+    size_t limit = 0;
     int *flags = nullptr;  // [0]: a wait gave up, [1]: an operand of the contraction at hand
                            // is not finite
 };
+constexpr size_t kContractBytes = (size_t)16 << 30;  // the largest limit
 constexpr int kContractSlot = 100, kContractSlots = 6;
-int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, ContractScratch &S);
+int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, size_t limit, ContractScratch &S);
 int fp64_contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int M, int N,
                   int64_t K, double alpha, const double *A, int64_t lda, int64_t sa,
                   const double *B, int64_t ldb, int64_t sb, double beta, double *C, int64_t ldc,
@@ -51,6 +57,6 @@ int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, 
                        int64_t ldc, int nrow_group, int64_t row_stride);
 int fp64_contract_check(const ContractScratch &S, cudaStream_t st);
 // Device bytes fp64_contract keeps for operands of these sizes.
-size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K);
+size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K, size_t limit);
 
 }  // namespace cutc

@@ -465,8 +465,8 @@ static size_t fixed_bytes(const Request &R)
         b += ((double)np * np + (double)np * nl) * 8;
     if (R.precision == CUTC_PLAIN_FP64)  // P, and the contractions' residues
         b += (double)np * n2 * 8 +
-             (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2),
-                              R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1));
+             (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2, kContractBytes),
+                              R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1, kContractBytes));
     else
         b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2);
     b += (double)pair_tc_fixed_bytes(R.n2, R.nN, pair_slices(R));
@@ -807,7 +807,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         note_launches(1);
     }
     if (R.precision == CUTC_PLAIN_FP64) {
-        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, contract));
+        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, kContractBytes, contract));
         CUTC_TRY(W.get(S_P, (size_t)np * n2 * 8, &p));
         d_P = (double *)p;
         if (!(R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == d_P)) {
@@ -1222,7 +1222,7 @@ int run_pair_only(Engine *E, cudaStream_t st, int i0, int n1b, int n1, int j0, i
     const PairTcMode mode = pair_tc_mode(coef.data(), exps.data(), (int)exps.size(), true, 0);
     if (mode.rows) {
         ContractScratch flags;  // (its wait flag alone)
-        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, flags));
+        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, 0, flags));
         PairTcPlan plan;
         CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, mode, n2b, nN, d_f2, n1b, flags.flags, plan));
         CUTC_TRY(pair_tc_tile_f64(st, plan, P, rn, a_en, E->n_sm));

@@ -62,7 +62,7 @@ static int x_ao_to_mo(Engine *E, cudaStream_t st, int n1, int nA, int n_mo, int 
         Xout = (double *)p;
     }
     ContractScratch contract;
-    CUTC_TRY(fp64_contract_begin(W, M_CONTRACT, st, contract));
+    CUTC_TRY(fp64_contract_begin(W, M_CONTRACT, st, 4 * budget, contract));
     const int64_t nA2 = (int64_t)nA * nA, nm2 = (int64_t)n_mo * n_mo;
     for (int64_t q0 = 0; q0 < nq; q0 += nb) {
         const int qb = (int)std::min<int64_t>(nb, nq - q0);

@@ -518,9 +518,10 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
         for (int h = 0; h < 2; h++) {
             if (m + h >= P.M)
                 break;
-            const int64_t row = P.out.nrow_group ? (int64_t)((m + h) / P.out.nrow_group) * P.out.row_stride +
-                                                       (m + h) % P.out.nrow_group
-                                                 : m + h;
+            const int gm = P.out.row0 + m + h;
+            const int64_t row = P.out.nrow_group ? (int64_t)(gm / P.out.nrow_group) * P.out.row_stride +
+                                                       gm % P.out.nrow_group
+                                                 : gm;
             double *dst = P.out.C + row + P.out.ldc * col;
             float f[L];
 #pragma unroll

@@ -79,8 +79,8 @@ struct ResiduePlanes {
 };
 
 // Where a contraction goes: C[row(m) + ldc col(n)] = alpha sum_k A[m, k] B[n, k] + beta C,
-// col(n) = (n / ncol_group) group_stride + col0 + n % ncol_group, and
-// row(m) = (m / nrow_group) row_stride + m % nrow_group (nrow_group 0: row(m) = m).
+// col(n) = (n / ncol_group) group_stride + col0 + n % ncol_group, and with M = row0 + m
+// row(m) = (M / nrow_group) row_stride + M % nrow_group (nrow_group 0: row(m) = M).
 struct ModularOut {
     double *C;
     int64_t ldc;
@@ -89,6 +89,7 @@ struct ModularOut {
     double alpha, beta;
     int nrow_group = 0;
     int64_t row_stride = 0;
+    int row0 = 0;
 };
 
 // Elements between the rows of a K panel of kp columns (whole 32-byte sectors; TMA takes
@@ -139,48 +140,74 @@ inline bool modular_whole(int n_mod, int64_t N, int64_t K, int64_t k_panel, size
     return K <= k_panel && modular_b_rows(n_mod, N, K, b_bytes) >= N;
 }
 
-// The contraction over K panels, gen_a(k0, kp, planes) and gen_b(n0, ncols, k0, kp, planes)
-// writing the residues of a panel (B's in groups of columns whose residues fit b_bytes);
-// gen_a may point planes.p at residues that are there already.  b_ready: B's are in slot_b
-// already (modular_whole only).
+// How a contraction is cut: rows of A whose residues are in memory at once, columns of B
+// likewise, and columns of results per pass.
+struct ModularBlocks {
+    int rows, group, pass;
+};
+
+// The contraction over K panels, gen_a(m0, rows, k0, kp, planes) and
+// gen_b(n0, ncols, k0, kp, planes) writing the residues of a panel; gen_a may point planes.p
+// at residues that are there already.  a.p, b_p and res: space for the residues of
+// blk.rows x k_panel, blk.group x k_panel and of the results of one pass.  b_ready: B's are
+// in b_p already (whole: k_panel >= K, blk.group >= N).
+template <class GenA, class GenB>
+int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K, int64_t k_panel,
+                            const ModularBlocks &blk, ResiduePlanes a, void *b_p, bool b_ready,
+                            unsigned short *res, const int *sa, const int *sb, ModularOut out,
+                            int *err, const int *skip, GenA gen_a, GenB gen_b)
+{
+    ResiduePlanes b;
+    b.p = b_p;
+    const bool b_whole = k_panel >= K && blk.group >= N && blk.pass >= N;
+    for (int m0 = 0; m0 < M; m0 += blk.rows) {
+        a.rows = std::min(blk.rows, M - m0);
+        out.row0 = m0;
+        bool a_ready = false;  // A's only panel stays for every pass
+        for (int n0 = 0; n0 < N; n0 += blk.pass) {
+            const int nc = std::min(blk.pass, N - n0);
+            for (int64_t k0 = 0; k0 < K; k0 += k_panel) {
+                const int64_t kp = std::min(k_panel, K - k0);
+                a.kp = b.kp = kp;
+                a.pitch = b.pitch = residue_pitch(kp);
+                if (!a_ready)
+                    CUTC_TRY(gen_a(m0, a.rows, k0, kp, a));
+                a_ready = a_ready || k_panel >= K;
+                for (int g = 0; g < nc; g += blk.group) {
+                    b.rows = std::min(blk.group, nc - g);
+                    if (!b_ready)
+                        CUTC_TRY(gen_b(n0 + g, b.rows, k0, kp, b));
+                    b_ready = b_ready || b_whole;
+                    CUTC_TRY(modular_gemm(st, n_mod, a, b, res + (int64_t)g * modular_ldm(a.rows),
+                                          nc, k0 > 0, err));
+                }
+            }
+            CUTC_TRY(modular_combine(st, n_mod, a.rows, n0, nc, res, sa + m0, sb + n0, out, err,
+                                     skip));
+        }
+    }
+    return CUTC_OK;
+}
+
+// The same with all rows of A at once and B's in groups of columns whose residues fit
+// b_bytes, the buffers from the workspace.
 template <class GenA, class GenB>
 int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, size_t b_bytes,
                      int n_mod, int M, int N, int64_t K, int64_t k_panel, ResiduePlanes a,
                      bool b_ready, const int *sa, const int *sb,
-                     const ModularOut &out, int *err, const int *skip, GenA gen_a, GenB gen_b)
+                     const ModularOut &out, int *err, GenA gen_a, GenB gen_b)
 {
     if (M <= 0 || N <= 0)
         return CUTC_OK;
-    const int pass = modular_pass_cols(n_mod, M, N);
-    const int group = std::min(pass, modular_b_rows(n_mod, N, std::min(K, k_panel), b_bytes));
-    void *p;
-    CUTC_TRY(W.get(slot_b, residue_bytes(n_mod, b_ready ? N : group, std::min(K, k_panel)), &p));
-    ResiduePlanes b;
-    b.p = p;
-    CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &p));
-    unsigned short *res = (unsigned short *)p;
-    a.rows = M;
-    bool a_ready = false;  // A's only panel stays for every pass
-    for (int n0 = 0; n0 < N; n0 += pass) {
-        const int nc = std::min(pass, N - n0);
-        for (int64_t k0 = 0; k0 < K; k0 += k_panel) {
-            const int64_t kp = std::min(k_panel, K - k0);
-            a.kp = b.kp = kp;
-            a.pitch = b.pitch = residue_pitch(kp);
-            if (!a_ready)
-                CUTC_TRY(gen_a(k0, kp, a));
-            a_ready = a_ready || k_panel >= K;
-            for (int g = 0; g < nc; g += group) {
-                b.rows = std::min(group, nc - g);
-                if (!b_ready)
-                    CUTC_TRY(gen_b(n0 + g, b.rows, k0, kp, b));
-                CUTC_TRY(modular_gemm(st, n_mod, a, b, res + (int64_t)g * modular_ldm(M), nc,
-                                      k0 > 0, err));
-            }
-        }
-        CUTC_TRY(modular_combine(st, n_mod, M, n0, nc, res, sa, sb + n0, out, err, skip));
-    }
-    return CUTC_OK;
+    ModularBlocks blk;
+    blk.rows = M;
+    blk.pass = modular_pass_cols(n_mod, M, N);
+    blk.group = std::min(blk.pass, modular_b_rows(n_mod, N, std::min(K, k_panel), b_bytes));
+    void *b, *res;
+    CUTC_TRY(W.get(slot_b, residue_bytes(n_mod, b_ready ? N : blk.group, std::min(K, k_panel)), &b));
+    CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &res));
+    return modular_contract_blocks(st, n_mod, M, N, K, k_panel, blk, a, b, b_ready,
+                                   (unsigned short *)res, sa, sb, out, err, nullptr, gen_a, gen_b);
 }
 
 }  // namespace cutc

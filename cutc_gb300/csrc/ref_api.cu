@@ -141,7 +141,7 @@ static int int2e_from_full_x(Engine *E, cudaStream_t st, int n1, int nA, const d
     double *S = (double *)p;
     const double one = 1.0, mhalf = -0.5;
     ContractScratch contract;
-    CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, contract));
+    CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, kContractBytes, contract));
     for (int g0 = 0; g0 < n1; g0 += K) {
         const int Kb = std::min(K, n1 - g0);
         // S0[g + Kb q], S[g + Kb m + 3 Kb q] for the block's points

@@ -240,8 +240,8 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
     const ModularOut out{Xb, np, nb, blk_rows, ib, 1.0, 0.0};
     CUTC_TRY(modular_contract(
         st, E->ws, sp.slot0 + SS_BX, sp.slot0 + SS_RES, x_residue_bytes(sp.n1t, R.n2), n_mod,
-        (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, false, sp.sc_ax, sp.sc_bx, out, sp.err, nullptr,
-        [&](int64_t k0, int64_t kp, ResiduePlanes &a) -> int {
+        (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, false, sp.sc_ax, sp.sc_bx, out, sp.err,
+        [&](int, int, int64_t k0, int64_t kp, ResiduePlanes &a) -> int {
             if (sp.ax_whole) {
                 a.p = p_panel(sp, n_mod, (int)np, k0);
                 return CUTC_OK;
@@ -301,8 +301,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a, nullptr));
     CUTC_TRY(modular_contract(
         st, W, slot0 + SS_BH, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, np, nb, pan_h, a, keep_b, sc_a,
-        sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err, nullptr,
-        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+        sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err,
+        [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_cols(st, n_mod, x3, np, np, k0, kp, o.pitch, sc_a, o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
@@ -312,8 +312,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
         CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a, nullptr));
         CUTC_TRY(modular_contract(
             st, W, slot0 + SS_BN, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, nl, k3, pan_n, a, keep_b, sc_a,
-            sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err, nullptr,
-            [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+            sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err,
+            [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
                 return residue_cols(st, n_mod, Xt, np, np, k0, kp, o.pitch, sc_a, o.p);
             },
             [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
@@ -397,8 +397,8 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
     sp.err = err;
     return modular_contract(
         st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
-        ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err, nullptr,
-        [&](int64_t k0, int64_t kp, const ResiduePlanes &o) {
+        ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err,
+        [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_rows(st, n_mod, sa, 0, M, K, k0, kp, o.pitch, sc_a, o.p, (int *)nullptr);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
