@@ -38,6 +38,7 @@ struct PlanMemo {
     uint64_t key = 0;   // 0: none
     uint64_t path = 0;  // the pair-term path of that build (its other buffers)
     size_t budget = 0;
+    size_t contract = 0;  // limit of the plain form's contraction scratch
     int64_t n1t = 0, kb = 0;
 };
 struct Workspace {
@@ -115,7 +116,8 @@ int get_engine(Engine **out);
 int make_engine(int dev, Engine **out);
 void destroy_engine(Engine *E);
 // Device bytes one build needs besides its molecule arrays, for a given r1-tile budget.
-size_t build_footprint(const Request &R, size_t tile_budget);
+// (contract: limit of the plain form's contraction scratch, 0: that of the budget).
+size_t build_footprint(const Request &R, size_t tile_budget, size_t contract = 0);
 int build_terms(const Request &R, std::vector<double> &coef, std::vector<int> &exps,
                 std::vector<int> &off);
 int run_build(Engine *E, const Request &R, cutc_stats *stats);

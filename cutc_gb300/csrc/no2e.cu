@@ -74,7 +74,9 @@ extern "C" int cutc_no_2e(const cutc_options *opt, int n_mo, int n_grid1, const 
     SplitPlan sp;
     if (opt->precision == CUTC_PLAIN_FP64) {
         // no_2e = 1/2 tmpC1^T X, then += 1/2 tmpC2^T tmpD2 (src/cutc_no.c:419-446)
-        CUTC_TRY(fp64_contract_begin(E->ws, kContractSlot, st, kContractBytes, contract));
+        const size_t limit = opt->max_work_bytes ? std::min(kContractBytes, opt->max_work_bytes)
+                                                 : kContractBytes;
+        CUTC_TRY(fp64_contract_begin(E->ws, kContractSlot, st, limit, contract));
         CUTC_TRY(fp64_contract(contract, st, true, (int)nm2, (int)nm2, k1, 0.5, C1, k1, 0, X,
                                k1, 0, 0.0, out, nm2, 0, 1));
         CUTC_TRY(fp64_contract(contract, st, true, (int)nm2, (int)nm2, n1, 0.5, C2, n1, 0, D2,
