@@ -426,8 +426,7 @@ __device__ __forceinline__ const CrtTab<N> &crt_tab()
         return c_crt15;
 }
 
-// v 2^k rounded to nearest even, in integer arithmetic (GB300's FP64 pipe is slow); results
-// outside the normal range by scalbn
+// v 2^k rounded to nearest even, in integer arithmetic (GB300's FP64 pipe is slow)
 __device__ __forceinline__ double scaled_double(__int128 v, int k)
 {
     const bool neg = v < 0;
@@ -438,16 +437,28 @@ __device__ __forceinline__ double scaled_double(__int128 v, int k)
     const int lz = ah ? __clzll((long long)ah) : 64 + __clzll((long long)(unsigned long long)a);
     a <<= lz;  // the leading bit at bit 127
     const unsigned long long h = (unsigned long long)(a >> 64), l = (unsigned long long)a;
-    unsigned long long m = h >> 11;  // 53 bits
-    const unsigned rest = (unsigned)h & 0x7ffu;
-    m += rest > 0x400u || (rest == 0x400u && (l != 0 || (m & 1))) ? 1 : 0;
     const int E = 1023 + 127 - lz + k;
-    double r;
-    if (E >= 1 && E <= 2045)  // m's leading bit (or its carry) adds one to the exponent field
-        r = __longlong_as_double((long long)(((unsigned long long)(E - 1) << 52) + m));
-    else
-        r = scalbn(__longlong_as_double((long long)((1022ull << 52) + m)), E - 1023);
-    return neg ? -r : r;
+    unsigned long long bits;
+    if (E >= 1 && E <= 2046) {  // m's leading bit (or its carry) adds one to the exponent field
+        unsigned long long m = h >> 11;  // 53 bits
+        const unsigned rest = (unsigned)h & 0x7ffu;
+        m += rest > 0x400u || (rest == 0x400u && (l != 0 || (m & 1))) ? 1 : 0;
+        bits = ((unsigned long long)(E - 1) << 52) + m;
+    } else if (E > 2046) {
+        bits = 0x7ffull << 52;
+    } else {  // subnormal: the multiple of 2^-1074 in place of the 53 bits
+        const int drop = 76 - E;
+        unsigned long long m = 0;
+        if (drop < 128)
+            m = (unsigned long long)(a >> drop);
+        if (drop <= 128) {
+            const unsigned __int128 rest = drop < 128 ? a << (128 - drop) : a;
+            const unsigned __int128 half = (unsigned __int128)1 << 127;
+            m += rest > half || (rest == half && (m & 1)) ? 1 : 0;
+        }
+        bits = m;
+    }
+    return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
 }
 
 // The integer of its limbs: v[l] an integer-valued float below 2^24 in magnitude.

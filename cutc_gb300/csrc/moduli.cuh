@@ -69,15 +69,15 @@ CUTC_HD constexpr int inverse(int a, int p)  // a^-1 mod p (p small: by search)
 }
 
 // rint(x 2^s) of an FP64 value with |x 2^s| < 2^63 (ties away from zero), in integer
-// arithmetic; subnormal x count as zero
+// arithmetic
 CUTC_HD long long scaled_int(double x, int s)
 {
     const unsigned long long bits = digits::double_bits(x);
     const int E = (int)((bits >> 52) & 0x7ff);
-    const int sh = E - 1075 + s;
-    const unsigned long long mant = (bits & ((1ull << 52) - 1)) | (1ull << 52);
+    const int sh = (E ? E : 1) - 1075 + s;
+    const unsigned long long mant = (bits & ((1ull << 52) - 1)) | (E ? 1ull << 52 : 0ull);
     unsigned long long T = 0;
-    if (E != 0 && sh > -54)
+    if (sh > -54)
         T = sh >= 0 ? mant << (sh & 63) : (mant + (1ull << (-sh - 1))) >> (-sh);
     return (bits >> 63) ? -(long long)T : (long long)T;
 }

@@ -148,9 +148,11 @@ __device__ __forceinline__ int scale_slow(unsigned long long mb, float bits, int
     const int E = (int)(mb >> 52);
     if (E >= 0x7ff)
         return kNotFinite;
-    if (E == 0)
+    if (mb == 0)
         return 0;
-    return (int)floorf(bits - 0.5f * log2f((float)K) - 0.0005f) - (E - 1022);
+    // max < 2^e (a subnormal's leading bit counts from 2^-1074)
+    const int e = E ? E - 1022 : -1010 - __clzll((long long)mb);
+    return (int)floorf(bits - 0.5f * log2f((float)K) - 0.0005f) - e;
 }
 
 // sc[r] for every row: one block per row (a fixed summation order, so the scale never
