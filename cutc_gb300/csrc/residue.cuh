@@ -129,30 +129,63 @@ __device__ __forceinline__ unsigned long long abs_bits(double v)
     return (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffull;
 }
 
-// The scale of a row from its maximum m and sum of squares ss in FP32 when both are well
-// inside the float range: floor(bits - log2 |row|_2).
-// Up to 2^20 columns the rounding of the sum stays far below the 0.0005.
+// The scale of a row of norm sqrt(ss) 2^e: floor(bits - log2 |row|_2), with the sum's even
+// power of two taken out first, so that a row times a power of two has the same digits.  The
+// 0.0005 covers the rounding of the sum (up to 2^20 columns in FP32).
+__device__ __forceinline__ int norm_scale(float ss, float bits, int e)
+{
+    const int b = __float_as_int(ss);
+    const int j = ((b >> 23) - 127) >> 1;
+    const float f = __int_as_float(b - j * (1 << 24));  // ss 4^-j, in [1, 4)
+    return (int)floorf(bits - 0.5f * log2f(f) - 0.0005f) - j - e;
+}
+
+constexpr int64_t kFloatSums = 1 << 20;  // columns up to which FP32 sums do
+
+// ... from the row's maximum m and sum of squares ss in FP32 when both are well inside the
+// float range.
 __device__ __forceinline__ bool scale_fast(float m, float ss, float bits, int64_t K, int *s)
 {
-    if (K > (1 << 20) || !(m >= 0x1p-50f && m <= 0x1p60f && ss <= 0x1p125f))
+    if (K > kFloatSums || !(m >= 0x1p-50f && m <= 0x1p60f && ss <= 0x1p125f))
         return false;
-    *s = (int)floorf(bits - 0.5f * log2f(ss) - 0.0005f);
+    *s = norm_scale(ss, bits, 0);
     return true;
 }
 
-// ... and from the largest |x| as bits otherwise (|row|_2 <= sqrt(K) max): rows of values
-// near the ends of the FP64 range, zero rows (scale 0) and rows with an infinity or a NaN
-// (kNotFinite).
-__device__ __forceinline__ int scale_slow(unsigned long long mb, float bits, int64_t K)
+// Other rows (values near the ends of the FP64 range, long rows) are summed a second time,
+// scaled by their largest |x|, given as bits: e with |x| < 2^e.
+__device__ __forceinline__ int max_exponent(unsigned long long mb)
 {
-    const int E = (int)(mb >> 52);
-    if (E >= 0x7ff)
+    const int E = (int)(mb >> 52);  // (a subnormal's leading bit counts from 2^-1074)
+    return E ? E - 1022 : mb ? -1010 - __clzll((long long)mb) : 0;
+}
+
+__device__ __forceinline__ float scaled_up(double x, int e) { return abs_up(scalbn(x, -e)); }
+
+// ... and their scale: ss is that sum.  Zero rows have scale 0, rows with an infinity or a NaN
+// kNotFinite.
+__device__ __forceinline__ int scale_slow(unsigned long long mb, float ss, float bits)
+{
+    if ((int)(mb >> 52) >= 0x7ff)
         return kNotFinite;
-    if (mb == 0)
-        return 0;
-    // max < 2^e (a subnormal's leading bit counts from 2^-1074)
-    const int e = E ? E - 1022 : -1010 - __clzll((long long)mb);
-    return (int)floorf(bits - 0.5f * log2f((float)K) - 0.0005f) - e;
+    return mb ? norm_scale(ss, bits, max_exponent(mb)) : 0;
+}
+
+// The sum of v over the block's 256 threads, in a fixed order, for thread 0.
+template <class T>
+__device__ __forceinline__ T block_sum(T v, T (&part)[8])
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+        v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();  // the previous values are read
+    if ((threadIdx.x & 31) == 0)
+        part[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 8; w++)
+            v += part[w];
+    return v;
 }
 
 // sc[r] for every row: one block per row (a fixed summation order, so the scale never
@@ -162,7 +195,8 @@ __global__ void __launch_bounds__(256)
 row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc, int *bad)
 {
     __shared__ float sm[8], sq[8];
-    __shared__ unsigned long long sb[8];
+    __shared__ double sd[8];
+    __shared__ unsigned long long sb[8], s_max;
     __shared__ int s_fast;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int r = blockIdx.x; r < rows; r += gridDim.x) {
@@ -174,21 +208,14 @@ row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc,
             ss = fmaf(v, v, ss);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
+        for (int o = 16; o > 0; o >>= 1)
             m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        }
-        __syncthreads();  // the previous row's shared values are read
-        if (lane == 0) {
-            sm[warp] = m;
-            sq[warp] = ss;
-        }
-        __syncthreads();
+        if (lane == 0)
+            sm[warp] = m;  // (read below before the next row's, behind block_sum's barriers)
+        ss = block_sum(ss, sq);
         if (threadIdx.x == 0) {
-            for (int w = 1; w < 8; w++) {
+            for (int w = 1; w < 8; w++)
                 m = fmaxf(m, sm[w]);
-                ss += sq[w];
-            }
             int s = 0;
             s_fast = scale_fast(m, ss, bits, K, &s);
             if (s_fast)
@@ -213,7 +240,28 @@ row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc,
         if (threadIdx.x == 0) {
             for (int w = 1; w < 8; w++)
                 mb = sb[w] > mb ? sb[w] : mb;
-            const int s = scale_slow(mb, bits, K);
+            s_max = mb;
+        }
+        __syncthreads();
+        mb = s_max;
+        const int e = max_exponent(mb);
+        if (K <= kFloatSums) {
+            ss = 0.0f;
+            for (int64_t k = threadIdx.x; k < K; k += 256) {
+                const float v = scaled_up(src(r, k), e);
+                ss = fmaf(v, v, ss);
+            }
+            ss = block_sum(ss, sq);
+        } else {
+            double s2 = 0.0;
+            for (int64_t k = threadIdx.x; k < K; k += 256) {
+                const float v = scaled_up(src(r, k), e);
+                s2 += (double)v * v;
+            }
+            ss = (float)block_sum(s2, sd);
+        }
+        if (threadIdx.x == 0) {
+            const int s = scale_slow(mb, ss, bits);
             sc[r] = s;
             if (s == kNotFinite && bad)
                 atomicExch(bad, 1);
@@ -352,6 +400,17 @@ row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_
     __shared__ unsigned long long sb[NG][RB + 1];
     const int t = threadIdx.x % RB, g = threadIdx.x / RB;
     const int r = blockIdx.x * RB + t;
+    // sums over the groups in a fixed order, left in a[0]
+    auto reduce = [&](auto &a, auto op) {
+        for (int h = NG / 2; h > 0; h >>= 1) {
+            __syncthreads();
+            if (g < h)
+                a[g][t] = op(a[g][t], a[g + h][t]);
+        }
+        __syncthreads();
+    };
+    auto add = [](auto x, auto y) { return x + y; };
+    auto larger = [](auto x, auto y) { return x > y ? x : y; };
     float m = 0.0f, ss = 0.0f;
     unsigned long long mb = 0;
     if (r < rows) {
@@ -368,19 +427,37 @@ row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_
     sm[g][t] = m;
     sq[g][t] = ss;
     sb[g][t] = mb;
-    for (int h = NG / 2; h > 0; h >>= 1) {  // a fixed order
-        __syncthreads();
-        if (g < h) {
-            sm[g][t] = fmaxf(sm[g][t], sm[g + h][t]);
-            sq[g][t] += sq[g + h][t];
-            sb[g][t] = sb[g + h][t] > sb[g][t] ? sb[g + h][t] : sb[g][t];
-        }
+    reduce(sm, larger);
+    reduce(sq, add);
+    reduce(sb, larger);
+    int s = 0;
+    const bool fast = scale_fast(sm[0][t], sq[0][t], bits, K, &s);
+    if (__syncthreads_or(r < rows && !fast)) {
+        mb = sb[0][t];
+        const int e = max_exponent(mb);
+        float s1 = 0.0f;
+        double s2 = 0.0;
+        if (r < rows && !fast)
+            for (int64_t k = g; k < K; k += NG) {
+                const float v = scaled_up(X[k * ld + r], e);
+                if (K <= kFloatSums)
+                    s1 = fmaf(v, v, s1);
+                else
+                    s2 += (double)v * v;
+            }
+        __syncthreads();  // sb[0] and sq[0] are read
+        double(*sd)[RB + 1] = reinterpret_cast<double(*)[RB + 1]>(sb);
+        sq[g][t] = s1;
+        sd[g][t] = s2;
+        if (K <= kFloatSums)
+            reduce(sq, add);
+        else
+            reduce(sd, add);
+        if (!fast)
+            s = scale_slow(mb, K <= kFloatSums ? sq[0][t] : (float)sd[0][t], bits);
     }
     if (g != 0 || r >= rows)
         return;
-    int s = 0;
-    if (!scale_fast(sm[0][t], sq[0][t], bits, K, &s))
-        s = scale_slow(sb[0][t], bits, K);
     sc[r] = s;
     if (s == kNotFinite && bad)
         atomicExch(bad, 1);
@@ -472,8 +549,19 @@ residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
                 const unsigned long long v = __shfl_xor_sync(0xffffffffu, mb, o);
                 mb = v > mb ? v : mb;
             }
+            const int e = max_exponent(mb);
+            float s2 = 0.0f;
+            if (ok)
+                for (int kk = gl * 8; kk < K; kk += 8 * G)  // (the order above)
+                    for (int k = kk; k < min(K, kk + 8); k++) {
+                        const float v = scaled_up(src(r0 + r, k), e);
+                        s2 = fmaf(v, v, s2);
+                    }
+#pragma unroll
+            for (int o = G / 2; o > 0; o >>= 1)
+                s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             if (!fast)
-                s = scale_slow(mb, bits, K);
+                s = scale_slow(mb, s2, bits);
             if (ok && s == kNotFinite && bad && gl == 0)
                 atomicExch(bad, 1);
         }
