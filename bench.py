@@ -33,6 +33,7 @@ import argparse
 import ctypes
 import dataclasses
 import json
+import math
 import os
 import subprocess
 import sys
@@ -105,6 +106,14 @@ def release_device():
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     cg.load().cutc_release()
+
+
+def split_products(n_slices, K):
+    """Residue products of a split-form contraction over K columns: the moduli whose rows are
+    rounded at 2^-beta of their norms, beta at least 9 slices' bits and sqrt(K)."""
+    bits = {8: 33.328, 9: 37.535, 10: 41.733, 11: 45.919, 12: 50.073, 13: 54.218, 15: 62.489}
+    need = 9 * n_slices + 0.5 * math.log2(K)
+    return next((n for n, b in bits.items() if b >= need), 17)
 
 
 def cuda_ms(fn, stream=None):
@@ -495,7 +504,7 @@ def run_ours(args):
         achieved = per_launch_flops / (per_launch_ms * 1e-3) / 1e12
         peak = float(peaks.get("bf16_tflops_sustained", peaks.get("bf16_tflops")))
         S = args.slices
-        n_products = 2 * S + 1 if prec == cg.SPLIT_BF16 else 0
+        n_products = split_products(S, p.n_grid2) if prec == cg.SPLIT_BF16 else 0
         packed = p.n_ao * (p.n_ao + 1) / 2.0 / nA2
         executed = achieved * packed * n_products if n_products else None
         roofline = {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -756,7 +765,7 @@ def large_leg(cg, args, warmup, steps, with_accuracy, sizes=(3000, 6000), full_b
     per_launch_ms = gemm_ms / max(1, gemm_launches)
     achieved = flops_x / max(1, gemm_launches) / (per_launch_ms * 1e-3) / 1e12
     S = args.slices
-    n_products = 2 * S + 1 if prec == cg.SPLIT_BF16 else 0
+    n_products = split_products(S, p.n_grid2) if prec == cg.SPLIT_BF16 else 0
     packed = p.n_ao * (p.n_ao + 1) / 2.0 / nA2
     executed = achieved * packed * n_products if n_products else None
     out = {"value": value, "unit": UNIT, "ms_per_build": t_full,
@@ -1186,7 +1195,7 @@ def run_kernel(args):
                "fp64_equiv_tflops": alg / ms / 1e9}
         if k == "split_gemm":
             S = args.slices
-            rec.update(slices=S, bf16_tflops_executed=alg * (2 * S + 1) / ms / 1e9,
+            rec.update(slices=S, bf16_tflops_executed=alg * split_products(S, args.k) / ms / 1e9,
                        note="call time includes both operands' residues and the results' sums")
         print(json.dumps(rec))
     elif k == "pair":

@@ -355,7 +355,10 @@ struct CombineParams {
 // W_i = (M / p_i) ((M / p_i)^-1 mod p_i), in 12-bit limbs (FP32 pairs, both lanes the same
 // value) and as fractions W_i / M.
 constexpr int kLimbBits = 12;
-constexpr int crt_limbs(int n) { return n <= 7 ? 5 : n <= 9 ? 7 : n <= 11 ? 8 : n <= 13 ? 10 : 11; }
+constexpr int crt_limbs(int n)
+{
+    return n <= 8 ? 6 : n <= 9 ? 7 : n <= 11 ? 8 : n <= 12 ? 9 : n <= 13 ? 10 : n <= 15 ? 11 : 12;
+}
 
 template <int N>
 struct CrtTab {
@@ -363,12 +366,61 @@ struct CrtTab {
     uint64_t w[N][L], frac[N];
 };
 
+// An unsigned integer of W 64-bit words.
+template <int W>
+struct Words {
+    unsigned long long w[W];
+    constexpr Words times(unsigned m) const
+    {
+        Words r{};
+        unsigned __int128 c = 0;
+        for (int i = 0; i < W; i++) {
+            c += (unsigned __int128)w[i] * m;
+            r.w[i] = (unsigned long long)c;
+            c >>= 64;
+        }
+        return r;
+    }
+    constexpr Words over(unsigned d, unsigned *rest) const
+    {
+        Words r{};
+        unsigned __int128 c = 0;
+        for (int i = W - 1; i >= 0; i--) {
+            c = (c << 64) | w[i];
+            r.w[i] = (unsigned long long)(c / d);
+            c %= d;
+        }
+        *rest = (unsigned)c;
+        return r;
+    }
+    constexpr unsigned bits12(int b) const
+    {
+        const int i = b / 64, s = b % 64;
+        unsigned long long v = i < W ? w[i] >> s : 0;
+        if (s > 52 && i + 1 < W)
+            v |= w[i + 1] << (64 - s);
+        return (unsigned)v & 0xfffu;
+    }
+    constexpr double value() const
+    {
+        double r = 0.0;
+        for (int i = W - 1; i >= 0; i--)
+            r = r * 18446744073709551616.0 + (double)w[i];
+        return r;
+    }
+};
+
+// Words that hold the results' integers: |V| < M / 2 with the sign (M < 2^126.01 of 15 moduli,
+// 2^142.4 of 17).
 template <int N>
-constexpr __int128 modulus()
+constexpr int kWords = N <= 15 ? 2 : 3;
+
+template <int N>
+constexpr Words<3> modulus()
 {
-    __int128 M = 1;
+    Words<3> M{{1, 0, 0}};
     for (int i = 0; i < N; i++)
-        M *= moduli::prime(i);
+        M = M.times((unsigned)moduli::prime(i));
     return M;
 }
 
@@ -390,47 +442,56 @@ template <int N>
 constexpr CrtTab<N> make_crt_tab()
 {
     CrtTab<N> t{};
-    const unsigned __int128 M = (unsigned __int128)modulus<N>();
+    const Words<3> M = modulus<N>();
     for (int i = 0; i < N; i++) {
         const int p = moduli::prime(i);
-        const unsigned __int128 q = M / (unsigned)p;
-        int inv = moduli::inverse((int)(q % (unsigned)p), p);
+        unsigned rest = 0, mod = 0;
+        const Words<3> q = M.over((unsigned)p, &rest);
+        (void)q.over((unsigned)p, &mod);
+        int inv = moduli::inverse((int)mod, p);
         if (inv < 0)
             inv += p;
-        const unsigned __int128 W = q * (unsigned)inv;
+        const Words<3> w = q.times((unsigned)inv);
         for (int l = 0; l < CrtTab<N>::L; l++)
-            t.w[i][l] = dup_code(float_code((int)(W >> (kLimbBits * l)) & 0xfff));
-        t.frac[i] = dup_code(positive_code((double)W / (double)M));
+            t.w[i][l] = dup_code(float_code((int)w.bits12(kLimbBits * l)));
+        t.frac[i] = dup_code(positive_code(w.value() / M.value()));
     }
     return t;
 }
 
-static __constant__ const CrtTab<7> c_crt7 = make_crt_tab<7>();
+static __constant__ const CrtTab<8> c_crt8 = make_crt_tab<8>();
 static __constant__ const CrtTab<9> c_crt9 = make_crt_tab<9>();
+static __constant__ const CrtTab<10> c_crt10 = make_crt_tab<10>();
 static __constant__ const CrtTab<11> c_crt11 = make_crt_tab<11>();
+static __constant__ const CrtTab<12> c_crt12 = make_crt_tab<12>();
 static __constant__ const CrtTab<13> c_crt13 = make_crt_tab<13>();
 static __constant__ const CrtTab<15> c_crt15 = make_crt_tab<15>();
+static __constant__ const CrtTab<17> c_crt17 = make_crt_tab<17>();
 
 template <int N>
 __device__ __forceinline__ const CrtTab<N> &crt_tab()
 {
-    if constexpr (N == 7)
-        return c_crt7;
+    if constexpr (N == 8)
+        return c_crt8;
     else if constexpr (N == 9)
         return c_crt9;
+    else if constexpr (N == 10)
+        return c_crt10;
     else if constexpr (N == 11)
         return c_crt11;
+    else if constexpr (N == 12)
+        return c_crt12;
     else if constexpr (N == 13)
         return c_crt13;
-    else
+    else if constexpr (N == 15)
         return c_crt15;
+    else
+        return c_crt17;
 }
 
-// v 2^k rounded to nearest even, in integer arithmetic (GB300's FP64 pipe is slow)
-__device__ __forceinline__ double scaled_double(__int128 v, int k)
+// (-1)^neg a 2^k rounded to nearest even, in integer arithmetic (GB300's FP64 pipe is slow)
+__device__ __forceinline__ double scaled_double(unsigned __int128 a, bool neg, int k)
 {
-    const bool neg = v < 0;
-    unsigned __int128 a = (unsigned __int128)(neg ? -v : v);
     const unsigned long long ah = (unsigned long long)(a >> 64);
     if (a == 0)
         return 0.0;
@@ -461,29 +522,77 @@ __device__ __forceinline__ double scaled_double(__int128 v, int k)
     return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
 }
 
-// The integer of its limbs: v[l] an integer-valued float below 2^24 in magnitude.
-template <int L>
-__device__ __forceinline__ __int128 limbs_value(const float (&v)[L])
+// (sum_l v[l] 2^12l - q M) 2^k as a double: v[l] integer-valued floats below 2^24 in
+// magnitude; all integer arithmetic is modulo 2^128 or 2^192, which hold the difference.
+template <int N>
+__device__ __forceinline__ double limbs_double(const float (&v)[CrtTab<N>::L], int q, int k)
 {
-    auto half = [&](int l0, int n) {  // up to 5 limbs, below 2^(48 + 24)
+    constexpr int L = CrtTab<N>::L, W = kWords<N>, top = (L - 1) / 3;
+    constexpr Words<3> M = modulus<N>();
+    auto part = [&](int g) {  // three limbs, below 2^(24 + 24) in magnitude
         long long s = 0;
+        const int n = g == top ? L - 3 * g : 3;
 #pragma unroll
         for (int l = n - 1; l >= 0; l--)
-            s = s * (1 << kLimbBits) + __float2int_rn(v[l0 + l]);
+            s = s * (1 << kLimbBits) + __float2int_rn(v[3 * g + l]);
         return s;
     };
-    // three limbs (2^48) to a 64-bit integer
-    __int128 r = 0;
+    if constexpr (W == 2) {
+        unsigned __int128 r = 0;
 #pragma unroll
-    for (int g = (L - 1) / 3; g >= 0; g--)
-        r = r * ((long long)1 << (3 * kLimbBits)) + half(3 * g, g == (L - 1) / 3 ? L - 3 * g : 3);
-    return r;
+        for (int g = top; g >= 0; g--)
+            r = (r << (3 * kLimbBits)) + (unsigned __int128)(__int128)part(g);
+        constexpr unsigned __int128 m = ((unsigned __int128)M.w[1] << 64) | M.w[0];
+        r -= (unsigned __int128)(__int128)q * m;
+        const bool neg = (long long)(r >> 64) < 0;
+        return scaled_double(neg ? -r : r, neg, k);
+    } else {
+        unsigned __int128 lo = 0;  // 192 bits: hi, lo
+        unsigned long long hi = 0;
+        auto add = [&](__int128 x) {  // (sign-extended)
+            const unsigned __int128 s = lo + (unsigned __int128)x;
+            hi += (x < 0 ? ~0ull : 0ull) + (s < lo ? 1ull : 0ull);
+            lo = s;
+        };
+#pragma unroll
+        for (int g = top; g >= 0; g--) {
+            hi = (hi << 36) | (unsigned long long)(lo >> 92);
+            lo <<= 36;
+            add(part(g));
+        }
+        static_assert(3 * kLimbBits == 36, "");
+        // -q M, word by word: |q| < 2^13
+        add(-((__int128)q * (long long)(M.w[0] & 0xffffffffull)));
+        add(-((__int128)q * (long long)(M.w[0] >> 32) * ((__int128)1 << 32)));
+        constexpr unsigned long long m1 = M.w[1] & 0xffffffffull, m2 = M.w[1] >> 32;
+        add(-((__int128)q * (long long)m1 * ((__int128)1 << 64)));
+        // the rest from 2^96 up
+        const __int128 t = -((__int128)q * (__int128)(m2 | (M.w[2] << 32)));
+        const unsigned __int128 tl = (unsigned __int128)t << 96;
+        const unsigned __int128 s = lo + tl;
+        hi += (unsigned long long)(t >> 32) + (s < lo ? 1ull : 0ull);
+        lo = s;
+        const bool neg = (long long)hi < 0;
+        if (neg) {
+            lo = -lo;
+            hi = ~hi + (lo == 0 ? 1ull : 0ull);
+        }
+        if (hi) {  // to 128 bits, what falls off kept as the last bit
+            const int n = 64 - __clzll((long long)hi);
+            const bool rest = (lo & (((unsigned __int128)1 << n) - 1)) != 0;
+            lo = ((unsigned __int128)hi << (128 - n)) | (lo >> n);
+            lo |= rest ? 1 : 0;
+            k += n;
+        }
+        return scaled_double(lo, neg, k);
+    }
 }
 
 // Residues -> the integer V = sum_i r_i W_i - q M (Chinese remainder theorem) -> FP64,
-// rounded once.  The limbs' sums stay below 2^24 (15 residues of 181 times 12 bits), so
-// their FP32 operations are exact; sum_i r_i W_i / M is off by less than 0.002, and
-// |V| <= 0.4914 M by the row scales, so q is its nearest integer.
+// rounded once.  The limbs' sums stay below 2^24 (17 residues of 181 times 12 bits), so
+// their FP32 operations are exact; sum_i r_i W_i / M is off by less than 0.0025 (17 roundings
+// of sums below 4096), and |V| <= 0.4935 M by the row scales (0.4914, and 0.0014 in each
+// log2 norm), so q is its nearest integer.
 // Consecutive threads take consecutive m, two per thread in f32x2 operations; bound by
 // these N (L + 1) operations and the integer work, where Garner's mixed-radix digits took
 // 5 N (N - 1) / 2.
@@ -543,10 +652,8 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
             if (failed || sm == kNotFinite || sn == kNotFinite) {
                 x = __longlong_as_double(0x7ff8000000000000ll);
             } else {
-                x = scaled_double(
-                    limbs_value<L>(f) -
-                        (__int128)((int)(h ? q >> 32 : q) - 0x4b400000) * modulus<N>(),
-                    P.alpha_exp - sm - sn);
+                x = limbs_double<N>(f, (int)(h ? q >> 32 : q) - 0x4b400000,
+                                    P.alpha_exp - sm - sn);
                 if (P.alpha_neg)
                     x = __longlong_as_double(__double_as_longlong(x) ^ (1ll << 63));
                 if (P.alpha_mul)
@@ -734,11 +841,14 @@ int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const 
     P.err = err;
     P.skip = skip;
     switch (n_mod) {
-    case 7: return launch_combine<7>(st, P);
+    case 8: return launch_combine<8>(st, P);
     case 9: return launch_combine<9>(st, P);
+    case 10: return launch_combine<10>(st, P);
     case 11: return launch_combine<11>(st, P);
+    case 12: return launch_combine<12>(st, P);
     case 13: return launch_combine<13>(st, P);
     case 15: return launch_combine<15>(st, P);
+    case 17: return launch_combine<17>(st, P);
     }
     cutc_set_error(CUTC_ERR_INVALID, "no combination of %d moduli", n_mod);
     return CUTC_ERR_INVALID;

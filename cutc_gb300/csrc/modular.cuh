@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "common.cuh"
 #include "engine.cuh"
@@ -63,13 +64,24 @@ constexpr ModuliTab make_moduli_tab()
 
 static __constant__ const ModuliTab c_tab = make_moduli_tab();
 
-// Moduli of the split form's contractions for n_slices BF16 slices (3 .. 7): operands
-// rounded at 2^-29, 2^-37, 2^-45, 2^-54, 2^-62 of their row norms, at least the precision
-// of that many 9-bit slices.
-constexpr int split_moduli(int n_slices) { return 2 * n_slices + 1; }
+// Moduli of a contraction over K columns with the precision of S 9-bit slices (3 .. 7).  S
+// slices round a row at 2^-9S of a power of two above its maximum; here it is rounded at
+// 2^-beta of its norm (to within a factor of 2, on both sides), at most sqrt(K) maxima.  With
+// beta >= 9 S + log2(K) / 2 no row of any kind has a coarser unit than its slices had.  Of the
+// numbers of moduli that are built; 7 slices beyond K = 41 000 keep 17, whose error stays
+// below that of the products which slices leave out (s + t >= S) up to K = 1.6e5, and below
+// FP64's rounding of the sum.
+inline int split_moduli(int S, int64_t K)
+{
+    const float need = 9.0f * (float)S + 0.5f * log2f((float)std::max<int64_t>(K, 1));
+    for (int n : {8, 9, 10, 11, 12, 13, 15})
+        if (moduli::row_bits(n) >= need)
+            return n;
+    return moduli::kMax;
+}
 // Moduli of the plain form's contractions: operands rounded at 2^-62 of their row norms,
 // below FP64's own rounding of the sums.
-constexpr int kPlainModuli = moduli::kMax;
+constexpr int kPlainModuli = 15;
 
 // BF16 residues of one K panel of an operand: planes[i][r][k], rows `pitch` apart.
 struct ResiduePlanes {

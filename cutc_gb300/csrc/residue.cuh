@@ -298,8 +298,8 @@ __device__ __forceinline__ void store_residues(const uint64_t (&chunk)[CH][4], _
 template <int CH>
 __device__ __forceinline__ void int_chunks(double x, int s, float (&c)[CH])
 {
-    const long long t = moduli::scaled_int(x, s);
-    const unsigned long long a = t < 0 ? 0ull - (unsigned long long)t : (unsigned long long)t;
+    using T = std::conditional_t<(CH <= 5), unsigned long long, unsigned __int128>;
+    const T a = moduli::scaled_magnitude<T>(x, s);
     const unsigned sign = (unsigned)(__double2hiint(x)) & 0x80000000u;
 #pragma unroll
     for (int j = 0; j < CH; j++) {
@@ -638,11 +638,14 @@ static int residue_rows(cudaStream_t st, int n_mod, Src src, int r0, int rows, i
                         int64_t k0, int64_t kp, int64_t pitch, int *sc, void *planes, int *bad)
 {
     switch (n_mod) {
-    case 7: return residue_rows<7>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 8: return residue_rows<8>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     case 9: return residue_rows<9>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 10: return residue_rows<10>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     case 11: return residue_rows<11>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 12: return residue_rows<12>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     case 13: return residue_rows<13>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     case 15: return residue_rows<15>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 17: return residue_rows<17>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
     }
     cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
     return CUTC_ERR_INVALID;
@@ -683,11 +686,14 @@ static inline int residue_cols(cudaStream_t st, int n_mod, const double *X, int6
                                int64_t k0, int64_t kp, int64_t pitch, const int *sc, void *planes)
 {
     switch (n_mod) {
-    case 7: return residue_cols<7>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 8: return residue_cols<8>(st, X, ld, rows, k0, kp, pitch, sc, planes);
     case 9: return residue_cols<9>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 10: return residue_cols<10>(st, X, ld, rows, k0, kp, pitch, sc, planes);
     case 11: return residue_cols<11>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 12: return residue_cols<12>(st, X, ld, rows, k0, kp, pitch, sc, planes);
     case 13: return residue_cols<13>(st, X, ld, rows, k0, kp, pitch, sc, planes);
     case 15: return residue_cols<15>(st, X, ld, rows, k0, kp, pitch, sc, planes);
+    case 17: return residue_cols<17>(st, X, ld, rows, k0, kp, pitch, sc, planes);
     }
     cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
     return CUTC_ERR_INVALID;

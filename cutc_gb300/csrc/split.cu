@@ -6,8 +6,8 @@
 //   N[p, l] = -1/2 sum_{m, r1} X_m[p, r1] S_m[l, r1]          (int_2e)
 // are C[M x N] = alpha * A[M x K] B[N x K]^T with FP64 operands and run as modular
 // contractions: exact integer products of the operands rounded on their row scales,
-// one BF16 tensor-core product per modulus (moduli.cuh).  n_slices chooses the number of
-// moduli (split_moduli): the precision of at least that many 9-bit slices.
+// one BF16 tensor-core product per modulus (moduli.cuh).  n_slices and K choose the number
+// of moduli (split_moduli): the precision of at least that many 9-bit slices.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -136,7 +136,7 @@ size_t split_fixed_bytes(const Request &R)
 {
     // residues of P (or of a K panel), the weighted AO values w chi_a on r2 they are formed
     // from, the int_2e operands' residues, and the residues of one pass of results
-    const int n_mod = split_moduli(R.n_slices);
+    const int n_mod = split_moduli(R.n_slices, std::max<int64_t>(R.n2, 3 * (int64_t)R.n1));
     const int64_t np = n_pairs(R.nA);
     size_t b = p_bytes(n_mod, np, R.n2, panel_k(R.n2, np, R.k_split)) + 8 * (size_t)R.nA * R.n2 +
                std::min(kMinResidueBytes, residue_bytes(n_mod, 4 * (int64_t)R.n1, R.n2)) +
@@ -189,9 +189,8 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
 {
     Workspace &W = E->ws;
     sp.slot0 = slot0;
-    sp.n_slices = R.n_slices;
     sp.n1t = n1t;
-    const int n_mod = split_moduli(R.n_slices);
+    const int n_mod = sp.n_mod = split_moduli(R.n_slices, R.n2);
     const int np = (int)n_pairs(R.nA);
     void *p;
     CUTC_TRY(W.get(slot0 + SS_ERR, 64, &p));
@@ -229,7 +228,7 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
                  int nb, double *Xb, int blk_rows, int ib, cudaEvent_t gemm_begin,
                  cudaEvent_t gemm_end)
 {
-    const int n_mod = split_moduli(sp.n_slices);
+    const int n_mod = sp.n_mod;
     const int64_t np = n_pairs(R.nA);
     SrcSym sa{sp.wchi2, sp.aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
     SrcDenseDF sb{G, (int64_t)R.n2};
@@ -266,8 +265,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     const int slot0 = sp.slot0;
     const int nA = R.nA;
     const int np = (int)n_pairs(nA), nl = (int)n_strict_pairs(nA);
-    const int n_mod = split_moduli(sp.n_slices);
     const int64_t k3 = 3 * (int64_t)nb;
+    const int n_mod = split_moduli(R.n_slices, k3);  // (of both contractions)
     const int64_t pan_h = int2e_panel_k(n_mod, nb, np, R.k_split);
     const int64_t pan_n = int2e_panel_k(n_mod, k3, np, R.k_split);
     void *p;
@@ -380,7 +379,7 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
                         SplitPlan &sp)
 {
     Workspace &W = E->ws;
-    const int n_mod = split_moduli(n_slices);
+    const int n_mod = split_moduli(n_slices, K);
     const int64_t pan = panel_k(K, M, 0);
     int *sc_a, *sc_b;
     void *p;

@@ -15,7 +15,7 @@ constexpr int kDefaultSlices = 5;
 
 struct SplitPlan {
     int slot0 = 0;
-    int n_slices = 0;
+    int n_mod = 0;                     // moduli of the X contraction
     int64_t n1t = 0;
     ResiduePlanes ax;                  // residues of P (a K panel, or all panels: ax_whole)
     bool ax_whole = false;
