@@ -456,8 +456,8 @@ static int pair_slices(const Request &R)
 
 // Device bytes of a build that do not grow with the r1 tile (besides the
 // molecule arrays): r2 terms, the P operand, H and N, int_2e output slabs.
-// contract: limit of the plain form's contraction scratch (contract_limit).
-static size_t fixed_bytes(const Request &R, size_t contract)
+// (R.scratch: contract_limit).
+static size_t fixed_bytes(const Request &R)
 {
     const int64_t n2 = R.n2, nA = R.nA, nN = R.nN;
     const int64_t np = n_pairs(nA), nl = std::max<int64_t>(1, n_strict_pairs(nA));
@@ -466,8 +466,8 @@ static size_t fixed_bytes(const Request &R, size_t contract)
         b += ((double)np * np + (double)np * nl) * 8;
     if (R.precision == CUTC_PLAIN_FP64)  // P, and the contractions' residues
         b += (double)np * n2 * 8 +
-             (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2, contract),
-                              R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1, contract));
+             (double)std::max(fp64_contract_bytes(np, 4 * (int64_t)R.n1, n2, R.scratch),
+                              R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1, R.scratch));
     else
         b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2);
     b += (double)pair_tc_fixed_bytes(R.n2, R.nN, pair_slices(R));
@@ -551,30 +551,32 @@ static void plan_rows(const Request &R, size_t budget, int64_t *n1t, int64_t *kb
     }
 }
 
-// The plain form's contraction scratch beside a tile and a block of `budget` bytes each:
-// half as much again.
+// The contractions' scratch beside a tile and a block of `budget` bytes each: half as much
+// again.
 static size_t contract_limit(size_t budget)
 {
     return std::min(kContractBytes, std::max<size_t>((size_t)64 << 20, budget / 2));
 }
 
-// The default budget and contraction limit for `free_b` bytes of free device memory.
-static size_t default_budget_bytes(const Request &R, size_t free_b, size_t *contract)
+// The default budget for `free_b` bytes of free device memory; sets R.scratch.
+static size_t default_budget_bytes(Request &R, size_t free_b)
 {
     size_t budget = std::min<size_t>((size_t)24 << 30, free_b / 4);
-    *contract = contract_limit(budget);
-    const size_t fixed = fixed_bytes(R, *contract);
+    R.scratch = contract_limit(budget);
+    const size_t fixed = fixed_bytes(R);
     if (free_b > fixed)
         budget = std::min<size_t>(budget, (size_t)((double)(free_b - fixed) * 0.4));
     return budget;
 }
 
-size_t build_footprint(const Request &R, size_t tile_budget, size_t contract)
+size_t build_footprint(const Request &R_in, size_t tile_budget, size_t scratch)
 {
+    Request R = R_in;
+    R.scratch = scratch ? scratch : contract_limit(tile_budget);
     const int64_t n1 = R.n1, n2 = R.n2, nA = R.nA, nN = R.nN;
     int64_t n1t, kb;
     plan_rows(R, tile_budget, &n1t, &kb);
-    double b = (double)fixed_bytes(R, contract ? contract : contract_limit(tile_budget)) + (double)n1t * r1_row_bytes(R) +
+    double b = (double)fixed_bytes(R) + (double)n1t * r1_row_bytes(R) +
                (double)kb * int2e_row_bytes(R);
     if (!(R.device_pointers || R.in_device))
         b += (4.0 * n1 + 4.0 * n2 + 3.0 * nN + 4.0 * n1 * nA + (double)n2 * nA) * 8;
@@ -730,7 +732,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     // complete, its share of the int_2e contractions (K = its rows) is added to H
     // and N in FP64.  Device memory is the fixed part plus one tile and one block,
     // each within the budget.
-    size_t budget = R.max_work_bytes, climit = contract_limit(budget);
+    size_t budget = R.max_work_bytes;
+    R.scratch = contract_limit(budget);
     int64_t n1t, kb;
     PlanMemo memo;
     const uint64_t key = plan_key(R);
@@ -744,14 +747,14 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     const bool default_budget = budget == 0;
     if (default_budget && E->ws.recall(key, &memo) && memo.path == path) {
         budget = memo.budget;  // the last build of this shape: its buffers fit this plan
-        climit = memo.contract;
+        R.scratch = memo.scratch;
         n1t = memo.n1t;
         kb = memo.kb;
     } else {
         if (default_budget) {
             size_t free_b = 0, total_b = 0;
             CUTC_CUDA_TRY(cudaMemGetInfo(&free_b, &total_b));
-            budget = default_budget_bytes(R, free_b, &climit);
+            budget = default_budget_bytes(R, free_b);
         }
         plan_rows(R, budget, &n1t, &kb);
     }
@@ -824,7 +827,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         note_launches(1);
     }
     if (R.precision == CUTC_PLAIN_FP64) {
-        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, climit, contract));
+        CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, R.scratch, contract));
         CUTC_TRY(W.get(S_P, (size_t)np * n2 * 8, &p));
         d_P = (double *)p;
         if (!(R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == d_P)) {
@@ -1156,11 +1159,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         }
         // a tile's X contraction is one FP64 launch, or the split form's K launches
         int x_launches = 1;
-        if (R.precision == CUTC_SPLIT_BF16) {
-            const int64_t nkb = ((int64_t)R.n2 + 31) / 32;
-            const int64_t per = split_k_blocks_per_launch(nkb * 32, n_pairs(R.nA), R.k_split);
-            x_launches = (int)((nkb + per - 1) / per);
-        }
+        if (R.precision == CUTC_SPLIT_BF16)
+            x_launches = (int)((R.n2 + sp.k_panel - 1) / sp.k_panel);
         stats->ms_x_gemm = ms_gemm;
         stats->n_x_gemm = n_tiles * x_launches;
         stats->ms_h2d = ev_ms(E->ev[0], E->ev[1]);
@@ -1176,7 +1176,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         memo.key = key;
         memo.path = path;
         memo.budget = budget;
-        memo.contract = climit;
+        memo.scratch = R.scratch;
         memo.n1t = n1t;
         memo.kb = kb;
         E->ws.remember(memo);
@@ -1595,12 +1595,13 @@ extern "C" int cutc_plan(const cutc_options *opt, int n_grid1, int n_grid2, int 
         R.tile_rows = atoi(tr);
     if (const char *ir = getenv("CUTC_INT2E_ROWS"))
         R.int2e_rows = atoi(ir);
-    size_t budget = opt->max_work_bytes, climit = contract_limit(budget);
+    size_t budget = opt->max_work_bytes;
+    R.scratch = contract_limit(budget);
     int64_t n1t, kb;
     PlanMemo memo;
     if (budget == 0 && engine_recall(plan_key(R), &memo)) {
         budget = memo.budget;  // as a build of this shape on the device's engine would
-        climit = memo.contract;
+        R.scratch = memo.scratch;
         n1t = memo.n1t;
         kb = memo.kb;
     } else {
@@ -1613,7 +1614,7 @@ extern "C" int cutc_plan(const cutc_options *opt, int n_grid1, int n_grid2, int 
                                cudaGetErrorString(e));
                 return CUTC_ERR_NO_DEVICE;
             }
-            budget = default_budget_bytes(R, free_b, &climit);
+            budget = default_budget_bytes(R, free_b);
         }
         plan_rows(R, budget, &n1t, &kb);
     }
@@ -1623,10 +1624,10 @@ extern "C" int cutc_plan(const cutc_options *opt, int n_grid1, int n_grid2, int 
     plan->n_blocks = (int)((n_grid1 + kb - 1) / kb);
     plan->slab_cols = int2e_slab_cols(n_ao);
     plan->budget_bytes = budget;
-    plan->fixed_bytes = fixed_bytes(R, climit);
+    plan->fixed_bytes = fixed_bytes(R);
     plan->tile_row_bytes = r1_row_bytes(R);
     plan->block_row_bytes = int2e_row_bytes(R);
-    plan->footprint_bytes = build_footprint(R, budget, climit);
+    plan->footprint_bytes = build_footprint(R, budget, R.scratch);
     if (R.precision == CUTC_SPLIT_BF16) {
         const int64_t nkb = ((int64_t)n_grid2 + 31) / 32;
         const int64_t per = split_k_blocks_per_launch(nkb * 32, n_pairs(n_ao), opt->k_split);

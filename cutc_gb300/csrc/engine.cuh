@@ -38,7 +38,7 @@ struct PlanMemo {
     uint64_t key = 0;   // 0: none
     uint64_t path = 0;  // the pair-term path of that build (its other buffers)
     size_t budget = 0;
-    size_t contract = 0;  // limit of the plain form's contraction scratch
+    size_t scratch = 0;  // limit of the contractions' scratch
     int64_t n1t = 0, kb = 0;
 };
 struct Workspace {
@@ -91,6 +91,7 @@ struct Request {
     int in_device = 0;        // molecule arrays (r1 .. aos2) on the device
     int out_device = 0;       // X and int_2e on the device
     size_t max_work_bytes = 0;
+    size_t scratch = (size_t)16 << 30;  // the contractions' residues take about this at most
     int tile_rows = 0;  // optional cap on r1 rows per X tile
     int int2e_rows = 0; // optional cap on r1 rows per int_2e block
     int pair_fp64 = 0;  // split form: FP64 pair terms
@@ -116,8 +117,8 @@ int get_engine(Engine **out);
 int make_engine(int dev, Engine **out);
 void destroy_engine(Engine *E);
 // Device bytes one build needs besides its molecule arrays, for a given r1-tile budget.
-// (contract: limit of the plain form's contraction scratch, 0: that of the budget).
-size_t build_footprint(const Request &R, size_t tile_budget, size_t contract = 0);
+// (scratch: limit of the contractions' scratch, 0: that of the budget).
+size_t build_footprint(const Request &R, size_t tile_budget, size_t scratch = 0);
 int build_terms(const Request &R, std::vector<double> &coef, std::vector<int> &exps,
                 std::vector<int> &off);
 int run_build(Engine *E, const Request &R, cutc_stats *stats);

@@ -729,15 +729,15 @@ static int planes_map(CUtensorMap *map, int n_mod, const ResiduePlanes &o, int b
     return encode_bf16_map(map, o.p, 3, dims, strides, box, 128);
 }
 
-int modular_pass_cols(int n_mod, int64_t M, int64_t N)
+int modular_pass_cols(int n_mod, int64_t M, int64_t N, size_t out_bytes)
 {
-    const int64_t per = ((int64_t)4 << 30) / (2 * n_mod * modular_ldm(M));
+    const int64_t per = (int64_t)out_bytes / (2 * n_mod * modular_ldm(M));
     return (int)std::min<int64_t>(N, std::max<int64_t>(256, per / 256 * 256));
 }
 
-size_t modular_out_bytes(int n_mod, int64_t M, int64_t N)
+size_t modular_out_bytes(int n_mod, int64_t M, int64_t N, size_t out_bytes)
 {
-    return (size_t)2 * n_mod * modular_ldm(M) * modular_pass_cols(n_mod, M, N);
+    return (size_t)2 * n_mod * modular_ldm(M) * modular_pass_cols(n_mod, M, N, out_bytes);
 }
 
 template <int BN, bool kResident>

@@ -115,9 +115,9 @@ inline size_t residue_bytes(int n_mod, int64_t rows, int64_t kp)
 }
 
 // Columns per pass of a contraction with M rows: the residues of the results of one pass
-// (2 bytes each and modulus) take at most 4 GiB.
-int modular_pass_cols(int n_mod, int64_t M, int64_t N);
-size_t modular_out_bytes(int n_mod, int64_t M, int64_t N);
+// (2 bytes each and modulus) take at most out_bytes (one tile's columns at least).
+int modular_pass_cols(int n_mod, int64_t M, int64_t N, size_t out_bytes);
+size_t modular_out_bytes(int n_mod, int64_t M, int64_t N, size_t out_bytes);
 
 // One K panel: residues of sum_k A[m, k] B[n, k] over the panel, for m < A.rows and
 // n < B.rows, into out[i][n][m] (rows modular_ldm(A.rows) apart, planes plane_cols rows),
@@ -202,10 +202,10 @@ int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K,
 }
 
 // The same with all rows of A at once and B's in groups of columns whose residues fit
-// b_bytes, the buffers from the workspace.
+// b_bytes and those of a pass of results out_bytes, the buffers from the workspace.
 template <class GenA, class GenB>
 int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, size_t b_bytes,
-                     int n_mod, int M, int N, int64_t K, int64_t k_panel, ResiduePlanes a,
+                     size_t out_bytes, int n_mod, int M, int N, int64_t K, int64_t k_panel, ResiduePlanes a,
                      bool b_ready, const int *sa, const int *sb,
                      const ModularOut &out, int *err, GenA gen_a, GenB gen_b)
 {
@@ -213,11 +213,11 @@ int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, si
         return CUTC_OK;
     ModularBlocks blk;
     blk.rows = M;
-    blk.pass = modular_pass_cols(n_mod, M, N);
+    blk.pass = modular_pass_cols(n_mod, M, N, out_bytes);
     blk.group = std::min(blk.pass, modular_b_rows(n_mod, N, std::min(K, k_panel), b_bytes));
     void *b, *res;
     CUTC_TRY(W.get(slot_b, residue_bytes(n_mod, b_ready ? N : blk.group, std::min(K, k_panel)), &b));
-    CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N), &res));
+    CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N, out_bytes), &res));
     return modular_contract_blocks(st, n_mod, M, N, K, k_panel, blk, a, b, b_ready,
                                    (unsigned short *)res, sa, sb, out, err, nullptr, gen_a, gen_b);
 }

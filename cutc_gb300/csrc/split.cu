@@ -87,39 +87,60 @@ static int64_t panel_k(int64_t K, int64_t M, int k_split)
     return std::min(K, (int64_t)split_k_blocks_per_launch(K, M, k_split) * kBK);
 }
 
+// The bytes below follow the build's scratch limit (R.scratch, half of its tile budget).
+//
 // Device bytes for the residues of B's columns: as many as the G tile they are formed
 // from takes (its rows are then read once per panel, in a few groups of columns), at
-// least 1 GiB, so that small contractions run in one group.
-constexpr size_t kMinResidueBytes = (size_t)1 << 30;
-static size_t x_residue_bytes(int64_t rows, int64_t n2)
+// least 1 GiB if the limit allows, so that small contractions run in one group.
+static size_t min_residue_bytes(const Request &R) { return std::min((size_t)1 << 30, R.scratch); }
+static size_t x_residue_bytes(const Request &R, int64_t rows)
 {
-    return std::max(kMinResidueBytes, (size_t)rows * 4 * (size_t)n2 * 8);
+    return std::max(min_residue_bytes(R), (size_t)rows * 4 * (size_t)R.n2 * 8);
 }
-// Device bytes of each operand's residues in the int_2e contractions.
-constexpr size_t kInt2eResidueBytes = (size_t)4 << 30;
+// Device bytes of each operand's residues in the int_2e contractions, and of a pass of results.
+static size_t operand_bytes(const Request &R) { return std::min((size_t)4 << 30, R.scratch / 2); }
 
 // K panel of the int_2e contractions: whole tensor-core chunks (256) whose residues of the
 // np rows of A fit.
-static int64_t int2e_panel_k(int n_mod, int64_t K, int64_t np, int k_split)
+static int64_t int2e_panel_k(const Request &R, int n_mod, int64_t K, int64_t np)
 {
-    const int64_t fit = (int64_t)(kInt2eResidueBytes / (2 * (size_t)n_mod * np)) / 256 * 256;
-    const int64_t cap = k_split > 0 ? panel_k(K, np, k_split) : K;
+    const int64_t fit = (int64_t)(operand_bytes(R) / (2 * (size_t)n_mod * np)) / 256 * 256;
+    const int64_t cap = R.k_split > 0 ? panel_k(K, np, R.k_split) : K;
     return std::min(cap, std::max<int64_t>(256, fit));
 }
 
 // P's residues stay for every r1 tile (and, in a scan, for every set) when all K panels
-// take at most 16 GiB; otherwise each tile forms a panel again (medium build, 7260 x 80 000:
-// 2.5 ms a tile).
-constexpr size_t kResidentBytes = (size_t)16 << 30;
-static bool p_resident(int n_mod, int64_t np, int64_t n2, int64_t k_panel)
+// take at most 16 GiB and twice the limit; otherwise each tile forms a panel again (medium
+// build, 7260 x 80 000: 3 ms a tile).
+static size_t resident_bytes(const Request &R) { return std::min((size_t)16 << 30, 2 * R.scratch); }
+
+// K panel of the residues of an operand of `rows` rows: the launch's, unless its residues take
+// more than `limit`; then a part of it, which takes no more than the operand's S BF16 slices
+// would.
+static int64_t residue_panel(int S, int n_mod, int64_t K, int64_t rows, int k_split, size_t limit)
 {
-    return k_panel >= n2 || (size_t)((n2 + k_panel - 1) / k_panel) *
-                                    residue_bytes(n_mod, np, k_panel) <= kResidentBytes;
+    const int64_t kp = panel_k(K, rows, k_split);
+    if (residue_bytes(n_mod, rows, kp) <= limit)
+        return kp;
+    const int parts = (n_mod + S - 1) / S;
+    return std::min(kp, (kp / parts + 511) / 512 * 512);
 }
-static size_t p_bytes(int n_mod, int64_t np, int64_t n2, int64_t k_panel)
+
+static int64_t x_panel(const Request &R, int n_mod)
 {
-    const int64_t panels = p_resident(n_mod, np, n2, k_panel) ? (n2 + k_panel - 1) / k_panel : 1;
-    return (size_t)panels * residue_bytes(n_mod, np, k_panel);
+    return residue_panel(R.n_slices, n_mod, R.n2, n_pairs(R.nA), R.k_split, resident_bytes(R));
+}
+
+static bool p_resident(const Request &R, int n_mod, int64_t k_panel)
+{
+    return k_panel >= R.n2 || (size_t)((R.n2 + k_panel - 1) / k_panel) *
+                                      residue_bytes(n_mod, n_pairs(R.nA), k_panel) <=
+                                  resident_bytes(R);
+}
+static size_t p_bytes(const Request &R, int n_mod, int64_t k_panel)
+{
+    const int64_t panels = p_resident(R, n_mod, k_panel) ? (R.n2 + k_panel - 1) / k_panel : 1;
+    return (size_t)panels * residue_bytes(n_mod, n_pairs(R.nA), k_panel);
 }
 
 size_t split_r1_row_bytes(const Request &R)
@@ -138,12 +159,14 @@ size_t split_fixed_bytes(const Request &R)
     // from, the int_2e operands' residues, and the residues of one pass of results
     const int n_mod = split_moduli(R.n_slices, std::max<int64_t>(R.n2, 3 * (int64_t)R.n1));
     const int64_t np = n_pairs(R.nA);
-    size_t b = p_bytes(n_mod, np, R.n2, panel_k(R.n2, np, R.k_split)) + 8 * (size_t)R.nA * R.n2 +
-               std::min(kMinResidueBytes, residue_bytes(n_mod, 4 * (int64_t)R.n1, R.n2)) +
+    size_t b = p_bytes(R, n_mod, x_panel(R, n_mod)) + 8 * (size_t)R.nA * R.n2 +
+               std::min(min_residue_bytes(R), residue_bytes(n_mod, 4 * (int64_t)R.n1, R.n2)) +
                modular_out_bytes(n_mod, np,
-                                 std::max<int64_t>(np, std::min<int64_t>(4 * (int64_t)R.n1, 1 << 30)));
+                                 std::max<int64_t>(np, std::min<int64_t>(4 * (int64_t)R.n1, 1 << 30)),
+                                 operand_bytes(R));
     if (!R.x_only)
-        b += std::min(kInt2eResidueBytes, residue_bytes(n_mod, np, 3 * (int64_t)R.n1)) * 3;
+        b += std::min(std::max(operand_bytes(R), residue_bytes(n_mod, np, 256)),
+                      residue_bytes(n_mod, np, 3 * (int64_t)R.n1)) * 3;
     return b;
 }
 
@@ -200,14 +223,14 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
     CUTC_TRY(make_pairs(W, slot0 + SS_PAIRS_ANTI, st, R.nA, true, &sp.pairs_anti));
     CUTC_TRY(scale_slot(W, slot0 + SS_AX_SC, np, &sp.sc_ax));
     CUTC_TRY(scale_slot(W, slot0 + SS_BX_SC, (int)(4 * n1t), &sp.sc_bx));
-    sp.k_panel = panel_k(R.n2, np, R.k_split);
-    CUTC_TRY(W.get(slot0 + SS_AX, p_bytes(n_mod, np, R.n2, sp.k_panel), &p));
+    sp.k_panel = x_panel(R, n_mod);
+    CUTC_TRY(W.get(slot0 + SS_AX, p_bytes(R, n_mod, sp.k_panel), &p));
     sp.ax.p = p;
     sp.ax.rows = np;
     CUTC_TRY(W.get(slot0 + SS_WCHI2, std::max<size_t>(1, (size_t)R.nA * R.n2) * 8, &p));
     sp.wchi2 = (const double *)p;
     sp.aos2v = aos2v;
-    sp.ax_whole = p_resident(n_mod, np, R.n2, sp.k_panel);
+    sp.ax_whole = p_resident(R, n_mod, sp.k_panel);
     if (R.mol_tag && E->tag_x == R.mol_tag && E->tag_x_buf == sp.ax.p)
         return CUTC_OK;  // the same molecule's scales (and residues) are already there
     CUTC_TRY(weighted_aos(st, R.n2, R.nA, wr2, aos2v, (int64_t)R.n2, (double *)p));
@@ -238,7 +261,8 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
     // column (c, i) of the tile -> column c blk_rows + ib + i of the block
     const ModularOut out{Xb, np, nb, blk_rows, ib, 1.0, 0.0};
     CUTC_TRY(modular_contract(
-        st, E->ws, sp.slot0 + SS_BX, sp.slot0 + SS_RES, x_residue_bytes(sp.n1t, R.n2), n_mod,
+        st, E->ws, sp.slot0 + SS_BX, sp.slot0 + SS_RES, x_residue_bytes(R, sp.n1t),
+        operand_bytes(R), n_mod,
         (int)np, 4 * nb, R.n2, sp.k_panel, sp.ax, false, sp.sc_ax, sp.sc_bx, out, sp.err,
         [&](int, int, int64_t k0, int64_t kp, ResiduePlanes &a) -> int {
             if (sp.ax_whole) {
@@ -267,8 +291,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     const int np = (int)n_pairs(nA), nl = (int)n_strict_pairs(nA);
     const int64_t k3 = 3 * (int64_t)nb;
     const int n_mod = split_moduli(R.n_slices, k3);  // (of both contractions)
-    const int64_t pan_h = int2e_panel_k(n_mod, nb, np, R.k_split);
-    const int64_t pan_n = int2e_panel_k(n_mod, k3, np, R.k_split);
+    const int64_t pan_h = int2e_panel_k(R, n_mod, nb, np);
+    const int64_t pan_n = int2e_panel_k(R, n_mod, k3, np);
     void *p;
     CUTC_TRY(W.get(slot0 + SS_WCHI1, std::max<size_t>(1, (size_t)nA * nb) * 8, &p));
     double *wchi = (double *)p;
@@ -282,9 +306,9 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     a.p = p;
     // With the whole r1 grid in one block the B operands depend on the molecule only,
     // and a build with the same molecule tag keeps them.
-    const bool whole = modular_whole(n_mod, np, nb, pan_h, kInt2eResidueBytes) &&
-                       modular_whole(n_mod, nl, k3, pan_n, kInt2eResidueBytes) &&
-                       modular_pass_cols(n_mod, np, np) >= np;
+    const bool whole = modular_whole(n_mod, np, nb, pan_h, operand_bytes(R)) &&
+                       modular_whole(n_mod, nl, k3, pan_n, operand_bytes(R)) &&
+                       modular_pass_cols(n_mod, np, np, operand_bytes(R)) >= np;
     const bool keep_b = whole && nb == R.n1 && R.mol_tag && E->tag_i == R.mol_tag &&
                         E->tag_i_buf == sc_h;
     SrcSym s0{wchi, aos1, (int64_t)nb, ld1, sp.pairs_sym};
@@ -299,8 +323,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     const double *x3 = Xt + 3 * (int64_t)nb * np;
     CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a, nullptr));
     CUTC_TRY(modular_contract(
-        st, W, slot0 + SS_BH, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, np, nb, pan_h, a, keep_b, sc_a,
-        sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err,
+        st, W, slot0 + SS_BH, slot0 + SS_RES, operand_bytes(R), operand_bytes(R), n_mod, np, np, nb,
+        pan_h, a, keep_b, sc_a, sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err,
         [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_cols(st, n_mod, x3, np, np, k0, kp, o.pitch, sc_a, o.p);
         },
@@ -310,8 +334,8 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     if (nl > 0) {
         CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a, nullptr));
         CUTC_TRY(modular_contract(
-            st, W, slot0 + SS_BN, slot0 + SS_RES, kInt2eResidueBytes, n_mod, np, nl, k3, pan_n, a, keep_b, sc_a,
-            sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err,
+            st, W, slot0 + SS_BN, slot0 + SS_RES, operand_bytes(R), operand_bytes(R), n_mod, np, nl, k3,
+            pan_n, a, keep_b, sc_a, sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err,
             [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
                 return residue_cols(st, n_mod, Xt, np, np, k0, kp, o.pitch, sc_a, o.p);
             },
@@ -380,7 +404,7 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
 {
     Workspace &W = E->ws;
     const int n_mod = split_moduli(n_slices, K);
-    const int64_t pan = panel_k(K, M, 0);
+    const int64_t pan = residue_panel(n_slices, n_mod, K, M, 0, (size_t)16 << 30);
     int *sc_a, *sc_b;
     void *p;
     CUTC_TRY(scale_slot(W, base, M, &sc_a));
@@ -395,7 +419,7 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
     CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, sc_b, (int *)nullptr));
     sp.err = err;
     return modular_contract(
-        st, W, base + 4, base + 5, (size_t)8 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
+        st, W, base + 4, base + 5, (size_t)8 << 30, (size_t)4 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
         ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err,
         [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
             return residue_rows(st, n_mod, sa, 0, M, K, k0, kp, o.pitch, sc_a, o.p, (int *)nullptr);
