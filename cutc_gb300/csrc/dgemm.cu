@@ -89,31 +89,20 @@ struct Args {
     const double *A, *B;
     double *C;
     int64_t lda, ldb, ldc, sa, sb, sc;
-    int tiles_m, tiles_n, batch;
-    const int *only_if;
+    int tiles_m, tiles_n;
 };
 
+// acc[i][j][h]: element (wm 64 + 8 i + lane / 4, wn 32 + 8 j + 2 (lane % 4) + h) of the 128 x 128
+// tile at (m0, n0) of A B, wm = warp % 2 and wn = warp / 2; smem: kSmem bytes.
 template <bool AK>
-__global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
+__device__ __forceinline__ void tile_product(const double *A, int64_t lda, const double *B,
+                                             int64_t ldb, int M, int N, int64_t K, int m0, int n0,
+                                             double *smem, double (&acc)[8][4][2])
 {
-    if (g.only_if && *g.only_if == 0)
-        return;
-    extern __shared__ __align__(16) double smem[];
     double *sA = smem;                       // kStages x kStageA
     double *sB = smem + kStages * kStageA;   // kStages x kStageB
-
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t per_batch = (int64_t)g.tiles_m * g.tiles_n;
-    // (one tile per block; a launch that waits for only_if has few blocks and walks them)
-    for (int64_t t = blockIdx.x; t < per_batch * g.batch; t += gridDim.x) {
-    const int z = (int)(t / per_batch);
-    const int64_t r = t - (int64_t)z * per_batch;
-    const int m0 = (int)(r % g.tiles_m) * kBM;  // m fastest: a wave shares the B tiles
-    const int n0 = (int)(r / g.tiles_m) * kBN;
-    const double *A = g.A + (int64_t)z * g.sa;
-    const double *B = g.B + (int64_t)z * g.sb;
-    double *C = g.C + (int64_t)z * g.sc;
-    const int64_t nkb = (g.K + kBK - 1) / kBK;
+    const int64_t nkb = (K + kBK - 1) / kBK;
 
     auto load = [&](int stage, int64_t kb) {
         const int64_t k0 = kb * kBK;
@@ -131,8 +120,8 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
             }
             const int gm = m0 + row;
             const int64_t gk = k0 + k;
-            const bool ok = gm < g.M && gk < g.K;
-            const double *src = ok ? (AK ? A + (int64_t)gm * g.lda + gk : A + gk * g.lda + gm) : A;
+            const bool ok = gm < M && gk < K;
+            const double *src = ok ? (AK ? A + (int64_t)gm * lda + gk : A + gk * lda + gm) : A;
             cp_async8(smem_u32(AK ? a + row * kLdRow + k : a + k * kLdCol + row), src, ok ? 8u : 0u);
         }
 #pragma unroll
@@ -141,8 +130,8 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
             const int row = e / kBK, k = e % kBK;
             const int gn = n0 + row;
             const int64_t gk = k0 + k;
-            const bool ok = gn < g.N && gk < g.K;
-            const double *src = ok ? B + (int64_t)gn * g.ldb + gk : B;
+            const bool ok = gn < N && gk < K;
+            const double *src = ok ? B + (int64_t)gn * ldb + gk : B;
             cp_async8(smem_u32(b + row * kLdRow + k), src, ok ? 8u : 0u);
         }
     };
@@ -150,7 +139,6 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
     // warp tile: rows wm * 64 .. + 64, columns wn * 32 .. + 32
     const int wm = warp & 1, wn = warp >> 1;
     const int fr = lane >> 2, fk = lane & 3;
-    double acc[8][4][2];
 #pragma unroll
     for (int i = 0; i < 8; i++)
 #pragma unroll
@@ -192,7 +180,26 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
         }
     }
     cp_async_wait<0>();
+    __syncthreads();  // the stages are free
+}
 
+template <bool AK>
+__global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
+{
+    extern __shared__ __align__(16) double smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t per_batch = (int64_t)g.tiles_m * g.tiles_n;
+    const int64_t t = blockIdx.x;
+    const int z = (int)(t / per_batch);
+    const int64_t r = t - (int64_t)z * per_batch;
+    const int m0 = (int)(r % g.tiles_m) * kBM;  // m fastest: a wave shares the B tiles
+    const int n0 = (int)(r / g.tiles_m) * kBN;
+    double *C = g.C + (int64_t)z * g.sc;
+    double acc[8][4][2];
+    tile_product<AK>(g.A + (int64_t)z * g.sa, g.lda, g.B + (int64_t)z * g.sb, g.ldb, g.M, g.N, g.K,
+                     m0, n0, smem, acc);
+    const int wm = warp & 1, wn = warp >> 1;
+    const int fr = lane >> 2, fk = lane & 3;
 #pragma unroll
     for (int i = 0; i < 8; i++) {
         const int m = m0 + wm * 64 + i * 8 + fr;
@@ -211,15 +218,120 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
             }
         }
     }
-    __syncthreads();  // the next tile's copies reuse the stages
+}
+
+// The results that a checked modular contraction left out (result_left), in FP64: M x N
+// results of one pass.  A block per SM walks the 128 x 128 tiles and lists each one's.  Few of
+// them are formed by a warp each, whose loads of 16 bytes per term the L2 feeds at about the
+// FP64 pipe's rate; more than kFewLeft by the whole tile's product.
+struct RestArgs {
+    int M, N;
+    int64_t K;
+    const double *A, *B;  // at the pass's first row and column
+    int64_t lda, ldb;
+    const unsigned short *sums;  // sums[n ldm + m]
+    int64_t ldm;
+    const int *sa, *sb;
+    int n0;
+    ModularOut out;
+    const int *left;
+};
+constexpr int kFewLeft = 2048;
+
+template <bool AK>
+__global__ void __launch_bounds__(kThreads, 1) contract_rest_kernel(const RestArgs g)
+{
+    if (*g.left == 0)
+        return;
+    extern __shared__ __align__(16) double smem[];
+    __shared__ unsigned short s_list[kFewLeft];
+    __shared__ int s_count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tiles_m = (g.M + kBM - 1) / kBM, tiles_n = (g.N + kBN - 1) / kBN;
+    auto left = [&](int m, int n) {
+        return m < g.M && n < g.N &&
+               result_left(g.sums[(int64_t)n * g.ldm + m], g.sa[m], g.sb[n]);
+    };
+    auto store = [&](int m, int n, double sum) {
+        const ModularOut &o = g.out;
+        const int gm = o.row0 + m, gn = g.n0 + n;
+        const int64_t row = o.nrow_group ? (int64_t)(gm / o.nrow_group) * o.row_stride + gm % o.nrow_group
+                                         : gm;
+        const int64_t col = (int64_t)(gn / o.ncol_group) * o.group_stride + o.col0 + gn % o.ncol_group;
+        double *c = o.C + row + o.ldc * col;
+        const double v = o.alpha * sum;
+        *c = o.beta == 0.0 ? v : v + o.beta * *c;
+    };
+    for (int64_t t = blockIdx.x; t < (int64_t)tiles_m * tiles_n; t += gridDim.x) {
+        const int m0 = (int)(t % tiles_m) * kBM, n0 = (int)(t / tiles_m) * kBN;
+        __syncthreads();  // the last tile's list is read
+        if (threadIdx.x == 0)
+            s_count = 0;
+        __syncthreads();
+        for (int k = threadIdx.x; k < kBM * kBN; k += kThreads)
+            if (left(m0 + k % kBM, n0 + k / kBM)) {
+                const int at = atomicAdd(&s_count, 1);
+                if (at < kFewLeft)
+                    s_list[at] = (unsigned short)k;
+            }
+        __syncthreads();
+        const int count = s_count;
+        if (count <= kFewLeft) {
+            for (int e = warp; e < count; e += kThreads / 32) {
+                const int m = m0 + s_list[e] % kBM, n = n0 + s_list[e] / kBM;
+                const double *a = AK ? g.A + (int64_t)m * g.lda : g.A + m;
+                const double *b = g.B + (int64_t)n * g.ldb;
+                double sum = 0.0;
+#pragma unroll 4
+                for (int64_t k = lane; k < g.K; k += 32)
+                    sum = fma(AK ? a[k] : a[k * g.lda], b[k], sum);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+                    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+                if (lane == 0)
+                    store(m, n, sum);
+            }
+            continue;
+        }
+        double acc[8][4][2];
+        tile_product<AK>(g.A, g.lda, g.B, g.ldb, g.M, g.N, g.K, m0, n0, smem, acc);
+        const int wm = warp & 1, wn = warp >> 1;
+        const int fr = lane >> 2, fk = lane & 3;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const int m = m0 + wm * 64 + i * 8 + fr, n = n0 + wn * 32 + j * 8 + 2 * fk + h;
+                    if (left(m, n))
+                        store(m, n, acc[i][j][h]);
+                }
     }
+}
+
+template <bool AK>
+int launch_rest(cudaStream_t st, const RestArgs &g, int n_sm)
+{
+    static std::atomic<unsigned long long> attr_done{0};
+    const unsigned long long bit = current_device_bit();
+    if (!(attr_done.load() & bit)) {
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(contract_rest_kernel<AK>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem));
+        attr_done.fetch_or(bit);
+    }
+    const int64_t tiles = ((int64_t)g.M + kBM - 1) / kBM * (((int64_t)g.N + kBN - 1) / kBN);
+    contract_rest_kernel<AK><<<(unsigned)std::min<int64_t>(tiles, n_sm), kThreads, kSmem, st>>>(g);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
 }
 
 }  // namespace
 
 int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double alpha,
               const double *A, int64_t lda, int64_t sa, const double *B, int64_t ldb, int64_t sb,
-              double beta, double *C, int64_t ldc, int64_t sc, int batch, const int *only_if)
+              double beta, double *C, int64_t ldc, int64_t sc, int batch)
 {
     if (M < 0 || N < 0 || K < 0 || batch < 0 || ldc < std::max(1, M) ||
         (K > 0 && (!A || !B || ldb < K || lda < (a_kmajor ? K : (int64_t)M))) || (M && N && !C)) {
@@ -253,8 +365,6 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
     g.sa = sa;
     g.sb = sb;
     g.sc = sc;
-    g.only_if = only_if;
-    g.batch = batch;
     g.tiles_m = (M + kBM - 1) / kBM;
     g.tiles_n = (N + kBN - 1) / kBN;
     const int64_t tiles = (int64_t)g.tiles_m * g.tiles_n * batch;
@@ -263,12 +373,10 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
                        (long long)tiles);
         return CUTC_ERR_INVALID;
     }
-    // a launch that mostly finds nothing to do has one block per SM
-    const unsigned grid = (unsigned)(only_if ? std::min<int64_t>(tiles, 152) : tiles);
     if (a_kmajor)
-        fp64_gemm_kernel<true><<<grid, kThreads, kSmem, st>>>(g);
+        fp64_gemm_kernel<true><<<(unsigned)tiles, kThreads, kSmem, st>>>(g);
     else
-        fp64_gemm_kernel<false><<<grid, kThreads, kSmem, st>>>(g);
+        fp64_gemm_kernel<false><<<(unsigned)tiles, kThreads, kSmem, st>>>(g);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
@@ -278,13 +386,16 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // FP64 contractions on the BF16 tensor cores
 // ---------------------------------------------------------------------------
 //
-// GB300's FP64 pipe gives 1.1 TF/s; 15 residue products at about 1.8 PF/s of BF16 give
-// more than 100 TF/s, with a smaller error: the operands are rounded at 2^-62 of their
-// row norms and nothing else until the result is rounded to FP64, where a sum of K FP64
-// terms rounds K times.  Below K = 16 the DMMA kernel does no more than one of its K steps
+// GB300's FP64 pipe gives 1.1 TF/s; 17 residue products and one of magnitudes at about
+// 1.8 PF/s of BF16 give about 100 TF/s.  The operands are rounded at 2^-70 of their row norms
+// and nothing else until the result is rounded to FP64, where a sum of K FP64 terms rounds K
+// times.  Where |a|_2 |b|_2 is so far above sum_k |a_k b_k| that this is not the smaller error
+// (rows that hardly overlap), where an operand is not finite, the FP64 GEMM's kernel forms the
+// result (modular.cuh, kCheckSum).  Below K = 16 the DMMA kernel does no more than one of its K steps
 // (65 us a wave of tiles), which the modular contraction's launches do not beat.
 
 constexpr int kMinContractK = 16;
+constexpr int kRestBlocks = 152;  // one per SM
 constexpr size_t kMinContractBytes = (size_t)16 << 20;  // no smaller blocks are tried
 enum ContractSlot { C_FLAGS, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
 static_assert(C_OUT + 1 == kContractSlots, "slots");
@@ -301,7 +412,7 @@ struct ContractPlan {
 
 static ContractPlan contract_plan(int64_t M, int64_t N, int64_t K, size_t limit)
 {
-    constexpr int n = kPlainModuli;
+    constexpr int n = kPlainPlanes;
     const size_t half = limit / 2, quarter = limit / 4;
     auto whole = [](size_t fit, int64_t all) {  // a multiple of 256, at least one, at most all
         return (int)std::min<int64_t>(all, std::max<int64_t>(256, (int64_t)(fit / 256 * 256)));
@@ -362,7 +473,7 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
 {
     constexpr int n_mod = kPlainModuli;
     Workspace &W = *S.W;
-    int *err = S.flags, *bad = S.flags + 1;
+    int *err = S.flags, *left = S.flags + 1;
     ContractPlan c;
     ResiduePlanes a;
     void *b = nullptr, *res = nullptr, *psa = nullptr, *psb = nullptr;
@@ -388,25 +499,41 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
     *done = true;
     int *sca = (int *)psa, *scb = (int *)psb;
     const int64_t pan = c.kp;
-    CUTC_CUDA_TRY(cudaMemsetAsync(bad, 0, 4, st));
+    CUTC_CUDA_TRY(cudaMemsetAsync(left, 0, 4, st));
     const SrcDense sa{A, lda}, sb{B, ldb};
     if (a_kmajor)
-        CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca, bad, c.blk.rows < M));
+        CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca));
     else
-        CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca, bad));
-    // Whether an operand is not finite has to be known before the first results are written:
-    // with several passes over the results short rows are looked at here, not block by block.
-    const bool passes = c.blk.pass < N || c.blk.rows < M;
-    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb, bad, passes));
+        CUTC_TRY(row_scales_cols(st, A, lda, M, K, n_mod, sca));
+    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, scb));
     return modular_contract_blocks(
-        st, n_mod, M, N, K, pan, c.blk, a, b, false, (unsigned short *)res, sca, scb, out, err, bad,
+        st, n_mod, M, N, K, pan, c.blk, a, b, false, (unsigned short *)res, sca, scb, out, err, left,
         [&](int m0, int rows, int64_t k0, int64_t kp, const ResiduePlanes &o) -> int {
-            return a_kmajor ? residue_rows<n_mod>(st, sa, m0, rows, K, k0, kp, o.pitch, sca, o.p, bad)
-                            : residue_cols<n_mod>(st, A + m0, lda, rows, k0, kp, o.pitch, sca + m0,
-                                                  o.p);
+            return a_kmajor ? residue_rows<n_mod, true>(st, sa, m0, rows, K, k0, kp, o.pitch, sca, o.p)
+                            : residue_cols<n_mod, true>(st, A + m0, lda, rows, k0, kp, o.pitch,
+                                                        sca + m0, o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-            return residue_rows<n_mod>(st, sb, n0, nc, K, k0, kp, o.pitch, scb, o.p, bad);
+            return residue_rows<n_mod, true>(st, sb, n0, nc, K, k0, kp, o.pitch, scb, o.p);
+        },
+        [&](int m0, int rows, int n0, int nc, const unsigned short *sums, const ModularOut &o) {
+            RestArgs g;
+            g.M = rows;
+            g.N = nc;
+            g.K = K;
+            g.A = A + (a_kmajor ? (int64_t)m0 * lda : m0);
+            g.B = B + (int64_t)n0 * ldb;
+            g.lda = lda;
+            g.ldb = ldb;
+            g.sums = sums;
+            g.ldm = modular_ldm(rows);
+            g.sa = sca + m0;
+            g.sb = scb + n0;
+            g.n0 = n0;
+            g.out = o;
+            g.left = left;
+            return a_kmajor ? launch_rest<true>(st, g, kRestBlocks)
+                            : launch_rest<false>(st, g, kRestBlocks);
         });
 }
 
@@ -430,8 +557,9 @@ int fp64_contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, int 
     bool done;
     CUTC_TRY(contract(S, st, a_kmajor, M, N * batch, K, A, lda, B, ldb,
                       ModularOut{C, ldc, N, batch > 1 ? sc / ldc : 0, 0, alpha, beta}, &done));
-    return fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc, batch,
-                     done ? S.flags + 1 : nullptr);
+    return done ? CUTC_OK
+                : fp64_gemm(st, a_kmajor, M, N, K, alpha, A, lda, sa, B, ldb, sb, beta, C, ldc, sc,
+                            batch);
 }
 
 int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, int64_t K,
@@ -442,12 +570,11 @@ int fp64_contract_rows(const ContractScratch &S, cudaStream_t st, int M, int N, 
     if (K >= kMinContractK)
         CUTC_TRY(contract(S, st, true, M, N, K, A, lda, B, ldb,
                           ModularOut{C, ldc, N, 0, 0, 1.0, 0.0, nrow_group, row_stride}, &done));
+    if (done)
+        return CUTC_OK;
     // the groups of rows as a batch: C of group z starts z row_stride further
-    const int *only_if = done ? S.flags + 1 : nullptr;
-    const int groups = M / nrow_group;
-    CUTC_TRY(fp64_gemm(st, true, nrow_group, N, K, 1.0, A, lda, (int64_t)nrow_group * lda, B, ldb,
-                       0, 0.0, C, ldc, row_stride, groups, only_if));
-    return CUTC_OK;
+    return fp64_gemm(st, true, nrow_group, N, K, 1.0, A, lda, (int64_t)nrow_group * lda, B, ldb, 0,
+                     0.0, C, ldc, row_stride, M / nrow_group);
 }
 
 }  // namespace cutc

@@ -15,23 +15,22 @@ namespace cutc {
 // B is K contiguous per column n (OP_N on a K x N column-major array).  With
 // beta == 0, C is not read.  Column-major C, as cuBLAS: the same call sites
 // keep their argument meaning.
-// only_if (may be null): the kernels return at once while *only_if is zero.
 int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double alpha,
               const double *A, int64_t lda, int64_t sa, const double *B, int64_t ldb, int64_t sb,
-              double beta, double *C, int64_t ldc, int64_t sc, int batch,
-              const int *only_if = nullptr);
+              double beta, double *C, int64_t ldc, int64_t sc, int batch);
 
-// The same contraction for callers with a workspace: a modular contraction on the BF16
-// tensor cores (modular.cuh) with operands rounded at 2^-62 of their row norms, below the
-// rounding of an FP64 sum, with fp64_gemm in its place for operands that hold an
-// infinity or a NaN (found on the device) and for K < 16.  S: from fp64_contract_begin; a
+// The same contraction for callers with a workspace: a checked modular contraction on the
+// BF16 tensor cores (modular.cuh), whose operands' rounding adds less to any result than FP64
+// sums round, with fp64_gemm's kernel for the results where it would not, for those of rows
+// that hold an infinity or a NaN (both found on the device), and with fp64_gemm for K < 16.  S: from fp64_contract_begin; a
 // bounded wait that gives up makes the results NaN and is reported by
 // fp64_contract_check.  Batches whose A is common and whose B rows follow one another
 // (sa = 0, sb = N ldb) are one contraction; others run one by one.
 //
 // Its residues take about `limit` bytes at most, whatever the sizes (contract_plan);
 // where that memory cannot be had it takes less, and fp64_gemm's path without any in the end.
-// The blocks do not change the results.
+// The blocks do not change the results (but for which kernel gives those at the edge of the
+// check).
 //
 // The scratch (kContractSlots slots from the given one) belongs to one stream until its
 // work is done: calls that wait for their results share kContractSlot, a call that returns
@@ -40,8 +39,8 @@ struct ContractScratch {
     Workspace *W = nullptr;
     int slot0 = 0;
     size_t limit = 0;
-    int *flags = nullptr;  // [0]: a wait gave up, [1]: an operand of the contraction at hand
-                           // is not finite
+    int *flags = nullptr;  // [0]: a wait gave up, [1]: results of the contraction at hand were
+                           // left to the FP64 kernel
 };
 constexpr size_t kContractBytes = (size_t)16 << 30;  // the largest limit
 constexpr int kContractSlot = 100, kContractSlots = 6;

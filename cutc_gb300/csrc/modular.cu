@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <type_traits>
 
 #include "modular.cuh"
 #include "tc.cuh"
@@ -51,21 +52,30 @@ struct ModCfg {
 
 // A residue r of a result is stored as the low half of the bits of the float r + kResidueBias,
 // whose high half is kResidueHigh.
-constexpr float kResidueBias = 12582912.0f + 512.0f;  // 1.5 * 2^23 + 2^9
+constexpr float kResidueBias = 12582912.0f + (float)kResidueOffset;  // 1.5 * 2^23 + 2^9
 constexpr unsigned kResidueHigh = 0x4b40u;
 
 struct ModGemmParams {
-    int n_mod, M, N, tiles_m, tiles_n;
+    int planes, M, N, tiles_m, tiles_n;
+    int magnitudes;            // the plane of magnitudes' sums, if any
     int nkb;                   // K blocks of the panel
     int accumulate;            // add to the residues in out
     unsigned short *out;       // out[i plane + n ldm + m]
     int64_t ldm, plane;
-    float p[moduli::kMax], inv[moduli::kMax];
+    float p[moduli::kMax + 1], inv[moduli::kMax + 1];  // 0: sums, not residues
     int *err;                  // set to a non-zero code if a bounded wait gave up
 };
 
-// kResident: the pair walks tasks of its own, a grid's width apart; else it has one.
-template <int BN, bool kResident>
+// The bits of a plane's entry: of a sum of magnitudes, zero stays zero and others are
+// 1 .. kMagnitudeCap; a residue is itself (the bounds are beyond it).
+__device__ __forceinline__ uint32_t bounded_sum(float x, bool sum)
+{
+    return __float_as_uint(x == 0.0f ? x : fminf(fmaxf(x, sum ? 1.0f : -1024.0f), (float)kMagnitudeCap));
+}
+
+// kResident: the pair walks tasks of its own, a grid's width apart; else it has one.  kMag:
+// plane P.magnitudes holds sums.
+template <int BN, bool kResident, bool kMag>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGemmThreads, 1)
 modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
                     const __grid_constant__ CUtensorMap tmB, const __grid_constant__ ModGemmParams P)
@@ -94,7 +104,7 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
     // (kGroupN column tiles sweep the row tiles, so concurrent pairs share their tiles of
     // A and B through L2).
     const int per_mod = P.tiles_m * P.tiles_n;
-    const int n_tasks = P.n_mod * per_mod, first = (int)(blockIdx.x >> 1);
+    const int n_tasks = P.planes * per_mod, first = (int)(blockIdx.x >> 1);
     const int stride = (int)(gridDim.x >> 1);
     struct Tile {
         int z, m0, n0;
@@ -311,7 +321,11 @@ modular_gemm_kernel(const __grid_constant__ CUtensorMap tmA,
             if (ok && m < P.M) {
 #pragma unroll
                 for (int j = 0; j < CP; j++) {
-                    const uint64_t w = tc::f2_add(acc[j], bias);
+                    uint64_t w = acc[j];
+                    if constexpr (kMag)
+                        w = tc::f2_pack(bounded_sum(tc::f2_lo(w), o.z == P.magnitudes),
+                                        bounded_sum(tc::f2_hi(w), o.z == P.magnitudes));
+                    w = tc::f2_add(w, bias);
                     if (2 * j < ncol)
                         dst[(int64_t)(2 * j) * P.ldm] = (unsigned short)w;
                     if (2 * j + 1 < ncol)
@@ -348,7 +362,8 @@ struct CombineParams {
     const int *sa, *sb;
     ModularOut out;
     int alpha_exp, alpha_neg, alpha_mul, beta_mode;  // beta_mode: 0, 1 or 2 (any other beta)
-    const int *err, *skip;
+    const int *err;
+    int *left;
 };
 
 // Tables of the Chinese remainder theorem for N moduli: V = sum_i r_i W_i mod M with
@@ -596,11 +611,9 @@ __device__ __forceinline__ double limbs_double(const float (&v)[CrtTab<N>::L], i
 // Consecutive threads take consecutive m, two per thread in f32x2 operations; bound by
 // these N (L + 1) operations and the integer work, where Garner's mixed-radix digits took
 // 5 N (N - 1) / 2.
-template <int N>
+template <int N, bool kChecked>
 __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
 {
-    if (P.skip && *P.skip)
-        return;
     const int m = 2 * (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (m >= P.M)
         return;
@@ -632,6 +645,9 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
         }
         const uint64_t q = tc::f2_add(t, magic);  // its bits: q + those of 1.5 * 2^23
         const int sn = P.sb[c], n = P.n0 + c;
+        unsigned sums = 0;
+        if constexpr (kChecked)
+            sums = *reinterpret_cast<const unsigned *>(src + N * P.plane);
         const int64_t col = (int64_t)(n / P.out.ncol_group) * P.out.group_stride + P.out.col0 +
                             n % P.out.ncol_group;
 #pragma unroll
@@ -648,6 +664,10 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
             for (int l = 0; l < L; l++)
                 f[l] = h ? tc::f2_hi(v[l]) : tc::f2_lo(v[l]);
             const int sm = h ? s1 : s0;
+            if (kChecked && result_left(h ? sums >> 16 : sums & 0xffffu, sm, sn)) {
+                *P.left = 1;
+                continue;
+            }
             double x;
             if (failed || sm == kNotFinite || sn == kNotFinite) {
                 x = __longlong_as_double(0x7ff8000000000000ll);
@@ -740,7 +760,7 @@ size_t modular_out_bytes(int n_mod, int64_t M, int64_t N, size_t out_bytes)
     return (size_t)2 * n_mod * modular_ldm(M) * modular_pass_cols(n_mod, M, N, out_bytes);
 }
 
-template <int BN, bool kResident>
+template <int BN, bool kResident, bool kMag>
 static int launch_gemm(cudaStream_t st, const ResiduePlanes &A, const ResiduePlanes &B,
                        ModGemmParams P)
 {
@@ -748,34 +768,35 @@ static int launch_gemm(cudaStream_t st, const ResiduePlanes &A, const ResiduePla
     static std::atomic<unsigned long long> attr_done{0};
     const unsigned long long bit = current_device_bit();
     if (!(attr_done.load() & bit)) {
-        CUTC_CUDA_TRY(cudaFuncSetAttribute(modular_gemm_kernel<BN, kResident>,
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(modular_gemm_kernel<BN, kResident, kMag>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
         attr_done.fetch_or(bit);
     }
     CUtensorMap ta, tb;
-    CUTC_TRY(planes_map(&ta, P.n_mod, A, 128));
-    CUTC_TRY(planes_map(&tb, P.n_mod, B, BN / 2));
+    CUTC_TRY(planes_map(&ta, P.planes, A, 128));
+    CUTC_TRY(planes_map(&tb, P.planes, B, BN / 2));
     P.tiles_m = (int)ceil_div(P.M, kTileM);
     P.tiles_n = (int)ceil_div(P.N, BN);
-    const int64_t tasks = (int64_t)P.n_mod * P.tiles_m * P.tiles_n;
+    const int64_t tasks = (int64_t)P.planes * P.tiles_m * P.tiles_n;
     if (tasks > INT32_MAX / 2) {
         cutc_set_error(CUTC_ERR_INVALID, "modular contraction of %lld tiles", (long long)tasks);
         return CUTC_ERR_INVALID;
     }
     const unsigned pairs = (unsigned)(kResident ? std::min<int64_t>(tasks, kPairs) : tasks);
-    modular_gemm_kernel<BN, kResident><<<2 * pairs, kGemmThreads, Cfg::kSmem, st>>>(ta, tb, P);
+    modular_gemm_kernel<BN, kResident, kMag><<<2 * pairs, kGemmThreads, Cfg::kSmem, st>>>(ta, tb, P);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
-int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
+int modular_gemm(cudaStream_t st, int n_mod, int planes, const ResiduePlanes &A, const ResiduePlanes &B,
                  unsigned short *out, int64_t plane_cols, bool accumulate, int *err)
 {
     if (A.rows <= 0 || B.rows <= 0 || A.kp <= 0)
         return CUTC_OK;
     ModGemmParams P{};
-    P.n_mod = n_mod;
+    P.planes = planes;
+    P.magnitudes = n_mod;
     P.M = A.rows;
     P.N = B.rows;
     P.nkb = (int)ceil_div(A.kp, kBK);
@@ -790,34 +811,38 @@ int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const Resid
     P.err = err;
     // narrow tiles for few columns, and where wide ones would leave the 76 SM pairs short
     // of work
-    const int64_t wide = (int64_t)n_mod * ceil_div(P.M, kTileM) * ceil_div(P.N, 256);
+    const int64_t wide = (int64_t)planes * ceil_div(P.M, kTileM) * ceil_div(P.N, 256);
     const int bn = P.N <= 64 ? 64 : (P.N <= 128 || wide < kPairs) ? 128 : 256;
     // Short panels: resident pairs walk the tasks, which hides a task's set-up and epilogue
     // behind the next one's MMAs.  Long ones: one pair per task, which the hardware starts
     // in order, so that concurrent tasks stay neighbours in L2.  M 7260, N 16384, resident
     // against one by one: K 1024 1.71 / 2.85 ms, 4096 6.04 / 7.07, 16384 25.1 / 24.4.
-    if (P.nkb <= kResidentBlocks)
-        return bn == 64    ? launch_gemm<64, true>(st, A, B, P)
-               : bn == 128 ? launch_gemm<128, true>(st, A, B, P)
-                           : launch_gemm<256, true>(st, A, B, P);
-    return bn == 64    ? launch_gemm<64, false>(st, A, B, P)
-           : bn == 128 ? launch_gemm<128, false>(st, A, B, P)
-                       : launch_gemm<256, false>(st, A, B, P);
+    const bool resident = P.nkb <= kResidentBlocks, mag = planes > n_mod;
+    auto launch = [&](auto width, auto res) {
+        constexpr int BN = decltype(width)::value;
+        constexpr bool kRes = decltype(res)::value;
+        return mag ? launch_gemm<BN, kRes, true>(st, A, B, P) : launch_gemm<BN, kRes, false>(st, A, B, P);
+    };
+    auto widths = [&](auto res) {
+        return bn == 64    ? launch(std::integral_constant<int, 64>{}, res)
+               : bn == 128 ? launch(std::integral_constant<int, 128>{}, res)
+                           : launch(std::integral_constant<int, 256>{}, res);
+    };
+    return resident ? widths(std::true_type{}) : widths(std::false_type{});
 }
 
-template <int N>
+template <int N, bool kChecked = false>
 static int launch_combine(cudaStream_t st, const CombineParams &P)
 {
     dim3 grid(ceil_div(P.M, 256), (unsigned)std::min(P.ncols, 65535));
-    combine_kernel<N><<<grid, 128, 0, st>>>(P);
+    combine_kernel<N, kChecked><<<grid, 128, 0, st>>>(P);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
 int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
-                    const int *sa, const int *sb, const ModularOut &out, const int *err,
-                    const int *skip)
+                    const int *sa, const int *sb, const ModularOut &out, const int *err, int *left)
 {
     if (M <= 0 || ncols <= 0)
         return CUTC_OK;
@@ -839,8 +864,10 @@ int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const 
     P.alpha_neg = !P.alpha_mul && out.alpha < 0;
     P.beta_mode = out.beta == 0.0 ? 0 : out.beta == 1.0 ? 1 : 2;
     P.err = err;
-    P.skip = skip;
-    switch (n_mod) {
+    P.left = left;
+    if (left && n_mod == kPlainModuli)
+        return launch_combine<kPlainModuli, true>(st, P);
+    switch (left ? 0 : n_mod) {
     case 8: return launch_combine<8>(st, P);
     case 9: return launch_combine<9>(st, P);
     case 10: return launch_combine<10>(st, P);

@@ -79,9 +79,23 @@ inline int split_moduli(int S, int64_t K)
             return n;
     return moduli::kMax;
 }
-// Moduli of the plain form's contractions: operands rounded at 2^-62 of their row norms,
-// below FP64's own rounding of the sums.
-constexpr int kPlainModuli = 15;
+// Moduli of the plain form's contractions: operands rounded at 2^-70 of their row norms.  That
+// is an error relative to |a|_2 |b|_2, where an FP64 sum's is relative to sum_k |a_k b_k|, so
+// a checked contraction forms that sum too, in one more product of the operands' magnitudes
+// (plane kPlainModuli, 8 bits of each), and leaves the results for which its error is not the
+// smaller one to the FP64 GEMM.
+//
+// With t the operands' integers, |t|_2 <= 2^70.674, the rounding of both makes an error of at
+// most 2^70.674 / sqrt(6) (rms, in units of the integer result).  Magnitudes enter as
+// |t| 2^-58, so that the plane's sum is s = sum |t_a t_b| 2^-116, and with s >= kCheckSum
+// that error is at most 0.17 2^-53 sum_k |a_k b_k|, about half of one rounding of an FP64
+// sum.  Sums are kept up to kMagnitudeCap; exact zeros (no k with both operands non-zero)
+// are told from small ones, because their results are exact.  With 15 moduli, 2^-62, the
+// check would fail for up to 8 % of the elements of a build (10 nuclei, 70 AOs: P against G's
+// -1/2 |grad u|^2); with 17 for fewer than one in 10^5.
+constexpr int kPlainModuli = moduli::kMax;
+constexpr int kPlainPlanes = kPlainModuli + 1;
+constexpr int kMagnitudeShift = 58, kMagnitudeCap = 32000, kCheckSum = 512;
 
 // BF16 residues of one K panel of an operand: planes[i][r][k], rows `pitch` apart.
 struct ResiduePlanes {
@@ -108,7 +122,7 @@ struct ModularOut {
 // multiples of 16 bytes).
 inline int64_t residue_pitch(int64_t kp) { return (kp + 15) / 16 * 16; }
 
-// Bytes of the residues of a panel.
+// Bytes of the residues of a panel (n_mod: its planes).
 inline size_t residue_bytes(int n_mod, int64_t rows, int64_t kp)
 {
     return (size_t)n_mod * rows * residue_pitch(kp) * 2;
@@ -121,18 +135,27 @@ size_t modular_out_bytes(int n_mod, int64_t M, int64_t N, size_t out_bytes);
 
 // One K panel: residues of sum_k A[m, k] B[n, k] over the panel, for m < A.rows and
 // n < B.rows, into out[i][n][m] (rows modular_ldm(A.rows) apart, planes plane_cols rows),
-// added to what is there when accumulate.  err: set when a bounded wait gave up.
+// added to what is there when accumulate.  err: set when a bounded wait gave up.  planes:
+// n_mod, or n_mod + 1 with the magnitudes' sums (plane n_mod).
 inline int64_t modular_ldm(int64_t M) { return (M + 7) / 8 * 8; }
-int modular_gemm(cudaStream_t st, int n_mod, const ResiduePlanes &A, const ResiduePlanes &B,
+int modular_gemm(cudaStream_t st, int n_mod, int planes, const ResiduePlanes &A, const ResiduePlanes &B,
                  unsigned short *out, int64_t plane_cols, bool accumulate, int *err);
 
 // The FP64 results from the residues: n0 .. n0 + ncols of the output's columns; sa and sb
 // are the row scales of A and B (sb of column n0 first).  A result with a scale of
-// kNotFinite, or after a wait that gave up, is NaN.  skip (may be null): nothing is
-// written when *skip is non-zero.
+// kNotFinite, or after a wait that gave up, is NaN.  Checked (left not null, res with the
+// magnitudes' sums): results of such scales and those whose sum is below kCheckSum are not
+// written, and *left is set to 1 when there are any (result_left tells which).
 int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
-                    const int *sa, const int *sb, const ModularOut &out, const int *err,
-                    const int *skip);
+                    const int *sa, const int *sb, const ModularOut &out, const int *err, int *left);
+
+// A plane's entry for a magnitudes' sum, and whether a checked result is left out.
+constexpr unsigned kResidueOffset = 512;
+__device__ __forceinline__ bool result_left(unsigned entry, int sm, int sn)
+{
+    const unsigned c = entry - kResidueOffset;
+    return sm == kNotFinite || sn == kNotFinite || (c != 0 && c < (unsigned)kCheckSum);
+}
 
 // cuTensorMapEncodeTiled of BF16 arrays: box[0] x box[1] tiles of the last two
 // dimensions; swizzle in bytes (64 or 128).
@@ -162,13 +185,16 @@ struct ModularBlocks {
 // gen_b(n0, ncols, k0, kp, planes) writing the residues of a panel; gen_a may point planes.p
 // at residues that are there already.  a.p, b_p and res: space for the residues of
 // blk.rows x k_panel, blk.group x k_panel and of the results of one pass.  b_ready: B's are
-// in b_p already (whole: k_panel >= K, blk.group >= N).
-template <class GenA, class GenB>
+// in b_p already (whole: k_panel >= K, blk.group >= N).  With left the contraction is checked:
+// rest(m0, rows, n0, ncols, sums, out) is called after each pass for the results left out
+// (sums: the magnitudes' plane, [n][m]).
+template <class GenA, class GenB, class Rest>
 int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K, int64_t k_panel,
                             const ModularBlocks &blk, ResiduePlanes a, void *b_p, bool b_ready,
                             unsigned short *res, const int *sa, const int *sb, ModularOut out,
-                            int *err, const int *skip, GenA gen_a, GenB gen_b)
+                            int *err, int *left, GenA gen_a, GenB gen_b, Rest rest)
 {
+    const int planes = n_mod + (left ? 1 : 0);
     ResiduePlanes b;
     b.p = b_p;
     const bool b_whole = k_panel >= K && blk.group >= N && blk.pass >= N;
@@ -190,12 +216,15 @@ int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K,
                     if (!b_ready)
                         CUTC_TRY(gen_b(n0 + g, b.rows, k0, kp, b));
                     b_ready = b_ready || b_whole;
-                    CUTC_TRY(modular_gemm(st, n_mod, a, b, res + (int64_t)g * modular_ldm(a.rows),
+                    CUTC_TRY(modular_gemm(st, n_mod, planes, a, b, res + (int64_t)g * modular_ldm(a.rows),
                                           nc, k0 > 0, err));
                 }
             }
             CUTC_TRY(modular_combine(st, n_mod, a.rows, n0, nc, res, sa + m0, sb + n0, out, err,
-                                     skip));
+                                     left));
+            if (left)
+                CUTC_TRY(rest(m0, a.rows, n0, nc, res + (int64_t)n_mod * nc * modular_ldm(a.rows),
+                              out));
         }
     }
     return CUTC_OK;
@@ -219,7 +248,10 @@ int modular_contract(cudaStream_t st, Workspace &W, int slot_b, int slot_out, si
     CUTC_TRY(W.get(slot_b, residue_bytes(n_mod, b_ready ? N : blk.group, std::min(K, k_panel)), &b));
     CUTC_TRY(W.get(slot_out, modular_out_bytes(n_mod, M, N, out_bytes), &res));
     return modular_contract_blocks(st, n_mod, M, N, K, k_panel, blk, a, b, b_ready,
-                                   (unsigned short *)res, sa, sb, out, err, nullptr, gen_a, gen_b);
+                                   (unsigned short *)res, sa, sb, out, err, nullptr, gen_a, gen_b,
+                                   [](int, int, int, int, const unsigned short *, const ModularOut &) {
+                                       return CUTC_OK;
+                                   });
 }
 
 }  // namespace cutc

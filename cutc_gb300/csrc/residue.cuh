@@ -192,7 +192,7 @@ __device__ __forceinline__ T block_sum(T v, T (&part)[8])
 // depends on scheduling); reads the row once.
 template <class Src>
 __global__ void __launch_bounds__(256)
-row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc, int *bad)
+row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc)
 {
     __shared__ float sm[8], sq[8];
     __shared__ double sd[8];
@@ -260,13 +260,36 @@ row_scale_kernel(Src src, int rows, int64_t K, float bits, int *__restrict__ sc,
             }
             ss = (float)block_sum(s2, sd);
         }
-        if (threadIdx.x == 0) {
-            const int s = scale_slow(mb, ss, bits);
-            sc[r] = s;
-            if (s == kNotFinite && bad)
-                atomicExch(bad, 1);
-        }
+        if (threadIdx.x == 0)
+            sc[r] = scale_slow(mb, ss, bits);
     }
+}
+
+// The magnitude |x| 2^s 2^-kMagnitudeShift as the bits of a BF16 number, truncated (at least
+// 2^-60 for x != 0, so that a product of two is not lost); integer arithmetic.
+__device__ __forceinline__ unsigned magnitude_bf16(double x, int s)
+{
+    unsigned long long b = abs_bits(x);
+    if (b == 0)
+        return 0;
+    int E = (int)(b >> 52);
+    if (E == 0) {  // subnormal: its leading bit to bit 52
+        const int lz = __clzll((long long)b) - 11;
+        b <<= lz;
+        E = 1 - lz;
+    }
+    const int e = E - 1023 + s - kMagnitudeShift;
+    return (unsigned)(max(e, -60) + 127) << 7 | (e >= -60 ? (unsigned)(b >> 45) & 0x7fu : 0u);
+}
+
+// ... of eight values, 16 bytes.
+__device__ __forceinline__ void store_magnitudes(const double (&x)[8], int s, __nv_bfloat16 *dst)
+{
+    unsigned w[4];
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+        w[q] = magnitude_bf16(x[2 * q], s) | magnitude_bf16(x[2 * q + 1], s) << 16;
+    *reinterpret_cast<uint4 *>(dst) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
 // The residues of eight integers per thread, chunk[j][q] holding the 13-bit chunks j of
@@ -362,10 +385,11 @@ __device__ __forceinline__ void residue_chunks(float2 x, int s, float (&v)[modul
 }
 
 // planes[i][r][k - k0] = residues of rint(src(r0 + r, k) 2^{sc[r0 + r]}) modulo p_i for
-// rows r < rows and k0 <= k < k0 + kp (zeros up to the row pitch).  Eight consecutive k
+// rows r < rows and k0 <= k < k0 + kp (zeros up to the row pitch), and with kMag the
+// magnitudes as plane N.  Eight consecutive k
 // per thread: one 16-byte store per plane.  Bound by the stores: 2 N bytes are written
 // per 8-byte element read.
-template <int N, class Src>
+template <int N, bool kMag, class Src>
 __global__ void __launch_bounds__(128)
 residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t pitch,
                     const int *__restrict__ sc, __nv_bfloat16 *__restrict__ planes)
@@ -376,15 +400,20 @@ residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t p
         return;
     for (int r = blockIdx.y; r < rows; r += gridDim.y) {
         const int s = max(sc[r0 + r], -4096);  // (kNotFinite: the result is NaN anyway)
+        typename ValueOf<Src::kDoubleFloat>::T x[8];
         float v[8][CH];
 #pragma unroll
-        for (int q = 0; q < 8; q++)
-            residue_chunks<N>(kk + q < kp ? value_of(src, r0 + r, k0 + kk + q)
-                                          : typename ValueOf<Src::kDoubleFloat>::T{},
-                              s, v[q]);
+        for (int q = 0; q < 8; q++) {
+            x[q] = kk + q < kp ? value_of(src, r0 + r, k0 + kk + q)
+                               : typename ValueOf<Src::kDoubleFloat>::T{};
+            residue_chunks<N>(x[q], s, v[q]);
+        }
+        __nv_bfloat16 *dst = planes + (int64_t)r * pitch + kk;
+        if constexpr (kMag)
+            store_magnitudes(x, s, dst + N * (int64_t)rows * pitch);
         uint64_t chunk[CH][4];
         pack_chunks<N>(v, chunk);
-        store_residues<N, CH>(chunk, planes + (int64_t)r * pitch + kk, (int64_t)rows * pitch);
+        store_residues<N, CH>(chunk, dst, (int64_t)rows * pitch);
     }
 }
 
@@ -393,7 +422,7 @@ residue_rows_kernel(Src src, int r0, int rows, int64_t k0, int64_t kp, int64_t p
 template <int RB>
 static __global__ void __launch_bounds__(1024)
 row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t K, float bits,
-                      int *__restrict__ sc, int *bad)
+                      int *__restrict__ sc)
 {
     constexpr int NG = 1024 / RB;
     __shared__ float sm[NG][RB + 1], sq[NG][RB + 1];
@@ -459,15 +488,13 @@ row_scale_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_
     if (g != 0 || r >= rows)
         return;
     sc[r] = s;
-    if (s == kNotFinite && bad)
-        atomicExch(bad, 1);
 }
 
 // The residues of such a matrix, as residue_rows_kernel: 32 rows x 64 columns per block
 // through shared memory (groups of eight columns four doubles further, so that eight
 // lanes reading eight columns apart take the minimum two wavefronts), so that reads run
 // along the rows and stores along the columns.
-template <int N>
+template <int N, bool kMag>
 __global__ void __launch_bounds__(256)
 residue_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t k0, int64_t kp,
                     int64_t pitch, const int *__restrict__ sc, __nv_bfloat16 *__restrict__ planes)
@@ -486,14 +513,19 @@ residue_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t 
         if (r0 + row >= rows || kb + kg * 8 >= pitch)
             continue;
         const int s = max(sc[r0 + row], -4096);
+        double x[8];
         float v[8][CH];
 #pragma unroll
-        for (int q = 0; q < 8; q++)
-            int_chunks<CH>(tile[(kg * 8 + q) * 32 + kg * 4 + row], s, v[q]);
+        for (int q = 0; q < 8; q++) {
+            x[q] = tile[(kg * 8 + q) * 32 + kg * 4 + row];
+            int_chunks<CH>(x[q], s, v[q]);
+        }
+        __nv_bfloat16 *dst = planes + (int64_t)(r0 + row) * pitch + kb + kg * 8;
+        if constexpr (kMag)
+            store_magnitudes(x, s, dst + N * (int64_t)rows * pitch);
         uint64_t chunk[CH][4];
         pack_chunks<N>(v, chunk);
-        store_residues<N, CH>(chunk, planes + (int64_t)(r0 + row) * pitch + kb + kg * 8,
-                              (int64_t)rows * pitch);
+        store_residues<N, CH>(chunk, dst, (int64_t)rows * pitch);
     }
 }
 
@@ -501,10 +533,10 @@ residue_cols_kernel(const double *__restrict__ X, int64_t ld, int rows, int64_t 
 // lane and step; a row of one step (K <= 8 G) is read once.  (A block per row for the scales
 // and another for the residues leave most of their threads without work: 600 900 rows of
 // 100 took 0.36 + 0.60 ms.)
-template <int N, int G, class Src>
+template <int N, bool kMag, int G, class Src>
 __global__ void __launch_bounds__(128)
 residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
-                     int *__restrict__ sc, int *bad, __nv_bfloat16 *__restrict__ planes)
+                     int *__restrict__ sc, __nv_bfloat16 *__restrict__ planes)
 {
     constexpr int CH = moduli::chunks(N);
     constexpr int kRows = 128 / G;  // rows per block
@@ -562,8 +594,6 @@ residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
                 s2 += __shfl_xor_sync(0xffffffffu, s2, o);
             if (!fast)
                 s = scale_slow(mb, s2, bits);
-            if (ok && s == kNotFinite && bad && gl == 0)
-                atomicExch(bad, 1);
         }
         if (!ok)
             continue;
@@ -578,6 +608,8 @@ residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
 #pragma unroll
             for (int q = 0; q < 8; q++)
                 residue_chunks<N>(x[q], s, v[q]);
+            if constexpr (kMag)
+                store_magnitudes(x, s, planes + r * pitch + kk + N * (int64_t)rows * pitch);
             uint64_t chunk[CH][4];
             pack_chunks<N>(v, chunk);
             store_residues<N, CH>(chunk, planes + r * pitch + kk, (int64_t)rows * pitch);
@@ -589,15 +621,14 @@ residue_short_kernel(Src src, int r0, int rows, int K, int pitch, float bits,
 // residues (residue_rows, one launch fewer); others beforehand (row_scales).
 constexpr int64_t kShortRow = 1024;
 
-// always: short rows too (their residues then find the same scales again).
 template <class Src>
 static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int64_t k_panel, int n_mod,
-                      int *sc, int *bad, bool always = false)
+                      int *sc)
 {
-    if (rows <= 0 || (K <= kShortRow && k_panel >= K && !always))
+    if (rows <= 0 || (K <= kShortRow && k_panel >= K))
         return CUTC_OK;
     row_scale_kernel<Src><<<std::min(rows, 1 << 20), 256, 0, st>>>(src, rows, K,
-                                                                    moduli::row_bits(n_mod), sc, bad);
+                                                                    moduli::row_bits(n_mod), sc);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
@@ -605,9 +636,9 @@ static int row_scales(cudaStream_t st, Src src, int rows, int64_t K, int64_t k_p
 
 // The planes of the K panel [k0, k0 + kp) for rows r0 .. r0 + rows; sc holds the scales of
 // all rows (row_scales) or receives them.
-template <int N, class Src>
+template <int N, bool kMag = false, class Src>
 static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t K, int64_t k0,
-                        int64_t kp, int64_t pitch, int *sc, void *planes, int *bad)
+                        int64_t kp, int64_t pitch, int *sc, void *planes)
 {
     if (rows <= 0 || kp <= 0)
         return CUTC_OK;
@@ -615,8 +646,8 @@ static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t K, i
     if (K <= kShortRow && kp == K) {
         auto launch = [&](auto g) {
             constexpr int G = decltype(g)::value;
-            residue_short_kernel<N, G, Src><<<std::min(ceil_div(rows, 128 / G), 1u << 16), 128, 0, st>>>(
-                src, r0, rows, (int)K, (int)pitch, moduli::row_bits(N), sc, bad, out);
+            residue_short_kernel<N, kMag, G, Src><<<std::min(ceil_div(rows, 128 / G), 1u << 16), 128, 0, st>>>(
+                src, r0, rows, (int)K, (int)pitch, moduli::row_bits(N), sc, out);
         };
         if (K <= 64)
             launch(std::integral_constant<int, 8>{});
@@ -626,7 +657,7 @@ static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t K, i
             launch(std::integral_constant<int, 32>{});
     } else {
         dim3 grid(ceil_div(pitch, 8 * 128), (unsigned)std::min(rows, 65535));
-        residue_rows_kernel<N, Src><<<grid, 128, 0, st>>>(src, r0, rows, k0, kp, pitch, sc, out);
+        residue_rows_kernel<N, kMag, Src><<<grid, 128, 0, st>>>(src, r0, rows, k0, kp, pitch, sc, out);
     }
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
@@ -635,24 +666,24 @@ static int residue_rows(cudaStream_t st, Src src, int r0, int rows, int64_t K, i
 
 template <class Src>
 static int residue_rows(cudaStream_t st, int n_mod, Src src, int r0, int rows, int64_t K,
-                        int64_t k0, int64_t kp, int64_t pitch, int *sc, void *planes, int *bad)
+                        int64_t k0, int64_t kp, int64_t pitch, int *sc, void *planes)
 {
     switch (n_mod) {
-    case 8: return residue_rows<8>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 9: return residue_rows<9>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 10: return residue_rows<10>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 11: return residue_rows<11>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 12: return residue_rows<12>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 13: return residue_rows<13>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 15: return residue_rows<15>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
-    case 17: return residue_rows<17>(st, src, r0, rows, K, k0, kp, pitch, sc, planes, bad);
+    case 8: return residue_rows<8>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 9: return residue_rows<9>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 10: return residue_rows<10>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 11: return residue_rows<11>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 12: return residue_rows<12>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 13: return residue_rows<13>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 15: return residue_rows<15>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
+    case 17: return residue_rows<17>(st, src, r0, rows, K, k0, kp, pitch, sc, planes);
     }
     cutc_set_error(CUTC_ERR_INVALID, "no residue kernel for %d moduli", n_mod);
     return CUTC_ERR_INVALID;
 }
 
 static inline int row_scales_cols(cudaStream_t st, const double *X, int64_t ld, int rows,
-                                  int64_t K, int n_mod, int *sc, int *bad)
+                                  int64_t K, int n_mod, int *sc)
 {
     if (rows <= 0)
         return CUTC_OK;
@@ -660,22 +691,22 @@ static inline int row_scales_cols(cudaStream_t st, const double *X, int64_t ld, 
     // a block)
     const float bits = moduli::row_bits(n_mod);
     if (rows <= 32 * 152)
-        row_scale_cols_kernel<8><<<ceil_div(rows, 8), 1024, 0, st>>>(X, ld, rows, K, bits, sc, bad);
+        row_scale_cols_kernel<8><<<ceil_div(rows, 8), 1024, 0, st>>>(X, ld, rows, K, bits, sc);
     else
-        row_scale_cols_kernel<32><<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K, bits, sc, bad);
+        row_scale_cols_kernel<32><<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K, bits, sc);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
-template <int N>
+template <int N, bool kMag = false>
 static int residue_cols(cudaStream_t st, const double *X, int64_t ld, int rows, int64_t k0,
                         int64_t kp, int64_t pitch, const int *sc, void *planes)
 {
     if (rows <= 0 || kp <= 0)
         return CUTC_OK;
     dim3 grid(ceil_div(pitch, 64), std::min(ceil_div(rows, 32), 65535u));
-    residue_cols_kernel<N><<<grid, 256, 0, st>>>(X, ld, rows, k0, kp, pitch, sc,
+    residue_cols_kernel<N, kMag><<<grid, 256, 0, st>>>(X, ld, rows, k0, kp, pitch, sc,
                                                  (__nv_bfloat16 *)planes);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);

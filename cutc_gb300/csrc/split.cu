@@ -235,12 +235,12 @@ int split_prepare_x(Engine *E, const Request &R, cudaStream_t st, const double *
         return CUTC_OK;  // the same molecule's scales (and residues) are already there
     CUTC_TRY(weighted_aos(st, R.n2, R.nA, wr2, aos2v, (int64_t)R.n2, (double *)p));
     SrcSym src{sp.wchi2, aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
-    CUTC_TRY(row_scales(st, src, np, (int64_t)R.n2, sp.k_panel, n_mod, sp.sc_ax, (int *)nullptr));
+    CUTC_TRY(row_scales(st, src, np, (int64_t)R.n2, sp.k_panel, n_mod, sp.sc_ax));
     if (sp.ax_whole)
         for (int64_t k0 = 0; k0 < R.n2; k0 += sp.k_panel) {
             const int64_t kp = std::min<int64_t>(sp.k_panel, R.n2 - k0);
             CUTC_TRY(residue_rows(st, n_mod, src, 0, np, R.n2, k0, kp, residue_pitch(kp), sp.sc_ax,
-                                  p_panel(sp, n_mod, np, k0), (int *)nullptr));
+                                  p_panel(sp, n_mod, np, k0)));
         }
     E->tag_x = R.mol_tag;
     E->tag_x_buf = sp.ax.p;
@@ -255,7 +255,7 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
     const int64_t np = n_pairs(R.nA);
     SrcSym sa{sp.wchi2, sp.aos2v, (int64_t)R.n2, (int64_t)R.n2, sp.pairs_sym};
     SrcDenseDF sb{G, (int64_t)R.n2};
-    CUTC_TRY(row_scales(st, sb, 4 * nb, (int64_t)R.n2, sp.k_panel, n_mod, sp.sc_bx, (int *)nullptr));
+    CUTC_TRY(row_scales(st, sb, 4 * nb, (int64_t)R.n2, sp.k_panel, n_mod, sp.sc_bx));
     if (gemm_begin)
         CUTC_CUDA_TRY(cudaEventRecord(gemm_begin, st));
     // column (c, i) of the tile -> column c blk_rows + ib + i of the block
@@ -269,12 +269,10 @@ int split_x_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp, co
                 a.p = p_panel(sp, n_mod, (int)np, k0);
                 return CUTC_OK;
             }
-            return residue_rows(st, n_mod, sa, 0, (int)np, R.n2, k0, kp, a.pitch, sp.sc_ax, a.p,
-                                (int *)nullptr);
+            return residue_rows(st, n_mod, sa, 0, (int)np, R.n2, k0, kp, a.pitch, sp.sc_ax, a.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &b) {
-            return residue_rows(st, n_mod, sb, n0, nc, R.n2, k0, kp, b.pitch, sp.sc_bx, b.p,
-                                (int *)nullptr);
+            return residue_rows(st, n_mod, sb, n0, nc, R.n2, k0, kp, b.pitch, sp.sc_bx, b.p);
         }));
     if (gemm_end)
         CUTC_CUDA_TRY(cudaEventRecord(gemm_end, st));
@@ -315,13 +313,13 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
     SrcAnti sn{wchi, aos1, nb, nA, ld1, sp.pairs_anti};
     if (!keep_b) {
         CUTC_TRY(weighted_aos(st, nb, nA, wr1, aos1, ld1, wchi));
-        CUTC_TRY(row_scales(st, s0, np, (int64_t)nb, pan_h, n_mod, sc_h, (int *)nullptr));
-        CUTC_TRY(row_scales(st, sn, nl, k3, pan_n, n_mod, sc_n, (int *)nullptr));
+        CUTC_TRY(row_scales(st, s0, np, (int64_t)nb, pan_h, n_mod, sc_h));
+        CUTC_TRY(row_scales(st, sn, nl, k3, pan_n, n_mod, sc_n));
     }
     const double beta = first ? 0.0 : 1.0;
     // Xt[(m nb + i) np + p]: X_3 is column block 3, X_012 the blocks 0..2
     const double *x3 = Xt + 3 * (int64_t)nb * np;
-    CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a, nullptr));
+    CUTC_TRY(row_scales_cols(st, x3, np, np, nb, n_mod, sc_a));
     CUTC_TRY(modular_contract(
         st, W, slot0 + SS_BH, slot0 + SS_RES, operand_bytes(R), operand_bytes(R), n_mod, np, np, nb,
         pan_h, a, keep_b, sc_a, sc_h, ModularOut{H, np, np, 0, 0, 1.0, beta}, sp.err,
@@ -329,10 +327,10 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
             return residue_cols(st, n_mod, x3, np, np, k0, kp, o.pitch, sc_a, o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-            return residue_rows(st, n_mod, s0, n0, nc, nb, k0, kp, o.pitch, sc_h, o.p, (int *)nullptr);
+            return residue_rows(st, n_mod, s0, n0, nc, nb, k0, kp, o.pitch, sc_h, o.p);
         }));
     if (nl > 0) {
-        CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a, nullptr));
+        CUTC_TRY(row_scales_cols(st, Xt, np, np, k3, n_mod, sc_a));
         CUTC_TRY(modular_contract(
             st, W, slot0 + SS_BN, slot0 + SS_RES, operand_bytes(R), operand_bytes(R), n_mod, np, nl, k3,
             pan_n, a, keep_b, sc_a, sc_n, ModularOut{N, np, nl, 0, 0, -0.5, beta}, sp.err,
@@ -340,8 +338,7 @@ int split_int2e_tile(Engine *E, const Request &R, cudaStream_t st, SplitPlan &sp
                 return residue_cols(st, n_mod, Xt, np, np, k0, kp, o.pitch, sc_a, o.p);
             },
             [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-                return residue_rows(st, n_mod, sn, n0, nc, k3, k0, kp, o.pitch, sc_n, o.p,
-                                    (int *)nullptr);
+                return residue_rows(st, n_mod, sn, n0, nc, k3, k0, kp, o.pitch, sc_n, o.p);
             }));
     }
     E->tag_i = whole && nb == R.n1 ? R.mol_tag : 0;
@@ -415,17 +412,17 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
     ResiduePlanes a;
     a.p = p;
     CUTC_CUDA_TRY(cudaMemsetAsync(err, 0, 4, st));
-    CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sc_a, (int *)nullptr));
-    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, sc_b, (int *)nullptr));
+    CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sc_a));
+    CUTC_TRY(row_scales(st, sb, N, K, pan, n_mod, sc_b));
     sp.err = err;
     return modular_contract(
         st, W, base + 4, base + 5, (size_t)8 << 30, (size_t)4 << 30, n_mod, M, N, K, pan, a, false, sc_a, sc_b,
         ModularOut{C, ldc, N, 0, 0, alpha, 0.0}, err,
         [&](int, int, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-            return residue_rows(st, n_mod, sa, 0, M, K, k0, kp, o.pitch, sc_a, o.p, (int *)nullptr);
+            return residue_rows(st, n_mod, sa, 0, M, K, k0, kp, o.pitch, sc_a, o.p);
         },
         [&](int n0, int nc, int64_t k0, int64_t kp, const ResiduePlanes &o) {
-            return residue_rows(st, n_mod, sb, n0, nc, K, k0, kp, o.pitch, sc_b, o.p, (int *)nullptr);
+            return residue_rows(st, n_mod, sb, n0, nc, K, k0, kp, o.pitch, sc_b, o.p);
         });
 }
 
