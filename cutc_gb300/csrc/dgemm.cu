@@ -221,9 +221,11 @@ __global__ void __launch_bounds__(kThreads, 1) fp64_gemm_kernel(const Args g)
 }
 
 // The results that a checked modular contraction left out (result_left), in FP64: M x N
-// results of one pass.  A block per SM walks the 128 x 128 tiles and lists each one's.  Few of
-// them are formed by a warp each, whose loads of 16 bytes per term the L2 feeds at about the
-// FP64 pipe's rate; more than kFewLeft by the whole tile's product.
+// results of one pass, by a block per SM.  Listed ones are formed by a warp each (12 000 x 300
+// results of K 12 000 with some dozens left: 0.70 ms when every block looked for its tiles'
+// own, 0.04 so).  With more than the list holds, the blocks walk the 128 x 128 tiles and
+// list each one's: up to kFewLeft are formed by a warp each, whose loads of 16 bytes per term
+// the L2 feeds at about the FP64 pipe's rate, more by the whole tile's product.
 struct RestArgs {
     int M, N;
     int64_t K;
@@ -234,14 +236,15 @@ struct RestArgs {
     const int *sa, *sb;
     int n0;
     ModularOut out;
-    const int *left;
+    const LeftResults *left;
 };
 constexpr int kFewLeft = 2048;
 
 template <bool AK>
 __global__ void __launch_bounds__(kThreads, 1) contract_rest_kernel(const RestArgs g)
 {
-    if (*g.left == 0)
+    const int total = g.left->count;
+    if (total == 0)
         return;
     extern __shared__ __align__(16) double smem[];
     __shared__ unsigned short s_list[kFewLeft];
@@ -262,6 +265,27 @@ __global__ void __launch_bounds__(kThreads, 1) contract_rest_kernel(const RestAr
         const double v = o.alpha * sum;
         *c = o.beta == 0.0 ? v : v + o.beta * *c;
     };
+    auto one = [&](int m, int n) {  // by a warp
+        const double *a = AK ? g.A + (int64_t)m * g.lda : g.A + m;
+        const double *b = g.B + (int64_t)n * g.ldb;
+        double sum = 0.0;
+#pragma unroll 8
+        for (int64_t k = lane; k < g.K; k += 32)
+            sum = fma(AK ? a[k] : a[k * g.lda], b[k], sum);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+            sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        if (lane == 0)
+            store(m, n, sum);
+    };
+    if (total <= kMaxListed) {
+        // (the blocks take neighbours of the list in turn)
+        for (int e = warp * gridDim.x + blockIdx.x; e < total; e += gridDim.x * (kThreads / 32)) {
+            const int2 at = g.left->at[e];
+            one(at.x, at.y);
+        }
+        return;
+    }
     for (int64_t t = blockIdx.x; t < (int64_t)tiles_m * tiles_n; t += gridDim.x) {
         const int m0 = (int)(t % tiles_m) * kBM, n0 = (int)(t / tiles_m) * kBN;
         __syncthreads();  // the last tile's list is read
@@ -277,20 +301,8 @@ __global__ void __launch_bounds__(kThreads, 1) contract_rest_kernel(const RestAr
         __syncthreads();
         const int count = s_count;
         if (count <= kFewLeft) {
-            for (int e = warp; e < count; e += kThreads / 32) {
-                const int m = m0 + s_list[e] % kBM, n = n0 + s_list[e] / kBM;
-                const double *a = AK ? g.A + (int64_t)m * g.lda : g.A + m;
-                const double *b = g.B + (int64_t)n * g.ldb;
-                double sum = 0.0;
-#pragma unroll 4
-                for (int64_t k = lane; k < g.K; k += 32)
-                    sum = fma(AK ? a[k] : a[k * g.lda], b[k], sum);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1)
-                    sum += __shfl_xor_sync(0xffffffffu, sum, o);
-                if (lane == 0)
-                    store(m, n, sum);
-            }
+            for (int e = warp; e < count; e += kThreads / 32)
+                one(m0 + s_list[e] % kBM, n0 + s_list[e] / kBM);
             continue;
         }
         double acc[8][4][2];
@@ -443,11 +455,12 @@ size_t fp64_contract_bytes(int64_t M, int64_t N, int64_t K, size_t limit)
 int fp64_contract_begin(Workspace &W, int slot0, cudaStream_t st, size_t limit, ContractScratch &S)
 {
     void *p;
-    CUTC_TRY(W.get(slot0 + C_FLAGS, 64, &p));
+    CUTC_TRY(W.get(slot0 + C_FLAGS, 64 + sizeof(LeftResults), &p));
     S.W = &W;
     S.limit = limit;
     S.slot0 = slot0;
     S.flags = (int *)p;
+    S.left = (LeftResults *)((char *)p + 64);
     CUTC_CUDA_TRY(cudaMemsetAsync(p, 0, 64, st));
     return CUTC_OK;
 }
@@ -473,7 +486,8 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
 {
     constexpr int n_mod = kPlainModuli;
     Workspace &W = *S.W;
-    int *err = S.flags, *left = S.flags + 1;
+    int *err = S.flags;
+    LeftResults *left = S.left;
     ContractPlan c;
     ResiduePlanes a;
     void *b = nullptr, *res = nullptr, *psa = nullptr, *psb = nullptr;
@@ -499,7 +513,6 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
     *done = true;
     int *sca = (int *)psa, *scb = (int *)psb;
     const int64_t pan = c.kp;
-    CUTC_CUDA_TRY(cudaMemsetAsync(left, 0, 4, st));
     const SrcDense sa{A, lda}, sb{B, ldb};
     if (a_kmajor)
         CUTC_TRY(row_scales(st, sa, M, K, pan, n_mod, sca));

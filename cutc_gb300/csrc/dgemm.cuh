@@ -35,12 +35,13 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // The scratch (kContractSlots slots from the given one) belongs to one stream until its
 // work is done: calls that wait for their results share kContractSlot, a call that returns
 // while its contractions still run has slots of its own.
+struct LeftResults;
 struct ContractScratch {
     Workspace *W = nullptr;
     int slot0 = 0;
     size_t limit = 0;
-    int *flags = nullptr;  // [0]: a wait gave up, [1]: results of the contraction at hand were
-                           // left to the FP64 kernel
+    int *flags = nullptr;  // [0]: a wait gave up
+    LeftResults *left = nullptr;
 };
 constexpr size_t kContractBytes = (size_t)16 << 30;  // the largest limit
 constexpr int kContractSlot = 100, kContractSlots = 6;

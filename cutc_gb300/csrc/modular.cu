@@ -363,7 +363,7 @@ struct CombineParams {
     ModularOut out;
     int alpha_exp, alpha_neg, alpha_mul, beta_mode;  // beta_mode: 0, 1 or 2 (any other beta)
     const int *err;
-    int *left;
+    LeftResults *left;
 };
 
 // Tables of the Chinese remainder theorem for N moduli: V = sum_i r_i W_i mod M with
@@ -665,7 +665,11 @@ __global__ void __launch_bounds__(128) combine_kernel(const CombineParams P)
                 f[l] = h ? tc::f2_hi(v[l]) : tc::f2_lo(v[l]);
             const int sm = h ? s1 : s0;
             if (kChecked && result_left(h ? sums >> 16 : sums & 0xffffu, sm, sn)) {
-                *P.left = 1;
+                if (*(volatile int *)&P.left->count < kMaxListed) {
+                    const int at = atomicAdd(&P.left->count, 1);
+                    if (at < kMaxListed)
+                        P.left->at[at] = make_int2(m + h, c);
+                }
                 continue;
             }
             double x;
@@ -842,7 +846,8 @@ static int launch_combine(cudaStream_t st, const CombineParams &P)
 }
 
 int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
-                    const int *sa, const int *sb, const ModularOut &out, const int *err, int *left)
+                    const int *sa, const int *sb, const ModularOut &out, const int *err,
+                    LeftResults *left)
 {
     if (M <= 0 || ncols <= 0)
         return CUTC_OK;

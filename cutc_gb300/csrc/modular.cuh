@@ -141,13 +141,21 @@ inline int64_t modular_ldm(int64_t M) { return (M + 7) / 8 * 8; }
 int modular_gemm(cudaStream_t st, int n_mod, int planes, const ResiduePlanes &A, const ResiduePlanes &B,
                  unsigned short *out, int64_t plane_cols, bool accumulate, int *err);
 
+// Results that a checked contraction leaves out of one pass.
+constexpr int kMaxListed = 1 << 15;
+struct LeftResults {
+    int count;             // may exceed kMaxListed
+    int2 at[kMaxListed];   // (row, column) in the pass's block
+};
+
 // The FP64 results from the residues: n0 .. n0 + ncols of the output's columns; sa and sb
 // are the row scales of A and B (sb of column n0 first).  A result with a scale of
 // kNotFinite, or after a wait that gave up, is NaN.  Checked (left not null, res with the
 // magnitudes' sums): results of such scales and those whose sum is below kCheckSum are not
-// written, and *left is set to 1 when there are any (result_left tells which).
+// written but counted and listed (result_left tells which, where the list is too short).
 int modular_combine(cudaStream_t st, int n_mod, int M, int n0, int ncols, const unsigned short *res,
-                    const int *sa, const int *sb, const ModularOut &out, const int *err, int *left);
+                    const int *sa, const int *sb, const ModularOut &out, const int *err,
+                    LeftResults *left);
 
 // A plane's entry for a magnitudes' sum, and whether a checked result is left out.
 constexpr unsigned kResidueOffset = 512;
@@ -192,7 +200,7 @@ template <class GenA, class GenB, class Rest>
 int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K, int64_t k_panel,
                             const ModularBlocks &blk, ResiduePlanes a, void *b_p, bool b_ready,
                             unsigned short *res, const int *sa, const int *sb, ModularOut out,
-                            int *err, int *left, GenA gen_a, GenB gen_b, Rest rest)
+                            int *err, LeftResults *left, GenA gen_a, GenB gen_b, Rest rest)
 {
     const int planes = n_mod + (left ? 1 : 0);
     ResiduePlanes b;
@@ -220,6 +228,8 @@ int modular_contract_blocks(cudaStream_t st, int n_mod, int M, int N, int64_t K,
                                           nc, k0 > 0, err));
                 }
             }
+            if (left)
+                CUTC_CUDA_TRY(cudaMemsetAsync(&left->count, 0, sizeof(int), st));
             CUTC_TRY(modular_combine(st, n_mod, a.rows, n0, nc, res, sa + m0, sb + n0, out, err,
                                      left));
             if (left)
