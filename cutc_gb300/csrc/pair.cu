@@ -241,6 +241,105 @@ int launch_pair_f64(cudaStream_t st, const PairArgs &P)
     return CUTC_OK;
 }
 
+// ---------------------------------------------------------------------------
+// marked pairs
+// ---------------------------------------------------------------------------
+
+// a r / (1 + a r) and, unless null, its gradient, of the distance vector d (zero below the
+// coalescence guard)
+__device__ __forceinline__ double scaled_distance(const double (&d)[3], double a, double *grad)
+{
+    const double d2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
+    if (grad)
+        grad[0] = grad[1] = grad[2] = 0.0;
+    if (!(d2 > 1e-15))
+        return 0.0;
+    const double r = sqrt(d2);
+    const double t = 1.0 / (1.0 + a * r);
+    if (grad) {
+        const double s = a * t * t / r;
+        for (int k = 0; k < 3; k++)
+            grad[k] = s * d[k];
+    }
+    return a * r * t;
+}
+
+// Every block takes 256 words of marks at a time, lists their pairs in shared memory and shares
+// them out over its threads, which form them as pair_f64_kernel does.
+constexpr int kMarkWords = 256;
+
+__global__ void __launch_bounds__(256)
+pair_f64_marked_kernel(PairArgs P, const double *__restrict__ rn, double a_en,
+                       const int *__restrict__ marked, const unsigned *__restrict__ marks, int words)
+{
+    if (*marked == 0)
+        return;
+    __shared__ unsigned short s_list[kMarkWords * 32];  // 32 word + bit
+    __shared__ int s_count;
+    const int64_t total = (int64_t)P.n1b * words;
+    for (int64_t w0 = (int64_t)blockIdx.x * kMarkWords; w0 < total; w0 += (int64_t)gridDim.x * kMarkWords) {
+        __syncthreads();  // the last words' list is read
+        if (threadIdx.x == 0)
+            s_count = 0;
+        __syncthreads();
+        unsigned bits = w0 + threadIdx.x < total ? marks[w0 + threadIdx.x] : 0u;
+        if (bits) {
+            int at = atomicAdd(&s_count, __popc(bits));
+            for (; bits; bits &= bits - 1)
+                s_list[at++] = (unsigned short)(32 * threadIdx.x + __ffs((int)bits) - 1);
+        }
+        __syncthreads();
+        const int count = s_count;
+        for (int e = threadIdx.x; e < count; e += 256) {
+            const int64_t w = w0 + s_list[e] / 32;
+            const int i = (int)(w / words), j = (int)(w % words) * 32 + s_list[e] % 32;
+            if (j >= P.n2)  // (marks of a tile that gave up are not set)
+                continue;
+            const double *p1 = P.r1 + 3 * (int64_t)(P.i0 + i), *p2 = P.r2 + 3 * (int64_t)j;
+            const double d12[3] = {p1[0] - p2[0], p1[1] - p2[1], p1[2] - p2[2]};
+            double gg[3], Gp[kTab], F1[kTab], F2[kTab];
+            powers(scaled_distance(d12, P.a_ee, gg), Gp, 1);
+            double u[3] = {0.0, 0.0, 0.0}, dudg = 0.0;
+            for (int A = 0; A < P.nN; A++) {
+                const double d1[3] = {p1[0] - rn[3 * A], p1[1] - rn[3 * A + 1], p1[2] - rn[3 * A + 2]};
+                double fg[3];
+                powers(scaled_distance(d1, a_en, fg), F1, 1);
+                powers(P.f2[(int64_t)A * P.n2 + j], F2, 1);
+                double dudf1 = 0.0;
+                for (int k = P.term_off[A]; k < P.term_off[A + 1]; k++) {
+                    const int ex = P.exps[k];
+                    const int m = ex & 7, n = (ex >> 3) & 7, o = (ex >> 6) & 7;
+                    const double cm = P.coef[3 * k], cn = P.coef[3 * k + 1], co = P.coef[3 * k + 2];
+                    dudf1 += (cm * F1[m > 0 ? m - 1 : 0] * F2[n] + cn * F1[n > 0 ? n - 1 : 0] * F2[m]) * Gp[o];
+                    dudg += co * Gp[o > 0 ? o - 1 : 0] * (F1[m] * F2[n] + F1[n] * F2[m]);
+                }
+                for (int k = 0; k < 3; k++)
+                    u[k] += dudf1 * fg[k];
+            }
+            for (int k = 0; k < 3; k++)
+                u[k] += dudg * gg[k];
+            double *out = P.G + (int64_t)i * P.ldg + j;
+            out[0] = u[0];
+            out[P.plane] = u[1];
+            out[2 * P.plane] = u[2];
+            out[3 * P.plane] = -0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+        }
+    }
+}
+
+int launch_pair_f64_marked(cudaStream_t st, const PairArgs &P, const double *rn, double a_en,
+                           const int *marked, const unsigned *marks, int words, int n_sm)
+{
+    if (P.n1b <= 0 || P.n2 <= 0)
+        return CUTC_OK;
+    const int64_t blocks = ((int64_t)P.n1b * words + kMarkWords - 1) / kMarkWords;
+    pair_f64_marked_kernel<<<(unsigned)std::min<int64_t>(blocks, 4 * n_sm), 256, 0, st>>>(
+        P, rn, a_en, marked, marks, words);
+    CUTC_CUDA_TRY(cudaGetLastError());
+    note_launches(1);
+    return CUTC_OK;
+}
+
 }  // namespace cutc
 
 // ---------------------------------------------------------------------------

@@ -81,5 +81,9 @@ int launch_r1_terms(cudaStream_t st, int i0, int n, int nN, const double *r1, co
 int launch_r2_terms(cudaStream_t st, int n2, int nN, const double *r2, const double *rn,
                     double a, double *f2);
 int launch_pair_f64(cudaStream_t st, const PairArgs &P);
+// The pairs (i, j) of the tile whose bit j % 32 of marks[i words + j / 32] is set, term by term
+// (P.t1 is not used); returns at once on the device while *marked is zero.
+int launch_pair_f64_marked(cudaStream_t st, const PairArgs &P, const double *rn, double a_en,
+                           const int *marked, const unsigned *marks, int words, int n_sm);
 
 }  // namespace cutc

@@ -32,6 +32,16 @@
 // operations per pair with 16 rows instead of 30 df multiply-adds (~450 operations) per
 // nucleus.
 //
+// F and the coefficients enter with an error relative to their rows' maxima, where a term by
+// term sum's is relative to the terms.  So FP64 results are checked: one more product, of the
+// operands' magnitudes to 8 bits (plane S, accumulators of its own), gives
+// v_c = sum_k |C[(r1, c)][k]| F[r2][k], and with it the sums of the terms' magnitudes and of the
+// errors, both as polynomials in g12.  The error of V_c is about sqrt(K) 2^-63 of the row
+// scales (rms, from the seven slices and the products left out); pairs for which four times
+// that is above 2^-53 of the terms (r2 near a nucleus whose terms all vanish there, small
+// values of few nuclei: fewer than one in 10^4 of 8 nuclei with 13 terms) are marked in a bit
+// mask and formed again term by term behind the kernel (pair.cu).
+//
 // FP64 epilogue: the diagonals down to 2^-43 of the row scales become one exact integer
 // and a double in integer arithmetic, the rest stays in FP32 beside it, and g12, its
 // gradient and the polynomial take FP64: 45 FP64 operations per pair with 16 rows, whatever
@@ -67,10 +77,14 @@ struct PairTcParams {
     int tiles_m, tiles_n, chunk;  // r2 tiles of 128 points, N tiles, N tiles per CTA
     int Mpad, Npad;               // padded rows of the F and coefficient slices
     const int *ea, *eb;           // row exponents of the F and the coefficient slices
-    const float *bscale;          // double-float: 2^(row exponent) of each coefficient row
+    const float *bscale;          // 2^(row exponent) of each coefficient row, 0 for a zero row
     const float2 *r1d;            // double-float: the tile's r1 points, [3 i + c]
     PairDfArgs P;                 // geometry and outputs
     double *G64;                  // FP64: in place of P.G
+    float check;                  // FP64: 2^8 / sqrt(K)
+    unsigned *marks;              // FP64: bit j % 32 of marks[i mark_words + j / 32]: (i, j) is
+    int mark_words;               // left out, and *marked is set
+    int *marked;
     int *err;
     // a group of K blocks of a longer contraction: from block kb0 on; the values so far are
     // added (not for the first group), and kept (not for the last) at
@@ -78,7 +92,7 @@ struct PairTcParams {
     int kb0, first, last;
     float2 *part;
     long long *partI;
-    float *partL;
+    float *partL, *partA;         // (and the magnitudes' sums)
 };
 
 // x 2^e for the scale of a value of row exponents e (clamped to the float range); NaN for
@@ -89,14 +103,6 @@ __device__ __forceinline__ float pow2f(int e)
         return __int_as_float(0x7fffffff);
     e = e < -126 ? -126 : (e > 127 ? 127 : e);
     return __int_as_float((e + 127) << 23);
-}
-
-// bscale[r] = 2^ex[r] as a float
-__global__ void exp_scale_kernel(const int *__restrict__ ex, int rows, float *__restrict__ bscale)
-{
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r < rows)
-        bscale[r] = pow2f(ex[r]);
 }
 
 // R: coefficient rows per r1 point (16 or 32).
@@ -115,14 +121,16 @@ struct PairTcCfg {
     static constexpr int kBufWarps = kEpiWarps / kBufs;  // epilogue warps of a buffer
     static constexpr int kCtlWarp = kEpiWarps;       // TMA loads and MMAs, lane 0
     static constexpr int kThreads = (kEpiWarps + 1) * 32;
+    static constexpr int kPlanes = S + (F64 ? 1 : 0);  // slices, and the magnitudes
     static constexpr int kASlice = kBM * kBK * 2;
     static constexpr int kBSlice = kBN * kBK * 2;
-    static constexpr int kABytes = KB * S * kASlice;
-    static constexpr int kBStage = KB * S * kBSlice;
+    static constexpr int kABytes = KB * kPlanes * kASlice;
+    static constexpr int kBStage = KB * kPlanes * kBSlice;
+    static constexpr int kBufCols = kBN * kPlanes;   // accumulator columns of a buffer
     static constexpr int kSmem = kABytes + kBufs * kBStage + 1024 + 256;
     static constexpr int kMaxN = 256;                // widest kind::f16 instruction at M = 128
     static_assert(kSmem <= 227 * 1024, "shared memory");
-    static_assert(kBufs * kBN * S <= (int)kTmemCols, "accumulators exceed tensor memory");
+    static_assert(kBufs * kBufCols <= (int)kTmemCols, "accumulators exceed tensor memory");
     static_assert(kMaxN % kBN == 0, "instruction splits on diagonal boundaries");
     static_assert(kBSlice % 512 == 0, "B slices must stack on 8-row swizzle atoms");
 };
@@ -378,12 +386,45 @@ __device__ __forceinline__ double minus_half(double x)
     return -0.5 * x;
 }
 
-// One pair in FP64 from its V values (hi + lo).  The reciprocal square root and the
+// Whether the error of a pair's values may be above that of a term by term sum (the check at
+// the top of this file): w[c] = 2^eb_c (check v_c - 1), the margin of V_c.
+template <int R>
+__device__ __forceinline__ bool pair_unsure(const float *w, float g, float gx, float gy, float gz)
+{
+    float ux, uy, uz, dudg;
+    if constexpr (R == 16) {
+        const float g2 = g * g;
+        auto poly = [&](int c) { return fmaf(fmaf(fmaf(w[c + 3], g, w[c + 2]), g, w[c + 1]), g2, w[c]); };
+        ux = poly(0);
+        uy = poly(4);
+        uz = poly(8);
+        dudg = fmaf(fmaf(w[14], g, w[13]), g, w[12]) * g;
+    } else {
+        auto poly = [&](int c, int n) {
+            float s = w[c + n - 1];
+#pragma unroll
+            for (int o = n - 2; o >= 0; o--)
+                s = fmaf(s, g, w[c + o]);
+            return s;
+        };
+        ux = poly(0, 7);
+        uy = poly(7, 7);
+        uz = poly(14, 7);
+        dudg = poly(21, 6);
+    }
+    // (a NaN is unsure)
+    return !(fmaf(dudg, fabsf(gx), ux) >= 0.f && fmaf(dudg, fabsf(gy), uy) >= 0.f &&
+             fmaf(dudg, fabsf(gz), uz) >= 0.f);
+}
+
+// One pair in FP64 from its V values (hi + lo); true, and nothing is written, when they are
+// unsure.  The reciprocal square root and the
 // reciprocal are FP32 seeds with one step each of third order in FP64 (the seeds' relative
 // errors of 2^-22 and 2^-23 become 2^-63 and below).
 template <int R>
-__device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, const double *V,
-                                         const float *W, double x2, double y2, double z2)
+__device__ __forceinline__ bool pair_f64(const PairTcParams &Q, int i, int j, const double *V,
+                                         const float *W, const float *w, double x2, double y2,
+                                         double z2)
 {
     const PairDfArgs &P = Q.P;
     const double *r1p = P.r1 + 3 * (int64_t)(P.i0 + i);
@@ -425,6 +466,8 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
         gz = s * dz;
     }
     const float gf = trunc_float(g);
+    if (pair_unsure<R>(w, gf, trunc_float(gx), trunc_float(gy), trunc_float(gz)))
+        return true;
     double ux, uy, uz, dudg;
     float lx, ly, lz, lg;
     if constexpr (R == 16) {
@@ -472,6 +515,7 @@ __device__ __forceinline__ void pair_f64(const PairTcParams &Q, int i, int j, co
     o[P.plane] = uy;
     o[2 * P.plane] = uz;
     o[3 * P.plane] = minus_half(fma(ux, ux, fma(uy, uy, uz * uz)));
+    return false;
 }
 
 // PART: one group of K blocks of a longer contraction (Q.kb0, Q.first, Q.last).
@@ -481,7 +525,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                const __grid_constant__ PairTcParams Q)
 {
     using Cfg = PairTcCfg<S, KB, R, F64>;
-    constexpr int D = S - 1, BN = Cfg::kBN;
+    constexpr int D = S - 1, BN = Cfg::kBN, NP = Cfg::kPlanes;
     constexpr int kCtlWarp = Cfg::kCtlWarp;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -546,9 +590,9 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                 for (int kb = 0; kb < KB; kb++)
 #pragma unroll
-                    for (int t = 0; t < S; t++)
+                    for (int t = 0; t < NP; t++)
                         tc::tma_load_2d(
-                            tc::smem_u32(sB + b * Cfg::kBStage + (kb * S + t) * Cfg::kBSlice), &tmB,
+                            tc::smem_u32(sB + b * Cfg::kBStage + (kb * NP + t) * Cfg::kBSlice), &tmB,
                             (kb0 + kb) * kBK, t * Q.Npad + n0, fb);
             };
             const uint32_t ab = tc::smem_u32(afull);
@@ -556,8 +600,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
             for (int kb = 0; kb < KB; kb++)
 #pragma unroll
-                for (int s = 0; s < S; s++)
-                    tc::tma_load_2d(tc::smem_u32(sA + (kb * S + s) * Cfg::kASlice), &tmA,
+                for (int s = 0; s < NP; s++)
+                    tc::tma_load_2d(tc::smem_u32(sA + (kb * NP + s) * Cfg::kASlice), &tmA,
                                     (kb0 + kb) * kBK, s * Q.Mpad + m0, ab);
             int loaded = 0;  // B tiles issued
             for (; loaded < min(NB, ntiles); loaded++)
@@ -579,7 +623,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 tc::fence_after_sync();
                 const uint32_t sb0 = tc::smem_u32(sB + b * Cfg::kBStage);
-                const uint32_t acc = tbase + (uint32_t)(BN * S * b);
+                const uint32_t acc = tbase + (uint32_t)(Cfg::kBufCols * b);
                 const uint32_t sa0 = tc::smem_u32(sA);
                 bool first = true;
 #pragma unroll
@@ -591,17 +635,23 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             // a_s x [b_0 .. b_{D-s}] -> diagonals s .. D, in instructions of
                             // at most kMaxN columns
                             const uint64_t ad = tc::smem_desc_sw64(
-                                sa0 + (kb * S + s) * Cfg::kASlice + k16 * 32);
+                                sa0 + (kb * NP + s) * Cfg::kASlice + k16 * 32);
 #pragma unroll
                             for (int t0 = 0; t0 <= D - s; t0 += Cfg::kMaxN / BN) {
                                 const int nt = min(Cfg::kMaxN / BN, D - s + 1 - t0);
                                 const uint64_t bd = tc::smem_desc_sw64(
-                                    sb0 + (kb * S + t0) * Cfg::kBSlice + k16 * 32);
+                                    sb0 + (kb * NP + t0) * Cfg::kBSlice + k16 * 32);
                                 tc::mma_bf16(acc + (uint32_t)(BN * (s + t0)), ad, bd,
                                              tc::idesc_bf16_f32(kBM, BN * nt), first ? 0u : 1u);
                             }
                             first = false;
                         }
+                        if constexpr (F64)  // the magnitudes' sums
+                            tc::mma_bf16(
+                                acc + (uint32_t)(BN * S),
+                                tc::smem_desc_sw64(sa0 + (kb * NP + S) * Cfg::kASlice + k16 * 32),
+                                tc::smem_desc_sw64(sb0 + (kb * NP + S) * Cfg::kBSlice + k16 * 32),
+                                tc::idesc_bf16_f32(kBM, BN), kb > 0 || k16 > 0 ? 1u : 0u);
                     }
                 }
                 tc::mma_commit(tc::smem_u32(&empty[b]));
@@ -654,11 +704,12 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 break;
             }
             tc::fence_after_sync();
-            const uint32_t cb = tbase + lane_off + (uint32_t)(BN * S * buf + R * pt0);
+            const uint32_t cb = tbase + lane_off + (uint32_t)(Cfg::kBufCols * buf + R * pt0);
             const int i0 = (t_begin + q) * Cfg::kPts + pt0;  // r1 row of the tile
             if constexpr (F64) {
                 double V[R];
-                float lo[R];
+                float lo[R], w[R];
+                const float *bs = Q.bscale + (int64_t)i0 * R;
                 const int *eb = Q.eb + (int64_t)i0 * R;
                 const bool out = jok && i0 < P.n1b;
 #pragma unroll
@@ -666,6 +717,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     long long I[8];
                     float rest[8];
                     read_f64_8<S, BN>(cb + (uint32_t)c, I, rest);
+                    float v[8];
+                    tc::tmem_ld8(cb + (uint32_t)(BN * S + c), v);
                     if constexpr (PART) {
                         if (out)
 #pragma unroll
@@ -674,23 +727,35 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                                 if (!Q.first) {
                                     I[k] += Q.partI[o];
                                     rest[k] += Q.partL[o];
+                                    v[k] += Q.partA[o];
                                 }
                                 if (!Q.last) {
                                     Q.partI[o] = I[k];
                                     Q.partL[o] = rest[k];
+                                    Q.partA[o] = v[k];
                                 }
                             }
                     }
 #pragma unroll
-                    for (int k = 0; k < 8; k++)
+                    for (int k = 0; k < 8; k++) {
                         scale_f64(I[k], rest[k], eb[c + k], ea, V + c + k, lo + c + k);
+                        w[c + k] = bs[c + k] * fmaf(Q.check, v[k], -1.0f);
+                    }
                 }
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
                     tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-                if (out && (!PART || Q.last))
-                    pair_f64<R>(Q, i0, j, V, lo, dx2, dy2, dz2);
+                if (!PART || Q.last) {
+                    const bool unsure = out && (pair_f64<R>(Q, i0, j, V, lo, w, dx2, dy2, dz2) ||
+                                                ea >= kNanExponent);
+                    const unsigned marks = __ballot_sync(0xffffffffu, unsure);
+                    if (lane == 0 && i0 < P.n1b && j < P.n2) {
+                        Q.marks[(int64_t)i0 * Q.mark_words + j / 32] = marks;
+                        if (marks)
+                            *Q.marked = 1;
+                    }
+                }
             } else {
                 uint64_t H[R / 16][8], L[R / 16][8], L2[R / 16][8];
 #pragma unroll
@@ -744,11 +809,13 @@ __device__ __forceinline__ int row_exponent(unsigned long long bits)
 
 // slices[(s * Mpad + r) * Kpad + k] for r < Mpad, k < Kpad (a multiple of 32; zeros outside
 // M x K), ex[r] = row exponent, of X[r * K + k]: one warp per row.  The digits are formed in
-// integer arithmetic (digits.cuh).
-template <int S>
+// integer arithmetic (digits.cuh).  kMag: the magnitudes on the row scale, truncated to BF16, as
+// plane S.  scale (may be null): 2^ex[r], 0 for a zero row, with kMag NaN for rows beyond 2^100
+// (which the check then leaves out).
+template <int S, bool kMag>
 __global__ void __launch_bounds__(256)
 slice_kernel(const double *__restrict__ X, int M, int K, int Kpad, int Mpad,
-             __nv_bfloat16 *__restrict__ slices, int *__restrict__ ex)
+             __nv_bfloat16 *__restrict__ slices, int *__restrict__ ex, float *__restrict__ scale)
 {
     const int lane = threadIdx.x & 31;
     const int64_t r = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
@@ -766,8 +833,11 @@ slice_kernel(const double *__restrict__ X, int M, int K, int Kpad, int Mpad,
         m = v > m ? v : m;
     }
     const int e = row_exponent(m);
-    if (lane == 0)
+    if (lane == 0) {
         ex[r] = e;
+        if (scale)
+            scale[r] = (m >> 52) == 0 ? 0.0f : pow2f(kMag && e > 100 ? kNanExponent : e);
+    }
     for (int k = lane; k < Kpad; k += 32) {
         const double x = r < M && k < K && e < kNanExponent ? X[r * K + k] : 0.0;
         int q[S];
@@ -776,6 +846,12 @@ slice_kernel(const double *__restrict__ X, int M, int K, int Kpad, int Mpad,
         for (int s = 0; s < S; s++)
             slices[((int64_t)s * Mpad + r) * Kpad + k] =
                 __float2bfloat16_rn(__int2float_rn(q[s]) * exp2f((float)(-8 - 9 * s)));
+        if constexpr (kMag) {
+            const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+            const int E = (int)(b >> 52 & 0x7ff) - 1023 - e + 127;
+            slices[((int64_t)S * Mpad + r) * Kpad + k] = __ushort_as_bfloat16(
+                (unsigned short)(E > 0 ? (unsigned)E << 7 | ((unsigned)(b >> 45) & 0x7fu) : 0u));
+        }
     }
 }
 
@@ -795,10 +871,13 @@ static int64_t pad_k(const PairTcMode &m, int64_t K)
     return round_up(std::max<int64_t>(K, 1), K <= one_group_k(m) ? kBK : kGroupBlocks * kBK);
 }
 
+static int planes(const PairTcMode &m) { return m.slices + (m.fp64 ? 1 : 0); }
+static int mark_words(int64_t n2) { return (int)((n2 + 31) / 32); }
+
 // r1 rows per sub-tile of a contraction in groups: its values so far take at most 2 GiB.
 static int64_t group_rows(const PairTcMode &m, int64_t n2, int64_t n1b)
 {
-    const int64_t per = n2 * m.rows * (m.fp64 ? 12 : 8);
+    const int64_t per = n2 * m.rows * (m.fp64 ? 16 : 8);
     return std::min(n1b, std::max<int64_t>(8, (((int64_t)2 << 30) / per) / 8 * 8));
 }
 
@@ -819,10 +898,10 @@ PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, bool f
     return m;
 }
 
-// Device bytes: per r2 point and r1 row, of K values in FP64 and in slices.
+// Device bytes: per r2 point and r1 row, of K values in FP64 and in slices (and magnitudes).
 static size_t operand_bytes(int64_t rows, int64_t K, int slices)
 {
-    return (size_t)rows * (8 * K + 2 * slices * round_up(K, kGroupBlocks * kBK) + 4);
+    return (size_t)rows * (8 * K + 2 * (slices + 1) * round_up(K, kGroupBlocks * kBK) + 4);
 }
 
 size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices)
@@ -855,23 +934,24 @@ static int alloc_operand(Workspace &W, int slot, int S, int64_t M, int row_mult,
 }
 
 template <int S>
-static int slice_rows(cudaStream_t st, const double *X, const SliceOperand &op)
+static int slice_rows(cudaStream_t st, const double *X, const SliceOperand &op, float *scale)
 {
-    slice_kernel<S><<<ceil_div(op.Mpad, 8), 256, 0, st>>>(X, op.M, (int)op.K, (int)op.Kpad, op.Mpad,
-                                                          (__nv_bfloat16 *)op.sl, op.ex);
+    slice_kernel<S, S == 7><<<ceil_div(op.Mpad, 8), 256, 0, st>>>(
+        X, op.M, (int)op.K, (int)op.Kpad, op.Mpad, (__nv_bfloat16 *)op.sl, op.ex, scale);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
-static int slice_rows(cudaStream_t st, int slices, const double *X, const SliceOperand &op)
+static int slice_rows(cudaStream_t st, int slices, const double *X, const SliceOperand &op,
+                      float *scale)
 {
-    return slices == 5   ? slice_rows<5>(st, X, op)
-           : slices == 6 ? slice_rows<6>(st, X, op)
-                         : slice_rows<7>(st, X, op);
+    return slices == 5   ? slice_rows<5>(st, X, op, scale)
+           : slices == 6 ? slice_rows<6>(st, X, op, scale)
+                         : slice_rows<7>(st, X, op, scale);  // (FP64)
 }
 
-enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale, kSlotPart };
+enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale, kSlotPart, kSlotMarks };
 
 int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &mode, int n2,
                     int n_nuc, const double *f2, int64_t n1t, int *err, PairTcPlan &plan)
@@ -891,14 +971,18 @@ int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &
     CUTC_TRY(W.get(slot0 + kSlotBscale, (size_t)round_up(rows, kPairBN) * 4, &p));
     plan.bscale = (float *)p;
     if (K > one_group_k(mode)) {
-        CUTC_TRY(W.get(slot0 + kSlotPart, (size_t)n2 * rows * (mode.fp64 ? 12 : 8), &p));
+        CUTC_TRY(W.get(slot0 + kSlotPart, (size_t)n2 * rows * (mode.fp64 ? 16 : 8), &p));
         plan.part = p;
     }
-    CUTC_TRY(alloc_operand(W, slot0 + kSlotAF, mode.slices, n2, kBM, K, Kpad, plan.AF));
-    CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, mode.slices, rows, kPairBN, K, Kpad, plan.BC));
+    if (mode.fp64) {
+        CUTC_TRY(W.get(slot0 + kSlotMarks, 64 + (size_t)plan.tile_rows * mark_words(n2) * 4, &p));
+        plan.marked = (int *)p;
+    }
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotAF, planes(mode), n2, kBM, K, Kpad, plan.AF));
+    CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, planes(mode), rows, kPairBN, K, Kpad, plan.BC));
     CUTC_TRY(launch_pair_tc_f(st, mode.powers(), n2, n_nuc, f2, plan.Fd));
     note_launches(1);
-    return slice_rows(st, mode.slices, plan.Fd, plan.AF);
+    return slice_rows(st, mode.slices, plan.Fd, plan.AF, nullptr);
 }
 
 // 2-D map over slices [rows_total][Kpad] BF16, box = kBK x box_rows, 64B swizzle.
@@ -972,16 +1056,11 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     SliceOperand B = plan.BC;
     B.M = m.rows * P.n1b;
     B.Mpad = (int)round_up(B.M, kPairBN);
-    CUTC_TRY(slice_rows(st, m.slices, plan.Cd, B));
-    if (!m.fp64) {
-        exp_scale_kernel<<<ceil_div(B.Mpad, 256), 256, 0, st>>>(B.ex, B.Mpad, plan.bscale);
-        CUTC_CUDA_TRY(cudaGetLastError());
-        note_launches(1);
-    }
+    CUTC_TRY(slice_rows(st, m.slices, plan.Cd, B, plan.bscale));
     CUtensorMap ta, tb;
-    CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)m.slices * plan.AF.Mpad, plan.AF.Kpad, kBM));
+    CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)planes(m) * plan.AF.Mpad, plan.AF.Kpad, kBM));
     const int bn = m.fp64 ? m.rows : kPairBN;
-    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)m.slices * B.Mpad, B.Kpad, bn));
+    CUTC_TRY(make_tmap(&tb, B.sl, (int64_t)planes(m) * B.Mpad, B.Kpad, bn));
     Q.tiles_m = plan.AF.Mpad / kBM;
     Q.tiles_n = B.Mpad / bn;
     Q.chunk = 1;
@@ -996,7 +1075,15 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     const bool part = plan.AF.K > one_group_k(m);
     Q.part = (float2 *)plan.part;
     Q.partI = (long long *)plan.part;
-    Q.partL = (float *)(Q.partI + (m.fp64 && part ? (int64_t)P.n2 * m.rows * P.n1b : 0));
+    const int64_t part_n = m.fp64 && part ? (int64_t)P.n2 * m.rows * P.n1b : 0;
+    Q.partL = (float *)(Q.partI + part_n);
+    Q.partA = Q.partL + part_n;
+    Q.check = 256.0f / std::sqrt((float)plan.AF.K);
+    Q.marked = plan.marked;
+    Q.marks = (unsigned *)(plan.marked + 16);
+    Q.mark_words = mark_words(P.n2);
+    if (m.fp64)
+        CUTC_CUDA_TRY(cudaMemsetAsync(plan.marked, 0, sizeof(int), st));
     for (int kb = 0; kb < KB; kb += part ? kGroupBlocks : KB) {
         Q.kb0 = kb;
         Q.first = kb == 0;
@@ -1048,6 +1135,12 @@ int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &A, const
         P.n1b = (int)std::min<int64_t>(plan.tile_rows, A.n1b - i);
         Q.G64 = A.G + i * A.ldg;
         CUTC_TRY(run_tile(st, plan, Q, rn, a_en, n_sm));
+        PairArgs R = A;
+        R.i0 = P.i0;
+        R.n1b = P.n1b;
+        R.G = Q.G64;
+        CUTC_TRY(launch_pair_f64_marked(st, R, rn, a_en, plan.marked,
+                                        (const unsigned *)(plan.marked + 16), mark_words(A.n2), n_sm));
     }
     return CUTC_OK;
 }

@@ -42,6 +42,7 @@ struct PairTcPlan {
     float *bscale = nullptr;    // 2^(row exponent) of the coefficient rows
     void *part = nullptr;       // the V values between the groups of a long contraction
     int64_t tile_rows = 0;      // r1 rows taken at once
+    int *marked = nullptr;      // FP64: set when pairs are left out; their bits 16 ints on
     int *err = nullptr;         // device flag set by a bounded wait that gave up
 };
 
@@ -52,7 +53,8 @@ int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &
 // The pair planes of one r1 tile.  Double-float: P.G as for launch_pair_df.
 int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, const double *rn,
                     double a_en, int n_sm);
-// FP64: P.G as for launch_pair_f64 (P.t1 is not used).
+// FP64: P.G as for launch_pair_f64 (P.t1 is not used), pairs that the check leaves out term by
+// term.
 int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &P, const double *rn,
                      double a_en, int n_sm);
 // Device bytes: fixed (F) and per r1 row of a tile, for the largest operands of the form.
