@@ -740,8 +740,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     // which pair-term buffers the build holds besides: the remembered plan is taken
     // only when they are the same
     const bool pair64 = R.precision == CUTC_PLAIN_FP64 || R.pair_fp64;
-    const PairTcMode pmode = pair_tc_mode(coef.data(), exps.data(), nt, pair64, R.n_slices);
-    uint64_t path = 1 + (R.pair_fp64 ? 2 : 0) + 64 * (uint64_t)pmode.rows;
+    const PairTcMode pmode = pair_tc_mode(coef.data(), exps.data(), nt, nN, pair64, R.n_slices);
+    uint64_t path = 1 + (R.pair_fp64 ? 2 : 0) + 64 * (uint64_t)pmode.rows + 4096 * (uint64_t)pmode.checked;
     if (!pair64)
         path += 8 * (uint64_t)pair_df_max_exp(exps.data(), nt);
     const bool default_budget = budget == 0;
@@ -1237,7 +1237,7 @@ int run_pair_only(Engine *E, cudaStream_t st, int i0, int n1b, int n1, int j0, i
     P.r1 = r1; P.r2 = r2w; P.t1 = d_t1; P.f2 = d_f2;
     P.coef = d_coef; P.exps = d_exps; P.term_off = d_off; P.a_ee = a_ee;
     P.G = G; P.ldg = ldg; P.plane = plane;
-    const PairTcMode mode = pair_tc_mode(coef.data(), exps.data(), (int)exps.size(), true, 0);
+    const PairTcMode mode = pair_tc_mode(coef.data(), exps.data(), (int)exps.size(), nN, true, 0);
     if (mode.rows) {
         ContractScratch flags;  // (its wait flag alone)
         CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, 0, flags));

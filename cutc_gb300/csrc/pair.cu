@@ -268,6 +268,7 @@ __device__ __forceinline__ double scaled_distance(const double (&d)[3], double a
 // them out over its threads, which form them as pair_f64_kernel does.
 constexpr int kMarkWords = 256;
 
+template <bool DF>
 __global__ void __launch_bounds__(256)
 pair_f64_marked_kernel(PairArgs P, const double *__restrict__ rn, double a_en,
                        const int *__restrict__ marked, const unsigned *__restrict__ marks, int words)
@@ -318,23 +319,33 @@ pair_f64_marked_kernel(PairArgs P, const double *__restrict__ rn, double a_en,
             }
             for (int k = 0; k < 3; k++)
                 u[k] += dudg * gg[k];
-            double *out = P.G + (int64_t)i * P.ldg + j;
-            out[0] = u[0];
-            out[P.plane] = u[1];
-            out[2 * P.plane] = u[2];
-            out[3 * P.plane] = -0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+            auto put = [&](int c, double v) {
+                const int64_t o = (int64_t)i * P.ldg + j + c * P.plane;
+                if constexpr (DF) {
+                    const float hi = (float)v;
+                    reinterpret_cast<float2 *>(P.G)[o] = make_float2(hi, (float)(v - (double)hi));
+                } else {
+                    P.G[o] = v;
+                }
+            };
+            for (int k = 0; k < 3; k++)
+                put(k, u[k]);
+            put(3, -0.5 * (u[0] * u[0] + u[1] * u[1] + u[2] * u[2]));
         }
     }
 }
 
 int launch_pair_f64_marked(cudaStream_t st, const PairArgs &P, const double *rn, double a_en,
-                           const int *marked, const unsigned *marks, int words, int n_sm)
+                           bool df, const int *marked, const unsigned *marks, int words, int n_sm)
 {
     if (P.n1b <= 0 || P.n2 <= 0)
         return CUTC_OK;
     const int64_t blocks = ((int64_t)P.n1b * words + kMarkWords - 1) / kMarkWords;
-    pair_f64_marked_kernel<<<(unsigned)std::min<int64_t>(blocks, 4 * n_sm), 256, 0, st>>>(
-        P, rn, a_en, marked, marks, words);
+    const unsigned grid = (unsigned)std::min<int64_t>(blocks, 4 * n_sm);
+    if (df)
+        pair_f64_marked_kernel<true><<<grid, 256, 0, st>>>(P, rn, a_en, marked, marks, words);
+    else
+        pair_f64_marked_kernel<false><<<grid, 256, 0, st>>>(P, rn, a_en, marked, marks, words);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;

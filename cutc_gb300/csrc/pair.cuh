@@ -82,8 +82,9 @@ int launch_r2_terms(cudaStream_t st, int n2, int nN, const double *r2, const dou
                     double a, double *f2);
 int launch_pair_f64(cudaStream_t st, const PairArgs &P);
 // The pairs (i, j) of the tile whose bit j % 32 of marks[i words + j / 32] is set, term by term
-// (P.t1 is not used); returns at once on the device while *marked is zero.
+// (P.t1 is not used); returns at once on the device while *marked is zero.  df: G takes (hi, lo)
+// float pairs.
 int launch_pair_f64_marked(cudaStream_t st, const PairArgs &P, const double *rn, double a_en,
-                           const int *marked, const unsigned *marks, int words, int n_sm);
+                           bool df, const int *marked, const unsigned *marks, int words, int n_sm);
 
 }  // namespace cutc

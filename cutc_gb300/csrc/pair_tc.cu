@@ -33,12 +33,13 @@
 // nucleus.
 //
 // F and the coefficients enter with an error relative to their rows' maxima, where a term by
-// term sum's is relative to the terms.  So FP64 results are checked: one more product, of the
+// term sum's is relative to the terms.  So FP64 results, and those in double-float of general
+// exponents and of more than 20 nuclei (from 6 slices), are checked: one more product, of the
 // operands' magnitudes to 8 bits (plane S, accumulators of its own), gives
 // v_c = sum_k |C[(r1, c)][k]| F[r2][k], and with it the sums of the terms' magnitudes and of the
 // errors, both as polynomials in g12.  The error of V_c is about sqrt(K) 2^-63 of the row
-// scales (rms, from the seven slices and the products left out); pairs for which four times
-// that is above 2^-53 of the terms (r2 near a nucleus whose terms all vanish there, small
+// scales with seven slices (rms, from the slices and the products left out), sqrt(K) 2^-54 with
+// six; pairs for which four times that is above 2^-53 (2^-45) of the terms (r2 near a nucleus whose terms all vanish there, small
 // values of few nuclei: fewer than one in 10^4 of 8 nuclei with 13 terms) are marked in a bit
 // mask and formed again term by term behind the kernel (pair.cu).
 //
@@ -81,8 +82,8 @@ struct PairTcParams {
     const float2 *r1d;            // double-float: the tile's r1 points, [3 i + c]
     PairDfArgs P;                 // geometry and outputs
     double *G64;                  // FP64: in place of P.G
-    float check;                  // FP64: 2^8 / sqrt(K)
-    unsigned *marks;              // FP64: bit j % 32 of marks[i mark_words + j / 32]: (i, j) is
+    float check;                  // checked: 2^8 / sqrt(K), double-float 2^7 / sqrt(K)
+    unsigned *marks;              // checked: bit j % 32 of marks[i mark_words + j / 32]: (i, j) is
     int mark_words;               // left out, and *marked is set
     int *marked;
     int *err;
@@ -106,7 +107,8 @@ __device__ __forceinline__ float pow2f(int e)
 }
 
 // R: coefficient rows per r1 point (16 or 32).
-template <int S, int KB, int R, bool F64>
+// CHK: with the magnitudes' product and the check (always with F64).
+template <int S, int KB, int R, bool F64, bool CHK>
 struct PairTcCfg {
     // Double-float: one accumulator set, and a warp per lane quarter and point of a tile
     // (16 warps with 16 rows, four per SM sub-partition, to hide the latency of their
@@ -121,7 +123,7 @@ struct PairTcCfg {
     static constexpr int kBufWarps = kEpiWarps / kBufs;  // epilogue warps of a buffer
     static constexpr int kCtlWarp = kEpiWarps;       // TMA loads and MMAs, lane 0
     static constexpr int kThreads = (kEpiWarps + 1) * 32;
-    static constexpr int kPlanes = S + (F64 ? 1 : 0);  // slices, and the magnitudes
+    static constexpr int kPlanes = S + (CHK ? 1 : 0);  // slices, and the magnitudes
     static constexpr int kASlice = kBM * kBK * 2;
     static constexpr int kBSlice = kBN * kBK * 2;
     static constexpr int kABytes = KB * kPlanes * kASlice;
@@ -195,10 +197,43 @@ __device__ __forceinline__ void scale_df16(const uint64_t (&H)[8], const uint64_
     }
 }
 
-// One pair in double-float from its V values.
+// Whether the error of a pair's values may be above that of a term by term sum (the check at
+// the top of this file): w[c] = 2^eb_c (check v_c - 1), the margin of V_c.
 template <int R>
-__device__ __forceinline__ void pair_df(const PairTcParams &Q, int i, int j, const df::D *V,
-                                        float2 x2, float2 y2, float2 z2, float sa, df::D a)
+__device__ __forceinline__ bool pair_unsure(const float *w, float g, float gx, float gy, float gz)
+{
+    float ux, uy, uz, dudg;
+    if constexpr (R == 16) {
+        const float g2 = g * g;
+        auto poly = [&](int c) { return fmaf(fmaf(fmaf(w[c + 3], g, w[c + 2]), g, w[c + 1]), g2, w[c]); };
+        ux = poly(0);
+        uy = poly(4);
+        uz = poly(8);
+        dudg = fmaf(fmaf(w[14], g, w[13]), g, w[12]) * g;
+    } else {
+        auto poly = [&](int c, int n) {
+            float s = w[c + n - 1];
+#pragma unroll
+            for (int o = n - 2; o >= 0; o--)
+                s = fmaf(s, g, w[c + o]);
+            return s;
+        };
+        ux = poly(0, 7);
+        uy = poly(7, 7);
+        uz = poly(14, 7);
+        dudg = poly(21, 6);
+    }
+    // (a NaN is unsure)
+    return !(fmaf(dudg, fabsf(gx), ux) >= 0.f && fmaf(dudg, fabsf(gy), uy) >= 0.f &&
+             fmaf(dudg, fabsf(gz), uz) >= 0.f);
+}
+
+// One pair in double-float from its V values; with CHK true, and nothing is written, when they
+// are unsure.
+template <int R, bool CHK>
+__device__ __forceinline__ bool pair_df(const PairTcParams &Q, int i, int j, const df::D *V,
+                                        const float *w, float2 x2, float2 y2, float2 z2, float sa,
+                                        df::D a)
 {
     const PairDfArgs &P = Q.P;
     const float2 *r1p = Q.r1d + 3 * (int64_t)i;
@@ -233,6 +268,9 @@ __device__ __forceinline__ void pair_df(const PairTcParams &Q, int i, int j, con
         gy = df::mul(sg, dy);
         gz = df::mul(sg, dz);
     }
+    if constexpr (CHK)
+        if (pair_unsure<R>(w, g.hi, gx.hi, gy.hi, gz.hi))
+            return true;
     df::D ux, uy, uz, dudg;
     if constexpr (R == 16) {
         const df::D g2 = df::sqr(g);
@@ -267,6 +305,7 @@ __device__ __forceinline__ void pair_df(const PairTcParams &Q, int i, int j, con
     o[P.plane] = make_float2(uy.hi, uy.lo);
     o[2 * P.plane] = make_float2(uz.hi, uz.lo);
     o[3 * P.plane] = make_float2(lv.hi, lv.lo);
+    return false;
 }
 
 // I 2^k for |I| < 2^53, exactly, in integer arithmetic (0 below the normal range, an
@@ -386,37 +425,6 @@ __device__ __forceinline__ double minus_half(double x)
     return -0.5 * x;
 }
 
-// Whether the error of a pair's values may be above that of a term by term sum (the check at
-// the top of this file): w[c] = 2^eb_c (check v_c - 1), the margin of V_c.
-template <int R>
-__device__ __forceinline__ bool pair_unsure(const float *w, float g, float gx, float gy, float gz)
-{
-    float ux, uy, uz, dudg;
-    if constexpr (R == 16) {
-        const float g2 = g * g;
-        auto poly = [&](int c) { return fmaf(fmaf(fmaf(w[c + 3], g, w[c + 2]), g, w[c + 1]), g2, w[c]); };
-        ux = poly(0);
-        uy = poly(4);
-        uz = poly(8);
-        dudg = fmaf(fmaf(w[14], g, w[13]), g, w[12]) * g;
-    } else {
-        auto poly = [&](int c, int n) {
-            float s = w[c + n - 1];
-#pragma unroll
-            for (int o = n - 2; o >= 0; o--)
-                s = fmaf(s, g, w[c + o]);
-            return s;
-        };
-        ux = poly(0, 7);
-        uy = poly(7, 7);
-        uz = poly(14, 7);
-        dudg = poly(21, 6);
-    }
-    // (a NaN is unsure)
-    return !(fmaf(dudg, fabsf(gx), ux) >= 0.f && fmaf(dudg, fabsf(gy), uy) >= 0.f &&
-             fmaf(dudg, fabsf(gz), uz) >= 0.f);
-}
-
 // One pair in FP64 from its V values (hi + lo); true, and nothing is written, when they are
 // unsure.  The reciprocal square root and the
 // reciprocal are FP32 seeds with one step each of third order in FP64 (the seeds' relative
@@ -519,12 +527,12 @@ __device__ __forceinline__ bool pair_f64(const PairTcParams &Q, int i, int j, co
 }
 
 // PART: one group of K blocks of a longer contraction (Q.kb0, Q.first, Q.last).
-template <int S, int KB, int R, bool F64, bool PART>
-__global__ void __launch_bounds__(PairTcCfg<S, KB, R, F64>::kThreads, 1)
+template <int S, int KB, int R, bool F64, bool CHK, bool PART>
+__global__ void __launch_bounds__(PairTcCfg<S, KB, R, F64, CHK>::kThreads, 1)
 pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const __grid_constant__ PairTcParams Q)
 {
-    using Cfg = PairTcCfg<S, KB, R, F64>;
+    using Cfg = PairTcCfg<S, KB, R, F64, CHK>;
     constexpr int D = S - 1, BN = Cfg::kBN, NP = Cfg::kPlanes;
     constexpr int kCtlWarp = Cfg::kCtlWarp;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -646,7 +654,7 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                             }
                             first = false;
                         }
-                        if constexpr (F64)  // the magnitudes' sums
+                        if constexpr (CHK)  // the magnitudes' sums
                             tc::mma_bf16(
                                 acc + (uint32_t)(BN * S),
                                 tc::smem_desc_sw64(sa0 + (kb * NP + S) * Cfg::kASlice + k16 * 32),
@@ -697,6 +705,14 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             z2 = P.r2d[2 * (int64_t)P.n2 + jc];
         }
         const float sa = F64 ? 0.f : pow2f(ea);
+        auto mark = [&](int i, bool unsure) {
+            const unsigned marks = __ballot_sync(0xffffffffu, unsure);
+            if (lane == 0 && i < P.n1b && j < P.n2) {
+                Q.marks[(int64_t)i * Q.mark_words + j / 32] = marks;
+                if (marks)
+                    *Q.marked = 1;
+            }
+        };
         const df::D a = df::make(P.a_ee_hi, P.a_ee_lo);
         for (int q = buf; q < ntiles; q += NB) {
             if (!tc::mbar_wait(tc::smem_u32(&tfull[buf]), (q / NB) & 1, s_abort)) {
@@ -746,43 +762,64 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 __syncwarp();
                 if (lane == 0)
                     tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-                if (!PART || Q.last) {
-                    const bool unsure = out && (pair_f64<R>(Q, i0, j, V, lo, w, dx2, dy2, dz2) ||
-                                                ea >= kNanExponent);
-                    const unsigned marks = __ballot_sync(0xffffffffu, unsure);
-                    if (lane == 0 && i0 < P.n1b && j < P.n2) {
-                        Q.marks[(int64_t)i0 * Q.mark_words + j / 32] = marks;
-                        if (marks)
-                            *Q.marked = 1;
-                    }
-                }
+                if (!PART || Q.last)
+                    mark(i0, out && (pair_f64<R>(Q, i0, j, V, lo, w, dx2, dy2, dz2) ||
+                                     ea >= kNanExponent));
             } else {
                 uint64_t H[R / 16][8], L[R / 16][8], L2[R / 16][8];
+                float w[R];
 #pragma unroll
-                for (int h = 0; h < R / 16; h++)
+                for (int h = 0; h < R / 16; h++) {
                     read_df16<S>(cb + 16u * h, H[h], L[h], L2[h]);
+                    if constexpr (CHK) {
+                        float v[16];
+                        tc::tmem_ld16(cb + (uint32_t)(BN * S) + 16u * h, v);
+#pragma unroll
+                        for (int k = 0; k < 16; k++)
+                            w[16 * h + k] = v[k];
+                    }
+                }
                 tc::fence_before_sync();
                 __syncwarp();
                 if (lane == 0)
                     tc::mbar_arrive(tc::smem_u32(&tempty[buf]));
-                if (jok && i0 < P.n1b) {
+                const bool out = jok && i0 < P.n1b;
+                bool unsure = false;
+                if (out) {
+                    const float *bs = Q.bscale + (int64_t)i0 * R;
                     df::D V[R];
 #pragma unroll
                     for (int h = 0; h < R / 16; h++)
-                        scale_df16(H[h], L[h], L2[h], Q.bscale + (int64_t)i0 * R + 16 * h, V + 16 * h);
+                        scale_df16(H[h], L[h], L2[h], bs + 16 * h, V + 16 * h);
                     if constexpr (PART) {
 #pragma unroll
                         for (int c = 0; c < R; c++) {
-                            float2 *o = Q.part + ((int64_t)i0 * R + c) * P.n2 + j;
+                            const int64_t at = ((int64_t)i0 * R + c) * P.n2 + j;
+                            float2 *o = Q.part + at;
                             if (!Q.first)
                                 V[c] = df::add(V[c], df::make(o->x, o->y));
                             if (!Q.last)
                                 *o = make_float2(V[c].hi, V[c].lo);
+                            if constexpr (CHK) {
+                                if (!Q.first)
+                                    w[c] += Q.partA[at];
+                                if (!Q.last)
+                                    Q.partA[at] = w[c];
+                            }
                         }
                     }
-                    if (!PART || Q.last)
-                        pair_df<R>(Q, i0, j, V, x2, y2, z2, sa, a);
+                    if (!PART || Q.last) {
+                        if constexpr (CHK)
+#pragma unroll
+                            for (int c = 0; c < R; c++)
+                                w[c] = bs[c] * fmaf(Q.check, w[c], -1.0f);
+                        unsure = pair_df<R, CHK>(Q, i0, j, V, w, x2, y2, z2, sa, a) ||
+                                 (CHK && ea >= kNanExponent);
+                    }
                 }
+                if constexpr (CHK)
+                    if (!PART || Q.last)
+                        mark(i0, unsure);
             }
         }
     }
@@ -861,40 +898,47 @@ slice_kernel(const double *__restrict__ X, int M, int K, int Kpad, int Mpad,
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
+// K of unchecked double-float contractions: 20 nuclei of 4 powers.
+constexpr int kPlainDfK = 80;
+
 // The K up to which the contraction is one group: the leading diagonals are exact (and the
 // operands fit shared memory).  A longer one runs in groups of kGroupBlocks K blocks whose
 // values are added between launches.
 constexpr int kGroupBlocks = 2;
-static int one_group_k(const PairTcMode &m) { return m.fp64 ? 64 : m.rows == 16 ? 80 : 85; }
+static int one_group_k(const PairTcMode &m) { return m.checked ? 64 : kPlainDfK; }
 static int64_t pad_k(const PairTcMode &m, int64_t K)
 {
     return round_up(std::max<int64_t>(K, 1), K <= one_group_k(m) ? kBK : kGroupBlocks * kBK);
 }
 
-static int planes(const PairTcMode &m) { return m.slices + (m.fp64 ? 1 : 0); }
+static int planes(const PairTcMode &m) { return m.slices + (m.checked ? 1 : 0); }
+// of a value between the groups: FP64 or double-float, and the magnitudes' sum
+static int part_bytes(const PairTcMode &m) { return m.fp64 ? 16 : 12; }
 static int mark_words(int64_t n2) { return (int)((n2 + 31) / 32); }
 
 // r1 rows per sub-tile of a contraction in groups: its values so far take at most 2 GiB.
 static int64_t group_rows(const PairTcMode &m, int64_t n2, int64_t n1b)
 {
-    const int64_t per = n2 * m.rows * (m.fp64 ? 16 : 8);
+    const int64_t per = n2 * m.rows * part_bytes(m);
     return std::min(n1b, std::max<int64_t>(8, (((int64_t)2 << 30) / per) / 8 * 8));
 }
 
-PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, bool fp64, int slices)
+PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, int n_nuc, bool fp64,
+                        int slices)
 {
     PairTcMode m;
     m.fp64 = fp64;
-    // 5 slices (representation error 2^-45, under the error of a 5-slice build's
-    // contractions), 6 for builds of 6 and 7 slices (2^-54, below the double-float
-    // epilogue), 7 for FP64 (2^-63)
-    m.slices = fp64 ? 7 : slices >= 6 ? 6 : 5;
     if (!fp64 && (getenv("CUTC_PAIR_DF") || getenv("CUTC_PAIR_DENSE")))
         return m;
     for (int k = 0; k < 3 * n_terms; k++)
         if (!std::isfinite(coef[k]))
             return m;
     m.rows = pair_df_sparse(exps, n_terms) ? 16 : 32;
+    m.checked = fp64 || m.rows == 32 || m.powers() * n_nuc > kPlainDfK;
+    // 5 slices (representation error 2^-45, under the error of a 5-slice build's operands), 6
+    // for builds of 6 and 7 slices and where the check is (2^-54, below the double-float
+    // epilogue), 7 for FP64 (2^-63)
+    m.slices = fp64 ? 7 : slices >= 6 || m.checked ? 6 : 5;
     return m;
 }
 
@@ -933,22 +977,23 @@ static int alloc_operand(Workspace &W, int slot, int S, int64_t M, int row_mult,
     return CUTC_OK;
 }
 
-template <int S>
+template <int S, bool kMag>
 static int slice_rows(cudaStream_t st, const double *X, const SliceOperand &op, float *scale)
 {
-    slice_kernel<S, S == 7><<<ceil_div(op.Mpad, 8), 256, 0, st>>>(
+    slice_kernel<S, kMag><<<ceil_div(op.Mpad, 8), 256, 0, st>>>(
         X, op.M, (int)op.K, (int)op.Kpad, op.Mpad, (__nv_bfloat16 *)op.sl, op.ex, scale);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
-static int slice_rows(cudaStream_t st, int slices, const double *X, const SliceOperand &op,
-                      float *scale)
+static int slice_rows(cudaStream_t st, const PairTcMode &m, const double *X,
+                      const SliceOperand &op, float *scale)
 {
-    return slices == 5   ? slice_rows<5>(st, X, op, scale)
-           : slices == 6 ? slice_rows<6>(st, X, op, scale)
-                         : slice_rows<7>(st, X, op, scale);  // (FP64)
+    return m.slices == 7 ? slice_rows<7, true>(st, X, op, scale)
+           : m.checked   ? slice_rows<6, true>(st, X, op, scale)
+           : m.slices == 6 ? slice_rows<6, false>(st, X, op, scale)
+                           : slice_rows<5, false>(st, X, op, scale);
 }
 
 enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale, kSlotPart, kSlotMarks };
@@ -971,10 +1016,10 @@ int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &
     CUTC_TRY(W.get(slot0 + kSlotBscale, (size_t)round_up(rows, kPairBN) * 4, &p));
     plan.bscale = (float *)p;
     if (K > one_group_k(mode)) {
-        CUTC_TRY(W.get(slot0 + kSlotPart, (size_t)n2 * rows * (mode.fp64 ? 16 : 8), &p));
+        CUTC_TRY(W.get(slot0 + kSlotPart, (size_t)n2 * rows * part_bytes(mode), &p));
         plan.part = p;
     }
-    if (mode.fp64) {
+    if (mode.checked) {
         CUTC_TRY(W.get(slot0 + kSlotMarks, 64 + (size_t)plan.tile_rows * mark_words(n2) * 4, &p));
         plan.marked = (int *)p;
     }
@@ -982,7 +1027,7 @@ int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &
     CUTC_TRY(alloc_operand(W, slot0 + kSlotBC, planes(mode), rows, kPairBN, K, Kpad, plan.BC));
     CUTC_TRY(launch_pair_tc_f(st, mode.powers(), n2, n_nuc, f2, plan.Fd));
     note_launches(1);
-    return slice_rows(st, mode.slices, plan.Fd, plan.AF, nullptr);
+    return slice_rows(st, mode, plan.Fd, plan.AF, nullptr);
 }
 
 // 2-D map over slices [rows_total][Kpad] BF16, box = kBK x box_rows, 64B swizzle.
@@ -995,15 +1040,15 @@ static int make_tmap(CUtensorMap *map, const void *base, int64_t rows_total, int
     return encode_bf16_map(map, base, 2, dims, strides, box, 64);
 }
 
-template <int S, int KB, int R, bool F64, bool PART>
+template <int S, int KB, int R, bool F64, bool CHK, bool PART>
 static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
                          PairTcParams Q, int n_sm)
 {
-    using Cfg = PairTcCfg<S, KB, R, F64>;
+    using Cfg = PairTcCfg<S, KB, R, F64, CHK>;
     static std::atomic<unsigned long long> attr_done{0};
     const unsigned long long bit = current_device_bit();
     if (!(attr_done.load() & bit)) {
-        CUTC_CUDA_TRY(cudaFuncSetAttribute(pair_tc_kernel<S, KB, R, F64, PART>,
+        CUTC_CUDA_TRY(cudaFuncSetAttribute(pair_tc_kernel<S, KB, R, F64, CHK, PART>,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem));
         attr_done.fetch_or(bit);
     }
@@ -1020,26 +1065,28 @@ static int launch_kernel(cudaStream_t st, const CUtensorMap &ta, const CUtensorM
         cutc_set_error(CUTC_ERR_INVALID, "pair grid of %lld CTAs", (long long)grid);
         return CUTC_ERR_INVALID;
     }
-    pair_tc_kernel<S, KB, R, F64, PART><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, Q);
+    pair_tc_kernel<S, KB, R, F64, CHK, PART><<<(unsigned)grid, Cfg::kThreads, Cfg::kSmem, st>>>(ta, tb, Q);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
     return CUTC_OK;
 }
 
-template <int S, int R, bool F64>
+template <int S, int R, bool F64, bool CHK>
 static int launch_kb(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
                      const PairTcParams &Q, int n_sm, int KB, bool part)
 {
-    if (part)
-        return launch_kernel<S, kGroupBlocks, R, F64, true>(st, ta, tb, Q, n_sm);
-    switch (KB) {
-    case 1: return launch_kernel<S, 1, R, F64, false>(st, ta, tb, Q, n_sm);
-    case 2: return launch_kernel<S, 2, R, F64, false>(st, ta, tb, Q, n_sm);
-    case 3:
-        if constexpr (!F64)
-            return launch_kernel<S, 3, R, F64, false>(st, ta, tb, Q, n_sm);
-        break;
-    }
+    if constexpr (CHK)
+        if (part)
+            return launch_kernel<S, kGroupBlocks, R, F64, CHK, true>(st, ta, tb, Q, n_sm);
+    if constexpr (!CHK || F64 || R == 32)  // (others have more than 80 K)
+        switch (KB) {
+        case 1: return launch_kernel<S, 1, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
+        case 2: return launch_kernel<S, 2, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
+        case 3:
+            if constexpr (!CHK)
+                return launch_kernel<S, 3, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
+            break;
+        }
     cutc_set_error(CUTC_ERR_INVALID, "pair contraction of %d K blocks", KB);
     return CUTC_ERR_INVALID;
 }
@@ -1056,7 +1103,7 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     SliceOperand B = plan.BC;
     B.M = m.rows * P.n1b;
     B.Mpad = (int)round_up(B.M, kPairBN);
-    CUTC_TRY(slice_rows(st, m.slices, plan.Cd, B, plan.bscale));
+    CUTC_TRY(slice_rows(st, m, plan.Cd, B, plan.bscale));
     CUtensorMap ta, tb;
     CUTC_TRY(make_tmap(&ta, plan.AF.sl, (int64_t)planes(m) * plan.AF.Mpad, plan.AF.Kpad, kBM));
     const int bn = m.fp64 ? m.rows : kPairBN;
@@ -1075,31 +1122,32 @@ static int run_tile(cudaStream_t st, PairTcPlan &plan, PairTcParams Q, const dou
     const bool part = plan.AF.K > one_group_k(m);
     Q.part = (float2 *)plan.part;
     Q.partI = (long long *)plan.part;
-    const int64_t part_n = m.fp64 && part ? (int64_t)P.n2 * m.rows * P.n1b : 0;
+    // the integers or double-float values, then (FP64) their rests, then the magnitudes' sums
+    const int64_t part_n = part ? (int64_t)P.n2 * m.rows * P.n1b : 0;
     Q.partL = (float *)(Q.partI + part_n);
-    Q.partA = Q.partL + part_n;
-    Q.check = 256.0f / std::sqrt((float)plan.AF.K);
+    Q.partA = Q.partL + (m.fp64 ? part_n : 0);
+    Q.check = (m.fp64 ? 256.0f : 128.0f) / std::sqrt((float)plan.AF.K);
     Q.marked = plan.marked;
     Q.marks = (unsigned *)(plan.marked + 16);
     Q.mark_words = mark_words(P.n2);
-    if (m.fp64)
+    if (m.checked)
         CUTC_CUDA_TRY(cudaMemsetAsync(plan.marked, 0, sizeof(int), st));
     for (int kb = 0; kb < KB; kb += part ? kGroupBlocks : KB) {
         Q.kb0 = kb;
         Q.first = kb == 0;
         Q.last = !part || kb + kGroupBlocks >= KB;
         if (m.fp64 && m.rows == 16)
-            CUTC_TRY((launch_kb<7, 16, true>(st, ta, tb, Q, n_sm, KB, part)));
+            CUTC_TRY((launch_kb<7, 16, true, true>(st, ta, tb, Q, n_sm, KB, part)));
         else if (m.fp64)
-            CUTC_TRY((launch_kb<7, 32, true>(st, ta, tb, Q, n_sm, KB, part)));
-        else if (m.slices == 6 && m.rows == 16)
-            CUTC_TRY((launch_kb<6, 16, false>(st, ta, tb, Q, n_sm, KB, part)));
+            CUTC_TRY((launch_kb<7, 32, true, true>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.rows == 32)
+            CUTC_TRY((launch_kb<6, 32, false, true>(st, ta, tb, Q, n_sm, KB, part)));
+        else if (m.checked)
+            CUTC_TRY((launch_kb<6, 16, false, true>(st, ta, tb, Q, n_sm, KB, part)));
         else if (m.slices == 6)
-            CUTC_TRY((launch_kb<6, 32, false>(st, ta, tb, Q, n_sm, KB, part)));
-        else if (m.rows == 16)
-            CUTC_TRY((launch_kb<5, 16, false>(st, ta, tb, Q, n_sm, KB, part)));
+            CUTC_TRY((launch_kb<6, 16, false, false>(st, ta, tb, Q, n_sm, KB, part)));
         else
-            CUTC_TRY((launch_kb<5, 32, false>(st, ta, tb, Q, n_sm, KB, part)));
+            CUTC_TRY((launch_kb<5, 16, false, false>(st, ta, tb, Q, n_sm, KB, part)));
     }
     return CUTC_OK;
 }
@@ -1116,6 +1164,16 @@ int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, cons
         Q.P.n1b = (int)std::min<int64_t>(plan.tile_rows, P.n1b - i);
         Q.P.G += i * P.ldg;
         CUTC_TRY(run_tile(st, plan, Q, rn, a_en, n_sm));
+        if (plan.mode.checked) {
+            PairArgs R{};
+            R.i0 = Q.P.i0; R.n1b = Q.P.n1b; R.n2 = P.n2; R.nN = P.nN;
+            R.r1 = P.r1; R.r2 = P.r2; R.f2 = P.f2;
+            R.coef = P.coef; R.exps = P.exps; R.term_off = P.term_off; R.a_ee = P.a_ee;
+            R.G = reinterpret_cast<double *>(Q.P.G); R.ldg = P.ldg; R.plane = P.plane;
+            CUTC_TRY(launch_pair_f64_marked(st, R, rn, a_en, true, plan.marked,
+                                            (const unsigned *)(plan.marked + 16), mark_words(P.n2),
+                                            n_sm));
+        }
     }
     return CUTC_OK;
 }
@@ -1139,7 +1197,7 @@ int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &A, const
         R.i0 = P.i0;
         R.n1b = P.n1b;
         R.G = Q.G64;
-        CUTC_TRY(launch_pair_f64_marked(st, R, rn, a_en, plan.marked,
+        CUTC_TRY(launch_pair_f64_marked(st, R, rn, a_en, false, plan.marked,
                                         (const unsigned *)(plan.marked + 16), mark_words(A.n2), n_sm));
     }
     return CUTC_OK;

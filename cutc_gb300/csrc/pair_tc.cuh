@@ -24,6 +24,7 @@ struct PairTcMode {
                        // (any in [0, 6]); 0: not on the tensor cores
     int slices = 5;    // BF16 slices per operand: 5 or 6 (double-float results), 7 (FP64)
     bool fp64 = false; // FP64 results
+    bool checked = false;  // results whose error may be above a term by term sum's are marked
     int powers() const { return rows == 16 ? 4 : 7; }
 };
 
@@ -31,7 +32,7 @@ struct PairTcMode {
 // FP64 results.  rows == 0 where the tensor-core kernel does not apply (a coefficient that
 // is not finite, or a kernel chosen by CUTC_PAIR_DF / CUTC_PAIR_DENSE for the double-float
 // form).
-PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, bool fp64,
+PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, int n_nuc, bool fp64,
                         int slices);
 
 struct PairTcPlan {
@@ -42,7 +43,7 @@ struct PairTcPlan {
     float *bscale = nullptr;    // 2^(row exponent) of the coefficient rows
     void *part = nullptr;       // the V values between the groups of a long contraction
     int64_t tile_rows = 0;      // r1 rows taken at once
-    int *marked = nullptr;      // FP64: set when pairs are left out; their bits 16 ints on
+    int *marked = nullptr;      // checked: set when pairs are left out; their bits 16 ints on
     int *err = nullptr;         // device flag set by a bounded wait that gave up
 };
 
