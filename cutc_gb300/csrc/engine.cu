@@ -470,7 +470,7 @@ static size_t fixed_bytes(const Request &R)
                               R.x_only ? (size_t)0 : fp64_contract_bytes(np, np, 3 * (int64_t)R.n1, R.scratch));
     else
         b += (double)split_fixed_bytes(R) + (3.0 + nN) * n2 * sizeof(float2);
-    b += (double)pair_tc_fixed_bytes(R.n2, R.nN, pair_slices(R));
+    b += (double)pair_tc_fixed_bytes(R.n2, R.nN, pair_slices(R), R.scratch);
     if (!(R.device_pointers || R.out_device) && !R.x_only)
         b += 2.0 * int2e_slab_cols(R.nA) * nA * nA * 8;
     return (size_t)b;
@@ -841,7 +841,7 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     }
     PairTcPlan ptc;
     if (pmode.rows)
-        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, pmode, n2, nN, d_f2, n1t,
+        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, pmode, n2, nN, d_f2, n1t, R.scratch,
                                  R.precision == CUTC_PLAIN_FP64 ? contract.flags : sp.err, ptc));
     CUTC_CUDA_TRY(cudaEventRecord(E->ev[2], st));
 
@@ -1225,27 +1225,48 @@ int run_pair_only(Engine *E, cudaStream_t st, int i0, int n1b, int n1, int j0, i
         CUTC_CUDA_TRY(cudaMemcpyAsync(d_exps, exps.data(), exps.size() * 4, cudaMemcpyHostToDevice, st));
     }
     CUTC_CUDA_TRY(cudaMemcpyAsync(d_off, off.data(), off.size() * 4, cudaMemcpyHostToDevice, st));
-    CUTC_TRY(W.get(S_T1, (size_t)n1b * nN * sizeof(NucTerm), &p));
-    NucTerm *d_t1 = (NucTerm *)p;
-    CUTC_TRY(W.get(S_F2, (size_t)nN * n2b * 8, &p));
-    double *d_f2 = (double *)p;
-    const double *r2w = r2 + 3 * (int64_t)j0;  // the r2 window
-    CUTC_TRY(launch_r2_terms(st, n2b, nN, r2w, rn, a_en, d_f2));
-    note_launches(1);
-    PairArgs P;
-    P.i0 = i0; P.n1b = n1b; P.n2 = n2b; P.nN = nN; P.n_terms = (int)exps.size();
-    P.r1 = r1; P.r2 = r2w; P.t1 = d_t1; P.f2 = d_f2;
-    P.coef = d_coef; P.exps = d_exps; P.term_off = d_off; P.a_ee = a_ee;
-    P.G = G; P.ldg = ldg; P.plane = plane;
+    PairArgs P{};
+    P.i0 = i0; P.n1b = n1b; P.nN = nN; P.n_terms = (int)exps.size();
+    P.r1 = r1; P.coef = d_coef; P.exps = d_exps; P.term_off = d_off; P.a_ee = a_ee;
+    P.ldg = ldg; P.plane = plane;
     const PairTcMode mode = pair_tc_mode(coef.data(), exps.data(), (int)exps.size(), nN, true, 0);
+    // the r2 points of a window, at j of the call's
+    auto window = [&](int j, int n) -> int {
+        CUTC_TRY(W.get(S_F2, (size_t)nN * n * 8, &p));
+        P.f2 = (const double *)p;
+        P.n2 = n;
+        P.r2 = r2 + 3 * ((int64_t)j0 + j);
+        P.G = G + j;
+        CUTC_TRY(launch_r2_terms(st, n, nN, P.r2, rn, a_en, (double *)p));
+        note_launches(1);
+        return CUTC_OK;
+    };
     if (mode.rows) {
         ContractScratch flags;  // (its wait flag alone)
         CUTC_TRY(fp64_contract_begin(W, kContractSlot, st, 0, flags));
-        PairTcPlan plan;
-        CUTC_TRY(pair_tc_prepare(W, S_PAIRTC, st, mode, n2b, nN, d_f2, n1b, flags.flags, plan));
-        CUTC_TRY(pair_tc_tile_f64(st, plan, P, rn, a_en, E->n_sm));
-        return fp64_contract_check(flags, st);
+        const int step = pair_tc_window(mode, nN);
+        int s = CUTC_OK;
+        for (int j = 0; j < n2b && s == CUTC_OK; j += step) {
+            const int n = std::min(step, n2b - j);
+            PairTcPlan plan;
+            s = window(j, n);
+            if (s == CUTC_OK)
+                s = pair_tc_prepare(W, S_PAIRTC, st, mode, n, nN, P.f2, n1b, kPairScratch,
+                                    flags.flags, plan);
+            if (s == CUTC_OK)
+                s = pair_tc_tile_f64(st, plan, P, rn, a_en, E->n_sm);
+            if (j > INT32_MAX - step)
+                break;
+        }
+        if (s == CUTC_OK)
+            return fp64_contract_check(flags, st);
+        if (s != CUTC_ERR_NO_MEMORY)
+            return s;  // (without memory for the operands: term by term)
     }
+    CUTC_TRY(W.get(S_T1, (size_t)n1b * nN * sizeof(NucTerm), &p));
+    NucTerm *d_t1 = (NucTerm *)p;
+    P.t1 = d_t1;
+    CUTC_TRY(window(0, n2b));
     CUTC_TRY(launch_r1_terms(st, i0, n1b, nN, r1, rn, a_en, d_t1));
     CUTC_TRY(launch_pair_f64(st, P));
     note_launches(2);

@@ -916,12 +916,6 @@ static int planes(const PairTcMode &m) { return m.slices + (m.checked ? 1 : 0); 
 static int part_bytes(const PairTcMode &m) { return m.fp64 ? 16 : 12; }
 static int mark_words(int64_t n2) { return (int)((n2 + 31) / 32); }
 
-// r1 rows per sub-tile of a contraction in groups: its values so far take at most 2 GiB.
-static int64_t group_rows(const PairTcMode &m, int64_t n2, int64_t n1b)
-{
-    const int64_t per = n2 * m.rows * part_bytes(m);
-    return std::min(n1b, std::max<int64_t>(8, (((int64_t)2 << 30) / per) / 8 * 8));
-}
 
 PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, int n_nuc, bool fp64,
                         int slices)
@@ -948,13 +942,31 @@ static size_t operand_bytes(int64_t rows, int64_t K, int slices)
     return (size_t)rows * (8 * K + 2 * (slices + 1) * round_up(K, kGroupBlocks * kBK) + 4);
 }
 
-size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices)
+// r1 rows per sub-tile: its coefficient operand, and in groups its values so far, take about
+// `limit` bytes each at most (eight rows at least).
+static int64_t sub_tile_rows(const PairTcMode &m, int64_t n2, int64_t K, int64_t n1b, size_t limit)
+{
+    size_t per = operand_bytes(m.rows, K, m.slices);
+    if (K > one_group_k(m))
+        per = std::max<size_t>(per, (size_t)n2 * m.rows * part_bytes(m));
+    return std::min(n1b, std::max<int64_t>(8, (int64_t)(limit / per) / 8 * 8));
+}
+
+static size_t sub_tile_bytes(size_t scratch) { return std::min(kPairScratch, scratch); }
+
+size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices, size_t scratch)
 {
     const int64_t K = 7 * (int64_t)n_nuc;
     size_t b = operand_bytes(round_up(n2, kBM), K, slices);
     if (K > 64)  // the values so far of a sub-tile
-        b += (size_t)2 << 30;
+        b += std::max(sub_tile_bytes(scratch), (size_t)n2 * 8 * 32 * 16);
     return b;
+}
+
+int pair_tc_window(const PairTcMode &m, int n_nuc)
+{
+    const size_t per = operand_bytes(kBM, (int64_t)m.powers() * n_nuc, m.slices);
+    return kBM * (int)std::max<size_t>(1, kPairScratch / per);
 }
 
 size_t pair_tc_row_bytes(int n_nuc, int slices)
@@ -999,12 +1011,13 @@ static int slice_rows(cudaStream_t st, const PairTcMode &m, const double *X,
 enum { kSlotAF = 0, kSlotBC = 2, kSlotF64 = 4, kSlotC64, kSlotR1d, kSlotBscale, kSlotPart, kSlotMarks };
 
 int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &mode, int n2,
-                    int n_nuc, const double *f2, int64_t n1t, int *err, PairTcPlan &plan)
+                    int n_nuc, const double *f2, int64_t n1t, size_t scratch, int *err,
+                    PairTcPlan &plan)
 {
     const int64_t K = (int64_t)mode.powers() * n_nuc, Kpad = pad_k(mode, K);
     plan.mode = mode;
     plan.err = err;
-    plan.tile_rows = K <= one_group_k(mode) ? n1t : group_rows(mode, n2, n1t);
+    plan.tile_rows = sub_tile_rows(mode, n2, K, n1t, sub_tile_bytes(scratch));
     const int64_t rows = (int64_t)mode.rows * plan.tile_rows;
     void *p;
     CUTC_TRY(W.get(slot0 + kSlotF64, (size_t)n2 * K * 8, &p));

@@ -48,9 +48,14 @@ struct PairTcPlan {
 };
 
 // Builds the F operand (powers of f2 on the n2 r2 points; f2 is [n_nuc][n2] FP64) and
-// reserves the coefficient operand for tiles of up to n1t rows.  err: the caller's flag.
+// reserves the coefficient operand for tiles of up to n1t rows, taken in sub-tiles whose
+// operands stay within kPairScratch and `scratch` bytes.  err: the caller's flag.
+constexpr size_t kPairScratch = (size_t)2 << 30;
 int pair_tc_prepare(Workspace &W, int slot0, cudaStream_t st, const PairTcMode &mode, int n2,
-                    int n_nuc, const double *f2, int64_t n1t, int *err, PairTcPlan &plan);
+                    int n_nuc, const double *f2, int64_t n1t, size_t scratch, int *err,
+                    PairTcPlan &plan);
+// r2 points whose F operand takes about kPairScratch bytes.
+int pair_tc_window(const PairTcMode &mode, int n_nuc);
 // The pair planes of one r1 tile.  Double-float: P.G as for launch_pair_df.
 int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, const double *rn,
                     double a_en, int n_sm);
@@ -59,7 +64,7 @@ int pair_tc_tile_df(cudaStream_t st, PairTcPlan &plan, const PairDfArgs &P, cons
 int pair_tc_tile_f64(cudaStream_t st, PairTcPlan &plan, const PairArgs &P, const double *rn,
                      double a_en, int n_sm);
 // Device bytes: fixed (F) and per r1 row of a tile, for the largest operands of the form.
-size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices);
+size_t pair_tc_fixed_bytes(int n2, int n_nuc, int slices, size_t scratch);
 size_t pair_tc_row_bytes(int n_nuc, int slices);
 
 }  // namespace cutc

@@ -13,7 +13,7 @@ def test_plain_contraction_scratch_follows_the_budget():
     assert fixed[0] < fixed[1] < fixed[2]
     assert fixed[2] - fixed[0] > 8 << 30
     # the rest: residues within 64 MiB (a tile's at least) and 512 MiB, scales, r2 terms
-    pair = 3 << 30
+    pair = 1 << 30
     assert fixed[0] < (192 << 20) + pair and fixed[1] < (640 << 20) + pair
 
 
@@ -26,6 +26,6 @@ def test_split_contraction_scratch_follows_the_budget():
     own = 8 * (np_ * np_ + np_ * nl)
     small, large = (cg.plan(n1, n2, nA, nN, cg.SPLIT_BF16, device_pointers=True,
                             max_work_bytes=b)["fixed_bytes"] - own for b in (1 << 20, 24 << 30))
-    pair = 3 << 30
+    pair = 1 << 30
     assert small < 10 * np_ * 40000 + (1 << 30) + pair
     assert large > 26 * np_ * n2
