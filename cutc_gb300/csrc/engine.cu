@@ -769,12 +769,14 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     }
 
     // ---- buffers -------------------------------------------------------------
-    NucTerm *d_t1;
+    NucTerm *d_t1 = nullptr;
     double *d_f2, *d_P = nullptr, *d_G, *d_Xt, *d_H = nullptr, *d_N = nullptr;
     double *d_S0 = nullptr, *d_Sl = nullptr;
     double *stage_x[2] = {nullptr, nullptr}, *stage_i[2] = {nullptr, nullptr};
-    CUTC_TRY(W.get(S_T1, (size_t)n1t * nN * sizeof(NucTerm), &p));
-    d_t1 = (NucTerm *)p;
+    if (!pmode.rows) {  // (the kernels that loop over the terms)
+        CUTC_TRY(W.get(S_T1, (size_t)n1t * nN * sizeof(NucTerm), &p));
+        d_t1 = (NucTerm *)p;
+    }
     CUTC_TRY(W.get(S_F2, (size_t)nN * n2 * 8, &p));
     d_f2 = (double *)p;
     CUTC_TRY(W.get(S_G, 4 * (size_t)n1t * n2 * 8, &p));
@@ -819,10 +821,12 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
         psparse = pexp == 4 && pair_df_sparse(exps.data(), nt) && !getenv("CUTC_PAIR_DENSE");
         CUTC_TRY(W.get(S_R2D, 3 * (size_t)n2 * sizeof(float2), &p));
         d_r2d = (float2 *)p;
-        CUTC_TRY(W.get(S_F2D, (size_t)nN * n2 * sizeof(float2), &p));
-        d_f2d = (float2 *)p;
-        CUTC_TRY(W.get(S_POLY, pair_df_poly_bytes(pexp, (int)n1t, nN), &p));
-        d_poly = (float2 *)p;
+        if (!pmode.rows) {
+            CUTC_TRY(W.get(S_F2D, (size_t)nN * n2 * sizeof(float2), &p));
+            d_f2d = (float2 *)p;
+            CUTC_TRY(W.get(S_POLY, pair_df_poly_bytes(pexp, (int)n1t, nN), &p));
+            d_poly = (float2 *)p;
+        }
         CUTC_TRY(launch_r2_df(st, n2, nN, d_r2, d_f2, d_r2d, d_f2d));
         note_launches(1);
     }

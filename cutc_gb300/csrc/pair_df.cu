@@ -102,6 +102,7 @@ __global__ void r1_poly_kernel(int i0, int n, int nN, const double *__restrict__
 }
 
 // r2 coordinates and f2A in df: r2d[c * n2 + j], f2d[A * n2 + j]
+// (f2d null: the points alone)
 __global__ void r2_df_kernel(int n2, int nN, const double *__restrict__ r2,
                              const double *__restrict__ f2, float2 *__restrict__ r2d,
                              float2 *__restrict__ f2d)
@@ -113,7 +114,7 @@ __global__ void r2_df_kernel(int n2, int nN, const double *__restrict__ r2,
         const df::D v = df::from_double(r2[3 * (int64_t)j + c]);
         r2d[(int64_t)c * n2 + j] = make_float2(v.hi, v.lo);
     }
-    for (int A = 0; A < nN; A++) {
+    for (int A = 0; f2d && A < nN; A++) {
         const df::D v = df::from_double(f2[(int64_t)A * n2 + j]);
         f2d[(int64_t)A * n2 + j] = make_float2(v.hi, v.lo);
     }
