@@ -64,6 +64,7 @@
 #include "digits.cuh"
 #include "modular.cuh"
 #include "pair_tc.cuh"
+#include "series.cuh"
 #include "tc.cuh"
 
 namespace cutc {
@@ -309,7 +310,9 @@ __device__ __forceinline__ bool pair_df(const PairTcParams &Q, int i, int j, con
 }
 
 // I 2^k for |I| < 2^53, exactly, in integer arithmetic (0 below the normal range, an
-// infinity above it)
+// infinity above it).  A V value is at most K units of the row scales, K 2^43 as an integer, and
+// K at most 7 powers of kMaxNuc nuclei in all groups together.
+static_assert(7 * kMaxNuc < 1024, "the V values' integers");
 __device__ __forceinline__ double int_double(long long I, int k)
 {
     const unsigned long long m = (unsigned long long)(I < 0 ? -I : I);
@@ -389,23 +392,6 @@ __device__ __forceinline__ void scale_f64(long long I, float rest, int eb, int e
     *lo = rest * pow2f(min(e, 127));
 }
 
-// a double as a float, truncated, with integer operations (0 below the float range)
-__device__ __forceinline__ float trunc_float(double x)
-{
-    const int hi = __double2hiint(x);
-    const int v = (hi & 0x7fffffff) - 0x38000000;
-    const unsigned m = ((unsigned)max(v, 0) << 3) | ((unsigned)__double2loint(x) >> 29);
-    const unsigned f = v < 0x00100000 ? 0u : v >= 0x0ff00000 ? 0x7f7fffffu : m;
-    return __uint_as_float(f | ((unsigned)hi & 0x80000000u));
-}
-
-// a positive normal float as a double, with integer operations
-__device__ __forceinline__ double exact_double(float x)
-{
-    const unsigned b = __float_as_uint(x);
-    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
-}
-
 // any float as a double (subnormals as zero, infinities and NaNs as infinities or NaNs)
 __device__ __forceinline__ double signed_double(float x)
 {
@@ -426,9 +412,7 @@ __device__ __forceinline__ double minus_half(double x)
 }
 
 // One pair in FP64 from its V values (hi + lo); true, and nothing is written, when they are
-// unsure.  The reciprocal square root and the
-// reciprocal are FP32 seeds with one step each of third order in FP64 (the seeds' relative
-// errors of 2^-22 and 2^-23 become 2^-63 and below).
+// unsure.
 template <int R>
 __device__ __forceinline__ bool pair_f64(const PairTcParams &Q, int i, int j, const double *V,
                                          const float *W, const float *w, double x2, double y2,
@@ -448,9 +432,7 @@ __device__ __forceinline__ bool pair_f64(const PairTcParams &Q, int i, int j, co
     if (db > __double_as_longlong(1e-15) && db <= 0x7ff0000000000000ll) {
         double y, z, d;
         if (hw < (1023 + 120) << 20) {
-            const double y0 = exact_double(rsqrtf(trunc_float(d2)));
-            const double e = fma(-(d2 * y0), y0, 1.0);
-            y = fma(e * y0, fma(e, 0.375, 0.5), y0);
+            y = rsqrt_series(d2);
             d = d2 * y;
         } else {  // distances beyond 2^60, and infinities
             d = sqrt(d2);
@@ -458,13 +440,7 @@ __device__ __forceinline__ bool pair_f64(const PairTcParams &Q, int i, int j, co
         }
         const double ad = a_one ? d : a * d;
         const double den = 1.0 + ad;
-        if (__double2hiint(den) < (1023 + 120) << 20) {
-            const double z0 = exact_double(__frcp_rn(trunc_float(den)));
-            const double e = fma(-den, z0, 1.0);
-            z = fma(z0, fma(e, e, e), z0);
-        } else {
-            z = 1.0 / den;
-        }
+        z = __double2hiint(den) < (1023 + 120) << 20 ? recip_series(den) : 1.0 / den;
         g = ad * z;
         double s = z * z * y;
         if (!a_one)
