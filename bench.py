@@ -203,7 +203,7 @@ def plain_rate_estimate(cg, p, sizes):
     release_device()
     return {"value_est": 1e3 / t_full, "unit": UNIT, "ms_per_build_est": t_full,
             "x_gemm_fp64_tflops": gemm[-1],
-            "x_gemm_kernel": "modular_gemm_kernel, 15 moduli (this library)",
+            "x_gemm_kernel": "modular_gemm_kernel, 17 moduli and the magnitudes (this library)",
             "basis": "plain FP64 form, device-resident, timed on %d and %d r1 rows (%.0f and %.0f ms) "
                      "and extrapolated linearly to n_grid1=%d" % (n_a, n_b, t_a, t_b, p.n_grid1)}
 
