@@ -115,20 +115,24 @@ static int64_t int2e_panel_k(const Request &R, int n_mod, int64_t K, int64_t np)
 static size_t resident_bytes(const Request &R) { return std::min((size_t)16 << 30, 2 * R.scratch); }
 
 // K panel of the residues of an operand of `rows` rows: the launch's, unless its residues take
-// more than `limit`; then a part of it, which takes no more than the operand's S BF16 slices
-// would.
+// more than `limit` and than the operand's S BF16 slices would; then equal parts of it that do
+// not (large build, 45 150 rows: 26 GB a panel in one part; cut in three, the contractions'
+// passes over the results' residues made the build 9 % slower).
 static int64_t residue_panel(int S, int n_mod, int64_t K, int64_t rows, int k_split, size_t limit)
 {
     const int64_t kp = panel_k(K, rows, k_split);
-    if (residue_bytes(n_mod, rows, kp) <= limit)
-        return kp;
-    const int parts = (n_mod + S - 1) / S;
-    return std::min(kp, (kp / parts + 511) / 512 * 512);
+    const size_t bytes = residue_bytes(n_mod, rows, kp);
+    const size_t allowed = std::max(limit, residue_bytes(S, rows, kp));
+    const int64_t parts = (int64_t)((bytes + allowed - 1) / allowed);
+    return parts <= 1 ? kp : std::min(kp, ((kp + parts - 1) / parts + 511) / 512 * 512);
 }
+
+constexpr size_t kPanelBytes = (size_t)32 << 30;  // of one panel (and four limits) at most
 
 static int64_t x_panel(const Request &R, int n_mod)
 {
-    return residue_panel(R.n_slices, n_mod, R.n2, n_pairs(R.nA), R.k_split, resident_bytes(R));
+    return residue_panel(R.n_slices, n_mod, R.n2, n_pairs(R.nA), R.k_split,
+                         std::min(kPanelBytes, 4 * R.scratch));
 }
 
 static bool p_resident(const Request &R, int n_mod, int64_t k_panel)
@@ -401,7 +405,7 @@ static int gemm_sources(Engine *E, cudaStream_t st, int base, int n_slices, int 
 {
     Workspace &W = E->ws;
     const int n_mod = split_moduli(n_slices, K);
-    const int64_t pan = residue_panel(n_slices, n_mod, K, M, 0, (size_t)16 << 30);
+    const int64_t pan = residue_panel(n_slices, n_mod, K, M, 0, kPanelBytes);
     int *sc_a, *sc_b;
     void *p;
     CUTC_TRY(scale_slot(W, base, M, &sc_a));
