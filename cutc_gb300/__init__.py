@@ -479,7 +479,7 @@ def no_2e(tmpC1, x_mo, tmpC2, tmpD2, n_mo, n_grid1, precision=PLAIN_FP64, n_slic
 
 def fp64_gemm_device(a_kmajor, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, stride_a=0,
                      stride_b=0, stride_c=0, batch=1):
-    """The plain form's FP64 DMMA GEMM on device tensors, with cuBLAS's
+    """An FP64 DMMA GEMM on device tensors, with cuBLAS's
     column-major argument meaning (cutc_fp64_gemm_dev); raises on a status."""
     s = load().cutc_fp64_gemm_dev(int(bool(a_kmajor)), M, N, K, alpha, _vp(A), lda, stride_a,
                                   _vp(B), ldb, stride_b, beta, _vp(C), ldc, stride_c, batch)

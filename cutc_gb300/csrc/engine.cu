@@ -852,10 +852,8 @@ int run_build(Engine *E, const Request &R_in, cutc_stats *stats)
     // ---- tiles ---------------------------------------------------------------
     // Host outputs leave through two device staging buffers, copied on the
     // transfer stream while the next tile computes.  Pinned (or managed) caller
-    // memory takes the copies directly; pageable caller memory gets them in two
-    // pinned buffers first, from which this thread copies while the device
-    // works on (no pageable cudaMemcpy, which holds the thread until the stream
-    // reaches it).
+    // memory takes the copies directly; pageable memory as told below, or through two
+    // pinned buffers, from which this thread copies while the device works on.
     StreamsDrain drain{st, E->xfer};
     cudaEvent_t ready[2] = {E->ev[3], E->ev[4]}, done[2] = {E->ev[9], E->ev[10]};
     bool busy[2] = {false, false};

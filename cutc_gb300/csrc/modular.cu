@@ -26,7 +26,8 @@ namespace cutc {
 // cap: M 7260, N 16384, K 16384 with 11 moduli takes 23.6 ms, 1817 TF/s of BF16 products
 // (cuBLAS: 1898 in a burst, 1704 sustained).  The 5-slice kernel that this replaces, with
 // a 128 x 48 tile of five stacked accumulators, ran 15 products at 1551 TF/s.  The medium
-// build (n_ao 120, 25k x 80k): 1361 -> 948 ms, with smaller errors (int_2e 1.7e-12 -> 3e-13).
+// build (n_ao 120, 25k x 80k, 13 moduli): 1361 -> 1110 ms, with smaller errors (int_2e
+// 1.7e-12 -> 1e-13).
 constexpr int kTileM = 256, kBK = 64;     // 64 BF16 = 128-byte rows (128B swizzle)
 constexpr int kChunkBlocks = 8;           // 512 K: sums of products of residues below 2^24
 constexpr int kEpiWarps = 16;             // 4 lane quarters x 4 column groups

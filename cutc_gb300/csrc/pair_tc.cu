@@ -48,8 +48,8 @@
 // gradient and the polynomial take FP64: 45 FP64 operations per pair with 16 rows, whatever
 // the number of nuclei, on a pipe of 2 per clock and SM, against about 11 per term in the
 // term-by-term kernel (pair.cu).  512 x 20 011 pairs, 8 nuclei with 13
-// terms each: 19.3 -> 1.20 ms.  General exponents in double-float, 2003 x 30 011 pairs, 6
-// nuclei, against pair_df_kernel<6>: 16.6 -> 4.5 ms.
+// terms each: 19.4 -> 1.22 ms.  General exponents in double-float, 2003 x 30 011 pairs, 6
+// nuclei, against pair_df_kernel<6>: 16.6 -> 5.1 ms.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>

@@ -72,13 +72,14 @@ typedef struct cutc_basis {
 
 typedef struct cutc_options {
     int precision;          /* CUTC_PLAIN_FP64 or CUTC_SPLIT_BF16 */
-    int n_slices;           /* split form: precision of the operands in 9-bit slices, 3..7
-                               (default 5) */
+    int n_slices;           /* split form: precision of the operands, 3..7 (default 5): no row is
+                               rounded more coarsely than that many 9-bit slices of it */
     double a_en;            /* e-n Jastrow scale: f = a r / (1 + a r); 1.0 = reference */
     double a_ee;            /* e-e Jastrow scale; 1.0 = reference */
     int x_components;       /* X components copied out: 3 (reference) or 4 */
     int device_pointers;    /* 1: every array argument is a device pointer */
-    size_t max_work_bytes;  /* device budget for the r1 tiles; 0 = automatic */
+    size_t max_work_bytes;  /* device budget for the r1 tiles (and half of it for the
+                               contractions' scratch); 0 = automatic */
     void *stream;           /* cudaStream_t to run on; NULL = the engine's stream */
     int pair_fp64;          /* split form: 1 = pair terms in FP64 instead of double-float */
     int k_split;            /* split form: max K per tensor-core launch; the partial results
@@ -214,7 +215,7 @@ int cutc_check_wait_limit(void);
  * The split-precision contraction alone, on device arrays of the current
  * device: C[m + ldc * n] = sum_k A[m * K + k] * B[n * K + k] for m < M, n < N,
  * with A and B FP64 row-major (K contiguous) and the product formed
- * exactly from operands rounded to the precision of n_slices 9-bit slices (3..7), on
+ * exactly from operands rounded no more coarsely than n_slices 9-bit slices (3..7) do, on
  * the tcgen05 tensor cores.  A row with an infinity or a NaN gives NaN results.
  * This is the kernel behind CUTC_SPLIT_BF16, exposed for callers that need the
  * GEMM itself.  Synchronous on the engine stream.  No reference counterpart.
