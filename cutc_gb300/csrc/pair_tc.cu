@@ -19,7 +19,8 @@
 // percent of what the kernels that loop over the nuclei take.
 //
 // A = the F slices of 128 r2 points, all of K, loaded once per CTA; B = the coefficient
-// slices in tiles of 64 rows (four r1 points, or two; one point for FP64 results), streamed;
+// slices in tiles of 64 rows (four r1 points, or two; one point for FP64 results), streamed
+// (whole tiles, or K block by K block where three checked blocks would not fit);
 // one stacked accumulator set in tensor memory (four or two for FP64 results).  The tensor-core work of a tile is a small part of its epilogue, so
 // one B stage per accumulator set suffices: the next tile's MMAs run as soon as the
 // epilogue has read the accumulators, and one control warp issues both the TMA loads and
@@ -128,9 +129,15 @@ struct PairTcCfg {
     static constexpr int kASlice = kBM * kBK * 2;
     static constexpr int kBSlice = kBN * kBK * 2;
     static constexpr int kABytes = KB * kPlanes * kASlice;
-    static constexpr int kBStage = KB * kPlanes * kBSlice;
+    // B comes in units: all of a tile's K with a stage per accumulator set, or one K block
+    // with two stages where the planes of three blocks do not fit
+    static constexpr bool kSplit = CHK && KB == 3;
+    static constexpr int kUnits = kSplit ? KB : 1;   // per tile
+    static constexpr int kUnitBlocks = KB / kUnits;
+    static constexpr int kStages = kSplit ? 2 : kBufs;
+    static constexpr int kBStage = kUnitBlocks * kPlanes * kBSlice;
     static constexpr int kBufCols = kBN * kPlanes;   // accumulator columns of a buffer
-    static constexpr int kSmem = kABytes + kBufs * kBStage + 1024 + 256;
+    static constexpr int kSmem = kABytes + kStages * kBStage + 1024 + 256;
     static constexpr int kMaxN = 256;                // widest kind::f16 instruction at M = 128
     static_assert(kSmem <= 227 * 1024, "shared memory");
     static_assert(kBufs * kBufCols <= (int)kTmemCols, "accumulators exceed tensor memory");
@@ -517,11 +524,12 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint8_t *sA = smem;
     uint8_t *sB = smem + Cfg::kABytes;
     constexpr int NB = Cfg::kBufs;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + NB * Cfg::kBStage);
+    constexpr int NS = Cfg::kStages, U = Cfg::kUnits;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sB + NS * Cfg::kBStage);
     uint64_t *afull = bars;            // the F tile has landed
-    uint64_t *full = bars + 1;         // a B stage holds a tile
-    uint64_t *empty = full + NB;       // the MMAs of the tile are done with the B stage
-    uint64_t *tfull = empty + NB;      // the accumulators hold the tile
+    uint64_t *full = bars + 1;         // a B stage holds a unit
+    uint64_t *empty = full + NS;       // the MMAs of the unit are done with the B stage
+    uint64_t *tfull = empty + NS;      // the accumulators hold the tile
     uint64_t *tempty = tfull + NB;     // its epilogue warps have read them
     uint64_t *drain = tempty + NB;
     uint32_t *s_tmem = reinterpret_cast<uint32_t *>(drain + 1);
@@ -535,9 +543,11 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     if (threadIdx.x == 0) {
         tc::mbar_init(tc::smem_u32(afull), 1);
-        for (int i = 0; i < NB; i++) {
+        for (int i = 0; i < NS; i++) {
             tc::mbar_init(tc::smem_u32(&full[i]), 1);
             tc::mbar_init(tc::smem_u32(&empty[i]), 1);
+        }
+        for (int i = 0; i < NB; i++) {
             tc::mbar_init(tc::smem_u32(&tfull[i]), 1);
             tc::mbar_init(tc::smem_u32(&tempty[i]), Cfg::kBufWarps);
         }
@@ -566,18 +576,20 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (warp == kCtlWarp) {
         if (lane == 0) {
             const int kb0 = PART ? Q.kb0 : 0;
-            auto load_b = [&](int q) {
-                const int b = q % NB;
+            constexpr int UB = Cfg::kUnitBlocks;
+            const int units = ntiles * U;
+            auto load_b = [&](int u) {
+                const int b = u % NS;
                 const uint32_t fb = tc::smem_u32(&full[b]);
                 tc::mbar_arrive_expect_tx(fb, Cfg::kBStage);
-                const int n0 = (t_begin + q) * BN;
+                const int n0 = (t_begin + u / U) * BN, k0 = kb0 + u % U * UB;
 #pragma unroll
-                for (int kb = 0; kb < KB; kb++)
+                for (int kb = 0; kb < UB; kb++)
 #pragma unroll
                     for (int t = 0; t < NP; t++)
                         tc::tma_load_2d(
                             tc::smem_u32(sB + b * Cfg::kBStage + (kb * NP + t) * Cfg::kBSlice), &tmB,
-                            (kb0 + kb) * kBK, t * Q.Npad + n0, fb);
+                            (k0 + kb) * kBK, t * Q.Npad + n0, fb);
             };
             const uint32_t ab = tc::smem_u32(afull);
             tc::mbar_arrive_expect_tx(ab, Cfg::kABytes);
@@ -587,68 +599,76 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 for (int s = 0; s < NP; s++)
                     tc::tma_load_2d(tc::smem_u32(sA + (kb * NP + s) * Cfg::kASlice), &tmA,
                                     (kb0 + kb) * kBK, s * Q.Mpad + m0, ab);
-            int loaded = 0;  // B tiles issued
-            for (; loaded < min(NB, ntiles); loaded++)
+            int loaded = 0;  // B units issued
+            for (; loaded < min(NS, units); loaded++)
                 load_b(loaded);
             bool ok = tc::mbar_wait(ab, 0, s_abort);
             if (!ok)
                 fail(12);
             for (int q = 0; q < ntiles && ok; q++) {
-                const int b = q % NB, round = q / NB;
+                const int set = q % NB, round = q / NB;
                 // the accumulators are free once their epilogue warps have read the last tile
                 if (round >= 1 &&
-                    !tc::mbar_wait(tc::smem_u32(&tempty[b]), (round - 1) & 1, s_abort)) {
+                    !tc::mbar_wait(tc::smem_u32(&tempty[set]), (round - 1) & 1, s_abort)) {
                     fail(13);
                     break;
                 }
-                if (!tc::mbar_wait(tc::smem_u32(&full[b]), round & 1, s_abort)) {
-                    fail(14);
-                    break;
-                }
-                tc::fence_after_sync();
-                const uint32_t sb0 = tc::smem_u32(sB + b * Cfg::kBStage);
-                const uint32_t acc = tbase + (uint32_t)(Cfg::kBufCols * b);
-                const uint32_t sa0 = tc::smem_u32(sA);
+                const uint32_t acc = tbase + (uint32_t)(Cfg::kBufCols * set);
                 bool first = true;
 #pragma unroll
-                for (int kb = 0; kb < KB; kb++) {
-#pragma unroll
-                    for (int k16 = 0; k16 < kBK / 16; k16++) {
-#pragma unroll
-                        for (int s = 0; s < S; s++) {
-                            // a_s x [b_0 .. b_{D-s}] -> diagonals s .. D, in instructions of
-                            // at most kMaxN columns
-                            const uint64_t ad = tc::smem_desc_sw64(
-                                sa0 + (kb * NP + s) * Cfg::kASlice + k16 * 32);
-#pragma unroll
-                            for (int t0 = 0; t0 <= D - s; t0 += Cfg::kMaxN / BN) {
-                                const int nt = min(Cfg::kMaxN / BN, D - s + 1 - t0);
-                                const uint64_t bd = tc::smem_desc_sw64(
-                                    sb0 + (kb * NP + t0) * Cfg::kBSlice + k16 * 32);
-                                tc::mma_bf16(acc + (uint32_t)(BN * (s + t0)), ad, bd,
-                                             tc::idesc_bf16_f32(kBM, BN * nt), first ? 0u : 1u);
-                            }
-                            first = false;
-                        }
-                        if constexpr (CHK)  // the magnitudes' sums
-                            tc::mma_bf16(
-                                acc + (uint32_t)(BN * S),
-                                tc::smem_desc_sw64(sa0 + (kb * NP + S) * Cfg::kASlice + k16 * 32),
-                                tc::smem_desc_sw64(sb0 + (kb * NP + S) * Cfg::kBSlice + k16 * 32),
-                                tc::idesc_bf16_f32(kBM, BN), kb > 0 || k16 > 0 ? 1u : 0u);
-                    }
-                }
-                tc::mma_commit(tc::smem_u32(&empty[b]));
-                tc::mma_commit(tc::smem_u32(&tfull[b]));
-                // refill a B stage once its MMAs have read it: with several stages, that of
-                // the tile before, so that this wait does not hold up the next MMAs
-                const int r = NB > 1 ? q - 1 : q;
-                if (r >= 0 && loaded < ntiles) {
-                    if (!tc::mbar_wait(tc::smem_u32(&empty[r % NB]), (r / NB) & 1, s_abort)) {
-                        fail(11);
+                for (int un = 0; un < U && ok; un++) {
+                    const int u = q * U + un, b = u % NS;
+                    if (!tc::mbar_wait(tc::smem_u32(&full[b]), (u / NS) & 1, s_abort)) {
+                        fail(14);
+                        ok = false;
                         break;
                     }
-                    load_b(loaded++);
+                    tc::fence_after_sync();
+                    const uint32_t sb0 = tc::smem_u32(sB + b * Cfg::kBStage);
+                    const uint32_t sa0 = tc::smem_u32(sA) + un * UB * NP * Cfg::kASlice;
+#pragma unroll
+                    for (int kb = 0; kb < UB; kb++) {
+#pragma unroll
+                        for (int k16 = 0; k16 < kBK / 16; k16++) {
+#pragma unroll
+                            for (int s = 0; s < S; s++) {
+                                // a_s x [b_0 .. b_{D-s}] -> diagonals s .. D, in instructions
+                                // of at most kMaxN columns
+                                const uint64_t ad = tc::smem_desc_sw64(
+                                    sa0 + (kb * NP + s) * Cfg::kASlice + k16 * 32);
+#pragma unroll
+                                for (int t0 = 0; t0 <= D - s; t0 += Cfg::kMaxN / BN) {
+                                    const int nt = min(Cfg::kMaxN / BN, D - s + 1 - t0);
+                                    const uint64_t bd = tc::smem_desc_sw64(
+                                        sb0 + (kb * NP + t0) * Cfg::kBSlice + k16 * 32);
+                                    tc::mma_bf16(acc + (uint32_t)(BN * (s + t0)), ad, bd,
+                                                 tc::idesc_bf16_f32(kBM, BN * nt), first ? 0u : 1u);
+                                }
+                                first = false;
+                            }
+                            if constexpr (CHK)  // the magnitudes' sums
+                                tc::mma_bf16(
+                                    acc + (uint32_t)(BN * S),
+                                    tc::smem_desc_sw64(sa0 + (kb * NP + S) * Cfg::kASlice + k16 * 32),
+                                    tc::smem_desc_sw64(sb0 + (kb * NP + S) * Cfg::kBSlice + k16 * 32),
+                                    tc::idesc_bf16_f32(kBM, BN),
+                                    un > 0 || kb > 0 || k16 > 0 ? 1u : 0u);
+                        }
+                    }
+                    tc::mma_commit(tc::smem_u32(&empty[b]));
+                    if (un == U - 1)
+                        tc::mma_commit(tc::smem_u32(&tfull[set]));
+                    // refill a B stage once its MMAs have read it: with several stages, that
+                    // of the unit before, so that this wait does not hold up the next MMAs
+                    const int r = NS > 1 ? u - 1 : u;
+                    if (r >= 0 && loaded < units) {
+                        if (!tc::mbar_wait(tc::smem_u32(&empty[r % NS]), (r / NS) & 1, s_abort)) {
+                            fail(11);
+                            ok = false;
+                            break;
+                        }
+                        load_b(loaded++);
+                    }
                 }
             }
             tc::mma_commit(tc::smem_u32(drain));
@@ -657,8 +677,8 @@ pair_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // let the copies still in flight land before the CTA goes away
             tc::mbar_wait(ab, 0, nullptr);
             if (*s_abort)
-                for (int q = max(0, loaded - NB); q < loaded; q++)
-                    tc::mbar_wait(tc::smem_u32(&full[q % NB]), (q / NB) & 1, nullptr);
+                for (int u = max(0, loaded - NS); u < loaded; u++)
+                    tc::mbar_wait(tc::smem_u32(&full[u % NS]), (u / NS) & 1, nullptr);
         }
     } else {
         // ---- epilogue: the warp's r1 points of each N tile, 32 r2 points ----------------
@@ -876,12 +896,14 @@ static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * 
 
 // K of unchecked double-float contractions: 20 nuclei of 4 powers.
 constexpr int kPlainDfK = 80;
+// The K of one group in double-float: exact leading diagonals.
+constexpr int kDfGroupK = 85;
 
 // The K up to which the contraction is one group: the leading diagonals are exact (and the
 // operands fit shared memory).  A longer one runs in groups of kGroupBlocks K blocks whose
 // values are added between launches.
 constexpr int kGroupBlocks = 2;
-static int one_group_k(const PairTcMode &m) { return m.checked ? 64 : kPlainDfK; }
+static int one_group_k(const PairTcMode &m) { return m.fp64 ? 64 : m.checked ? kDfGroupK : kPlainDfK; }
 static int64_t pad_k(const PairTcMode &m, int64_t K)
 {
     return round_up(std::max<int64_t>(K, 1), K <= one_group_k(m) ? kBK : kGroupBlocks * kBK);
@@ -904,7 +926,13 @@ PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, int n_
         if (!std::isfinite(coef[k]))
             return m;
     m.rows = pair_df_sparse(exps, n_terms) ? 16 : 32;
-    m.checked = fp64 || m.rows == 32 || m.powers() * n_nuc > kPlainDfK;
+    const int K = m.powers() * n_nuc;
+    m.checked = fp64 || m.rows == 32 || K > kPlainDfK;
+    // 32 rows of double-float values a pair between groups of K cost more than the loop over the
+    // nuclei (2003 x 30 011 pairs: 57 ms in two groups, 110 in three; the loop 38, 46 and 96 ms
+    // with 13, 16 and 24 nuclei)
+    if (!fp64 && m.rows == 32 && K > kDfGroupK)
+        return PairTcMode{};
     // 5 slices (representation error 2^-45, under the error of a 5-slice build's operands), 6
     // for builds of 6 and 7 slices and where the check is (2^-54, below the double-float
     // epilogue), 7 for FP64 (2^-63)
@@ -1064,18 +1092,18 @@ template <int S, int R, bool F64, bool CHK>
 static int launch_kb(cudaStream_t st, const CUtensorMap &ta, const CUtensorMap &tb,
                      const PairTcParams &Q, int n_sm, int KB, bool part)
 {
-    if constexpr (CHK)
+    if constexpr (F64 || (CHK && R == 16))
         if (part)
             return launch_kernel<S, kGroupBlocks, R, F64, CHK, true>(st, ta, tb, Q, n_sm);
-    if constexpr (!CHK || F64 || R == 32)  // (others have more than 80 K)
-        switch (KB) {
-        case 1: return launch_kernel<S, 1, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
-        case 2: return launch_kernel<S, 2, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
-        case 3:
-            if constexpr (!CHK)
-                return launch_kernel<S, 3, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
-            break;
-        }
+    if constexpr (F64 || !CHK || R == 32) {  // (others have more than 80 K)
+        if (KB == 1)
+            return launch_kernel<S, 1, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
+        if (KB == 2)
+            return launch_kernel<S, 2, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
+    }
+    if constexpr (!F64)
+        if (KB == 3)
+            return launch_kernel<S, 3, R, F64, CHK, false>(st, ta, tb, Q, n_sm);
     cutc_set_error(CUTC_ERR_INVALID, "pair contraction of %d K blocks", KB);
     return CUTC_ERR_INVALID;
 }
