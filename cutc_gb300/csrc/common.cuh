@@ -74,4 +74,20 @@ inline unsigned long long current_device_bit()
     return 1ull << (dev & 63);
 }
 
+// SMs of the current device (152 on GB300).
+inline int device_sms()
+{
+    static std::atomic<int> sms[64];
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::atomic<int> &c = sms[dev & 63];
+    int n = c.load();
+    if (n <= 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0)
+            n = 152;
+        c.store(n);
+    }
+    return n;
+}
+
 }  // namespace cutc

@@ -407,7 +407,6 @@ int fp64_gemm(cudaStream_t st, bool a_kmajor, int M, int N, int64_t K, double al
 // (65 us a wave of tiles), which the modular contraction's launches do not beat.
 
 constexpr int kMinContractK = 16;
-constexpr int kRestBlocks = 152;  // one per SM
 constexpr size_t kMinContractBytes = (size_t)16 << 20;  // no smaller blocks are tried
 enum ContractSlot { C_FLAGS, C_SCA, C_SCB, C_RA, C_RB, C_OUT };
 static_assert(C_OUT + 1 == kContractSlots, "slots");
@@ -545,8 +544,8 @@ static int contract(const ContractScratch &S, cudaStream_t st, bool a_kmajor, in
             g.n0 = n0;
             g.out = o;
             g.left = left;
-            return a_kmajor ? launch_rest<true>(st, g, kRestBlocks)
-                            : launch_rest<false>(st, g, kRestBlocks);
+            return a_kmajor ? launch_rest<true>(st, g, device_sms())
+                            : launch_rest<false>(st, g, device_sms());
         });
 }
 

@@ -34,7 +34,6 @@ constexpr int kEpiWarps = 16;             // 4 lane quarters x 4 column groups
 constexpr int kTmaWarp = kEpiWarps, kMmaWarp = kEpiWarps + 1;
 constexpr int kGemmThreads = (kEpiWarps + 2) * 32;
 constexpr int kGroupN = 8;                // column tiles per raster group
-constexpr int kPairs = 76;                // CTA pairs of GB300's 152 SMs
 constexpr int kResidentBlocks = 128;      // K blocks up to which pairs stay resident (8192 K)
 
 template <int BN>
@@ -787,7 +786,7 @@ static int launch_gemm(cudaStream_t st, const ResiduePlanes &A, const ResiduePla
         cutc_set_error(CUTC_ERR_INVALID, "modular contraction of %lld tiles", (long long)tasks);
         return CUTC_ERR_INVALID;
     }
-    const unsigned pairs = (unsigned)(kResident ? std::min<int64_t>(tasks, kPairs) : tasks);
+    const unsigned pairs = (unsigned)(kResident ? std::min<int64_t>(tasks, device_sms() / 2) : tasks);
     modular_gemm_kernel<BN, kResident, kMag><<<2 * pairs, kGemmThreads, Cfg::kSmem, st>>>(ta, tb, P);
     CUTC_CUDA_TRY(cudaGetLastError());
     note_launches(1);
@@ -814,10 +813,10 @@ int modular_gemm(cudaStream_t st, int n_mod, int planes, const ResiduePlanes &A,
         P.inv[i] = 1.0f / (float)moduli::prime(i);
     }
     P.err = err;
-    // narrow tiles for few columns, and where wide ones would leave the 76 SM pairs short
+    // narrow tiles for few columns, and where wide ones would leave the SM pairs (76) short
     // of work
     const int64_t wide = (int64_t)planes * ceil_div(P.M, kTileM) * ceil_div(P.N, 256);
-    const int bn = P.N <= 64 ? 64 : (P.N <= 128 || wide < kPairs) ? 128 : 256;
+    const int bn = P.N <= 64 ? 64 : (P.N <= 128 || wide < device_sms() / 2) ? 128 : 256;
     // Short panels: resident pairs walk the tasks, which hides a task's set-up and epilogue
     // behind the next one's MMAs.  Long ones: one pair per task, which the hardware starts
     // in order, so that concurrent tasks stay neighbours in L2.  M 7260, N 16384, resident

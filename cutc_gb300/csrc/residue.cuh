@@ -690,7 +690,7 @@ static inline int row_scales_cols(cudaStream_t st, const double *X, int64_t ld, 
     // few rows: 64-byte runs and four times the blocks (300 rows of 9000: 100 us with 32 rows
     // a block)
     const float bits = moduli::row_bits(n_mod);
-    if (rows <= 32 * 152)
+    if (rows <= 32 * device_sms())
         row_scale_cols_kernel<8><<<ceil_div(rows, 8), 1024, 0, st>>>(X, ld, rows, K, bits, sc);
     else
         row_scale_cols_kernel<32><<<ceil_div(rows, 32), 1024, 0, st>>>(X, ld, rows, K, bits, sc);
