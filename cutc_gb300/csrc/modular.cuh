@@ -89,7 +89,8 @@ inline int split_moduli(int S, int64_t K)
 // most 2^70.674 / sqrt(6) (rms, in units of the integer result).  Magnitudes enter as
 // |t| 2^-58, so that the plane's sum is s = sum |t_a t_b| 2^-116, and with s >= kCheckSum
 // that error is at most 0.17 2^-53 sum_k |a_k b_k|, about half of one rounding of an FP64
-// sum.  Sums are kept up to kMagnitudeCap; exact zeros (no k with both operands non-zero)
+// sum (0.34 where the sum is of many K panels, each of which rounds it).  Sums are kept up to
+// kMagnitudeCap; exact zeros (no k with both operands non-zero)
 // are told from small ones, because their results are exact.  With 15 moduli, 2^-62, the
 // check would fail for up to 8 % of the elements of a build (10 nuclei, 70 AOs: P against G's
 // -1/2 |grad u|^2); with 17 for fewer than one in 10^5.

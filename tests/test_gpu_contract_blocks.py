@@ -19,3 +19,34 @@ def test_blocks_of_a_small_budget():
     assert np.array_equal(X, Xs)
     # int_2e: the blocks' shares are added in FP64
     assert np.abs(I - Is).max() <= 2e-15 * np.abs(I).max()
+
+
+def test_check_of_many_panels():
+    """cutc_no_2e under a budget that cuts K = 330 000 into 645 panels: the largest values of
+    tmpC1 meet zeros, and every panel adds a little to the sums of magnitudes.  The error stays
+    relative to sum |a b|."""
+    import torch
+    n_mo, n1 = 6, 110_000
+    m2 = n_mo * n_mo
+    rng = np.random.default_rng(12)
+    C1, X = rng.normal(size=(m2, 3 * n1)), rng.normal(size=(m2, 3 * n1))
+    C2, D2 = rng.normal(size=(m2, n1)), rng.normal(size=(m2, n1))
+    C1[:, :3] *= 1e10
+    X[:, :3] = 0.0
+    dev = [torch.from_numpy(a).cuda() for a in (C1, X, C2, D2)]
+    out = torch.empty((m2, m2), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    opt = cg.options(cg.PLAIN_FP64, device_pointers=True, max_work_bytes=1 << 20)
+    import ctypes
+    assert cg.load().cutc_no_2e(ctypes.byref(opt), n_mo, n1, *[t.data_ptr() for t in dev],
+                                out.data_ptr()) == cg.CUTC_OK
+    ld = np.longdouble
+
+    def step(a):
+        a = (a + a.T).reshape(n_mo, n_mo, n_mo, n_mo)
+        return a.transpose(0, 2, 1, 3).reshape(m2, m2)
+
+    ref = step(0.5 * (C1.astype(ld) @ X.T.astype(ld)) + 0.5 * (C2.astype(ld) @ D2.T.astype(ld)))
+    mag = step(0.5 * (np.abs(C1) @ np.abs(X).T) + 0.5 * (np.abs(C2) @ np.abs(D2).T))
+    err = np.abs(np.asarray(out.cpu().numpy() - ref, dtype=np.float64))
+    assert np.all(err <= 4 * 2.0 ** -53 * mag), (err / mag).max() * 2.0 ** 53
