@@ -933,6 +933,17 @@ PairTcMode pair_tc_mode(const double *coef, const int *exps, int n_terms, int n_
     // with 13, 16 and 24 nuclei)
     if (!fp64 && m.rows == 32 && K > kDfGroupK)
         return PairTcMode{};
+    // Few nuclei with general exponents: where every term vanishes at its nucleus a large part
+    // of the pairs is marked, and forming them again costs more than the loops over all pairs
+    // (2003 x 30 011 pairs, 11 terms, double-float: one nucleus 9.8 to 14.3 ms, the loop 3.8; two
+    // 4.0 with powers 0 among the terms, 7.1 to 10.5 without, the loop 6.3; three at most 6.0, the
+    // loop 8.9.  512 x 20 011 in FP64: one nucleus 2.6 with powers 0, 3.4 to 3.7 without, the
+    // loop 3.0; two at most 3.1, the loop 4.9)
+    bool vanish = true;
+    for (int k = 0; k < n_terms; k++)
+        vanish = vanish && (exps[k] & 7) && (exps[k] >> 3 & 7);
+    if (m.rows == 32 && ((n_nuc == 1 && (!fp64 || vanish)) || (n_nuc == 2 && !fp64 && vanish)))
+        return PairTcMode{};
     // 5 slices (representation error 2^-45, under the error of a 5-slice build's operands), 6
     // for builds of 6 and 7 slices and where the check is (2^-54, below the double-float
     // epilogue), 7 for FP64 (2^-63)
